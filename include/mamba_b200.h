@@ -308,9 +308,10 @@ MAMBA_B200_API int mamba_b200_conv1d_bwd(void* handle, void* stream, const mamba
  *   the state after the window (NULL = not written); read first when carry_in = 1.
  * 16-bit storage with hd <= 64 and N <= 128 (multiples of 8; tiles are padded to
  * 64 / 128 columns with zeros inside the kernel, so the reference's own limits
- * hd 32, N 64 are covered) and no carried state runs the chunked form on tcgen05
- * tensor cores with the running state in TMEM (no chunk-state or K_scaled tensors
- * in HBM); every other case runs the sequential definition.
+ * hd 32, N 64 are covered) runs the chunked form on tcgen05 tensor cores with the
+ * running state in TMEM (no chunk-state or K_scaled tensors in HBM); a carried state
+ * is kept to f32 accuracy there (rounded operands are split in two).  Every other
+ * case, and a carried window of a few steps, runs the sequential definition.
  * hd and N are not limited to the reference's hd <= 32, N <= 64
  * (src/mamba3_siso/config.rs:66-99); N <= 128.
  */
@@ -328,7 +329,7 @@ typedef struct mamba_b200_m3_ssd_args {
     float* ssm_state;
     float* k_state;
     float* v_state;
-    int carry_in;         /* 1: continue from the given state (sequential kernel) */
+    int carry_in;         /* 1: continue from the given state */
     int force_sequential; /* 1: never take the tensor-core path (for comparison) */
     /* Optional (Bn != NULL; tensor-core path only, else MAMBA_B200_ERR_SHAPE): the per-head
      * K and Q are built inside the kernel and K, Q above are ignored.  Replaces

@@ -8,9 +8,9 @@
 //    never touch HBM (the reference writes [B, chunks, nh, hd, N] f32 of them).
 //    Per chunk: G = Q K^T, decay/causal mask in registers, Y1 = M V,
 //    Y2 = Q S_in^T, S^T <- exp(dA_end) S^T + K^T (w o V).
-//  * m3_ssd_seq_kernel — the sequential definition (one thread per
-//    (sample, head, p), state in registers) for every other shape / dtype and
-//    whenever a recurrent state is carried in.
+//    With a carried state the same kernel starts from it (CARRY).
+//  * m3_ssd_seq_kernel — the sequential definition (eight rows p per warp, state in
+//    registers) for every other shape / dtype and for short carried windows.
 #include <string.h>
 
 #include <type_traits>
@@ -46,79 +46,146 @@ struct M3Params {
 // ---------------------------------------------------------------------------
 // Sequential definition, src/mamba3_siso/cpu/forward.rs:85-138 / kernels/mamba3_ssd.cu:229-348:
 //   h = alpha h + (beta v_prev) k_prev + (gamma x) k ;  y = <h, q> + D x
-// grid (nh, B), block hd threads (rounded up to a warp); k, q, k_prev staged in
-// shared memory per step.
+// A warp owns R rows p of one (sample, head); its lanes split the state index (n = lane + 32 i),
+// so the state, K and Q move as whole 128-byte rows and no block barrier is needed.  The dot
+// products of a step are reduced by a halving butterfly that leaves row r in one lane group.
+// With few heads the chain of one step bounds it (0.37 us a step at 1 x 4 heads of 64 x 128; loads
+// are requested PF steps ahead), with many the issue slots (1.5 us at 8 x 32 heads); one thread per
+// row with 128 states in registers and two block barriers a step, which it replaces, took 8 us.
+// grid (nh, B, ceil(hd / rows of a CTA)).
 // ---------------------------------------------------------------------------
-template <typename Tact, int NMAX>
-__global__ void m3_ssd_seq_kernel(const M3Params p) {
-    extern __shared__ float sm[];
-    float* ks = sm;                // [2][N] current / previous k
-    float* qs = sm + 2 * p.N;      // [N]
-    const int h = blockIdx.x, b = blockIdx.y, pp = threadIdx.x;
+template <typename Tact, int NI, int R>
+__global__ void __launch_bounds__(256) m3_ssd_seq_kernel(const M3Params p) {
+    constexpr int PF = 4;  // steps requested ahead
+    const int h = blockIdx.x, b = blockIdx.y, lane = threadIdx.x & 31;
     const int N = p.N, hd = p.hd, nh = p.nh, T = p.T;
-    const bool act = pp < hd;
-    float st[NMAX];
+    const int p0 = (blockIdx.z * (blockDim.x >> 5) + (threadIdx.x >> 5)) * R;
+    const long long bh = static_cast<long long>(b) * nh + h;
+    // lane -> output row of this warp after the butterfly: R == 8: bits 4..2, R == 2: bit 4
+    const int rl = R == 8 ? ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1) : (lane >> 4) & 1;
+    const bool rok = p0 + rl < hd;
+    const bool writer = rok && (R == 8 ? (lane & 3) == 0 : (lane & 15) == 0);
+    bool nok[NI];
 #pragma unroll
-    for (int n = 0; n < NMAX; ++n) st[n] = 0.0f;
-    float vprev = 0.0f;
+    for (int i = 0; i < NI; ++i) nok[i] = lane + 32 * i < N;
+    float st[R][NI], kp[NI], vp[R];
+#pragma unroll
+    for (int i = 0; i < NI; ++i) kp[i] = 0.0f;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        vp[r] = 0.0f;
+#pragma unroll
+        for (int i = 0; i < NI; ++i) st[r][i] = 0.0f;
+    }
     if (p.carry_in) {
-        if (act) {
 #pragma unroll
-            for (int n = 0; n < NMAX; ++n)
-                if (n < N) st[n] = p.ssm_state[((static_cast<long long>(b) * nh + h) * hd + pp) * N + n];
-            vprev = p.v_state[(static_cast<long long>(b) * nh + h) * hd + pp];
-        }
-        for (int n = threadIdx.x; n < N; n += blockDim.x)
-            ks[N + n] = p.k_state[(static_cast<long long>(b) * nh + h) * N + n];
-    } else {
-        for (int n = threadIdx.x; n < N; n += blockDim.x) ks[N + n] = 0.0f;
+        for (int r = 0; r < R; ++r)
+            if (p0 + r < hd) {
+                vp[r] = p.v_state[bh * hd + p0 + r];
+#pragma unroll
+                for (int i = 0; i < NI; ++i)
+                    if (nok[i]) st[r][i] = p.ssm_state[(bh * hd + p0 + r) * N + lane + 32 * i];
+            }
+#pragma unroll
+        for (int i = 0; i < NI; ++i)
+            if (nok[i]) kp[i] = p.k_state[bh * N + lane + 32 * i];
+        __syncthreads();  // the CTA's warps have read k_state before one of them overwrites it
     }
-    const Tact* xb = static_cast<const Tact*>(p.x);
-    const Tact* Kb = static_cast<const Tact*>(p.K);
-    const Tact* Qb = static_cast<const Tact*>(p.Q);
-    Tact* yb = static_cast<Tact*>(p.y);
+    if (p0 >= hd) return;
+    const Tact* xb = static_cast<const Tact*>(p.x) + static_cast<long long>(b) * T * nh * hd + h * hd + p0 + rl;
+    const Tact* Kb = static_cast<const Tact*>(p.K) + (static_cast<long long>(b) * T * nh + h) * N + lane;
+    const Tact* Qb = static_cast<const Tact*>(p.Q) + (static_cast<long long>(b) * T * nh + h) * N + lane;
+    Tact* yb = static_cast<Tact*>(p.y) + static_cast<long long>(b) * T * nh * hd + h * hd + p0 + rl;
     const float Dv = p.Dh[h];
-    for (int t = 0; t < T; ++t) {
+    Tact kr[PF][NI], qr[PF][NI], xr[PF];
+    float sa[PF], sd[PF], sg[PF];
+    auto request = [&](int t, int s) {
+        if (t >= T) return;
         const long long th = (static_cast<long long>(b) * T + t) * nh + h;
-        const int cur = t & 1, prv = cur ^ 1;  // ks[cur] <- k_t ; ks[prv] holds k_{t-1}
-        __syncthreads();
-        for (int n = threadIdx.x; n < N; n += blockDim.x) {
-            ks[cur * N + n] = to_f(Kb[th * N + n]);
-            qs[n] = to_f(Qb[th * N + n]);
-        }
-        __syncthreads();
-        const float alpha = ex2(p.adt[th] * kLog2e);
-        const float beta = alpha * p.dt[th] * (1.0f - p.trap[th]);
-        const float gamma = p.trap[th] * p.dt[th];
-        if (act) {
-            const float xv = to_f(xb[(static_cast<long long>(b) * T + t) * nh * hd + h * hd + pp]);
-            const float bv = beta * vprev, gx = gamma * xv;
-            float acc = 0.0f;
-            const float* kc = ks + cur * N;
-            const float* kp = ks + prv * N;
+        const long long kq = static_cast<long long>(t) * nh * N;
+        sa[s] = p.adt[th]; sd[s] = p.dt[th]; sg[s] = p.trap[th];
 #pragma unroll
-            for (int n = 0; n < NMAX; ++n)
-                if (n < N) {
-                    st[n] = fmaf(alpha, st[n], fmaf(bv, kp[n], gx * kc[n]));
-                    acc = fmaf(st[n], qs[n], acc);
+        for (int i = 0; i < NI; ++i)
+            if (nok[i]) {
+                kr[s][i] = Kb[kq + 32 * i];
+                qr[s][i] = Qb[kq + 32 * i];
+            }
+        if (rok) xr[s] = xb[static_cast<long long>(t) * nh * hd];
+    };
+#pragma unroll
+    for (int s = 0; s < PF; ++s) request(s, s);
+    for (int tb = 0; tb < T; tb += PF) {
+#pragma unroll
+        for (int s = 0; s < PF; ++s) {
+            const int t = tb + s;
+            if (t < T) {
+                const float alpha = ex2(sa[s] * kLog2e);
+                const float beta = alpha * sd[s] * (1.0f - sg[s]), gamma = sg[s] * sd[s];
+                const float xv = rok ? to_f(xr[s]) : 0.0f;
+                float k[NI], q[NI], acc[R];
+#pragma unroll
+                for (int i = 0; i < NI; ++i) {
+                    k[i] = nok[i] ? to_f(kr[s][i]) : 0.0f;
+                    q[i] = nok[i] ? to_f(qr[s][i]) : 0.0f;
                 }
-            yb[(static_cast<long long>(b) * T + t) * nh * hd + h * hd + pp] = from_f<Tact>(fmaf(Dv, xv, acc));
-            vprev = xv;
-        }
-    }
-    // T == 0 leaves the state untouched; otherwise ks[(T-1)&1] holds the last k.
-    if (T > 0) {
-        if (p.ssm_state && act) {
 #pragma unroll
-            for (int n = 0; n < NMAX; ++n)
-                if (n < N) p.ssm_state[((static_cast<long long>(b) * nh + h) * hd + pp) * N + n] = st[n];
+                for (int r = 0; r < R; ++r) {
+                    const int src = R == 8 ? ((r >> 2) & 1) * 16 + ((r >> 1) & 1) * 8 + (r & 1) * 4 : r * 16;
+                    const float xb_r = __shfl_sync(0xffffffffu, xv, src);
+                    const float bv = beta * vp[r], gx = gamma * xb_r;
+                    acc[r] = 0.0f;
+#pragma unroll
+                    for (int i = 0; i < NI; ++i) {
+                        st[r][i] = fmaf(alpha, st[r][i], fmaf(bv, kp[i], gx * k[i]));
+                        acc[r] = fmaf(st[r][i], q[i], acc[r]);
+                    }
+                    vp[r] = xb_r;
+                }
+#pragma unroll
+                for (int i = 0; i < NI; ++i) kp[i] = k[i];
+                request(t + PF, s);
+                // halving butterfly over the lanes: R sums, one per lane group
+                int m = 16;
+#pragma unroll
+                for (int w = R / 2; w >= 1; w >>= 1, m >>= 1) {
+                    const bool up = (lane & m) != 0;
+#pragma unroll
+                    for (int r = 0; r < w; ++r) {
+                        const float give = up ? acc[r] : acc[r + w], keep = up ? acc[r + w] : acc[r];
+                        acc[r] = keep + __shfl_xor_sync(0xffffffffu, give, m);
+                    }
+                }
+                float y = acc[0];
+#pragma unroll
+                for (int mm = R == 8 ? 2 : 8; mm >= 1; mm >>= 1) y += __shfl_xor_sync(0xffffffffu, y, mm);
+                if (writer) yb[static_cast<long long>(t) * nh * hd] = from_f<Tact>(fmaf(Dv, xv, y));
+            }
         }
-        if (p.v_state && act) p.v_state[(static_cast<long long>(b) * nh + h) * hd + pp] = vprev;
-        __syncthreads();
-        if (p.k_state)
-            for (int n = threadIdx.x; n < N; n += blockDim.x)
-                p.k_state[(static_cast<long long>(b) * nh + h) * N + n] = ks[((T - 1) & 1) * N + n];
     }
+    if (gridDim.z == 1 && threadIdx.x < 32 && p.k_state) {
+#pragma unroll
+        for (int i = 0; i < NI; ++i)
+            if (nok[i]) p.k_state[bh * N + lane + 32 * i] = kp[i];
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+        if (p0 + r < hd) {
+            if (p.ssm_state)
+#pragma unroll
+                for (int i = 0; i < NI; ++i)
+                    if (nok[i]) p.ssm_state[(bh * hd + p0 + r) * N + lane + 32 * i] = st[r][i];
+            if (p.v_state && lane == 0) p.v_state[bh * hd + p0 + r] = vp[r];
+        }
+}
+
+// k_state after the window when several CTAs share a (sample, head): any of them may still be
+// reading the entering k_state when another has finished.
+template <typename Tact>
+__global__ void m3_seq_kstate_kernel(const M3Params p) {
+    const int h = blockIdx.x, b = blockIdx.y;
+    const Tact* kl = static_cast<const Tact*>(p.K) + ((static_cast<long long>(b) * p.T + p.T - 1) * p.nh + h) * p.N;
+    for (int n = threadIdx.x; n < p.N; n += blockDim.x)
+        p.k_state[(static_cast<long long>(b) * p.nh + h) * p.N + n] = to_f(kl[n]);
 }
 
 // ---------------------------------------------------------------------------
@@ -136,6 +203,9 @@ constexpr int CS = 128, HD = 64, NS = 128;
 // 16-bit copy of the new state for the next chunk's Y2; then f32 vectors, barriers.
 constexpr uint32_t kQ0 = 0, kK0 = 65536, kV0 = 131072, kQKStride = 32768, kVStride = 16384;
 constexpr uint32_t kM = 163840, kVw = 196608, kS = 196608;
+// carried state: one Q, K and V buffer; remainders of M, w o V and the state copy behind them
+constexpr uint32_t kCarryK = 32768, kCarryV = 65536, kMlo = 81920, kVwLo = 114688, kSlo = kVwLo;
+static_assert(kVwLo + 16384 <= kM, "carry layout");
 // f32 dA[128], scale[128], gamma[128], dA*log2(e)[128], dt[128] per chunk, two sets: a chunk's
 // set is written while slower threads may still read the previous chunk's
 constexpr uint32_t kVec = 212992, kVecSet = 5 * 128;
@@ -157,7 +227,17 @@ constexpr uint32_t cG = 0, cY1 = 256, cY2 = 320, cS = 384, kTmemCols = 512;
 // (src/mamba3_siso/cpu/forward.rs:336-375; kernels/mamba3_ops.cu:279-310, :400-440,
 // :575-640).  The in-chunk sums run in f32 (shuffle scans over the rows), the angle
 // entering a chunk is carried in f64.
-template <typename Th, bool GEN>
+//
+// CARRY: continue from ssm_state / k_state / v_state.  In the shifted form the state that enters
+// is S = h + dt_0 (1 - trap_0) k_prev v_prev^T, so it is loaded into TMEM and the first chunk is
+// a chunk like any other.  A carried state is kept to f32 accuracy as the sequential definition
+// keeps it: every rounded MMA operand (M, w o V, the state copy) is a 16-bit value plus a second
+// one with the rounding that was left, two products each (K, Q and V are 16-bit inputs and
+// exact), which leaves 2^-17 of each term.  The second tiles take the room of the second Q / K /
+// V buffers: Q of the next chunk is requested when the first MMA group has read it, K and V when
+// the second has.  8 x 256 steps x 32 heads of 64 x 128, bf16: 43 us (2050 us sequentially), the
+// state within 3e-6 of the sequential kernel's.
+template <typename Th, bool GEN, bool CARRY>
 __global__ void __launch_bounds__(256, 1) m3_ssd_fwd_tc_kernel(const __grid_constant__ M3Params p) {
     extern __shared__ __align__(1024) unsigned char smem[];
     // two threads per step: thread (row, half) owns row `row` of the chunk (TMEM lane
@@ -409,6 +489,23 @@ __global__ void __launch_bounds__(256, 1) m3_ssd_fwd_tc_kernel(const __grid_cons
     // One elected thread issues the five boxes of a chunk (Q and K: two 64-column sub-tiles
     // each, V: one); rows past the end of the sequence and columns past the head's width
     // arrive as zeros.
+    auto issue_carry_q = [&](int c) {
+        if (threadIdx.x == 0) {
+            mbar_expect_tx(&full[0], kQKStride);
+#pragma unroll
+            for (int sub = 0; sub < 2; ++sub)
+                tma_load_4d(smem + kQ0 + sub * kSwSub, &p.tm_q, &full[0], 64 * sub, h, c * CS, b);
+        }
+    };
+    auto issue_carry_kv = [&](int c) {
+        if (threadIdx.x == 0) {
+            mbar_expect_tx(&full[1], kQKStride + kVStride);
+#pragma unroll
+            for (int sub = 0; sub < 2; ++sub)
+                tma_load_4d(smem + kCarryK + sub * kSwSub, &p.tm_k, &full[1], 64 * sub, h, c * CS, b);
+            tma_load_4d(smem + kCarryV, &p.tm_v, &full[1], 0, h, c * CS, b);
+        }
+    };
     auto issue_tiles = [&](int c) {
         if (threadIdx.x == 0) {
             const int buf = c & 1, t0 = c * CS;
@@ -422,9 +519,47 @@ __global__ void __launch_bounds__(256, 1) m3_ssd_fwd_tc_kernel(const __grid_cons
             tma_load_4d(smem + kV0 + buf * kVStride, &p.tm_v, &full[buf], 0, h, t0, b);
         }
     };
-    issue_tiles(0);
+    if (CARRY) {
+        issue_carry_q(0);
+        issue_carry_kv(0);
+    } else {
+        issue_tiles(0);
+    }
     stage_scalars(0);
     if (GEN) load_vel(0);
+    // 16-bit copy of this thread's state row (and the remainders): the B operand of Y2
+    auto copy_state = [&](const float* sv) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            uint32_t w[4], lo[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                w[i] = pack2<Th>(sv[8 * j + 2 * i], sv[8 * j + 2 * i + 1]);
+                if (CARRY) {
+                    const float2 r = unpack2<Th>(w[i]);
+                    lo[i] = pack2<Th>(sv[8 * j + 2 * i] - r.x, sv[8 * j + 2 * i + 1] - r.y);
+                }
+            }
+            *reinterpret_cast<uint4*>(smem + kS + sw_chunk(tid, half * 4 + j)) = make_uint4(w[0], w[1], w[2], w[3]);
+            if (CARRY)
+                *reinterpret_cast<uint4*>(smem + kSlo + sw_chunk(tid, half * 4 + j)) =
+                    make_uint4(lo[0], lo[1], lo[2], lo[3]);
+        }
+    };
+    if (CARRY) {
+        const long long bh = static_cast<long long>(b) * nh + h, th0 = static_cast<long long>(b) * T * nh + h;
+        const float kc = tid < nsv ? p.dt[th0] * (1.0f - p.trap[th0]) * p.k_state[bh * nsv + tid] : 0.0f;
+        float sv[32];
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+            const int pp = half * 32 + i;
+            sv[i] = pp < hdv && tid < nsv ? fmaf(kc, p.v_state[bh * hdv + pp], p.ssm_state[(bh * hdv + pp) * nsv + tid])
+                                          : 0.0f;
+        }
+        tmem_st32(lane_addr + cS + half * 32, sv);
+        copy_state(sv);
+        fence_proxy_async();  // (published by the barriers ahead of the first MMA group)
+    }
 
     for (int c = 0; c < nchunks; ++c) {
         const int t0 = c * CS, nv = min(CS, T - t0);
@@ -432,12 +567,19 @@ __global__ void __launch_bounds__(256, 1) m3_ssd_fwd_tc_kernel(const __grid_cons
         const float* dA = vec + (c & 1) * kVecSet;
         const float* scl = dA + 128;
         const float* gam = dA + 256;
-        const uint32_t tQ = kQ0 + (c & 1) * kQKStride, tK = kK0 + (c & 1) * kQKStride, tV = kV0 + (c & 1) * kVStride;
+        const uint32_t tQ = kQ0 + (CARRY ? 0u : (c & 1) * kQKStride);
+        const uint32_t tK = CARRY ? kCarryK : kK0 + (c & 1) * kQKStride;
+        const uint32_t tV = CARRY ? kCarryV : kV0 + (c & 1) * kVStride;
         // ---- 1. copies of the next chunk's tiles into the other buffers (their last readers,
         //         the MMAs of chunk c - 1, have completed); per-row scalars; this chunk's tiles ----
-        if (c + 1 < nchunks) issue_tiles(c + 1);
+        if (!CARRY && c + 1 < nchunks) issue_tiles(c + 1);
         scalars(c, c & 1);
-        ok = mbar_wait(&full[c & 1], (c >> 1) & 1, p.status) && ok;
+        if (CARRY) {
+            ok = mbar_wait(&full[0], c & 1, p.status) && ok;
+            ok = mbar_wait(&full[1], c & 1, p.status) && ok;
+        } else {
+            ok = mbar_wait(&full[c & 1], (c >> 1) & 1, p.status) && ok;
+        }
         if (GEN) {
             gen_apply(c, c & 1);
             fence_proxy_async();  // the rewritten K / Q pieces, before the tensor core reads them
@@ -455,15 +597,21 @@ __global__ void __launch_bounds__(256, 1) m3_ssd_fwd_tc_kernel(const __grid_cons
 #pragma unroll
             for (int k = 0; k < NS / 16; ++k)
                 mma(tmem + cG, desc_sw_k(sbase + tQ, k), desc_sw_k(sbase + tK, k), idG, k > 0);
-            if (c > 0) {
+            if (CARRY || c > 0) {
 #pragma unroll
                 for (int k = 0; k < NS / 16; ++k)  // N = p, K = n
                     mma(tmem + cY2, desc_sw_k(sbase + tQ, k), desc_sw_mn(sbase + kS, k), idY, k > 0);
+            }
+            if (CARRY) {
+#pragma unroll
+                for (int k = 0; k < NS / 16; ++k)
+                    mma(tmem + cY2, desc_sw_k(sbase + tQ, k), desc_sw_mn(sbase + kSlo, k), idY, true);
             }
             commit(&bars[0]);
         }
         ok = mbar_wait(&bars[0], c & 1, p.status) && ok;
         fence_after();
+        if (CARRY && c + 1 < nchunks) issue_carry_q(c + 1);
         // ---- 3. decay / causal mask -> M (over the Q tile); w o V (over the old state
         //         copy); rescale the running state ----
         {
@@ -472,13 +620,20 @@ __global__ void __launch_bounds__(256, 1) m3_ssd_fwd_tc_kernel(const __grid_cons
 #pragma unroll
                 for (int j = half * (HD / 16); j < (half + 1) * (HD / 16); ++j) {
                     const uint4 v = *reinterpret_cast<const uint4*>(smem + tV + sw_chunk(tid, j));
-                    uint32_t w4[4] = {v.x, v.y, v.z, v.w};
+                    uint32_t w4[4] = {v.x, v.y, v.z, v.w}, lo[4];
 #pragma unroll
                     for (int q4 = 0; q4 < 4; ++q4) {
                         const float2 f = unpack2<Th>(w4[q4]);
                         w4[q4] = pack2<Th>(f.x * wt, f.y * wt);
+                        if (CARRY) {
+                            const float2 r = unpack2<Th>(w4[q4]);
+                            lo[q4] = pack2<Th>(f.x * wt - r.x, f.y * wt - r.y);
+                        }
                     }
                     *reinterpret_cast<uint4*>(smem + kVw + sw_chunk(tid, j)) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
+                    if (CARRY)
+                        *reinterpret_cast<uint4*>(smem + kVwLo + sw_chunk(tid, j)) =
+                            make_uint4(lo[0], lo[1], lo[2], lo[3]);
                 }
             }
             const float* dAl = dA + 384;  // dA * log2(e)
@@ -490,7 +645,7 @@ __global__ void __launch_bounds__(256, 1) m3_ssd_fwd_tc_kernel(const __grid_cons
                 constexpr bool DIAG = decltype(diag_tag)::value;
                 float g[32];
                 tmem_ld32(lane_addr + cG + q4 * 32, g);
-                uint32_t packed[16];
+                uint32_t packed[16], rest[16];
 #pragma unroll
                 for (int i = 0; i < 32; i += 4) {
                     const float4 da4 = *reinterpret_cast<const float4*>(dAl + q4 * 32 + i);
@@ -509,24 +664,37 @@ __global__ void __launch_bounds__(256, 1) m3_ssd_fwd_tc_kernel(const __grid_cons
                     }
                     packed[i / 2] = pack2<Th>(m[0], m[1]);
                     packed[i / 2 + 1] = pack2<Th>(m[2], m[3]);
+                    if (CARRY) {
+                        const float2 r0 = unpack2<Th>(packed[i / 2]), r1 = unpack2<Th>(packed[i / 2 + 1]);
+                        rest[i / 2] = pack2<Th>(m[0] - r0.x, m[1] - r0.y);
+                        rest[i / 2 + 1] = pack2<Th>(m[2] - r1.x, m[3] - r1.y);
+                    }
                 }
 #pragma unroll
                 for (int j = 0; j < 4; ++j)
                     *reinterpret_cast<uint4*>(smem + kM + sw_chunk(tid, q4 * 4 + j)) =
                         make_uint4(packed[4 * j], packed[4 * j + 1], packed[4 * j + 2], packed[4 * j + 3]);
+                if (CARRY)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        *reinterpret_cast<uint4*>(smem + kMlo + sw_chunk(tid, q4 * 4 + j)) =
+                            make_uint4(rest[4 * j], rest[4 * j + 1], rest[4 * j + 2], rest[4 * j + 3]);
             };
             for (int q4 = 2 * half; q4 < 2 * half + 2; ++q4) {
                 if (q4 > warp) {  // wholly above the diagonal for every row of this warp
 #pragma unroll
-                    for (int j = 0; j < 4; ++j)
+                    for (int j = 0; j < 4; ++j) {
                         *reinterpret_cast<uint4*>(smem + kM + sw_chunk(tid, q4 * 4 + j)) = make_uint4(0, 0, 0, 0);
+                        if (CARRY)
+                            *reinterpret_cast<uint4*>(smem + kMlo + sw_chunk(tid, q4 * 4 + j)) = make_uint4(0, 0, 0, 0);
+                    }
                 } else if (q4 == warp) {
                     mask_block(std::true_type{}, q4);
                 } else {
                     mask_block(std::false_type{}, q4);
                 }
             }
-            if (c > 0) {  // S^T row `tid` (state index n = tid) *= exp(dA_end)
+            if (CARRY || c > 0) {  // S^T row `tid` (state index n = tid) *= exp(dA_end)
                 const float e_end = ex2(dA[nv - 1] * kLog2e);
                 float sv[32];
                 tmem_ld32(lane_addr + cS + half * 32, sv);
@@ -549,17 +717,26 @@ __global__ void __launch_bounds__(256, 1) m3_ssd_fwd_tc_kernel(const __grid_cons
                 mma(tmem + cY1, desc_sw_k(sbase + kM, k), desc_sw_mn(sbase + tV, k), idY, k > 0);
 #pragma unroll
             for (int k = 0; k < CS / 16; ++k)  // M = n, N = p, K = t
-                mma(tmem + cS, desc_sw_mn(sbase + tK, k), desc_sw_mn(sbase + kVw, k), idS, c > 0 || k > 0);
+                mma(tmem + cS, desc_sw_mn(sbase + tK, k), desc_sw_mn(sbase + kVw, k), idS, CARRY || c > 0 || k > 0);
+            if (CARRY) {
+#pragma unroll
+                for (int k = 0; k < CS / 16; ++k)
+                    mma(tmem + cY1, desc_sw_k(sbase + kMlo, k), desc_sw_mn(sbase + tV, k), idY, true);
+#pragma unroll
+                for (int k = 0; k < CS / 16; ++k)
+                    mma(tmem + cS, desc_sw_mn(sbase + tK, k), desc_sw_mn(sbase + kVwLo, k), idS, true);
+            }
             commit(&bars[1]);
         }
         ok = mbar_wait(&bars[1], c & 1, p.status) && ok;
         fence_after();
+        if (CARRY && c + 1 < nchunks) issue_carry_kv(c + 1);
         // ---- 5. epilogue: y row; 16-bit copy of the new state for the next chunk ----
         {
             const float e_t = ex2(dA[tid] * kLog2e);
             const int q2 = half;
             float y1[32], y2[32];
-            if (c > 0) {
+            if (CARRY || c > 0) {
                 tmem_ld32x2(lane_addr + cY1 + q2 * 32, y1, lane_addr + cY2 + q2 * 32, y2);
 #pragma unroll
                 for (int i = 0; i < 32; ++i) y1[i] = fmaf(e_t, y2[i], y1[i]);
@@ -574,11 +751,7 @@ __global__ void __launch_bounds__(256, 1) m3_ssd_fwd_tc_kernel(const __grid_cons
             float sv[32];
             tmem_ld32(lane_addr + cS + q2 * 32, sv);
             if (c + 1 < nchunks) {
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    *reinterpret_cast<uint4*>(smem + kS + sw_chunk(tid, q2 * 4 + j)) =
-                        make_uint4(pack2<Th>(sv[8 * j], sv[8 * j + 1]), pack2<Th>(sv[8 * j + 2], sv[8 * j + 3]),
-                                   pack2<Th>(sv[8 * j + 4], sv[8 * j + 5]), pack2<Th>(sv[8 * j + 6], sv[8 * j + 7]));
+                copy_state(sv);
             } else if (p.ssm_state) {  // final state [b, h, p, n], n = tid
 #pragma unroll
                 for (int i = 0; i < 32; ++i)
@@ -634,29 +807,43 @@ __global__ void __launch_bounds__(256, 1) m3_ssd_fwd_tc_kernel(const __grid_cons
 }  // namespace tc
 
 int m3_configure(Ctx* c) {
-    const void* fns[4] = {reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false>),
-                          reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__half, false>),
-                          reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, true>),
-                          reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__half, true>)};
+    const void* fns[6] = {reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, false>),
+                          reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__half, false, false>),
+                          reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, true, false>),
+                          reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__half, true, false>),
+                          reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, true>),
+                          reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__half, false, true>)};
     for (const void* fn : fns)
         MB200_CUDA_CHECK(c, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::kSmem));
     return MAMBA_B200_OK;
 }
 
+// Eight rows a warp share one K / Q load and one butterfly; two rows a warp when that leaves
+// fewer than eight warps per SM (the step's chain, not the arithmetic, is then the time).
+template <typename Tact, int NI>
+static void launch_seq_ni(const M3Params& p, int sms, cudaStream_t st) {
+    const bool few = static_cast<long long>(p.B) * p.nh * ((p.hd + 7) / 8) < 8LL * sms;
+    const int rows = few ? 2 : 8, warps = min(8, (p.hd + rows - 1) / rows);
+    const dim3 grid(p.nh, p.B, (p.hd + rows * warps - 1) / (rows * warps));
+    if (few) m3_ssd_seq_kernel<Tact, NI, 2><<<grid, warps * 32, 0, st>>>(p);
+    else m3_ssd_seq_kernel<Tact, NI, 8><<<grid, warps * 32, 0, st>>>(p);
+    if (grid.z > 1 && p.k_state) m3_seq_kstate_kernel<Tact><<<dim3(p.nh, p.B), 128, 0, st>>>(p);
+}
 template <typename Tact>
-static void launch_seq(const M3Params& p, cudaStream_t st) {
-    dim3 grid(p.nh, p.B);
-    const int threads = ((p.hd + 31) / 32) * 32;
-    const size_t smem = sizeof(float) * 3 * p.N;
-    if (p.N <= 16) m3_ssd_seq_kernel<Tact, 16><<<grid, threads, smem, st>>>(p);
-    else if (p.N <= 32) m3_ssd_seq_kernel<Tact, 32><<<grid, threads, smem, st>>>(p);
-    else if (p.N <= 64) m3_ssd_seq_kernel<Tact, 64><<<grid, threads, smem, st>>>(p);
-    else m3_ssd_seq_kernel<Tact, 128><<<grid, threads, smem, st>>>(p);
+static void launch_seq(const M3Params& p, int sms, cudaStream_t st) {
+    if (p.N <= 32) launch_seq_ni<Tact, 1>(p, sms, st);
+    else if (p.N <= 64) launch_seq_ni<Tact, 2>(p, sms, st);
+    else launch_seq_ni<Tact, 4>(p, sms, st);
 }
 
 }  // namespace mb200
 
 using namespace mb200;
+
+// A carried window of at most this many steps takes the sequential kernel: a 128-row chunk costs
+// the tensor-core kernel the same time whether it holds 1 step or 128 (15 us at 4 heads, 32 us at
+// 256), and the sequential kernel reaches that after 30 and 18 steps.
+constexpr int kCarrySeqSteps = 20;
 
 extern "C" MAMBA_B200_API int mamba_b200_m3_ssd_fwd(void* handle, void* stream,
                                                     const mamba_b200_m3_ssd_args* ap) {
@@ -696,7 +883,7 @@ extern "C" MAMBA_B200_API int mamba_b200_m3_ssd_fwd(void* handle, void* stream,
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
     bool tensor_core = a.dtype != MAMBA_B200_F32 && a.hd <= tc::HD && a.hd % 8 == 0 && a.N <= tc::NS &&
-                       a.N % 8 == 0 && !a.carry_in &&
+                       a.N % 8 == 0 && (!a.carry_in || (!gen && a.T > kCarrySeqSteps)) &&
                        !a.force_sequential && al16(a.x) && al16(a.y) &&
                        (gen ? al16(a.Bn) && al16(a.Cn) && al16(a.angle_vel) : al16(a.K) && al16(a.Q));
     // the tile maps; when the driver refuses one (no encoder, a stride beyond its range) the
@@ -717,16 +904,18 @@ extern "C" MAMBA_B200_API int mamba_b200_m3_ssd_fwd(void* handle, void* stream,
                    make_tmap_3d(c, &p.tm_trap, MAMBA_B200_F32, a.trap, a.nh, a.nh, a.T, a.B, 4, 129);
         dim3 grid(a.nh, a.B);
         if (a.dtype == MAMBA_B200_BF16) {
-            if (gen) tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, true><<<grid, 256, tc::kSmem, st>>>(p);
-            else tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false><<<grid, 256, tc::kSmem, st>>>(p);
+            if (gen) tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, true, false><<<grid, 256, tc::kSmem, st>>>(p);
+            else if (a.carry_in) tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, true><<<grid, 256, tc::kSmem, st>>>(p);
+            else tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, false><<<grid, 256, tc::kSmem, st>>>(p);
         } else {
-            if (gen) tc::m3_ssd_fwd_tc_kernel<__half, true><<<grid, 256, tc::kSmem, st>>>(p);
-            else tc::m3_ssd_fwd_tc_kernel<__half, false><<<grid, 256, tc::kSmem, st>>>(p);
+            if (gen) tc::m3_ssd_fwd_tc_kernel<__half, true, false><<<grid, 256, tc::kSmem, st>>>(p);
+            else if (a.carry_in) tc::m3_ssd_fwd_tc_kernel<__half, false, true><<<grid, 256, tc::kSmem, st>>>(p);
+            else tc::m3_ssd_fwd_tc_kernel<__half, false, false><<<grid, 256, tc::kSmem, st>>>(p);
         }
     } else {
-        if (a.dtype == MAMBA_B200_F32) launch_seq<float>(p, st);
-        else if (a.dtype == MAMBA_B200_F16) launch_seq<__half>(p, st);
-        else launch_seq<__nv_bfloat16>(p, st);
+        if (a.dtype == MAMBA_B200_F32) launch_seq<float>(p, c->sm_count, st);
+        else if (a.dtype == MAMBA_B200_F16) launch_seq<__half>(p, c->sm_count, st);
+        else launch_seq<__nv_bfloat16>(p, c->sm_count, st);
     }
     MB200_CUDA_CHECK(c, cudaGetLastError());
     return MAMBA_B200_OK;

@@ -153,3 +153,36 @@ def test_tensor_core_kernel_at_config4_size_agrees_with_sequential_and_is_linear
     y12 = mb.m3_ssd_fwd(x12, K, Q, dt, trap, adt, Dh).float()
     torch.cuda.synchronize()
     assert float((y12 - (y_tc + y2)).abs().max() / y12.abs().max()) <= TOL["bf16"]
+
+
+# a stream in windows: the tensor-core kernel from a carried state (windows beyond the short ones the
+# sequential kernel keeps), ragged windows around the 128-step chunk, padded head / state sizes, and a
+# head count that is no multiple of 4; state held to the f32 bar because the carried form splits every
+# rounded operand in two
+CARRY_SHAPES = [((25, 1, 40), 1, 2, 64, 128), ((128, 256, 3), 2, 4, 64, 128), ((1, 129, 300), 1, 3, 64, 128),
+                ((60, 70), 2, 2, 32, 64), ((30, 127, 128), 1, 2, 24, 40), ((200, 1, 1), 1, 40, 72, 96)]
+
+
+@pytest.mark.parametrize("dt", ["bf16", "f16", "f32"])
+@pytest.mark.parametrize("shape", CARRY_SHAPES, ids=lambda s: "T%s_B%dnh%dhd%dN%d" % ("_".join(map(str, s[0])), *s[1:]))
+def test_windows_of_a_stream_carry_state(cuda_dev, shape, dt):
+    import torch
+
+    import mamba_rs_b200 as mb
+    cuts, B, nh, hd, N = shape
+    i = rounded(synth.m3_ssd_inputs(B, sum(cuts), nh, hd, N, seed=sum(cuts)), dt)
+    whole = oracle.m3_ssd_fwd(*[i[k] for k in ARGS])
+    td = torch_dtype(dt)
+    ssm, ks, vs = (torch.zeros(*s, device=cuda_dev) for s in ((B, nh, hd, N), (B, nh, N), (B, nh, hd)))
+    ys, lo = [], 0
+    for n in cuts:
+        sl = {k: (np.ascontiguousarray(i[k][:, lo:lo + n]) if k != "Dh" else i[k]) for k in ARGS}
+        ys.append(mb.m3_ssd_fwd(*[to_dev(sl[k], cuda_dev, td if k in ("x", "K", "Q") else None) for k in ARGS],
+                                ssm_state=ssm, k_state=ks, v_state=vs, carry_in=True))
+        lo += n
+    torch.cuda.synchronize()
+    mb.ffi.default_handle(0).check_status()
+    assert rel_err(torch.cat(ys, 1).float().cpu().numpy(), whole["y"]) <= TOL[dt]
+    assert rel_err(ssm.cpu().numpy(), whole["ssm_state"]) <= 1e-4
+    np.testing.assert_array_equal(ks.cpu().numpy(), whole["k_state"])
+    np.testing.assert_array_equal(vs.cpu().numpy(), whole["v_state"])
