@@ -484,6 +484,54 @@ MAMBA_B200_API int mamba_b200_adamw_step(void* handle, void* stream, float* para
                           float* v, float lr, float beta1, float beta2, float eps, float weight_decay,
                           const float* bias_factors, void* param_lp, int lp_dtype, long long n);
 
+/*
+ * One token per sequence through every layer of a Mamba-1 backbone, in one cooperative launch
+ * (the grid stays resident and meets at barriers in `workspace`): replaces the per-layer launch
+ * sequence of GpuMambaBackbone::step (src/mamba_ssm/gpu/inference.rs:1515-1855, :1062-1215) and,
+ * with next_ids != NULL, GpuMambaLM's greedy decode step around it (src/module/gpu_lm.rs:560-679).
+ * Weights are two arenas with the same layout, the compute-dtype copy `lp` (in_proj, x_proj,
+ * dt_proj, out_proj, embedding) and the f32 master (norms, conv, D): parameter `o_*` of layer l
+ * starts at l * layer_stride + o_*; norm_w at l * layer_stride.  GEMM weights are [in, out]
+ * row-major, conv_w [d_inner, K], a_neg [n_layers, d_inner, N] f32.
+ *   conv_state [n_layers, batch_capacity, d_inner, K], ssm_state [n_layers, batch_capacity,
+ *   d_inner, N] f32: updated in place (the first B sequences).
+ *   backbone: residual [B, d_model] f32 holds the input rows and is updated in place; out
+ *   [B, d_model] (compute dtype) = rmsnorm(residual) * norm_f.
+ *   LM: `steps` tokens are taken one after the other (one launch each): the row embedding[next_ids[b]]
+ *   starts the residual stream (an id outside [0, vocab) starts from zero), tokens[b * tokens_ld + i]
+ *   (may be NULL) records the id, logits [B, vocab] are the last step's, next_ids the greedy choice
+ *   (lowest index among equals).
+ * mamba_b200_decode_workspace_bytes returns what `workspace` must hold, 0 when the kernel does not
+ * take this model or batch (N 16, K 4, d_model a multiple of 8 up to 1024, B <= 64): call the
+ * operators one by one then.  The workspace's first 256 bytes must be zero before the first
+ * launch and are zero again after each; one workspace serves one launch at a time.
+ */
+typedef struct mamba_b200_decode_args {
+    int dtype;
+    int B, batch_capacity, d_model, d_inner, N, K, dt_rank, n_layers, vocab;
+    float eps;
+    const void* lp;
+    const float* master;
+    const float* a_neg;
+    long long layer_stride;
+    long long o_in_proj, o_conv_w, o_conv_b, o_x_proj, o_dt_proj_w, o_dt_proj_b, o_d_param, o_out_proj;
+    long long o_norm_f, o_embedding; /* from the start of the arenas */
+    float* conv_state;
+    float* ssm_state;
+    float* residual;
+    void* out;
+    int* next_ids;
+    int* tokens;
+    long long tokens_ld;
+    void* logits;
+    int steps;
+    void* workspace; /* 16-byte aligned */
+    long long workspace_bytes;
+} mamba_b200_decode_args;
+
+MAMBA_B200_API long long mamba_b200_decode_workspace_bytes(void* handle, const mamba_b200_decode_args* args);
+MAMBA_B200_API int mamba_b200_decode_step(void* handle, void* stream, const mamba_b200_decode_args* args);
+
 #ifdef __cplusplus
 }
 #endif

@@ -39,6 +39,26 @@ bool make_tmap_3d(Ctx* c, CUtensorMap* map, int dtype, const void* base, long lo
     return r == CUDA_SUCCESS;
 }
 
+bool make_tmap_stack(Ctx* c, CUtensorMap* map, int dtype, const void* base, int cols, int rows, int layers,
+                     long long stride, int box_cols, int box_rows) {
+    if (!c->encode_tiled || !base) return false;
+    const size_t es = dtype_size(dtype);
+    if ((reinterpret_cast<uintptr_t>(base) & 15) != 0 || (cols * es) % 16 != 0 || (stride * es) % 16 != 0 ||
+        (box_cols * es) % 16 != 0 || box_cols > 256 || box_rows > 256)
+        return false;
+    CUtensorMapDataType dt = dtype == MAMBA_B200_F32   ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
+                             : dtype == MAMBA_B200_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
+                                                       : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+    cuuint64_t dims[3] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows), static_cast<cuuint64_t>(layers)};
+    cuuint64_t strides[2] = {static_cast<cuuint64_t>(cols) * es, static_cast<cuuint64_t>(stride) * es};
+    cuuint32_t box[3] = {static_cast<cuuint32_t>(box_cols), static_cast<cuuint32_t>(box_rows), 1};
+    cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = reinterpret_cast<EncodeTiledFn>(c->encode_tiled)(
+        map, dt, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+        CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS;
+}
+
 bool make_tmap_head_tile(Ctx* c, CUtensorMap* map, int dtype, const void* base, int cols, int heads, int T,
                          int B) {
     if (!c->encode_tiled || !base || dtype == MAMBA_B200_F32) return false;
@@ -64,6 +84,7 @@ int m3_bwd_configure(Ctx* c);   // m3_ssd_bwd.cu
 int norm_configure(Ctx* c);     // norm.cu
 int conv_configure(Ctx* c);     // m1_step_conv.cu
 int train_ops_configure(Ctx* c);  // train_ops.cu
+int decode_configure(Ctx* c);     // decode.cu
 
 }  // namespace mb200
 
@@ -106,6 +127,8 @@ extern "C" MAMBA_B200_API int mamba_b200_init(int device, void** handle) {
     rc = conv_configure(c);
     if (rc) return rc;
     rc = train_ops_configure(c);
+    if (rc) return rc;
+    rc = decode_configure(c);
     if (rc) return rc;
     return MAMBA_B200_OK;
 }

@@ -107,6 +107,21 @@ class M3SsdBwdArgs(C.Structure):
     ]
 
 
+class DecodeArgs(C.Structure):
+    _fields_ = [
+        ("dtype", C.c_int), ("B", C.c_int), ("batch_capacity", C.c_int), ("d_model", C.c_int), ("d_inner", C.c_int),
+        ("N", C.c_int), ("K", C.c_int), ("dt_rank", C.c_int), ("n_layers", C.c_int), ("vocab", C.c_int),
+        ("eps", C.c_float),
+        ("lp", C.c_void_p), ("master", C.c_void_p), ("a_neg", C.c_void_p), ("layer_stride", C.c_longlong),
+        ("o_in_proj", C.c_longlong), ("o_conv_w", C.c_longlong), ("o_conv_b", C.c_longlong), ("o_x_proj", C.c_longlong),
+        ("o_dt_proj_w", C.c_longlong), ("o_dt_proj_b", C.c_longlong), ("o_d_param", C.c_longlong),
+        ("o_out_proj", C.c_longlong), ("o_norm_f", C.c_longlong), ("o_embedding", C.c_longlong),
+        ("conv_state", C.c_void_p), ("ssm_state", C.c_void_p), ("residual", C.c_void_p), ("out", C.c_void_p),
+        ("next_ids", C.c_void_p), ("tokens", C.c_void_p), ("tokens_ld", C.c_longlong), ("logits", C.c_void_p),
+        ("steps", C.c_int), ("workspace", C.c_void_p), ("workspace_bytes", C.c_longlong),
+    ]
+
+
 _lib = None
 
 
@@ -157,6 +172,8 @@ def lib() -> C.CDLL:
         bind("mamba_b200_embedding_gather", [vp, vp, it, vp, vp, vp, ll, it, it])
         bind("mamba_b200_softmax_xent", [vp, vp, it, vp, vp, vp, vp, fl, ll, it, ll])
         bind("mamba_b200_adamw_step", [vp, vp, vp, vp, vp, vp, fl, fl, fl, fl, fl, vp, vp, it, ll])
+        bind("mamba_b200_decode_workspace_bytes", [vp, C.POINTER(DecodeArgs)], ll)
+        bind("mamba_b200_decode_step", [vp, vp, C.POINTER(DecodeArgs)])
         bind("mamba_b200_m3_ssd_fwd", [vp, vp, C.POINTER(M3SsdArgs)])
         bind("mamba_b200_m3_ssd_bwd", [vp, vp, C.POINTER(M3SsdBwdArgs)])
         bind("mamba_b200_m3_ssd_bwd_workspace_bytes", [C.c_int] * 5, C.c_longlong)

@@ -20,12 +20,13 @@ torch supplies device memory, streams and the process group, nothing else.
 """
 from __future__ import annotations
 
+import ctypes as C
 import math
 from dataclasses import dataclass
 
 import torch
 
-from . import ops
+from . import ffi, ops
 from .parallel import BucketedGradReducer
 
 __all__ = ["MambaConfig", "MambaWeights", "GpuMambaBackbone", "GpuMambaLM", "MambaLMTrainer"]
@@ -79,7 +80,8 @@ class MambaWeights:
         self.master = torch.zeros(self.n, device=device)
         self.grad = torch.zeros(self.n, device=device)
         self.lp = torch.zeros(self.n, device=device, dtype=dtype) if dtype != torch.float32 else self.master
-        self.a_neg = [torch.empty(di, N, device=device) for _ in range(cfg.n_layers)]
+        self._a_neg_all = torch.empty(cfg.n_layers, di, N, device=device)
+        self.a_neg = list(self._a_neg_all)
 
     # ---- views ----
     def _views(self, flat, l):
@@ -159,6 +161,60 @@ class MambaWeights:
         return self
 
 
+class _DecodePlan:
+    """Arguments and workspace of the whole-model decode launch (``mamba_b200_decode_step``) for one
+    engine and batch size; ``ok`` is False where the kernel does not take the model or batch."""
+
+    def __init__(self, bb: "GpuMambaBackbone", B: int, lm: "GpuMambaLM | None" = None):
+        w, c = bb.w, bb.cfg
+        self.key = self.pointers(bb)
+        self.handle = ffi.default_handle(w.device.index or 0)
+        a = self.args = ffi.DecodeArgs()
+        a.dtype = ops.dtype_code(w.dtype)
+        a.B, a.batch_capacity, a.d_model, a.d_inner = B, bb.batch, c.d_model, c.d_inner
+        a.N, a.K, a.dt_rank, a.n_layers = c.d_state, c.d_conv, c.dt_rank, c.n_layers
+        a.vocab, a.eps = (w.vocab if lm else 0), c.rms_norm_eps
+        a.lp, a.master, a.a_neg, a.conv_state, a.ssm_state = self.key
+        a.layer_stride = w.layer_size
+        offset, o = {}, 0
+        for k in _LAYER_FIELDS:
+            offset[k], o = o, o + math.prod(w.shapes[k])
+        a.o_in_proj, a.o_conv_w, a.o_conv_b = offset["in_proj_w"], offset["conv_w"], offset["conv_b"]
+        a.o_x_proj, a.o_dt_proj_w, a.o_dt_proj_b = offset["x_proj_w"], offset["dt_proj_w"], offset["dt_proj_b"]
+        a.o_d_param, a.o_out_proj = offset["d_param"], offset["out_proj_w"]
+        a.o_norm_f = c.n_layers * w.layer_size
+        a.o_embedding = a.o_norm_f + c.d_model
+        a.steps = 1
+        lib = ffi.lib()
+        # the kernel walks the decay rates as one [n_layers, d_inner, N] array
+        whole = all(t.data_ptr() == w._a_neg_all[l].data_ptr() for l, t in enumerate(w.a_neg))
+        a.workspace_bytes = lib.mamba_b200_decode_workspace_bytes(self.handle.ptr, C.byref(a)) if whole else 0
+        self.ok = a.workspace_bytes > 0
+        if self.ok:
+            self.ws = torch.zeros(a.workspace_bytes, dtype=torch.uint8, device=w.device)
+            a.workspace = self.ws.data_ptr()
+            if lm is not None:
+                self.res = torch.empty(B, c.d_model, device=w.device)
+                a.residual = self.res.data_ptr()
+        self._call, self._ref = lib.mamba_b200_decode_step, C.byref(a)
+
+    @staticmethod
+    def pointers(bb):
+        w = bb.w
+        return (w.lp.data_ptr(), w.master.data_ptr(), w._a_neg_all.data_ptr(), bb.conv.data_ptr(), bb.ssm.data_ptr())
+
+    def launch(self):
+        dev = self.handle.device
+        stream = torch.cuda.current_stream(dev).cuda_stream
+        if torch.cuda.current_device() == dev:
+            rc = self._call(self.handle.ptr, stream, self._ref)
+        else:
+            with torch.cuda.device(dev):
+                rc = self._call(self.handle.ptr, stream, self._ref)
+        if rc:
+            self.handle.check(rc, "mamba_b200_decode_step")
+
+
 class GpuMambaBackbone:
     """Prefill + decode over a residual stream [B, T, d_model] f32
     (``GpuMambaBackbone``, src/mamba_ssm/gpu/inference.rs:1515-1855): ``prefill_sequence``
@@ -171,6 +227,16 @@ class GpuMambaBackbone:
         self.conv = torch.zeros(c.n_layers, batch, c.d_inner, c.d_conv, device=dev)
         self.ssm = torch.zeros(c.n_layers, batch, c.d_inner, c.d_state, device=dev)
         self._ws = {}
+        self._plans = {}
+
+    def _plan(self, B):
+        """The decode launch for B sequences, rebuilt when a buffer it points at was replaced."""
+        p = self._plans.get(B)
+        if p is None or p.key != _DecodePlan.pointers(self):
+            if len(self._plans) >= 8:
+                self._plans.clear()
+            p = self._plans[B] = _DecodePlan(self, B)
+        return p
 
     def reset(self):
         self.conv.zero_()
@@ -210,9 +276,18 @@ class GpuMambaBackbone:
         return out.view(B, T, dm)
 
     def step(self, temporal: torch.Tensor) -> torch.Tensor:
-        """One token per sequence: temporal [B, d_model] f32 -> [B, d_model] (compute dtype)."""
+        """One token per sequence: temporal [B, d_model] f32 -> [B, d_model] (compute dtype).  The
+        input tensor is used as the residual stream (updated in place).  One launch for the whole
+        model where ``mamba_b200_decode_step`` takes it, else the operators one by one."""
         c, w = self.cfg, self.w
         B, dm = temporal.shape
+        plan = self._plan(B)
+        if (plan.ok and B <= self.batch and temporal.is_cuda and temporal.dtype == torch.float32
+                and temporal.is_contiguous() and temporal.data_ptr() % 16 == 0):
+            out = torch.empty(B, dm, device=temporal.device, dtype=w.dtype)
+            plan.args.residual, plan.args.out = temporal.data_ptr(), out.data_ptr()
+            plan.launch()
+            return out
         di, N, dr = c.d_inner, c.d_state, c.dt_rank
         res = temporal
         branch = None
@@ -237,8 +312,9 @@ class GpuMambaBackbone:
 class GpuMambaLM:
     """Token-level wrapper with a tied head (``GpuMambaLM``, src/module/gpu_lm.rs:136-679):
     ``prefill`` runs whole prompts through the backbone and returns the logits of the last
-    position, ``generate_greedy`` decodes token by token.  One decode step (embedding row,
-    24-layer step, head GEMM, argmax) is captured in a CUDA graph on first use and replayed,
+    position, ``generate_greedy`` decodes token by token: one launch per token
+    (``mamba_b200_decode_step``) where the model allows it.  Otherwise one decode step (embedding
+    row, 24-layer step, head GEMM, argmax) is captured in a CUDA graph on first use and replayed,
     as the reference captures its step (src/mamba_ssm/gpu/inference.rs:1608-1630)."""
 
     def __init__(self, weights: MambaWeights, batch: int):
@@ -250,6 +326,7 @@ class GpuMambaLM:
         self.next_ids = torch.zeros(batch, dtype=torch.int32, device=dev)
         self.logits = torch.empty(batch, weights.vocab, device=dev, dtype=weights.dtype)
         self._graph = None
+        self._dec = None
 
     def prefill(self, ids: torch.Tensor) -> torch.Tensor:
         """ids [B, T] int32 -> logits of the last position [B, vocab]; leaves the greedy
@@ -272,6 +349,14 @@ class GpuMambaLM:
     def generate_greedy(self, n: int, use_graph: bool = True) -> torch.Tensor:
         """n greedy tokens after a prefill; returns them as [B, n] int32."""
         out = torch.empty(self.batch, n, dtype=torch.int32, device=self.w.device)
+        if self._dec is None or self._dec.key != _DecodePlan.pointers(self.backbone):
+            self._dec = _DecodePlan(self.backbone, self.batch, self)
+        if self._dec.ok and n > 0:
+            a = self._dec.args
+            a.next_ids, a.logits, a.steps = self.next_ids.data_ptr(), self.logits.data_ptr(), n
+            a.tokens, a.tokens_ld = out.data_ptr(), n
+            self._dec.launch()
+            return out
         if use_graph and self._graph is None:
             dev = self.w.device
             keep = (self.backbone.conv.clone(), self.backbone.ssm.clone(), self.next_ids.clone())
