@@ -450,6 +450,11 @@ MAMBA_B200_API int mamba_b200_conv1d_bwd_static(void* handle, void* stream, cons
 MAMBA_B200_API int mamba_b200_residual_rmsnorm_fwd(void* handle, void* stream, int dtype, float* residual,
                                     const void* branch, const float* scale, void* y, float* rms_out,
                                     int rows, int dim, float eps);
+/* The same with the sum written to residual_out and `residual` kept: what a trainer that saves the
+ * stream of every layer would otherwise copy.  Without a branch residual_out is not written. */
+MAMBA_B200_API int mamba_b200_residual_rmsnorm_fwd_to(void* handle, void* stream, int dtype, const float* residual,
+                                       const void* branch, const float* scale, float* residual_out, void* y,
+                                       float* rms_out, int rows, int dim, float eps);
 MAMBA_B200_API long long mamba_b200_residual_rmsnorm_bwd_workspace_bytes(int rows, int dim);
 MAMBA_B200_API int mamba_b200_residual_rmsnorm_bwd(void* handle, void* stream, int dtype, const void* dy,
                                     const float* x, const float* scale, const float* rms_saved,
@@ -466,7 +471,7 @@ MAMBA_B200_API int mamba_b200_residual_rmsnorm_bwd(void* handle, void* stream, i
  *             (table in the storage dtype; an id outside [0, vocab) gives a zero row).
  *   softmax_xent    : per row of logits [rows, ld] (V used columns, storage dtype):
  *             loss_rows[r] = logsumexp(l) - l[target]; with d_logits != NULL also
- *             d_logits = (softmax(l) - onehot(target)) * grad_scale.  target < 0 marks a
+ *             d_logits = (softmax(l) - onehot(target)) * grad_scale (may be the logits themselves).  target < 0 marks a
  *             row that does not count (loss 0, zero gradient).  One read of the logits,
  *             one write of the gradient when a row fits shared memory (V * size <= 208 KB).
  *   adamw_step      : adamw_step_f32_capturable (kernels/adamw.cu:30-61; decoupled decay,

@@ -44,9 +44,8 @@ __global__ void __launch_bounds__(256) embedding_gather_kernel(const Tact* __res
 // count: loss 0, zero gradient.  The row is kept in shared memory in its storage
 // dtype between the two passes when it fits, so the logits are read once.
 template <typename Tact, bool VEC>
-__global__ void __launch_bounds__(512) softmax_xent_kernel(const Tact* __restrict__ logits,
-                                                           const int* __restrict__ targets, float* __restrict__ loss,
-                                                           Tact* __restrict__ dlogits, float grad_scale, int V,
+__global__ void __launch_bounds__(512) softmax_xent_kernel(const Tact* logits, const int* __restrict__ targets,
+                                                           float* __restrict__ loss, Tact* dlogits, float grad_scale, int V,
                                                            long long ld, int cache_row) {
     extern __shared__ __align__(16) unsigned char xsm[];
     __shared__ float red_m[16], red_s[16];
@@ -98,6 +97,8 @@ __global__ void __launch_bounds__(512) softmax_xent_kernel(const Tact* __restric
         m = mm;
     }
     const int warp = tid >> 5, lane = tid & 31, nw = blockDim.x >> 5;
+    const bool counted = tgt >= 0 && tgt < V;
+    const float lt = tid == 0 && counted ? to_f(row[tgt]) : 0.0f;  // before d_logits may overwrite it
     if (lane == 0) {
         red_m[warp] = m;
         red_s[warp] = s;
@@ -108,8 +109,7 @@ __global__ void __launch_bounds__(512) softmax_xent_kernel(const Tact* __restric
     float S = 0.0f;
     for (int w = 0; w < nw; ++w)
         if (red_m[w] != -INFINITY) S += red_s[w] * ex2((red_m[w] - M) * kLog2e);
-    const bool counted = tgt >= 0 && tgt < V;
-    if (tid == 0) loss[r] = counted ? (M + lg2(S) * kLn2) - to_f(row[tgt]) : 0.0f;
+    if (tid == 0) loss[r] = counted ? (M + lg2(S) * kLn2) - lt : 0.0f;
     if (!dlogits) return;
     const float inv = counted ? grad_scale / S : 0.0f;
     Tact* drow = dlogits + r * ld;

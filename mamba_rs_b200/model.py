@@ -82,6 +82,7 @@ class MambaWeights:
         self.lp = torch.zeros(self.n, device=device, dtype=dtype) if dtype != torch.float32 else self.master
         self._a_neg_all = torch.empty(cfg.n_layers, di, N, device=device)
         self.a_neg = list(self._a_neg_all)
+        self._view_cache = {}
 
     # ---- views ----
     def _views(self, flat, l):
@@ -93,11 +94,22 @@ class MambaWeights:
             o += n
         return out
 
+    def _cached(self, key, flat, make):
+        """Views of an arena are made once and kept while the arena is the same tensor."""
+        got = self._view_cache.get(key)
+        if got is None or got[0] is not flat:
+            got = self._view_cache[key] = (flat, make())
+        return got[1]
+
     def layer(self, l, which="lp"):
-        return self._views(getattr(self, which), l)
+        flat = getattr(self, which)
+        return self._cached((which, l), flat, lambda: self._views(flat, l))
 
     def tail(self, which="lp"):
         flat = getattr(self, which)
+        return self._cached((which, "tail"), flat, lambda: self._tail_views(flat))
+
+    def _tail_views(self, flat):
         o = self.cfg.n_layers * self.layer_size
         dm = self.cfg.d_model
         out = dict(norm_f=flat[o:o + dm])
@@ -115,8 +127,19 @@ class MambaWeights:
         """master -> compute copy, and a_neg = -exp(a_log) (trainer.rs:78-111)."""
         if self.lp is not self.master:
             self.lp.copy_(self.master)
-        for l in range(self.cfg.n_layers):
-            torch.exp(self.layer(l, "master")["a_log"], out=self.a_neg[l]).neg_()
+        self.refresh_a_neg()
+
+    def refresh_a_neg(self):
+        """a_neg = -exp(a_log) of every layer, over the whole arena at once (unless a layer's tensor
+        was replaced)."""
+        whole = all(t.data_ptr() == self._a_neg_all[l].data_ptr() for l, t in enumerate(self.a_neg))
+        if whole:
+            a = self.layer(0, "master")["a_log"]
+            logs = torch.as_strided(self.master, self._a_neg_all.shape, (self.layer_size, *a.stride()), a.storage_offset())
+            torch.exp(logs, out=self._a_neg_all).neg_()
+        else:
+            for l in range(self.cfg.n_layers):
+                torch.exp(self.layer(l, "master")["a_log"], out=self.a_neg[l]).neg_()
 
     def init_random(self, seed: int):
         """MambaWeights::init (src/weights.rs:107-160): Kaiming-uniform projections,
@@ -159,6 +182,109 @@ class MambaWeights:
         self.tail("master")["norm_f"].copy_(torch.as_tensor(norm_f, dtype=torch.float32))
         self.refresh()
         return self
+
+
+class _Launcher:
+    """The library's entry points on one device's current stream, with the arguments a plan has
+    prepared: what a layer's launches cost on the host is then the call itself."""
+
+    def __init__(self, device):
+        self.handle = ffi.default_handle(device.index or 0)
+        self.dev, self.h, self.lib = self.handle.device, self.handle.ptr, ffi.lib()
+        self.stream = 0
+
+    def begin(self):
+        """Reads the current stream; returns the context the launches of one pass run in."""
+        self.stream = torch._C._cuda_getCurrentRawStream(self.dev)
+        return ops._on(torch.device("cuda", self.dev))
+
+    def call(self, fn, *args):
+        rc = fn(self.h, self.stream, *args)
+        if rc:
+            self.handle.check(rc, getattr(fn, "__name__", "kernel call"))
+
+
+class _PrefillPlan:
+    """Everything about a prefill of B x T tokens that does not change from call to call: the C
+    argument structs of every layer and the weights' views.  Activations come from the caching
+    allocator on each call (they are the same for every layer, and are given back); the structs are
+    pointed at them again when their addresses have changed."""
+
+    def __init__(self, bb: "GpuMambaBackbone", B: int, T: int):
+        w, c = bb.w, bb.cfg
+        self.key = self.pointers(bb)
+        self.bb, self.B, self.T, self.where = bb, B, T, None
+        self.run_on = _Launcher(w.device)
+        di, N, dr, xd = c.d_inner, c.d_state, c.dt_rank, c.xdbl_dim
+        self.dt, self.es = ops.dtype_code(w.dtype), w.lp.element_size()
+        self.ws_bytes = ops.selective_scan_fwd_workspace_bytes(B, T, di, N)
+        self.layers = []
+        for l in range(c.n_layers):
+            p, pm = w.layer(l), w.layer(l, "master")
+            cv, sc = ffi.Conv1dArgs(), ffi.SscanFwdArgs()
+            cv.dtype, cv.B, cv.T, cv.D, cv.K = self.dt, B, T, di, c.d_conv
+            cv.ld_x, cv.ld_u = 2 * di, di
+            cv.conv_w, cv.conv_b, cv.conv_state = pm["conv_w"].data_ptr(), pm["conv_b"].data_ptr(), bb.conv[l].data_ptr()
+            sc.dtype, sc.B, sc.T, sc.D, sc.N = self.dt, B, T, di, N
+            sc.ld_x, sc.ld_delta, sc.delta_softplus, sc.ld_bc, sc.ld_z, sc.z_mode, sc.ld_y = di, di, 1, xd, 2 * di, 1, di
+            sc.a_neg, sc.Dp, sc.ssm_state = w.a_neg[l].data_ptr(), pm["d_param"].data_ptr(), bb.ssm[l].data_ptr()
+            sc.workspace_bytes = self.ws_bytes
+            self.layers.append((pm["norm_w"].data_ptr(), p["in_proj_w"], C.byref(cv), p["x_proj_w"], p["dt_proj_b"],
+                                p["dt_proj_w"], C.byref(sc), p["out_proj_w"], cv, sc))
+        self.norm_f = w.tail("master")["norm_f"].data_ptr()
+
+    @staticmethod
+    def pointers(bb):
+        return _DecodePlan.pointers(bb) + tuple(a.data_ptr() for a in bb.w.a_neg)
+
+    def point(self, proj, u, xdbl, delta, y, ws):
+        di, N, dr, es = self.bb.cfg.d_inner, self.bb.cfg.d_state, self.bb.cfg.dt_rank, self.es
+        self.where = (proj, u, xdbl, delta, y, ws)
+        for layer in self.layers:
+            cv, sc = layer[-2:]
+            cv.x, cv.u = proj, u
+            sc.x, sc.delta, sc.Bm, sc.Cm = u, delta, xdbl + dr * es, xdbl + (dr + N) * es
+            sc.z, sc.y, sc.workspace = proj + di * es, y, ws
+
+    def run(self, temporal, last_only=False):
+        """The backbone over temporal [B, T, d_model] (updated in place).  last_only: only the last
+        position's normalised row is wanted, so the last out_proj and the last norm take that row."""
+        bb, B, T = self.bb, self.B, self.T
+        c, w = bb.cfg, bb.w
+        dm, di, dr, BT = c.d_model, c.d_inner, c.dt_rank, B * T
+        new = lambda *shape: torch.empty(shape, dtype=w.dtype, device=temporal.device)  # noqa: E731
+        post, proj, u, xdbl, delta, y = new(BT, dm), new(BT, 2 * di), new(BT, di), new(BT, c.xdbl_dim), new(BT, di), new(BT, di)
+        ws = torch.empty(self.ws_bytes, dtype=torch.uint8, device=temporal.device)
+        where = (proj.data_ptr(), u.data_ptr(), xdbl.data_ptr(), delta.data_ptr(), y.data_ptr(), ws.data_ptr())
+        if where != self.where:
+            self.point(*where)
+        branch, dtx = post, xdbl[:, :dr]  # the norm reads its branch row before it writes the row over it
+        go, lib = self.run_on, self.run_on.lib
+        norm, conv, scan = lib.mamba_b200_residual_rmsnorm_fwd, lib.mamba_b200_conv1d_fwd, lib.mamba_b200_sscan_fwd
+        res_p, post_p = temporal.data_ptr(), post.data_ptr()
+        mm, addmm = torch.mm, torch.addmm
+        with go.begin():
+            br = None
+            for norm_w, w_in, cv, w_x, b_dt, w_dt, sc, w_out, *_ in self.layers:
+                go.call(norm, self.dt, res_p, br, norm_w, post_p, None, BT, dm, c.rms_norm_eps)
+                mm(post, w_in, out=proj)                                    # [BT, 2 di]: x | z in place
+                go.call(conv, cv)
+                mm(u, w_x, out=xdbl)                                        # [BT, dr + 2N]: dt | B | C in place
+                addmm(b_dt, dtx, w_dt, out=delta)
+                go.call(scan, sc)
+                if last_only and w_out is self.layers[-1][7]:
+                    break
+                mm(y, w_out, out=branch)
+                br = post_p
+            if last_only:
+                rows = temporal.view(B, T, dm)[:, -1].contiguous()
+                last = y.view(B, T, di)[:, -1] @ self.layers[-1][7]
+                out = torch.empty_like(last)
+                go.call(norm, self.dt, rows.data_ptr(), last.data_ptr(), self.norm_f, out.data_ptr(), None, B, dm, c.rms_norm_eps)
+                return out
+            out = new(BT, dm)
+            go.call(norm, self.dt, res_p, br, self.norm_f, out.data_ptr(), None, BT, dm, c.rms_norm_eps)
+        return out.view(B, T, dm)
 
 
 class _DecodePlan:
@@ -226,8 +352,7 @@ class GpuMambaBackbone:
         dev, c = weights.device, weights.cfg
         self.conv = torch.zeros(c.n_layers, batch, c.d_inner, c.d_conv, device=dev)
         self.ssm = torch.zeros(c.n_layers, batch, c.d_inner, c.d_state, device=dev)
-        self._ws = {}
-        self._plans = {}
+        self._plans, self._prefills = {}, {}
 
     def _plan(self, B):
         """The decode launch for B sequences, rebuilt when a buffer it points at was replaced."""
@@ -242,38 +367,24 @@ class GpuMambaBackbone:
         self.conv.zero_()
         self.ssm.zero_()
 
-    def _fwd_ws(self, B, T):
-        key = (B, T)
-        if key not in self._ws:
-            c = self.cfg
-            self._ws[key] = torch.empty(ops.selective_scan_fwd_workspace_bytes(B, T, c.d_inner, c.d_state),
-                                        dtype=torch.uint8, device=self.w.device)
-        return self._ws[key]
-
     def prefill_sequence(self, temporal: torch.Tensor) -> torch.Tensor:
         """temporal [B, T, d_model] f32 (embedded inputs) -> norm_f(residual) [B, T, d_model]
         in the compute dtype.  The input tensor is used as the residual stream (updated in place)."""
-        c, w = self.cfg, self.w
+        return self._prefill(temporal, False)
+
+    def _prefill(self, temporal, last_only):
         B, T, dm = temporal.shape
-        di, N, dr = c.d_inner, c.d_state, c.dt_rank
-        res = temporal.view(B * T, dm)
-        branch = None
-        for l in range(c.n_layers):
-            p = w.layer(l)
-            post, _ = ops.residual_rmsnorm_fwd(res, branch, w.layer(l, "master")["norm_w"], eps=c.rms_norm_eps,
-                                               out_dtype=w.dtype)
-            proj = post @ p["in_proj_w"]                                   # [BT, 2 di]: x | z in place
-            pv = proj.view(B, T, 2 * di)
-            u = ops.conv1d_fwd(pv[..., :di], w.layer(l, "master")["conv_w"], w.layer(l, "master")["conv_b"], self.conv[l])
-            xdbl = u.view(B * T, di) @ p["x_proj_w"]                       # [BT, dr + 2N]: dt | B | C in place
-            delta = torch.addmm(p["dt_proj_b"], xdbl[:, :dr], p["dt_proj_w"])
-            xv = xdbl.view(B, T, c.xdbl_dim)
-            y = ops.selective_scan_fwd(u, delta.view(B, T, di), xv[..., dr:dr + N], xv[..., dr + N:], w.a_neg[l],
-                                       w.layer(l, "master")["d_param"], pv[..., di:], ssm_state=self.ssm[l],
-                                       workspace=self._fwd_ws(B, T))
-            branch = y.view(B * T, di) @ p["out_proj_w"]
-        out, _ = ops.residual_rmsnorm_fwd(res, branch, w.tail("master")["norm_f"], eps=c.rms_norm_eps, out_dtype=w.dtype)
-        return out.view(B, T, dm)
+        ops._require_cuda(temporal)
+        if temporal.dtype != torch.float32 or not temporal.is_contiguous() or dm != self.cfg.d_model:
+            raise TypeError("temporal is contiguous float32 [B, T, d_model]")
+        if B > self.batch:
+            raise ValueError(f"{B} sequences, the engine's state holds {self.batch}")
+        p = self._prefills.get((B, T))
+        if p is None or p.key != _PrefillPlan.pointers(self):
+            if len(self._prefills) >= 64:
+                self._prefills.clear()
+            p = self._prefills[B, T] = _PrefillPlan(self, B, T)
+        return p.run(temporal, last_only)
 
     def step(self, temporal: torch.Tensor) -> torch.Tensor:
         """One token per sequence: temporal [B, d_model] f32 -> [B, d_model] (compute dtype).  The
@@ -334,8 +445,8 @@ class GpuMambaLM:
         B, T = ids.shape
         emb = self.w.tail()["embedding"]
         temporal = ops.embedding_gather(emb, ids.contiguous()).view(B, T, -1)
-        hidden = self.backbone.prefill_sequence(temporal)
-        torch.matmul(hidden[:, -1], emb.t(), out=self.logits)
+        hidden = self.backbone._prefill(temporal, True)
+        torch.matmul(hidden, emb.t(), out=self.logits)
         self.next_ids.copy_(self.logits.argmax(dim=1))
         return self.logits
 
@@ -380,6 +491,91 @@ class GpuMambaLM:
         return out
 
 
+class _TrainPlan:
+    """What a training step on B x T tokens does not work out again each time: the C argument structs
+    of every layer, forward and backward, and the weights' views.  Activations and gradients come from
+    the caching allocator in each step; the structs are pointed at them when their addresses changed."""
+
+    class Layer:
+        __slots__ = ("norm_w", "g_norm", "w_in", "w_in_t", "w_x", "w_x_t", "b_dt", "w_dt", "w_dt_t", "w_out", "w_out_t",
+                     "conv", "scan", "conv_b", "scan_b", "structs")
+
+    def __init__(self, w: MambaWeights, B: int, T: int, save: int):
+        c = w.cfg
+        self.key, self.B, self.T, self.w = self.pointers(w), B, T, w
+        self.run_on = _Launcher(w.device)
+        di, N, K, xd, S = c.d_inner, c.d_state, c.d_conv, c.xdbl_dim, save
+        self.blocks = (T + S - 1) // S
+        self.dt, self.es = ops.dtype_code(w.dtype), w.lp.element_size()
+        lib = ffi.lib()
+        self.fwd_ws = ops.selective_scan_fwd_workspace_bytes(B, T, di, N)
+        self.bwd_ws = max(ops.selective_scan_bwd_workspace_bytes(B, T, di, N),
+                          lib.mamba_b200_conv1d_bwd_workspace_bytes(B, T, di, K),
+                          lib.mamba_b200_residual_rmsnorm_bwd_workspace_bytes(B * T, c.d_model), 1)
+        self.norm_f = w.tail("master")["norm_f"].data_ptr()
+        self.fwd_at = self.bwd_at = None
+        self.layers = []
+        for l in range(c.n_layers):
+            p, pm, g, lay = w.layer(l), w.layer(l, "master"), w.layer(l, "grad"), self.Layer()
+            lay.norm_w, lay.g_norm = pm["norm_w"].data_ptr(), g["norm_w"].data_ptr()
+            lay.w_in, lay.w_x, lay.b_dt, lay.w_dt, lay.w_out = (p[k] for k in ("in_proj_w", "x_proj_w", "dt_proj_b", "dt_proj_w", "out_proj_w"))
+            lay.w_in_t, lay.w_x_t, lay.w_dt_t, lay.w_out_t = (t.t() for t in (lay.w_in, lay.w_x, lay.w_dt, lay.w_out))
+            cv, sc, cb, sb = ffi.Conv1dArgs(), ffi.SscanFwdArgs(), ffi.Conv1dArgs(), ffi.SscanBwdArgs()
+            for q in (cv, cb):
+                q.dtype, q.B, q.T, q.D, q.K, q.ld_x = self.dt, B, T, di, K, 2 * di
+                q.conv_w, q.conv_b = pm["conv_w"].data_ptr(), pm["conv_b"].data_ptr()
+            cv.ld_u = cb.ld_du = di
+            cb.ld_dx, cb.dconv_w, cb.dconv_b, cb.workspace_bytes = 2 * di, g["conv_w"].data_ptr(), g["conv_b"].data_ptr(), self.bwd_ws
+            for q in (sc, sb):
+                q.dtype, q.B, q.T, q.D, q.N = self.dt, B, T, di, N
+                q.ld_delta, q.delta_softplus, q.ld_bc, q.ld_z, q.z_mode = di, 1, xd, 2 * di, 1
+                q.a_neg, q.Dp, q.save_stride = w.a_neg[l].data_ptr(), pm["d_param"].data_ptr(), S
+            sc.ld_x = sc.ld_y = sb.ld_u = sb.ld_dy = sb.ld_du = sb.ld_ddelta = di
+            sc.workspace_bytes, sb.workspace_bytes, sb.ld_dz = self.fwd_ws, self.bwd_ws, 2 * di
+            sb.dA_log, sb.dD = g["a_log"].data_ptr(), g["d_param"].data_ptr()
+            lay.structs = (cv, sc, cb, sb)
+            lay.conv, lay.scan, lay.conv_b, lay.scan_b = (C.byref(q) for q in lay.structs)
+            self.layers.append(lay)
+
+    @staticmethod
+    def pointers(w):
+        return (w.lp.data_ptr(), w.master.data_ptr(), w.grad.data_ptr()) + tuple(a.data_ptr() for a in w.a_neg)
+
+    def _at(self, l, proj, u, xdbl, delta, cs):
+        """Addresses of layer l's saved x, z, u, B, C, delta and block states."""
+        c, es, BT = self.w.cfg, self.es, self.B * self.T
+        di, N, xd = c.d_inner, c.d_state, c.xdbl_dim
+        x, b = proj + es * BT * 2 * di * l, xdbl + es * (BT * xd * l + c.dt_rank)
+        return (x, x + es * di, u + es * BT * di * l, b, b + es * N, delta + es * BT * di * l,
+                cs + 4 * self.B * self.blocks * di * N * l)
+
+    def point_forward(self, proj, u, xdbl, delta, y, cs, ws):
+        at = tuple(t.data_ptr() for t in (proj, u, xdbl, delta, y, cs, ws))
+        if at == self.fwd_at:
+            return
+        self.fwd_at = at
+        step = self.es * self.B * self.T * self.w.cfg.d_inner
+        for l, lay in enumerate(self.layers):
+            cv, sc = lay.structs[:2]
+            x, z, u_l, b, c_, d, s_ = self._at(l, at[0], at[1], at[2], at[3], at[5])
+            cv.x, cv.u = x, u_l
+            sc.x, sc.delta, sc.Bm, sc.Cm, sc.z, sc.y, sc.chunk_states, sc.workspace = u_l, d, b, c_, z, at[4] + step * l, s_, at[6]
+
+    def point_backward(self, acts, d_y, d_u, d_delta, d_proj, d_bc, ws):
+        at = tuple(t.data_ptr() for t in (acts["proj"], acts["u"], acts["xdbl"], acts["delta"], acts["cs"], d_y, d_u, d_delta, d_proj, d_bc, ws))
+        if at == self.bwd_at:
+            return
+        self.bwd_at = at
+        dz = at[8] + self.es * self.w.cfg.d_inner
+        dc = at[9] + 4 * self.B * self.T * self.w.cfg.d_state
+        for l, lay in enumerate(self.layers):
+            cb, sb = lay.structs[2:]
+            x, z, u_l, b, c_, d, s_ = self._at(l, *at[:5])
+            sb.u, sb.delta, sb.Bm, sb.Cm, sb.z, sb.chunk_states, sb.dy = u_l, d, b, c_, z, s_, at[5]
+            sb.d_u, sb.d_delta, sb.d_z, sb.dBm, sb.dCm, sb.workspace = at[6], at[7], dz, at[9], dc, at[10]
+            cb.x, cb.d_u, cb.d_x, cb.workspace = x, at[6], at[8], at[10]
+
+
 class MambaLMTrainer:
     """A next-token training step on the device: embedding gather, the backbone forward
     with block-boundary state saves, tied-head logits, softmax cross-entropy, the manual
@@ -402,6 +598,7 @@ class MambaLMTrainer:
         self.bias = torch.ones(2, device=weights.device)
         self._acts = None
         self._pending = 0
+        self._plans = {}
 
     # ---- forward ----
     def forward(self, ids: torch.Tensor) -> torch.Tensor:
@@ -410,81 +607,116 @@ class MambaLMTrainer:
         c, w = self.cfg, self.w
         B, T1 = ids.shape
         T = T1 - 1
-        di, N, dr, dm = c.d_inner, c.d_state, c.dt_rank, c.d_model
-        S = self.SAVE
+        dm, BT, L = c.d_model, B * T, c.n_layers
+        dev, plan = w.device, self._plan(B, T)
         emb = w.tail()["embedding"]
         inp = ids[:, :-1].contiguous()
-        res = ops.embedding_gather(emb, inp)                      # [BT, dm] f32 residual stream
-        acts, branch = [], None
-        for l in range(c.n_layers):
-            p, pm = w.layer(l), w.layer(l, "master")
-            post, rms = ops.residual_rmsnorm_fwd(res, branch, pm["norm_w"], eps=c.rms_norm_eps, out_dtype=w.dtype)
-            x_res = res.clone()                                    # the stream this norm saw
-            proj = post @ p["in_proj_w"]
-            pv = proj.view(B, T, 2 * di)
-            u = ops.conv1d_fwd(pv[..., :di], pm["conv_w"], pm["conv_b"])
-            xdbl = u.view(B * T, di) @ p["x_proj_w"]
-            delta = torch.addmm(p["dt_proj_b"], xdbl[:, :dr], p["dt_proj_w"])
-            xv = xdbl.view(B, T, c.xdbl_dim)
-            cs = torch.empty(B, (T + S - 1) // S, di, N, device=res.device)
-            y = ops.selective_scan_fwd(u, delta.view(B, T, di), xv[..., dr:dr + N], xv[..., dr + N:], w.a_neg[l],
-                                       pm["d_param"], pv[..., di:], chunk_states=cs, save_stride=S)
-            branch = y.view(B * T, di) @ p["out_proj_w"]
-            acts.append(dict(x_res=x_res, rms=rms, post=post, proj=proj, u=u, xdbl=xdbl, delta=delta, cs=cs, y=y))
-        hidden, rms_f = ops.residual_rmsnorm_fwd(res, branch, w.tail("master")["norm_f"], eps=c.rms_norm_eps,
-                                                 out_dtype=w.dtype)
+        go, lib = plan.run_on, plan.run_on.lib
+        new = lambda *shape: torch.empty(shape, dtype=w.dtype, device=dev)  # noqa: E731
+        f32 = lambda *shape: torch.empty(shape, device=dev)  # noqa: E731
+        # saved activations, one tensor per kind over all layers: residual stream as each norm saw it
+        # ([0] is the embedding), row rms, normalised rows, x | z, u, dt | B | C, delta, y, block states
+        di = c.d_inner
+        res, rms = f32(L + 1, BT, dm), f32(L + 1, BT)
+        post, proj, u, xdbl = new(L, BT, dm), new(L, BT, 2 * di), new(L, BT, di), new(L, BT, c.xdbl_dim)
+        delta, y, cs = new(L, BT, di), new(L, BT, di), f32(L, B, plan.blocks, di, c.d_state)
+        branch, hidden, ws = new(BT, dm), new(BT, dm), torch.empty(plan.fwd_ws, dtype=torch.uint8, device=dev)
+        plan.point_forward(proj, u, xdbl, delta, y, cs, ws)
+        norm, conv, scan = lib.mamba_b200_residual_rmsnorm_fwd_to, lib.mamba_b200_conv1d_fwd, lib.mamba_b200_sscan_fwd
+        ops.embedding_gather(emb, inp, res[0])
+        mm, addmm, dr = torch.mm, torch.addmm, c.dt_rank
+        res_p, rms_p, post_p, branch_p = res.data_ptr(), rms.data_ptr(), post.data_ptr(), branch.data_ptr()
+        with go.begin():
+            acts = list(zip(post.unbind(), proj.unbind(), u.unbind(), xdbl.unbind(), delta.unbind(), y.unbind()))
+            for l, (lay, (post_l, proj_l, u_l, xdbl_l, delta_l, y_l)) in enumerate(zip(plan.layers, acts)):
+                # the stream this layer's norm saw is kept in res[l]; the embedding is there already
+                go.call(norm, plan.dt, res_p + 4 * BT * dm * max(l - 1, 0), branch_p if l else None, lay.norm_w,
+                        res_p + 4 * BT * dm * l, post_p + plan.es * BT * dm * l, rms_p + 4 * BT * l, BT, dm, c.rms_norm_eps)
+                mm(post_l, lay.w_in, out=proj_l)
+                go.call(conv, lay.conv)
+                mm(u_l, lay.w_x, out=xdbl_l)
+                addmm(lay.b_dt, xdbl_l[:, :dr], lay.w_dt, out=delta_l)
+                go.call(scan, lay.scan)
+                mm(y_l, lay.w_out, out=branch)
+            go.call(norm, plan.dt, res_p + 4 * BT * dm * (L - 1), branch_p, plan.norm_f, res_p + 4 * BT * dm * L,
+                    hidden.data_ptr(), rms_p + 4 * BT * L, BT, dm, c.rms_norm_eps)
         logits = hidden @ emb.t()                                  # tied head, [BT, V]
         tgt = ids[:, 1:].contiguous().view(-1)
-        loss_rows, dlogits = ops.softmax_xent(logits, tgt, grad_scale=1.0 / (B * T))
-        self._acts = dict(layers=acts, res_f=res, rms_f=rms_f, hidden=hidden, dlogits=dlogits, inp=inp, B=B, T=T)
-        return loss_rows.sum() / (B * T)
+        # the gradient takes the logits' place: every row is read before it is written
+        loss_rows, dlogits = ops.softmax_xent(logits, tgt, grad_scale=1.0 / BT, dlogits=logits)
+        self._acts = dict(layers=acts, res=res, rms=rms, proj=proj, u=u, xdbl=xdbl, delta=delta, cs=cs, hidden=hidden,
+                          dlogits=dlogits, inp=inp, B=B, T=T, plan=plan)
+        return loss_rows.sum() / BT
+
+    def _plan(self, B, T):
+        p = self._plans.get((B, T))
+        if p is None or p.key != _TrainPlan.pointers(self.w):
+            if len(self._plans) >= 16:
+                self._plans.clear()
+            p = self._plans[B, T] = _TrainPlan(self.w, B, T, self.SAVE)
+        return p
+
+    def _accumulate(self, g, a, b):
+        """g (f32) += a.T @ b, the product accumulated into g by the GEMM itself."""
+        if a.dtype == torch.float32:
+            g.addmm_(a.t(), b)
+        else:
+            torch.addmm(g, a.t(), b, out_dtype=torch.float32, out=g)
 
     # ---- backward + optimiser ----
     def backward_step(self, accumulate_only: bool = False):
         c, w, a = self.cfg, self.w, self._acts
         if a is None:
             raise RuntimeError("backward_step needs a forward first")
-        B, T = a["B"], a["T"]
-        di, N, dr, dm = c.d_inner, c.d_state, c.dt_rank, c.d_model
-        S = self.SAVE
-        L = c.n_layers
+        B, T, plan = a["B"], a["T"], a["plan"]
+        di, N, dr, dm, L, BT = c.d_inner, c.d_state, c.dt_rank, c.d_model, c.n_layers, B * T
+        dev, dt = w.device, w.dtype
         red = None if accumulate_only else BucketedGradReducer(w.grad, w.bucket_bounds(), group=self.group, average=True)
         emb = w.tail()["embedding"]
         gt = w.tail("grad")
-        dl = a["dlogits"]
-        gt["embedding"].add_((dl.t() @ a["hidden"]).float())       # head weight gradient
-        d_hidden = dl @ emb                                         # [BT, dm]
-        d_res = torch.zeros(B * T, dm, device=w.device)
-        ops.residual_rmsnorm_bwd(d_hidden, a["res_f"], w.tail("master")["norm_f"], a["rms_f"], d_res, gt["norm_f"])
-        for l in reversed(range(L)):
-            p, pm, g, s = w.layer(l), w.layer(l, "master"), w.layer(l, "grad"), a["layers"][l]
-            pv = s["proj"].view(B, T, 2 * di)
-            xv = s["xdbl"].view(B, T, c.xdbl_dim)
-            d_out = d_res.to(w.dtype)                               # gradient of this layer's branch output
-            g["out_proj_w"].add_((s["y"].view(B * T, di).t() @ d_out).float())
-            d_y = (d_out @ p["out_proj_w"].t()).view(B, T, di)
-            sb = ops.selective_scan_bwd(s["u"], s["delta"].view(B, T, di), xv[..., dr:dr + N], xv[..., dr + N:],
-                                        w.a_neg[l], pm["d_param"], d_y, s["cs"], S, pv[..., di:],
-                                        dA_log=g["a_log"], dD=g["d_param"])
-            d_delta = sb["d_delta"].view(B * T, di)
-            g["dt_proj_b"].add_(d_delta.float().sum(0))
-            g["dt_proj_w"].add_((s["xdbl"][:, :dr].t() @ d_delta).float())
-            d_xdbl = torch.empty(B * T, c.xdbl_dim, device=w.device, dtype=w.dtype)
-            d_xdbl[:, :dr] = d_delta @ p["dt_proj_w"].t()
-            d_xdbl[:, dr:dr + N] = sb["dB"].view(B * T, N)
-            d_xdbl[:, dr + N:] = sb["dC"].view(B * T, N)
-            g["x_proj_w"].add_((s["u"].view(B * T, di).t() @ d_xdbl).float())
-            d_u = sb["d_u"].view(B * T, di) + d_xdbl @ p["x_proj_w"].t()   # backward_mixed.rs:350-580
-            cg = ops.conv1d_bwd(pv[..., :di], pm["conv_w"], pm["conv_b"], d_u.view(B, T, di), None, dconv_w=g["conv_w"],
-                                dconv_b=g["conv_b"])
-            d_proj = torch.cat([cg["d_x"].view(B * T, di), sb["d_z"].view(B * T, di)], dim=1)
-            g["in_proj_w"].add_((s["post"].t() @ d_proj).float())
-            d_post = d_proj @ p["in_proj_w"].t()
-            ops.residual_rmsnorm_bwd(d_post, s["x_res"], pm["norm_w"], s["rms"], d_res, g["norm_w"])
-            if red is not None:
-                red.bucket_ready(l)                                  # its all-reduce runs under layers l-1 .. 0
+        dl, acc = a["dlogits"], self._accumulate
+        acc(gt["embedding"], dl, a["hidden"])                       # head weight gradient
+        d_post = dl @ emb                                           # [BT, dm], here of the final norm
+        a["dlogits"] = dl = None
+        new = lambda *shape: torch.empty(shape, dtype=dt, device=dev)  # noqa: E731
+        d_res = torch.zeros(BT, dm, device=dev)
+        d_y, d_u, d_delta, d_proj, d_xdbl = new(BT, di), new(BT, di), new(BT, di), new(BT, 2 * di), new(BT, c.xdbl_dim)
+        d_bc = torch.empty(2, BT, N, device=dev)
+        d_out = d_res if dt == torch.float32 else new(BT, dm)
+        ws = torch.empty(plan.bwd_ws, dtype=torch.uint8, device=dev)
+        plan.point_backward(a, d_y, d_u, d_delta, d_proj, d_bc, ws)
+        go, lib = plan.run_on, plan.run_on.lib
+        norm, conv, scan = lib.mamba_b200_residual_rmsnorm_bwd, lib.mamba_b200_conv1d_bwd, lib.mamba_b200_sscan_bwd
+        res_p, rms_p, dres_p, ws_p = a["res"].data_ptr(), a["rms"].data_ptr(), d_res.data_ptr(), ws.data_ptr()
+        d_dt_in, d_bc_out, d_bc_in = d_xdbl[:, :dr], d_xdbl[:, dr:].view(BT, 2, N), d_bc.transpose(0, 1)
+        mm, addmm = torch.mm, torch.addmm
+        with go.begin():
+            dp = d_post.data_ptr()
+            go.call(norm, plan.dt, dp, res_p + 4 * BT * dm * L, plan.norm_f, rms_p + 4 * BT * L, dres_p, gt["norm_f"].data_ptr(),
+                    BT, dm, ws_p, plan.bwd_ws)
+            for l in range(L - 1, -1, -1):
+                lay, g = plan.layers[l], w.layer(l, "grad")
+                post, proj, u, xdbl, delta, y = a["layers"][l]
+                if d_out is not d_res:
+                    d_out.copy_(d_res)                              # gradient of this layer's branch output
+                acc(g["out_proj_w"], y, d_out)
+                mm(d_out, lay.w_out_t, out=d_y)
+                go.call(scan, lay.scan_b)
+                g["dt_proj_b"].add_(torch.sum(d_delta, 0, dtype=torch.float32))
+                acc(g["dt_proj_w"], xdbl[:, :dr], d_delta)
+                mm(d_delta, lay.w_dt_t, out=d_dt_in)
+                d_bc_out.copy_(d_bc_in)
+                acc(g["x_proj_w"], u, d_xdbl)
+                addmm(d_u, d_xdbl, lay.w_x_t, out=d_u)              # backward_mixed.rs:350-580
+                go.call(conv, lay.conv_b)
+                acc(g["in_proj_w"], post, d_proj)
+                mm(d_proj, lay.w_in_t, out=d_post)
+                go.call(norm, plan.dt, dp, res_p + 4 * BT * dm * l, lay.norm_w, rms_p + 4 * BT * l, dres_p, lay.g_norm,
+                        BT, dm, ws_p, plan.bwd_ws)
+                if red is not None:
+                    red.bucket_ready(l)                              # its all-reduce runs under layers l-1 .. 0
         # embedding rows: the residual gradient flows into the gathered rows
-        gt["embedding"].index_add_(0, a["inp"].view(-1).long(), d_res)
+        gt["embedding"].index_add_(0, a["inp"].view(-1), d_res)
         self._acts = None
         self._pending += 1
         if accumulate_only:
@@ -496,11 +728,11 @@ class MambaLMTrainer:
         self._pending = 0
         self.t += 1
         b1, b2 = self.betas
-        self.bias.copy_(torch.tensor([1.0 / (1.0 - b1 ** self.t), 1.0 / (1.0 - b2 ** self.t)]))
+        self.bias[:1].fill_(1.0 / (1.0 - b1 ** self.t))
+        self.bias[1:].fill_(1.0 / (1.0 - b2 ** self.t))
         ops.adamw_step(w.master, w.grad, self.m, self.v, self.bias, lr=self.lr, beta1=b1, beta2=b2, eps=self.eps,
                        weight_decay=self.wd, param_lp=None if w.lp is w.master else w.lp)
-        for l in range(L):
-            torch.exp(w.layer(l, "master")["a_log"], out=w.a_neg[l]).neg_()
+        w.refresh_a_neg()
         w.grad.zero_()
 
     def step(self, ids: torch.Tensor) -> torch.Tensor:

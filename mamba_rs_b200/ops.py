@@ -21,9 +21,12 @@ __all__ = ["selective_scan_fwd", "selective_scan_fwd_workspace_bytes", "selectiv
            "ssm_parallel_scan_fwd_nosave", "ssm_scan_fwd_save", "ssm_scan_bwd", "conv1d_fwd_nosave", "selective_scan_step", "conv1d_fwd", "conv1d_bwd", "m3_ssd_fwd", "m3_ssd_fwd_fused_kq", "m3_ssd_bwd", "dtype_code"]
 
 
+_DTYPES = {torch.float32: ffi.F32, torch.float16: ffi.F16, torch.bfloat16: ffi.BF16}
+
+
 def dtype_code(dt: torch.dtype) -> int:
     try:
-        return {torch.float32: ffi.F32, torch.float16: ffi.F16, torch.bfloat16: ffi.BF16}[dt]
+        return _DTYPES[dt]
     except KeyError:
         raise TypeError(f"unsupported storage dtype {dt} (WeightDtype is f32 / f16 / bf16)")
 
@@ -45,11 +48,30 @@ def _rows(t: torch.Tensor, name: str) -> int:
 
 
 def _ptr(t):
-    return C.c_void_p(0 if t is None else t.data_ptr())
+    return None if t is None else t.data_ptr()
 
 
 def _stream(dev):
-    return C.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
+    """The current stream of a device as the integer the C ABI takes (no Stream object is built)."""
+    return torch._C._cuda_getCurrentRawStream(dev.index or 0)
+
+
+class _on:
+    """``with torch.cuda.device(dev)`` that costs nothing when the device is current already."""
+
+    __slots__ = ("dev", "guard")
+
+    def __init__(self, dev):
+        self.dev, self.guard = dev, None
+
+    def __enter__(self):
+        if torch._C._cuda_getDevice() != (self.dev.index or 0):
+            self.guard = torch.cuda.device(self.dev)
+            self.guard.__enter__()
+
+    def __exit__(self, *exc):
+        if self.guard is not None:
+            self.guard.__exit__(*exc)
 
 
 def selective_scan_fwd(x, delta, Bm, Cm, a_neg, Dp, z=None, *, z_mode=None,
@@ -98,7 +120,7 @@ def selective_scan_fwd(x, delta, Bm, Cm, a_neg, Dp, z=None, *, z_mode=None,
     if workspace is not None:
         _require_cuda(workspace)
         a.workspace, a.workspace_bytes = _ptr(workspace), workspace.numel() * workspace.element_size()
-    with torch.cuda.device(dev):
+    with _on(dev):
         rc = ffi.lib().mamba_b200_sscan_fwd(h.ptr, _stream(dev), C.byref(a))
     h.check(rc, "mamba_b200_sscan_fwd")
     return y
@@ -117,10 +139,10 @@ def ssm_parallel_scan_fwd_nosave(h_state, y_out, delta, u, Bm, Cm, a_neg, Dp, *,
         if not t.is_contiguous():
             raise ValueError("compat entry point takes contiguous tensors")
     fn = ffi.lib().mamba_b200_ssm_scan_fwd_nosave
-    with torch.cuda.device(dev):
-        rc = fn(hd.ptr, _stream(dev), C.c_int(dtype_code(delta.dtype)), _ptr(h_state), _ptr(y_out),
-                _ptr(delta), _ptr(u), _ptr(Bm), _ptr(Cm), _ptr(a_neg), _ptr(Dp), C.c_int(Bsz),
-                C.c_int(T), C.c_int(D), C.c_int(N))
+    with _on(dev):
+        rc = fn(hd.ptr, _stream(dev), dtype_code(delta.dtype), _ptr(h_state), _ptr(y_out),
+                _ptr(delta), _ptr(u), _ptr(Bm), _ptr(Cm), _ptr(a_neg), _ptr(Dp), Bsz,
+                T, D, N)
     hd.check(rc, "mamba_b200_ssm_scan_fwd_nosave")
     return y_out
 
@@ -139,9 +161,9 @@ def ssm_scan_fwd_save(h_state, y_out, h_saved, delta, u, Bm, Cm, a_neg, Dp, *, h
     for t in (y_out, delta, u, Bm, Cm, a_neg, Dp, h_state):
         if not t.is_contiguous():
             raise ValueError("compat entry point takes contiguous tensors")
-    with torch.cuda.device(dev):
+    with _on(dev):
         rc = ffi.lib().mamba_b200_ssm_scan_fwd_save(
-            hd.ptr, _stream(dev), C.c_int(dtype_code(delta.dtype)), _ptr(h_state), _ptr(y_out), _ptr(h_saved),
+            hd.ptr, _stream(dev), dtype_code(delta.dtype), _ptr(h_state), _ptr(y_out), _ptr(h_saved),
             _ptr(delta), _ptr(u), _ptr(Bm), _ptr(Cm), _ptr(a_neg), _ptr(Dp), Bsz, T, D, N)
     hd.check(rc, "mamba_b200_ssm_scan_fwd_save")
     return y_out
@@ -169,11 +191,11 @@ def ssm_scan_bwd(h_saved, delta, u, Bm, Cm, a_neg, Dp, dy, *, d_D=None, d_a_log=
     if workspace is None:
         workspace = torch.empty(max(selective_scan_bwd_workspace_bytes(Bsz, T, D, N), 1), dtype=torch.uint8,
                                 device=dev)
-    with torch.cuda.device(dev):
+    with _on(dev):
         rc = ffi.lib().mamba_b200_ssm_scan_bwd(
-            hd.ptr, _stream(dev), C.c_int(dtype_code(delta.dtype)), _ptr(h_saved), _ptr(delta), _ptr(u), _ptr(Bm),
+            hd.ptr, _stream(dev), dtype_code(delta.dtype), _ptr(h_saved), _ptr(delta), _ptr(u), _ptr(Bm),
             _ptr(Cm), _ptr(a_neg), _ptr(Dp), _ptr(dy), _ptr(d_delta), _ptr(d_u), _ptr(dB), _ptr(dC), _ptr(d_D),
-            _ptr(d_a_log), Bsz, T, D, N, _ptr(workspace), C.c_longlong(workspace.numel()))
+            _ptr(d_a_log), Bsz, T, D, N, _ptr(workspace), workspace.numel())
     hd.check(rc, "mamba_b200_ssm_scan_bwd")
     return dict(d_delta=d_delta, d_u=d_u, dB=dB, dC=dC, dD=d_D, dA_log=d_a_log)
 
@@ -187,8 +209,8 @@ def conv1d_fwd_nosave(u_out, state, x, conv_w, conv_b, *, handle=None):
     for t in (u_out, state, x, conv_w, conv_b):
         if not t.is_contiguous():
             raise ValueError("compat entry point takes contiguous tensors")
-    with torch.cuda.device(dev):
-        rc = ffi.lib().mamba_b200_conv1d_fwd_nosave(hd.ptr, _stream(dev), C.c_int(dtype_code(x.dtype)), _ptr(u_out),
+    with _on(dev):
+        rc = ffi.lib().mamba_b200_conv1d_fwd_nosave(hd.ptr, _stream(dev), dtype_code(x.dtype), _ptr(u_out),
                                                     _ptr(state), _ptr(x), _ptr(conv_w), _ptr(conv_b), Bsz, T, D,
                                                     conv_w.shape[1])
     hd.check(rc, "mamba_b200_conv1d_fwd_nosave")
@@ -245,7 +267,7 @@ def selective_scan_bwd(u, delta, Bm, Cm, a_neg, Dp, dy, chunk_states, save_strid
     a.d_z, a.ld_dz = _ptr(d_z), D
     a.dBm, a.dCm, a.dA_log, a.dD = _ptr(dB), _ptr(dC), _ptr(dA_log), _ptr(dD)
     a.workspace, a.workspace_bytes = _ptr(workspace), workspace.numel()
-    with torch.cuda.device(dev):
+    with _on(dev):
         rc = ffi.lib().mamba_b200_sscan_bwd(h.ptr, _stream(dev), C.byref(a))
     h.check(rc, "mamba_b200_sscan_bwd")
     return dict(d_u=d_u, d_delta=d_delta, d_z=d_z, dB=dB, dC=dC, dA_log=dA_log, dD=dD)
@@ -278,7 +300,7 @@ def selective_scan_step(x, delta, Bm, Cm, a_neg, Dp, ssm_state, z=None, *, z_mod
     a.ssm_state = _ptr(ssm_state)
     a.y, a.ld_y = _ptr(y), y.stride(0)
     a.u_out, a.ld_u = _ptr(u_out), (u_out.stride(0) if u_out is not None else 0)
-    with torch.cuda.device(dev):
+    with _on(dev):
         rc = ffi.lib().mamba_b200_sscan_step(h.ptr, _stream(dev), C.byref(a))
     h.check(rc, "mamba_b200_sscan_step")
     return y
@@ -298,7 +320,7 @@ def conv1d_fwd(x, conv_w, conv_b, conv_state=None, u=None, *, handle=None):
     a.x, a.ld_x = _ptr(x), _rows(x, "x")
     a.conv_w, a.conv_b, a.conv_state = _ptr(conv_w), _ptr(conv_b), _ptr(conv_state)
     a.u, a.ld_u = _ptr(u), _rows(u, "u")
-    with torch.cuda.device(dev):
+    with _on(dev):
         rc = ffi.lib().mamba_b200_conv1d_fwd(h.ptr, _stream(dev), C.byref(a))
     h.check(rc, "mamba_b200_conv1d_fwd")
     return u
@@ -328,7 +350,7 @@ def conv1d_bwd(x, conv_w, conv_b, d_u, conv_state0=None, *, dconv_w=None, dconv_
     a.d_x, a.ld_dx = _ptr(d_x), D
     a.dconv_w, a.dconv_b = _ptr(dconv_w), _ptr(dconv_b)
     a.workspace, a.workspace_bytes = _ptr(workspace), workspace.numel()
-    with torch.cuda.device(dev):
+    with _on(dev):
         rc = ffi.lib().mamba_b200_conv1d_bwd(h.ptr, _stream(dev), C.byref(a))
     h.check(rc, "mamba_b200_conv1d_bwd")
     return dict(d_x=d_x, dconv_w=dconv_w, dconv_b=dconv_b)
@@ -361,7 +383,7 @@ def m3_ssd_fwd(x, K, Q, dt, trap, adt, Dh, *, ssm_state=None, k_state=None, v_st
     a.y = _ptr(y)
     a.ssm_state, a.k_state, a.v_state = _ptr(ssm_state), _ptr(k_state), _ptr(v_state)
     a.carry_in, a.force_sequential = int(carry_in), int(force_sequential)
-    with torch.cuda.device(dev):
+    with _on(dev):
         rc = ffi.lib().mamba_b200_m3_ssd_fwd(h.ptr, _stream(dev), C.byref(a))
     h.check(rc, "mamba_b200_m3_ssd_fwd")
     return y
@@ -401,7 +423,7 @@ def m3_ssd_fwd_fused_kq(x, Bn, Cn, b_bias, c_bias, angle_vel, dt, trap, adt, Dh,
     a.Bn, a.Cn, a.b_bias, a.c_bias = _ptr(Bn), _ptr(Cn), _ptr(b_bias), _ptr(c_bias)
     a.angle_vel, a.angle_state = _ptr(angle_vel), _ptr(angle_state)
     a.ng, a.n_angles = ng, (angle_vel.shape[2] if angle_vel is not None else 0)
-    with torch.cuda.device(dev):
+    with _on(dev):
         rc = ffi.lib().mamba_b200_m3_ssd_fwd(h.ptr, _stream(dev), C.byref(a))
     h.check(rc, "mamba_b200_m3_ssd_fwd")
     return y
@@ -443,7 +465,7 @@ def m3_ssd_bwd(x, K, Q, dt, trap, adt, Dh, dy, *, dD=None, workspace=None, handl
     a.dx, a.dK, a.dQ = _ptr(dx), _ptr(dK), _ptr(dQ)
     a.d_adt, a.d_dt, a.d_trap, a.dD = _ptr(d_adt), _ptr(d_dt), _ptr(d_trap), _ptr(dD)
     a.workspace, a.workspace_bytes = _ptr(workspace), workspace.numel()
-    with torch.cuda.device(dev):
+    with _on(dev):
         rc = ffi.lib().mamba_b200_m3_ssd_bwd(h.ptr, _stream(dev), C.byref(a))
     h.check(rc, "mamba_b200_m3_ssd_bwd")
     return dict(dx=dx, dK=dK, dQ=dQ, d_adt=d_adt, d_dt=d_dt, d_trap=d_trap, dD=dD)
@@ -465,7 +487,7 @@ def residual_rmsnorm_fwd(residual, branch, scale, *, eps=1e-5, out_dtype=None, y
         y = torch.empty((rows, dim), dtype=dt, device=dev)
     if rms_out is None:
         rms_out = torch.empty(rows, dtype=torch.float32, device=dev)
-    with torch.cuda.device(dev):
+    with _on(dev):
         rc = ffi.lib().mamba_b200_residual_rmsnorm_fwd(h.ptr, _stream(dev), dtype_code(dt), _ptr(residual), _ptr(branch),
                                                        _ptr(scale), _ptr(y), _ptr(rms_out), rows, dim, float(eps))
     h.check(rc, "mamba_b200_residual_rmsnorm_fwd")
@@ -482,7 +504,7 @@ def residual_rmsnorm_bwd(dy, x, scale, rms_saved, d_residual, d_scale, *, worksp
     need = int(ffi.lib().mamba_b200_residual_rmsnorm_bwd_workspace_bytes(rows, dim))
     if workspace is None:
         workspace = torch.empty(max(need, 1), dtype=torch.uint8, device=dev)
-    with torch.cuda.device(dev):
+    with _on(dev):
         rc = ffi.lib().mamba_b200_residual_rmsnorm_bwd(h.ptr, _stream(dev), dtype_code(dy.dtype), _ptr(dy), _ptr(x),
                                                        _ptr(scale), _ptr(rms_saved), _ptr(d_residual), _ptr(d_scale),
                                                        rows, dim, _ptr(workspace), workspace.numel())
@@ -501,7 +523,7 @@ def embedding_gather(table, ids, out=None, *, handle=None):
         raise TypeError("ids are contiguous int32, the table is contiguous")
     if out is None:
         out = torch.empty((ids.numel(), dim), dtype=torch.float32, device=dev)
-    with torch.cuda.device(dev):
+    with _on(dev):
         rc = ffi.lib().mamba_b200_embedding_gather(h.ptr, _stream(dev), dtype_code(table.dtype), _ptr(table), _ptr(ids),
                                                    _ptr(out), ids.numel(), dim, vocab)
     h.check(rc, "mamba_b200_embedding_gather")
@@ -520,7 +542,7 @@ def softmax_xent(logits, targets, *, grad_scale=1.0, want_grad=True, dlogits=Non
     loss = torch.empty(rows, dtype=torch.float32, device=dev)
     if want_grad and dlogits is None:
         dlogits = torch.empty_strided(logits.shape, logits.stride(), dtype=logits.dtype, device=dev)
-    with torch.cuda.device(dev):
+    with _on(dev):
         rc = ffi.lib().mamba_b200_softmax_xent(h.ptr, _stream(dev), dtype_code(logits.dtype), _ptr(logits), _ptr(targets),
                                                _ptr(loss), _ptr(dlogits if want_grad else None), float(grad_scale),
                                                rows, V, logits.stride(0))
@@ -538,7 +560,7 @@ def adamw_step(param, grad, m, v, bias_factors, *, lr, beta1=0.9, beta2=0.999, e
     for t in (param, grad, m, v, bias_factors):
         if t.dtype != torch.float32 or not t.is_contiguous():
             raise TypeError("AdamW state is contiguous float32")
-    with torch.cuda.device(dev):
+    with _on(dev):
         rc = ffi.lib().mamba_b200_adamw_step(h.ptr, _stream(dev), _ptr(param), _ptr(grad), _ptr(m), _ptr(v), float(lr),
                                              float(beta1), float(beta2), float(eps), float(weight_decay),
                                              _ptr(bias_factors), _ptr(param_lp),
