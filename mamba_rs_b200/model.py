@@ -213,7 +213,7 @@ class _PrefillPlan:
     def __init__(self, bb: "GpuMambaBackbone", B: int, T: int):
         w, c = bb.w, bb.cfg
         self.key = self.pointers(bb)
-        self.bb, self.B, self.T, self.where = bb, B, T, None
+        self.cfg, self.dtype, self.B, self.T, self.where = c, w.dtype, B, T, None  # (not bb: it keeps this plan)
         self.run_on = _Launcher(w.device)
         di, N, dr, xd = c.d_inner, c.d_state, c.dt_rank, c.xdbl_dim
         self.dt, self.es = ops.dtype_code(w.dtype), w.lp.element_size()
@@ -238,7 +238,7 @@ class _PrefillPlan:
         return _DecodePlan.pointers(bb) + tuple(a.data_ptr() for a in bb.w.a_neg)
 
     def point(self, proj, u, xdbl, delta, y, ws):
-        di, N, dr, es = self.bb.cfg.d_inner, self.bb.cfg.d_state, self.bb.cfg.dt_rank, self.es
+        di, N, dr, es = self.cfg.d_inner, self.cfg.d_state, self.cfg.dt_rank, self.es
         self.where = (proj, u, xdbl, delta, y, ws)
         for layer in self.layers:
             cv, sc = layer[-2:]
@@ -249,10 +249,9 @@ class _PrefillPlan:
     def run(self, temporal, last_only=False):
         """The backbone over temporal [B, T, d_model] (updated in place).  last_only: only the last
         position's normalised row is wanted, so the last out_proj and the last norm take that row."""
-        bb, B, T = self.bb, self.B, self.T
-        c, w = bb.cfg, bb.w
+        c, B, T = self.cfg, self.B, self.T
         dm, di, dr, BT = c.d_model, c.d_inner, c.dt_rank, B * T
-        new = lambda *shape: torch.empty(shape, dtype=w.dtype, device=temporal.device)  # noqa: E731
+        new = lambda *shape: torch.empty(shape, dtype=self.dtype, device=temporal.device)  # noqa: E731
         post, proj, u, xdbl, delta, y = new(BT, dm), new(BT, 2 * di), new(BT, di), new(BT, c.xdbl_dim), new(BT, di), new(BT, di)
         ws = torch.empty(self.ws_bytes, dtype=torch.uint8, device=temporal.device)
         where = (proj.data_ptr(), u.data_ptr(), xdbl.data_ptr(), delta.data_ptr(), y.data_ptr(), ws.data_ptr())
