@@ -403,6 +403,23 @@ __global__ void __launch_bounds__(256) bwd_reduce_bc_kernel(const float* __restr
     }
 }
 
+// Segment hand-over of the two-lane backward: slot s of seg_dh arrives holding the dh segment s leaves
+// where it begins when started from zero and leaves holding the true one, which segment s - 1 starts
+// from.  (Slot 0 is not used: nothing precedes segment 0.)
+__global__ void sscan_bwd_carry_kernel(float* seg_dh, const float* seg_sum, const float* a_neg, int B, int S, int D, int N) {
+    const long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
+    const long long DN = static_cast<long long>(D) * N;
+    if (i >= B * DN) return;
+    const long long b = i / DN, dn = i - b * DN, d = dn / N;
+    const float a2 = a_neg[dn] * kLog2e;
+    float run = 0.0f;
+    for (int s = S - 1; s >= 1; --s) {
+        const long long at = (b * S + s) * DN + dn;
+        run = fmaf(ex2(a2 * seg_sum[(b * S + s) * D + d]), run, seg_dh[at]);
+        seg_dh[at] = run;
+    }
+}
+
 // dA_log[D,N] += sum_b part_a, dD[D] += sum_b part_d, in sample order
 // (kernels/mamba_ssm.cu:703-715, :750-763).
 __global__ void bwd_reduce_params_kernel(const float* __restrict__ part_a,
@@ -526,10 +543,10 @@ static const BwdTable& bwd_table() {
     return table;
 }
 
-// Two-lane kernels (8 < d_state <= 16): [dtype][stride index][flags].
+// Two-lane kernels (8 < d_state <= 16, save stride 32): [dtype][0][flags].
 struct Bwd2Table {
-    BwdKernelFn fn[3][2][4];
-    size_t smem[3][2];
+    BwdKernelFn fn[3][1][8];
+    size_t smem[3][1];
 };
 
 static const Bwd2Table& bwd2_table() {
@@ -548,8 +565,8 @@ int m1_bwd_configure(Ctx* c) {
     MB200_CUDA_CHECK(c, bwd_wide_configure());
     const Bwd2Table& t2 = bwd2_table();
     for (int dt = 0; dt < 3; ++dt)
-        for (int si = 0; si < 2; ++si)
-            for (int f = 0; f < 4; ++f) {
+        for (int si = 0; si < 1; ++si)
+            for (int f = 0; f < 8; ++f) {
                 MB200_CUDA_CHECK(c, cudaFuncSetAttribute(reinterpret_cast<const void*>(t2.fn[dt][si][f]),
                                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                          static_cast<int>(t2.smem[dt][si])));
@@ -568,11 +585,34 @@ int m1_bwd_configure(Ctx* c) {
     return MAMBA_B200_OK;
 }
 
+// Time segments of the two-lane backward.  A wave is the 12 one-warp CTAs per SM that are resident
+// together; splitting costs the first pass, about three tenths of the whole (measured: 0.28 at
+// 2 x 8192 x 5120).  The count with the least waves x blocks per segment wins, the smaller one on a
+// tie; a segment keeps at least two blocks.  (The workspace is sized without a handle, so for the
+// B200's SM count.)
+constexpr int kBwdMaxSegs = 32;
+static int bwd_segments(int B, int T, int D, int N) {
+    if (N <= 8 || N > 16) return 1;
+    const long long warps = static_cast<long long>(B) * ((D + 15) / 16), wave = 12 * 148;
+    const int nblk = (T + 31) / 32;
+    int best = 1;
+    double cost = static_cast<double>((warps + wave - 1) / wave) * nblk;
+    for (int s = 2; s <= kBwdMaxSegs && 2 * s <= nblk; ++s) {
+        const double c = 1.3 * static_cast<double>((warps * s + wave - 1) / wave) * ((nblk + s - 1) / s);
+        if (c < 0.97 * cost) {
+            cost = c;
+            best = s;
+        }
+    }
+    return best;
+}
+
 static int bwd_ns(int N) { return N <= 4 ? 4 : (N <= 8 ? 8 : 16); }
 
 
 static void bwd_ws_layout(int B, int T, int D, int N, size_t* off_a, size_t* off_d, size_t* off_dense,
-                          size_t* total) {
+                          size_t* total, size_t* off_dh = nullptr, size_t* off_sum = nullptr) {
+    const size_t segs = bwd_segments(B, T, D, N);
     // channel tiles of the dB/dC partials: 16 channels per CTA for the two-lane
     // kernel (d_state > 8), 32 for the one-lane kernel
     size_t tiles = N > 8 ? (D + 15) / 16 : (D + 31) / 32, V = 2 * bwd_ns(N);
@@ -583,15 +623,19 @@ static void bwd_ws_layout(int B, int T, int D, int N, size_t* off_a, size_t* off
     }
     size_t bc = sizeof(float) * static_cast<size_t>(B) * tiles * T * V;
     bc = (bc + 255) & ~size_t(255);
-    size_t a = sizeof(float) * static_cast<size_t>(B) * D * N;
+    size_t a = sizeof(float) * static_cast<size_t>(B) * segs * D * N;
     a = (a + 255) & ~size_t(255);
-    const size_t dd = sizeof(float) * static_cast<size_t>(B) * D;
+    const size_t dd = sizeof(float) * static_cast<size_t>(B) * segs * D;
     *off_a = bc;
     *off_d = bc + a;
     *off_dense = bc + a + ((dd + 255) & ~size_t(255));
     // states every 32 steps, rebuilt from a stride-64 save (two-lane kernel only)
     const size_t dense = (N > 8 && N <= 16) ? sizeof(float) * static_cast<size_t>(B) * ((T + 31) / 32) * D * N : 0;
     *total = *off_dense + ((dense + 255) & ~size_t(255));
+    if (off_dh) *off_dh = *total;
+    if (segs > 1) *total += a;
+    if (off_sum) *off_sum = *total;
+    if (segs > 1) *total += (dd + 255) & ~size_t(255);
 }
 
 }  // namespace mb200
@@ -623,8 +667,8 @@ static int launch_bwd(Ctx* c, void* stream, const mamba_b200_sscan_bwd_args& a, 
     if (a.ld_u < a.D || a.ld_delta < a.D || a.ld_dy < a.D || a.ld_bc < a.N || a.ld_du < a.D ||
         a.ld_ddelta < a.D || (a.z_mode && (a.ld_z < a.D || a.ld_dz < a.D)))
         return fail(c, MAMBA_B200_ERR_ARG, "sscan_bwd: a row stride is smaller than its row");
-    size_t off_a, off_d, off_dense, total;
-    bwd_ws_layout(a.B, a.T, a.D, a.N, &off_a, &off_d, &off_dense, &total);
+    size_t off_a, off_d, off_dense, total, off_dh, off_sum;
+    bwd_ws_layout(a.B, a.T, a.D, a.N, &off_a, &off_d, &off_dense, &total, &off_dh, &off_sum);
     if (a.workspace_bytes < static_cast<long long>(total))
         return fail(c, MAMBA_B200_ERR_ARG, "sscan_bwd: workspace %lld < %zu bytes", a.workspace_bytes, total);
     if (reinterpret_cast<uintptr_t>(a.workspace) % 256)
@@ -702,10 +746,30 @@ static int launch_bwd(Ctx* c, void* stream, const mamba_b200_sscan_bwd_args& a, 
     const int flags = (a.delta_softplus ? 1 : 0) | (a.z_mode ? 2 : 0);
     const int tiles = (a.D + DT - 1) / DT;
     dim3 grid(tiles, a.B);
+    int segs = 1;
     if (two_lane) {
         const Bwd2Table& t2 = bwd2_table();
-        const int si = S == 32 ? 0 : 1;
-        t2.fn[a.dtype][si][flags]<<<grid, 32, t2.smem[a.dtype][si], st>>>(p);
+        segs = bwd_segments(a.B, a.T, a.D, a.N);
+        if (segs > 1) {
+            const int nblk = (a.T + S - 1) / S;
+            p.seg_blocks = (nblk + segs - 1) / segs;
+            segs = (nblk + p.seg_blocks - 1) / p.seg_blocks;
+        }
+        if (segs > 1) {
+            p.seg_dh = reinterpret_cast<float*>(ws + off_dh);
+            p.seg_sum = reinterpret_cast<float*>(ws + off_sum);
+            grid.z = segs - 1;
+            t2.fn[a.dtype][0][4 | flags]<<<grid, 32, t2.smem[a.dtype][0], st>>>(p);
+            MB200_CUDA_CHECK(c, cudaGetLastError());
+            const long long n = static_cast<long long>(a.B) * a.D * a.N;
+            sscan_bwd_carry_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, st>>>(p.seg_dh, p.seg_sum, a.a_neg, a.B, segs,
+                                                                                          a.D, a.N);
+            MB200_CUDA_CHECK(c, cudaGetLastError());
+            grid.z = segs;
+        } else {
+            p.seg_blocks = 0;
+        }
+        t2.fn[a.dtype][0][flags]<<<grid, 32, t2.smem[a.dtype][0], st>>>(p);
     } else {
         t.fn[a.dtype][vi][flags]<<<grid, 32, t.smem[a.dtype][vi], st>>>(p);
     }
@@ -715,7 +779,7 @@ static int launch_bwd(Ctx* c, void* stream, const mamba_b200_sscan_bwd_args& a, 
         p.part_bc, a.dBm, a.dCm, a.B, a.T, a.N, ns, tiles, bc_vec);
     MB200_CUDA_CHECK(c, cudaGetLastError());
     const int np = a.D * a.N;
-    bwd_reduce_params_kernel<<<(np + 255) / 256, 256, 0, st>>>(p.part_a, p.part_d, a.dA_log, a.dD, a.B,
+    bwd_reduce_params_kernel<<<(np + 255) / 256, 256, 0, st>>>(p.part_a, p.part_d, a.dA_log, a.dD, a.B * segs,
                                                              a.D, a.N);
     MB200_CUDA_CHECK(c, cudaGetLastError());
     return MAMBA_B200_OK;

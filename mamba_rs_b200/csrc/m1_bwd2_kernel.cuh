@@ -23,6 +23,14 @@
 //     finished in pairs (lanes 0-15 the even row, lanes 16-31 the odd one), so the
 //     elementwise output code runs once per two rows without divergence.
 // Results differ from the one-lane kernel only by summation order.
+//
+// Few (sample, channel tile) pairs leave the GPU idle: 640 warps of a 2 x 8192 x 5120 shard are one
+// per scheduler, where a step takes 1030 cycles against 1290 / 2.6 with the chip full.  The blocks
+// are then split into time segments (grid.z) that run side by side, each from the gradient of the
+// state that leaves it.  That gradient is exact: a first launch (FLAGS bit 2) walks every segment but
+// the first from zero, dh <- exp(delta a) (dh + dy gate C) alone, and keeps dh and the sum of the
+// deltas where the segment begins; sscan_bwd_carry_kernel chains them (the decay of a segment is one
+// exponential of its summed deltas).
 #pragma once
 #include <string.h>
 
@@ -49,8 +57,12 @@ struct BwdParams {
     // h_saved [B, T+1, D, N] through the compat entry point)
     long long cs_ld_b, cs_ld_k;
     float *part_bc;  // [B][tiles][T][2N]
-    float *part_a;   // [B][D][N]
-    float *part_d;   // [B][D]
+    float *part_a;   // [B][segments][D][N]
+    float *part_d;   // [B][segments][D]
+    // time segments: [B][segments][D][N] dh where segment s begins (first pass: from zero; after the
+    // carry: the true one), [B][segments][D] sum of its deltas
+    float *seg_dh, *seg_sum;
+    int seg_blocks;  // blocks per segment (0: one segment)
     int B, T, D, N, S;
     int z_mode;
     unsigned tma_mask;  // bit per tensor map, in declaration order
@@ -99,11 +111,11 @@ struct Bwd2Traits {
     static_assert(SB % 2 == 0, "rows are finished in pairs");
 };
 
-// FLAGS: bit0 softplus on delta, bit1 gate present.
+// FLAGS: bit0 softplus on delta, bit1 gate present, bit2 the segments' first pass (dh only).
 template <typename Tact, int S, int FLAGS>
 __global__ void __maxnreg__(kBwd2MaxRegs) sscan_bwd2_kernel(const __grid_constant__ BwdParams p) {
     using Tr = Bwd2Traits<Tact, S>;
-    constexpr bool kSoftplus = (FLAGS & 1) != 0, kGate = (FLAGS & 2) != 0;
+    constexpr bool kSoftplus = (FLAGS & 1) != 0, kGate = (FLAGS & 2) != 0, kDhOnly = (FLAGS & 4) != 0;
     constexpr int DT = 16, SB = Tr::SB, NSUB = Tr::NSUB, NP = 16, THREADS = 32;
     extern __shared__ __align__(128) unsigned char smem[];
     float* Bf = reinterpret_cast<float*>(smem + Tr::OFF_BF);
@@ -119,7 +131,10 @@ __global__ void __maxnreg__(kBwd2MaxRegs) sscan_bwd2_kernel(const __grid_constan
     const int n0 = part * 8;
     const int T = p.T, D = p.D, N = p.N;
     const bool d_ok = d < D;
-    const int nblk = (T + S - 1) / S;
+    const int nblk = (T + S - 1) / S, nseg = gridDim.z, seg = blockIdx.z + (kDhOnly ? 1 : 0);
+    const int nsegs = kDhOnly ? nseg + 1 : nseg;  // the first pass has no CTA for segment 0
+    const int k_lo = p.seg_blocks > 0 ? seg * p.seg_blocks : 0;
+    const int k_hi = p.seg_blocks > 0 ? min(nblk, (seg + 1) * p.seg_blocks) : nblk;
     const bool gate_is_silu = p.z_mode == 1;
 
     auto st_u = [&](int s) { return reinterpret_cast<Tact*>(smem + 0 * s); };
@@ -134,11 +149,11 @@ __global__ void __maxnreg__(kBwd2MaxRegs) sscan_bwd2_kernel(const __grid_constan
 
     const unsigned lm = p.tma_mask;
     uint32_t tx_bytes = 0;
-    if (lm & kBU) tx_bytes += sizeof(Tact) * S * DT;
+    if (!kDhOnly && (lm & kBU)) tx_bytes += sizeof(Tact) * S * DT;
     if (lm & kBDl) tx_bytes += sizeof(Tact) * S * DT;
     if (kGate && (lm & kBZ)) tx_bytes += sizeof(Tact) * S * DT;
     if (lm & kBDy) tx_bytes += sizeof(Tact) * S * DT;
-    if (lm & kBB) tx_bytes += sizeof(Tact) * S * N;
+    if (!kDhOnly && (lm & kBB)) tx_bytes += sizeof(Tact) * S * N;
     if (lm & kBC) tx_bytes += sizeof(Tact) * S * N;
     const unsigned all_loads = kBU | kBDl | kBZ | kBDy | kBB | kBC;
     const bool any_plain = (lm & all_loads) != all_loads;
@@ -147,11 +162,11 @@ __global__ void __maxnreg__(kBwd2MaxRegs) sscan_bwd2_kernel(const __grid_constan
         const int t0 = k * S;
         if (!tx_bytes) return;
         mbar_expect_tx(&bars[s], tx_bytes);
-        if (lm & kBU) tma_load_3d(st_u(s), &p.tm_u, &bars[s], d0, t0, b);
+        if (!kDhOnly && (lm & kBU)) tma_load_3d(st_u(s), &p.tm_u, &bars[s], d0, t0, b);
         if (lm & kBDl) tma_load_3d(st_dl(s), &p.tm_dl, &bars[s], d0, t0, b);
         if (kGate && (lm & kBZ)) tma_load_3d(st_z(s), &p.tm_z, &bars[s], d0, t0, b);
         if (lm & kBDy) tma_load_3d(st_dy(s), &p.tm_dy, &bars[s], d0, t0, b);
-        if (lm & kBB) tma_load_3d(st_b(s), &p.tm_b, &bars[s], 0, t0, b);
+        if (!kDhOnly && (lm & kBB)) tma_load_3d(st_b(s), &p.tm_b, &bars[s], 0, t0, b);
         if (lm & kBC) tma_load_3d(st_c(s), &p.tm_c, &bars[s], 0, t0, b);
     };
 
@@ -205,23 +220,31 @@ __global__ void __maxnreg__(kBwd2MaxRegs) sscan_bwd2_kernel(const __grid_constan
     float accD = 0.0f;
 #pragma unroll
     for (int j = 0; j < 4; ++j) dh[j] = accA[j] = make_float2(0.0f, 0.0f);
+    float sum_dl = 0.0f;
+    if (!kDhOnly && seg + 1 < nsegs && d_ok) {  // what the next segment hands back
+        const float* src = p.seg_dh + ((static_cast<long long>(b) * nsegs + seg + 1) * D + d) * N + n0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            dh[j] = make_float2(n0 + 2 * j < N ? src[2 * j] : 0.0f, n0 + 2 * j + 1 < N ? src[2 * j + 1] : 0.0f);
+    }
 
     auto run_blocks = [&](auto geo_tag) {
-        for (int it = 0; it < nblk; ++it) {
-            const int k = nblk - 1 - it, s = 0, t0 = k * S;
+        uint32_t phase = 0;
+        for (int k = k_hi - 1; k >= k_lo; --k, phase ^= 1) {
+            const int s = 0, t0 = k * S;
             const int nv = min(S, T - t0);
             // One stage: the previous block's readers finished at the warp barrier that
             // ended it; other resident CTAs cover this load's latency.
             if (tid == 0) issue(k, 0);
             if (any_plain) {
-                if (!(lm & kBU)) bwd_load_plain(st_u(s), static_cast<const Tact*>(p.u), p.ld_u, b, T, t0, d0, D, S, DT, THREADS);
+                if (!kDhOnly && !(lm & kBU)) bwd_load_plain(st_u(s), static_cast<const Tact*>(p.u), p.ld_u, b, T, t0, d0, D, S, DT, THREADS);
                 if (!(lm & kBDl)) bwd_load_plain(st_dl(s), static_cast<const Tact*>(p.dl), p.ld_dl, b, T, t0, d0, D, S, DT, THREADS);
                 if (kGate && !(lm & kBZ)) bwd_load_plain(st_z(s), static_cast<const Tact*>(p.z), p.ld_z, b, T, t0, d0, D, S, DT, THREADS);
                 if (!(lm & kBDy)) bwd_load_plain(st_dy(s), static_cast<const Tact*>(p.dy), p.ld_dy, b, T, t0, d0, D, S, DT, THREADS);
-                if (!(lm & kBB)) bwd_load_plain(st_b(s), static_cast<const Tact*>(p.bm), p.ld_bc, b, T, t0, 0, N, S, N, THREADS);
+                if (!kDhOnly && !(lm & kBB)) bwd_load_plain(st_b(s), static_cast<const Tact*>(p.bm), p.ld_bc, b, T, t0, 0, N, S, N, THREADS);
                 if (!(lm & kBC)) bwd_load_plain(st_c(s), static_cast<const Tact*>(p.cm), p.ld_bc, b, T, t0, 0, N, S, N, THREADS);
             }
-            if (tx_bytes) mbar_wait(&bars[0], it & 1, p.status);
+            if (tx_bytes) mbar_wait(&bars[0], phase, p.status);
             __syncwarp();
 
             // ---- 1. per-block elementwise caches ----
@@ -243,7 +266,7 @@ __global__ void __maxnreg__(kBwd2MaxRegs) sscan_bwd2_kernel(const __grid_constan
                 const Tact* rc = st_c(s);
                 for (int i = tid; i < S * NP; i += THREADS) {
                     const int r = i / NP, n = i - r * NP;
-                    Bf[i] = n < N ? to_f(rb[r * N + n]) : 0.0f;
+                    if (!kDhOnly) Bf[i] = n < N ? to_f(rb[r * N + n]) : 0.0f;
                     Cf[i] = n < N ? to_f(rc[r * N + n]) : 0.0f;
                 }
             }
@@ -254,6 +277,24 @@ __global__ void __maxnreg__(kBwd2MaxRegs) sscan_bwd2_kernel(const __grid_constan
             const float* rgy = gy + col;
             const float* Bp = Bf + n0;
             const float* Cp = Cf + n0;
+
+            if constexpr (kDhOnly) {
+                // rows past the end carry no gradient and are the first ones walked: dh is still zero
+#pragma unroll 4
+                for (int r = S - 1; r >= 0; --r) {
+                    const float dlv = rdl[r * DT];
+                    const float2 dyp2 = splat2(rgy[r * DT]);
+                    float2 e[4];
+                    decay(geo_tag, dlv, e);
+                    StateVec<float, 8> Cq;
+                    Cq.load(Cp + r * NP);
+                    sum_dl += dlv;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) dh[j] = mul2(e[j], fma2(dyp2, Cq.pair(j), dh[j]));
+                }
+                __syncwarp();
+                continue;
+            }
 
             auto fwd_step = [&](int r, float2* h) {
                 const float dlv = rdl[r * DT], duv = dlv * to_f(ru[r * DT]);
@@ -403,35 +444,45 @@ __global__ void __maxnreg__(kBwd2MaxRegs) sscan_bwd2_kernel(const __grid_constan
     if (geo) run_blocks(std::true_type{});
     else run_blocks(std::false_type{});
 
-    // per-sample parameter-gradient partials
+    if constexpr (kDhOnly) {
+        if (d_ok) {
+            const long long at = (static_cast<long long>(b) * nsegs + seg) * D + d;
+            if (part == 0) p.seg_sum[at] = sum_dl;
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                if (n0 + j < N) p.seg_dh[at * N + n0 + j] = (j & 1) ? dh[j / 2].y : dh[j / 2].x;
+        }
+        return;
+    }
+    // per-sample (and segment) parameter-gradient partials
     accD += __shfl_xor_sync(0xffffffffu, accD, 16);
     if (d_ok) {
-        if (part == 0) p.part_d[static_cast<long long>(b) * D + d] = accD;
+        const long long at = (static_cast<long long>(b) * nsegs + seg) * D + d;
+        if (part == 0) p.part_d[at] = accD;
 #pragma unroll
         for (int j = 0; j < 8; ++j)
             if (n0 + j < N)
-                p.part_a[(static_cast<long long>(b) * D + d) * N + n0 + j] =
+                p.part_a[at * N + n0 + j] =
                     ((j & 1) ? accA[j / 2].y : accA[j / 2].x) * p.a_neg[static_cast<long long>(d) * N + n0 + j];
     }
 }
 
 template <typename Tact>
-static void fill_bwd2(BwdKernelFn (*fn)[4], size_t* smem) {
+static void fill_bwd2(BwdKernelFn (*fn)[8], size_t* smem) {
     fn[0][0] = sscan_bwd2_kernel<Tact, 32, 0>;
     fn[0][1] = sscan_bwd2_kernel<Tact, 32, 1>;
     fn[0][2] = sscan_bwd2_kernel<Tact, 32, 2>;
     fn[0][3] = sscan_bwd2_kernel<Tact, 32, 3>;
-    fn[1][0] = sscan_bwd2_kernel<Tact, 64, 0>;
-    fn[1][1] = sscan_bwd2_kernel<Tact, 64, 1>;
-    fn[1][2] = sscan_bwd2_kernel<Tact, 64, 2>;
-    fn[1][3] = sscan_bwd2_kernel<Tact, 64, 3>;
+    fn[0][4] = sscan_bwd2_kernel<Tact, 32, 4>;
+    fn[0][5] = sscan_bwd2_kernel<Tact, 32, 5>;
+    fn[0][6] = sscan_bwd2_kernel<Tact, 32, 6>;
+    fn[0][7] = sscan_bwd2_kernel<Tact, 32, 7>;
     smem[0] = Bwd2Traits<Tact, 32>::SMEM;
-    smem[1] = Bwd2Traits<Tact, 64>::SMEM;
 }
 
-// [stride index: 0 = 32, 1 = 64][flags]; one translation unit per storage dtype
-void bwd2_kernels_f32(BwdKernelFn (*fn)[4], size_t* smem);
-void bwd2_kernels_f16(BwdKernelFn (*fn)[4], size_t* smem);
-void bwd2_kernels_bf16(BwdKernelFn (*fn)[4], size_t* smem);
+// [0][flags] (save stride 32); one translation unit per storage dtype
+void bwd2_kernels_f32(BwdKernelFn (*fn)[8], size_t* smem);
+void bwd2_kernels_f16(BwdKernelFn (*fn)[8], size_t* smem);
+void bwd2_kernels_bf16(BwdKernelFn (*fn)[8], size_t* smem);
 
 }  // namespace mb200

@@ -139,3 +139,23 @@ def test_backward_full_size_config2_properties(cuda_dev):
     assert rel_err(f(g1["d_u"])[..., dsel], ref["d_x"]) <= TOL["bf16"]
     assert rel_err(f(g1["d_delta"])[..., dsel], ref["d_delta"]) <= TOL["bf16"]
     assert rel_err(f(g1["d_z"])[..., dsel], ref["d_z"]) <= TOL["bf16"]
+
+
+# few (sample, channel tile) pairs: the blocks are split into time segments with an exact carry of dh;
+# lengths around whole segments and blocks, an unaligned channel count, both save strides
+SEG_SHAPES = [(1, 64, 16, 16), (1, 129, 24, 16), (1, 1030, 16, 12), (2, 700, 33, 16), (1, 4100, 8, 16)]
+
+
+@pytest.mark.parametrize("dt", ["f32", "bf16", "f16"])
+@pytest.mark.parametrize("S", [32, 64])
+@pytest.mark.parametrize("shape", SEG_SHAPES, ids=lambda s: "B%dT%dD%dN%d" % s)
+def test_time_segments_of_the_backward_match_oracle(cuda_dev, shape, S, dt):
+    B, T, D, N = shape
+    q = quantised_inputs(B, T, D, N, 0, dt, seed=T, a_mode="random" if T % 2 else "s4d")
+    ssm0, _ = random_states(B, D, N, 0, seed=T + 1)
+    dg = synth.round_to(np.random.default_rng(T).standard_normal((B, T, D)).astype(np.float32), dt)
+    ref = oracle.m1_fused_bwd(q["x"], q["delta_raw"], q["Bm"], q["Cm"], q["z"], q["a_neg"], q["Dp"], dg, ssm_state0=ssm0)
+    g = gpu_fwd_bwd(q, dg, dt, cuda_dev, ssm0, S)
+    for gk, rk in (("d_u", "d_x"), ("d_delta", "d_delta"), ("d_z", "d_z"), ("dB", "dB"), ("dC", "dC"),
+                   ("dA_log", "dA_log"), ("dD", "dD")):
+        assert rel_err(g[gk], ref[rk]) <= TOL[dt], gk
