@@ -105,7 +105,7 @@ typedef struct mamba_b200_sscan_fwd_args {
     int save_stride;     /* 32 or 64 when chunk_states != NULL; 32 is the backward's fast setting */
     void* workspace;     /* optional caller-owned scratch, 256-byte aligned, or NULL.  With it, a
                             launch whose batch x channels cannot fill the GPU is cut along the
-                            sequence into up to 16 segments that run side by side (a first pass
+                            sequence into up to 64 segments that run side by side (a first pass
                             for the segments' leaving states, an exact carry, then the full pass);
                             without it the sequence is always walked by one CTA per channel tile. */
     long long workspace_bytes; /* >= mamba_b200_sscan_fwd_workspace_bytes(B,T,D,N) uses every segment */

@@ -158,6 +158,88 @@ struct StateVec<__half, NS> : StateVecHalf<__half, NS> {
     }
 };
 
+// A [rows x box_cols] tile of a [T, ld] matrix into shared memory with plain loads by THREADS threads,
+// for tensors that break a TMA layout rule (odd row lengths in 16-bit storage, views): out-of-range
+// elements become zero.  Sixteen loads per thread are in flight; one at a time, the tile of 32 x 64
+// took 5 us and the scan of an odd channel count five times as long as that of an even one.
+// box_cols: an int, or a StaticInt where the compiler should know it.
+template <int V>
+struct StaticInt {
+    __device__ constexpr operator int() const { return V; }
+};
+template <int THREADS, typename Tact, typename Cols>
+__device__ __forceinline__ void plain_tile(Tact* dst, const Tact* src, long long ld, int t_first, int rows, int T, int c_first,
+                                           Cols box_cols, int cols_total, int tid) {
+    constexpr int U = 16;
+    const int cols = box_cols, total = rows * cols;
+#pragma unroll 1
+    for (int i0 = tid; i0 < total; i0 += THREADS * U) {
+        Tact v[U];
+#pragma unroll
+        for (int j = 0; j < U; ++j) {
+            const int i = i0 + THREADS * j, r = i / cols, c = i - r * cols, t = t_first + r, col = c_first + c;
+            v[j] = from_f<Tact>(0.0f);
+            if (i < total && t >= 0 && t < T && col < cols_total) v[j] = src[static_cast<long long>(t) * ld + col];
+        }
+#pragma unroll
+        for (int j = 0; j < U; ++j)
+            if (i0 + THREADS * j < total) dst[i0 + THREADS * j] = v[j];
+    }
+}
+
+// The same for 16-bit storage and COLS columns with a 4-byte aligned matrix: lanes fetch words of two
+// elements and rows that start on an odd element (odd ld) are shifted into place with the neighbour
+// lane's word.  Half the accesses of plain_tile.  `src` is the whole matrix, the tile's rows are row0 + t:
+// no word outside it is touched (a row that starts on an odd element has one before it, and the last
+// column of an odd count is fetched alone; an odd ld with an even count goes to plain_tile).
+template <int COLS, typename Tact>
+__device__ __forceinline__ void plain_tile_words(Tact* dst, const Tact* src, long long ld, long long row0, int t_first, int rows,
+                                                 int T, int c_first, int cols_total, int lane) {
+    static_assert(sizeof(Tact) == 2 && COLS % 2 == 0 && COLS <= 64, "one row in at most a warp");
+    constexpr int LPR = COLS / 2, RPI = 32 / LPR, U = 16;
+    const int l = lane % LPR, c = c_first + 2 * l;
+    const unsigned short* s16 = reinterpret_cast<const unsigned short*>(src);
+#pragma unroll 1
+    for (int r0 = lane / LPR; r0 - lane / LPR < rows; r0 += RPI * U) {
+        uint32_t w[U], x[U];
+#pragma unroll
+        for (int j = 0; j < U; ++j) {
+            const int r = r0 + RPI * j, t = t_first + r;
+            const long long e = (row0 + t) * ld + c;  // this lane's first element
+            const bool row = r < rows && t >= 0 && t < T;
+            const bool odd = ((row0 + t) * ld + c_first) & 1;
+            w[j] = x[j] = 0;
+            if (row && c < cols_total) {
+                if (odd || c + 1 < cols_total) w[j] = *reinterpret_cast<const uint32_t*>(s16 + (odd ? e - 1 : e));
+                else w[j] = s16[e];
+            }
+            if (row && odd && l == LPR - 1 && c + 1 < cols_total) x[j] = s16[e + 1];
+        }
+#pragma unroll
+        for (int j = 0; j < U; ++j) {
+            const int r = r0 + RPI * j, t = t_first + r;
+            const bool odd = ((row0 + t) * ld + c_first) & 1;
+            const uint32_t nb = __shfl_down_sync(0xffffffffu, w[j], 1);
+            if (odd) w[j] = (w[j] >> 16) | ((l == LPR - 1 ? x[j] : nb) << 16);
+            if (c >= cols_total) w[j] = 0;
+            else if (c + 1 >= cols_total) w[j] &= 0xffffu;
+            if (r < rows) *reinterpret_cast<uint32_t*>(dst + r * COLS + 2 * l) = w[j];
+        }
+    }
+}
+// A tile of COLS channels, whichever way its matrix allows.
+template <int COLS, typename Tact>
+__device__ __forceinline__ void plain_channels(Tact* dst, const Tact* src, long long ld, long long row0, int t_first, int rows,
+                                               int T, int c_first, int cols_total, int lane) {
+    if constexpr (sizeof(Tact) == 2 && COLS <= 64) {
+        if (reinterpret_cast<uintptr_t>(src) % 4 == 0 && (ld % 2 == 0 || cols_total % 2 != 0)) {
+            plain_tile_words<COLS>(dst, src, ld, row0, t_first, rows, T, c_first, cols_total, lane);
+            return;
+        }
+    }
+    plain_tile<32>(dst, src + row0 * ld, ld, t_first, rows, T, c_first, StaticInt<COLS>{}, cols_total, lane);
+}
+
 // ---- mbarrier + TMA ----------------------------------------------------------
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));

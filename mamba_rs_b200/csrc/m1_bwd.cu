@@ -177,12 +177,12 @@ __global__ void __launch_bounds__(32) sscan_bwd_kernel(const __grid_constant__ B
         const int nv = min(S, T - t0);
         if (lane == 0 && it + 1 < nblk) issue(k - 1, s ^ 1);
         if (any_plain) {
-            if (!(lm & kBU)) bwd_load_plain(st_u(s), static_cast<const Tact*>(p.u), p.ld_u, b, T, t0, d0, D, S, DT);
-            if (!(lm & kBDl)) bwd_load_plain(st_dl(s), static_cast<const Tact*>(p.dl), p.ld_dl, b, T, t0, d0, D, S, DT);
-            if (kGate && !(lm & kBZ)) bwd_load_plain(st_z(s), static_cast<const Tact*>(p.z), p.ld_z, b, T, t0, d0, D, S, DT);
-            if (!(lm & kBDy)) bwd_load_plain(st_dy(s), static_cast<const Tact*>(p.dy), p.ld_dy, b, T, t0, d0, D, S, DT);
-            if (!(lm & kBB)) bwd_load_plain(st_b(s), static_cast<const Tact*>(p.bm), p.ld_bc, b, T, t0, 0, N, S, N);
-            if (!(lm & kBC)) bwd_load_plain(st_c(s), static_cast<const Tact*>(p.cm), p.ld_bc, b, T, t0, 0, N, S, N);
+            if (!(lm & kBU)) plain_tile<32>(st_u(s), static_cast<const Tact*>(p.u) + static_cast<long long>(b) * T * p.ld_u, p.ld_u, t0, S, T, d0, StaticInt<DT>{}, D, lane);
+            if (!(lm & kBDl)) plain_tile<32>(st_dl(s), static_cast<const Tact*>(p.dl) + static_cast<long long>(b) * T * p.ld_dl, p.ld_dl, t0, S, T, d0, StaticInt<DT>{}, D, lane);
+            if (kGate && !(lm & kBZ)) plain_tile<32>(st_z(s), static_cast<const Tact*>(p.z) + static_cast<long long>(b) * T * p.ld_z, p.ld_z, t0, S, T, d0, StaticInt<DT>{}, D, lane);
+            if (!(lm & kBDy)) plain_tile<32>(st_dy(s), static_cast<const Tact*>(p.dy) + static_cast<long long>(b) * T * p.ld_dy, p.ld_dy, t0, S, T, d0, StaticInt<DT>{}, D, lane);
+            if (!(lm & kBB)) plain_tile<32>(st_b(s), static_cast<const Tact*>(p.bm) + static_cast<long long>(b) * T * p.ld_bc, p.ld_bc, t0, S, T, 0, N, N, lane);
+            if (!(lm & kBC)) plain_tile<32>(st_c(s), static_cast<const Tact*>(p.cm) + static_cast<long long>(b) * T * p.ld_bc, p.ld_bc, t0, S, T, 0, N, N, lane);
         }
         if (lane == 0) tma_wait_read0();  // output tiles of the previous block fully read
         if (tx_bytes) mbar_wait(&bars[s], (it >> 1) & 1, p.status);
@@ -545,7 +545,7 @@ static const BwdTable& bwd_table() {
 
 // Two-lane kernels (8 < d_state <= 16, save stride 32): [dtype][0][flags].
 struct Bwd2Table {
-    BwdKernelFn fn[3][1][8];
+    BwdKernelFn fn[3][1][16];
     size_t smem[3][1];
 };
 
@@ -566,7 +566,7 @@ int m1_bwd_configure(Ctx* c) {
     const Bwd2Table& t2 = bwd2_table();
     for (int dt = 0; dt < 3; ++dt)
         for (int si = 0; si < 1; ++si)
-            for (int f = 0; f < 8; ++f) {
+            for (int f = 0; f < 16; ++f) {
                 MB200_CUDA_CHECK(c, cudaFuncSetAttribute(reinterpret_cast<const void*>(t2.fn[dt][si][f]),
                                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                          static_cast<int>(t2.smem[dt][si])));
@@ -749,6 +749,8 @@ static int launch_bwd(Ctx* c, void* stream, const mamba_b200_sscan_bwd_args& a, 
     int segs = 1;
     if (two_lane) {
         const Bwd2Table& t2 = bwd2_table();
+        const unsigned loads = kBU | kBDl | kBZ | kBDy | kBB | kBC;
+        const int flags2 = flags | ((m & loads) != loads ? 8 : 0);
         segs = bwd_segments(a.B, a.T, a.D, a.N);
         if (segs > 1) {
             const int nblk = (a.T + S - 1) / S;
@@ -759,7 +761,7 @@ static int launch_bwd(Ctx* c, void* stream, const mamba_b200_sscan_bwd_args& a, 
             p.seg_dh = reinterpret_cast<float*>(ws + off_dh);
             p.seg_sum = reinterpret_cast<float*>(ws + off_sum);
             grid.z = segs - 1;
-            t2.fn[a.dtype][0][4 | flags]<<<grid, 32, t2.smem[a.dtype][0], st>>>(p);
+            t2.fn[a.dtype][0][4 | flags2]<<<grid, 32, t2.smem[a.dtype][0], st>>>(p);
             MB200_CUDA_CHECK(c, cudaGetLastError());
             const long long n = static_cast<long long>(a.B) * a.D * a.N;
             sscan_bwd_carry_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, st>>>(p.seg_dh, p.seg_sum, a.a_neg, a.B, segs,
@@ -769,7 +771,7 @@ static int launch_bwd(Ctx* c, void* stream, const mamba_b200_sscan_bwd_args& a, 
         } else {
             p.seg_blocks = 0;
         }
-        t2.fn[a.dtype][0][flags]<<<grid, 32, t2.smem[a.dtype][0], st>>>(p);
+        t2.fn[a.dtype][0][flags2]<<<grid, 32, t2.smem[a.dtype][0], st>>>(p);
     } else {
         t.fn[a.dtype][vi][flags]<<<grid, 32, t.smem[a.dtype][vi], st>>>(p);
     }

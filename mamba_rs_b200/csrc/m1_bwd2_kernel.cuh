@@ -35,6 +35,7 @@
 #include <string.h>
 
 #include <type_traits>
+#include <utility>
 
 #include "common.cuh"
 #include "internal.h"
@@ -75,20 +76,6 @@ enum : unsigned {
 
 typedef void (*BwdKernelFn)(const BwdParams);
 
-template <typename Tact>
-__device__ __forceinline__ void bwd_load_plain(Tact* dst, const Tact* src, long long ld, int b, int T,
-                                               int t0, int c0, int cols, int rows, int box_cols,
-                                               int nthreads = 32) {
-    const Tact zero = from_f<Tact>(0.0f);
-    for (int i = threadIdx.x; i < rows * box_cols; i += nthreads) {
-        int r = i / box_cols, c = i - r * box_cols;
-        int t = t0 + r, col = c0 + c;
-        Tact v = zero;
-        if (t < T && col < cols) v = src[(static_cast<long long>(b) * T + t) * ld + col];
-        dst[i] = v;
-    }
-}
-
 template <typename Tact, int S>
 struct Bwd2Traits {
     static constexpr int DT = 16, THREADS = 32, SB = kBwd2SubBlock, NSUB = S / SB, NP = 16;
@@ -111,11 +98,13 @@ struct Bwd2Traits {
     static_assert(SB % 2 == 0, "rows are finished in pairs");
 };
 
-// FLAGS: bit0 softplus on delta, bit1 gate present, bit2 the segments' first pass (dh only).
+// FLAGS: bit0 softplus on delta, bit1 gate present, bit2 the segments' first pass (dh only), bit3 some
+// tensor needs plain loads (kept out of the aligned kernel: its registers are at the cap).
 template <typename Tact, int S, int FLAGS>
 __global__ void __maxnreg__(kBwd2MaxRegs) sscan_bwd2_kernel(const __grid_constant__ BwdParams p) {
     using Tr = Bwd2Traits<Tact, S>;
     constexpr bool kSoftplus = (FLAGS & 1) != 0, kGate = (FLAGS & 2) != 0, kDhOnly = (FLAGS & 4) != 0;
+    constexpr bool kPlain = (FLAGS & 8) != 0;
     constexpr int DT = 16, SB = Tr::SB, NSUB = Tr::NSUB, NP = 16, THREADS = 32;
     extern __shared__ __align__(128) unsigned char smem[];
     float* Bf = reinterpret_cast<float*>(smem + Tr::OFF_BF);
@@ -155,8 +144,6 @@ __global__ void __maxnreg__(kBwd2MaxRegs) sscan_bwd2_kernel(const __grid_constan
     if (lm & kBDy) tx_bytes += sizeof(Tact) * S * DT;
     if (!kDhOnly && (lm & kBB)) tx_bytes += sizeof(Tact) * S * N;
     if (lm & kBC) tx_bytes += sizeof(Tact) * S * N;
-    const unsigned all_loads = kBU | kBDl | kBZ | kBDy | kBB | kBC;
-    const bool any_plain = (lm & all_loads) != all_loads;
 
     auto issue = [&](int k, int s) {  // one thread
         const int t0 = k * S;
@@ -236,13 +223,19 @@ __global__ void __maxnreg__(kBwd2MaxRegs) sscan_bwd2_kernel(const __grid_constan
             // One stage: the previous block's readers finished at the warp barrier that
             // ended it; other resident CTAs cover this load's latency.
             if (tid == 0) issue(k, 0);
-            if (any_plain) {
-                if (!kDhOnly && !(lm & kBU)) bwd_load_plain(st_u(s), static_cast<const Tact*>(p.u), p.ld_u, b, T, t0, d0, D, S, DT, THREADS);
-                if (!(lm & kBDl)) bwd_load_plain(st_dl(s), static_cast<const Tact*>(p.dl), p.ld_dl, b, T, t0, d0, D, S, DT, THREADS);
-                if (kGate && !(lm & kBZ)) bwd_load_plain(st_z(s), static_cast<const Tact*>(p.z), p.ld_z, b, T, t0, d0, D, S, DT, THREADS);
-                if (!(lm & kBDy)) bwd_load_plain(st_dy(s), static_cast<const Tact*>(p.dy), p.ld_dy, b, T, t0, d0, D, S, DT, THREADS);
-                if (!kDhOnly && !(lm & kBB)) bwd_load_plain(st_b(s), static_cast<const Tact*>(p.bm), p.ld_bc, b, T, t0, 0, N, S, N, THREADS);
-                if (!(lm & kBC)) bwd_load_plain(st_c(s), static_cast<const Tact*>(p.cm), p.ld_bc, b, T, t0, 0, N, S, N, THREADS);
+            if constexpr (kPlain) {
+                if (!kDhOnly && !(lm & kBU))
+                    plain_channels<DT>(st_u(s), static_cast<const Tact*>(p.u), p.ld_u, static_cast<long long>(b) * T, t0, S, T, d0, D, tid);
+                if (!(lm & kBDl))
+                    plain_channels<DT>(st_dl(s), static_cast<const Tact*>(p.dl), p.ld_dl, static_cast<long long>(b) * T, t0, S, T, d0, D, tid);
+                if (kGate && !(lm & kBZ))
+                    plain_channels<DT>(st_z(s), static_cast<const Tact*>(p.z), p.ld_z, static_cast<long long>(b) * T, t0, S, T, d0, D, tid);
+                if (!(lm & kBDy))
+                    plain_channels<DT>(st_dy(s), static_cast<const Tact*>(p.dy), p.ld_dy, static_cast<long long>(b) * T, t0, S, T, d0, D, tid);
+                if (!kDhOnly && !(lm & kBB))
+                    plain_tile<32>(st_b(s), static_cast<const Tact*>(p.bm) + static_cast<long long>(b) * T * p.ld_bc, p.ld_bc, t0, S, T, 0, N, N, tid);
+                if (!(lm & kBC))
+                    plain_tile<32>(st_c(s), static_cast<const Tact*>(p.cm) + static_cast<long long>(b) * T * p.ld_bc, p.ld_bc, t0, S, T, 0, N, N, tid);
             }
             if (tx_bytes) mbar_wait(&bars[0], phase, p.status);
             __syncwarp();
@@ -467,22 +460,19 @@ __global__ void __maxnreg__(kBwd2MaxRegs) sscan_bwd2_kernel(const __grid_constan
     }
 }
 
+template <typename Tact, int... F>
+static void fill_bwd2_flags(BwdKernelFn* fn, std::integer_sequence<int, F...>) {
+    ((fn[F] = sscan_bwd2_kernel<Tact, 32, F>), ...);
+}
 template <typename Tact>
-static void fill_bwd2(BwdKernelFn (*fn)[8], size_t* smem) {
-    fn[0][0] = sscan_bwd2_kernel<Tact, 32, 0>;
-    fn[0][1] = sscan_bwd2_kernel<Tact, 32, 1>;
-    fn[0][2] = sscan_bwd2_kernel<Tact, 32, 2>;
-    fn[0][3] = sscan_bwd2_kernel<Tact, 32, 3>;
-    fn[0][4] = sscan_bwd2_kernel<Tact, 32, 4>;
-    fn[0][5] = sscan_bwd2_kernel<Tact, 32, 5>;
-    fn[0][6] = sscan_bwd2_kernel<Tact, 32, 6>;
-    fn[0][7] = sscan_bwd2_kernel<Tact, 32, 7>;
+static void fill_bwd2(BwdKernelFn (*fn)[16], size_t* smem) {
+    fill_bwd2_flags<Tact>(fn[0], std::make_integer_sequence<int, 16>{});
     smem[0] = Bwd2Traits<Tact, 32>::SMEM;
 }
 
 // [0][flags] (save stride 32); one translation unit per storage dtype
-void bwd2_kernels_f32(BwdKernelFn (*fn)[8], size_t* smem);
-void bwd2_kernels_f16(BwdKernelFn (*fn)[8], size_t* smem);
-void bwd2_kernels_bf16(BwdKernelFn (*fn)[8], size_t* smem);
+void bwd2_kernels_f32(BwdKernelFn (*fn)[16], size_t* smem);
+void bwd2_kernels_f16(BwdKernelFn (*fn)[16], size_t* smem);
+void bwd2_kernels_bf16(BwdKernelFn (*fn)[16], size_t* smem);
 
 }  // namespace mb200

@@ -6,7 +6,27 @@
 
 namespace mb200 {
 
-constexpr int kMaxSegments = 16;
+constexpr int kMaxSegments = 64;
+
+// Time segments of a launch that was lent a workspace (see launch_fwd), chosen from the consumer warps
+// it has per warp scheduler.  A warp alone on its scheduler takes 225 cycles a step, with 2.6 beside
+// each other 340 for all of them, and the state-only first pass costs half of a full one, so from 1.15
+// warps per scheduler one piece is as fast (8 x 2048 x 1536: 288 us in one piece, 303 in four; at 6
+// sequences 248 and 239).  Below that the sequence is cut into at least 16 pieces, and into more until
+// the schedulers are full (1 x 8192 x 64), none shorter than about 32 steps; sequences under 192 steps
+// stay whole (1 x 128 x 1536: 21 us whole, 24 in four).
+static int fwd_segments(int B, int T, int D, int N) {
+    int lpc = 1;
+    while (8 * lpc < N) lpc *= 2;
+    const int cw = lpc >= 16 ? 8 : 4, dt = cw * (32 / lpc);
+    const double per_sched = static_cast<double>(B) * ((D + dt - 1) / dt) * cw / (4 * 148);
+    if (per_sched >= 1.15 || T < 192) return 1;
+    int s = static_cast<int>(2.6 / per_sched) + 1;
+    if (s < 16) s = 16;
+    if (s > kMaxSegments) s = kMaxSegments;
+    const int most = (T + 31) / 32;
+    return s < most ? s : most;
+}
 
 struct FwdTable {
     FwdVariant v[3][kMaxFwdVariants];
@@ -158,12 +178,10 @@ static int launch_fwd(Ctx* c, cudaStream_t stream, const mamba_b200_sscan_fwd_ar
     // keeping the sum of its deltas), a small kernel chains them into the true
     // entering states, and the second launch runs every segment in full.
     const int tiles = (a.D + v->dt - 1) / v->dt;
-    const long long warps = static_cast<long long>(tiles) * a.B * (v->threads / 32 - 1);
     const int nchunks = (a.T + v->tc - 1) / v->tc;
     int segs = 1;
     if (a.workspace && a.workspace_bytes > 0) {
-        const long long want = 8ll * c->sm_count;  // two warps per scheduler
-        while (segs < kMaxSegments && warps * segs < want && nchunks / (segs * 2) >= 4) segs *= 2;
+        segs = fwd_segments(a.B, a.T, a.D, a.N);
         size_t o1, o2, o3;
         while (segs > 1 && fwd_ws_bytes(a.B, a.D, a.N, segs, &o1, &o2, &o3) > static_cast<size_t>(a.workspace_bytes))
             segs /= 2;
@@ -206,10 +224,9 @@ static int launch_fwd(Ctx* c, cudaStream_t stream, const mamba_b200_sscan_fwd_ar
 using namespace mb200;
 
 extern "C" MAMBA_B200_API long long mamba_b200_sscan_fwd_workspace_bytes(int B, int T, int D, int N) {
-    (void)T;
-    if (B <= 0 || D <= 0 || N <= 0 || N > 256) return 0;
+    if (B <= 0 || T <= 0 || D <= 0 || N <= 0 || N > 256) return 0;
     size_t o1, o2, o3;
-    return static_cast<long long>(fwd_ws_bytes(B, D, N, kMaxSegments, &o1, &o2, &o3));
+    return static_cast<long long>(fwd_ws_bytes(B, D, N, fwd_segments(B, T, D, N), &o1, &o2, &o3));
 }
 
 extern "C" MAMBA_B200_API int mamba_b200_sscan_fwd(void* handle, void* stream, const mamba_b200_sscan_fwd_args* args) {

@@ -159,19 +159,14 @@ sscan_fwd_kernel(const __grid_constant__ FwdParams p) {
         if (use_z && (load_mask & kTmaZ)) tx_bytes += sizeof(Tact) * TC * DT;
         if (load_mask & kTmaB) tx_bytes += sizeof(Tact) * TC * N;
         if (!kStateOnly && (load_mask & kTmaC)) tx_bytes += sizeof(Tact) * TC * N;
-        const Tact zero = from_f<Tact>(0.0f);
-        // Copies one [rows x cols] tile with plain loads (a tensor that breaks a TMA
-        // layout rule): out-of-range elements become zero, as TMA would fill them.
-        auto plain = [&](Tact* dst, const void* src, long long ld, int t_first, int rows, int c_first,
-                         int box_cols, int cols_total) {
-            const Tact* g = static_cast<const Tact*>(src);
-            for (int i = lane; i < rows * box_cols; i += 32) {
-                const int r = i / box_cols, cc = i - r * box_cols;
-                const int t = t_first + r, col = c_first + cc;
-                Tact v = zero;
-                if (t >= 0 && t < T && col < cols_total) v = g[(static_cast<long long>(b) * T + t) * ld + col];
-                dst[i] = v;
-            }
+        // Copies one [rows x box_cols] tile with plain loads (a tensor that breaks a TMA layout
+        // rule): out-of-range elements become zero, as TMA would fill them.
+        auto plain = [&](Tact* dst, const void* src, long long ld, int t_first, int rows) {
+            plain_channels<DT>(dst, static_cast<const Tact*>(src), ld, static_cast<long long>(b) * T, t_first, rows, T, d0, D, lane);
+        };
+        auto plain_bc = [&](Tact* dst, const void* src, int t_first) {
+            plain_tile<32>(dst, static_cast<const Tact*>(src) + static_cast<long long>(b) * T * p.ld_bc, p.ld_bc, t_first, TC, T, 0, N,
+                           N, lane);
         };
         auto issue = [&](int c) {  // whole warp
             const int s = c % STAGES, t0 = (c_begin + c) * TC;
@@ -182,15 +177,11 @@ sscan_fwd_kernel(const __grid_constant__ FwdParams p) {
             const bool any_plain = (load_mask & (kTmaX | kTmaDl | kTmaB)) != (kTmaX | kTmaDl | kTmaB) ||
                                    (use_z && !(load_mask & kTmaZ)) || (!kStateOnly && !(load_mask & kTmaC));
             if (any_plain) {
-                if (!(load_mask & kTmaX)) plain(xdst, p.x, p.ld_x, xr0, kConv ? TC + kHaloRows : TC, d0, DT, D);
-                if (!(load_mask & kTmaDl))
-                    plain(reinterpret_cast<Tact*>(st + Tr::OFF_DL), p.dl, p.ld_dl, t0, TC, d0, DT, D);
-                if (use_z && !(load_mask & kTmaZ))
-                    plain(reinterpret_cast<Tact*>(st + Tr::OFF_Z), p.z, p.ld_z, t0, TC, d0, DT, D);
-                if (!(load_mask & kTmaB))
-                    plain(reinterpret_cast<Tact*>(st + Tr::OFF_RB), p.bm, p.ld_bc, t0, TC, 0, N, N);
-                if (!kStateOnly && !(load_mask & kTmaC))
-                    plain(reinterpret_cast<Tact*>(st + Tr::OFF_RC), p.cm, p.ld_bc, t0, TC, 0, N, N);
+                if (!(load_mask & kTmaX)) plain(xdst, p.x, p.ld_x, xr0, kConv ? TC + kHaloRows : TC);
+                if (!(load_mask & kTmaDl)) plain(reinterpret_cast<Tact*>(st + Tr::OFF_DL), p.dl, p.ld_dl, t0, TC);
+                if (use_z && !(load_mask & kTmaZ)) plain(reinterpret_cast<Tact*>(st + Tr::OFF_Z), p.z, p.ld_z, t0, TC);
+                if (!(load_mask & kTmaB)) plain_bc(reinterpret_cast<Tact*>(st + Tr::OFF_RB), p.bm, t0);
+                if (!kStateOnly && !(load_mask & kTmaC)) plain_bc(reinterpret_cast<Tact*>(st + Tr::OFF_RC), p.cm, t0);
                 __syncwarp();
             }
             if (lane == 0) {

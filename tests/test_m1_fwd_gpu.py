@@ -305,3 +305,30 @@ def test_time_segments_with_exact_carry_match_oracle(cuda_dev, shape, dt):
     torch.cuda.synchronize()
     assert rel_err(y.float().cpu().numpy(), y1.float().cpu().numpy()) <= TOL[dt]
     assert rel_err(ssm.cpu().numpy(), ssm1.cpu().numpy()) <= 1e-4
+
+
+# rows that no TMA map describes: odd channel counts (rows start on odd elements in 16-bit storage), an odd
+# row stride around an even count, a base 2 bytes off a word; more than one sample and channel tile
+@pytest.mark.parametrize("dt", ["f32", "bf16", "f16"])
+@pytest.mark.parametrize("case", [(2, 70, 65, 65, 0), (3, 33, 129, 129, 0), (2, 40, 64, 67, 0), (2, 40, 31, 48, 1), (1, 200, 1, 1, 0)],
+                         ids=lambda c: "B%dT%dD%dld%doff%d" % c)
+def test_unaligned_rows_take_plain_loads(cuda_dev, case, dt):
+    import torch
+
+    import mamba_rs_b200 as mb
+    B, T, D, ld, off = case
+    q = quantised_inputs(B, T, D, 16, 0, dt, seed=D, a_mode="random")
+    ref = oracle.m1_fused_fwd(q["x"], q["delta_raw"], q["Bm"], q["Cm"], q["z"], q["a_neg"], q["Dp"])
+    td = torch_dtype(dt)
+
+    def view(a):  # [B,T,D] inside rows of ld elements, `off` elements into the buffer
+        flat = torch.full((B * T * ld + off,), float("nan"), device=cuda_dev, dtype=td)
+        v = flat[off:].view(B, T, ld)[..., :D]
+        v.copy_(to_dev(a, cuda_dev, td))
+        return v
+
+    y = mb.selective_scan_fwd(view(q["x"]), view(q["delta_raw"]), to_dev(q["Bm"], cuda_dev, td), to_dev(q["Cm"], cuda_dev, td),
+                              to_dev(q["a_neg"], cuda_dev), to_dev(q["Dp"], cuda_dev), view(q["z"]))
+    torch.cuda.synchronize()
+    mb.ffi.default_handle(0).check_status()
+    assert rel_err(y.float().cpu().numpy(), ref["y"]) <= TOL[dt]
