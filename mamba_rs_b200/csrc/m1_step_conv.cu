@@ -6,6 +6,7 @@
 // once (plus a K-1 row halo per time chunk).
 #include <string.h>
 
+#include <algorithm>
 #include <atomic>
 #include <initializer_list>
 
@@ -232,374 +233,252 @@ __global__ void __launch_bounds__(128) conv1d_bwd_kernel(const ConvParams p) {
 }
 
 // ---------------------------------------------------------------------------
-// Vector variants (d_conv <= 4, rows and pointers aligned to the vector): a
-// thread owns VEC adjacent channels and moves them with one 4- to 16-byte access
-// per step, kConvUnr steps of loads in flight.  Same arithmetic, in the same
-// order per channel, as the scalar kernels above.  The defaults (8-byte accesses
-// forward, 2 channels backward, 32-step forward chunks, 2 steps in flight) are the
-// fastest of the combinations timed at B 16, L 2048, D 1536, bf16: wider vectors
-// and deeper unrolling cost more in registers (occupancy) than they save.
+// Register kernels for d_conv <= 4 and rows aligned to the vector (the model shapes).  A warp owns 8 steps
+// of 32 x VEC channels and requests every row it needs, halo included, before it computes: 11 row pieces a
+// lane forward, 25 backward, so a thread's loads overlap each other whatever the number of warps; a CTA is
+// up to eight warps over 64 adjacent steps, whose halos meet in L1.  Bound by HBM at model sizes (8 x 2048 x
+// 1536 bf16: forward 23 us, 4.4 TB/s, backward with its reduction 62 us) and by one round of load latency at
+// small ones (1 x 1021 x 1536: 4.1 and 11 us; 1 x 32 x 1536 f32: 2.3 and 7.7).  The walks of 32 and 64 steps
+// with two loads in flight that these replace took 30 and 75, 7.6 and 14.3, 6.5 and 27 us.
 // ---------------------------------------------------------------------------
-constexpr int kConvKV = 4;     // widest d_conv of the vector kernels
-constexpr int kConvFwdTT = 32;      // timesteps per thread, forward
-constexpr int kConvUnr = 2;         // steps of loads in flight per thread
-constexpr int kConvFwdBytes = 8;    // bytes one forward thread moves per step
-// (a backward thread owns 2 channels with 16-bit storage, 4 with f32)
+constexpr int kConvKV = 4;                 // widest d_conv of these kernels
+constexpr int kConvRT = 8;                 // steps of a warp
+constexpr int kConvWarps = kConvTT / kConvRT;
 
 template <typename Tact, int VEC>
-__device__ __forceinline__ void load_vec(const Tact* ptr, float* out) {
-    constexpr int BYTES = sizeof(Tact) * VEC;
-    static_assert(BYTES == 16 || BYTES == 8 || BYTES == 4, "vector access of 4, 8 or 16 bytes");
-    uint32_t w[BYTES / 4];
-    if constexpr (BYTES == 16) {
-        const uint4 v = *reinterpret_cast<const uint4*>(ptr);
-        w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
-    } else if constexpr (BYTES == 8) {
-        const uint2 v = *reinterpret_cast<const uint2*>(ptr);
-        w[0] = v.x; w[1] = v.y;
-    } else {
-        w[0] = *reinterpret_cast<const uint32_t*>(ptr);
-    }
+struct RawVec {
+    static constexpr int W = sizeof(Tact) * VEC / 4;
+    uint32_t w[W];
+    __device__ __forceinline__ void zero() {
 #pragma unroll
-    for (int i = 0; i < BYTES / 4; ++i) {
-        if (sizeof(Tact) == 4) {
-            out[i] = __uint_as_float(w[i]);
+        for (int i = 0; i < W; ++i) w[i] = 0;
+    }
+    __device__ __forceinline__ void load(const Tact* p) {
+        if constexpr (W == 4) {
+            const uint4 v = *reinterpret_cast<const uint4*>(p);
+            w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
+        } else if constexpr (W == 2) {
+            const uint2 v = *reinterpret_cast<const uint2*>(p);
+            w[0] = v.x; w[1] = v.y;
         } else {
-            const Tact* h = reinterpret_cast<const Tact*>(&w[i]);
-            out[2 * i] = to_f(h[0]);
-            out[2 * i + 1] = to_f(h[1]);
+            w[0] = *reinterpret_cast<const uint32_t*>(p);
         }
     }
-}
-template <typename Tact, int VEC>
-__device__ __forceinline__ void store_vec(Tact* ptr, const float* v) {
-    constexpr int BYTES = sizeof(Tact) * VEC;
-    __align__(16) Tact tmp[VEC];
+    __device__ __forceinline__ void store(Tact* p) const {
+        if constexpr (W == 4) *reinterpret_cast<uint4*>(p) = make_uint4(w[0], w[1], w[2], w[3]);
+        else if constexpr (W == 2) *reinterpret_cast<uint2*>(p) = make_uint2(w[0], w[1]);
+        else *reinterpret_cast<uint32_t*>(p) = w[0];
+    }
+    __device__ __forceinline__ float get(int v) const {
+        if constexpr (sizeof(Tact) == 4) {
+            return __uint_as_float(w[v]);
+        } else {
+            const float2 f = unpack2<Tact>(w[v / 2]);
+            return (v & 1) ? f.y : f.x;
+        }
+    }
+    __device__ __forceinline__ void set(const float* f) {
 #pragma unroll
-    for (int i = 0; i < VEC; ++i) tmp[i] = from_f<Tact>(v[i]);
-    if (BYTES == 16) *reinterpret_cast<uint4*>(ptr) = *reinterpret_cast<const uint4*>(tmp);
-    else if (BYTES == 8) *reinterpret_cast<uint2*>(ptr) = *reinterpret_cast<const uint2*>(tmp);
-    else *reinterpret_cast<uint32_t*>(ptr) = *reinterpret_cast<const uint32_t*>(tmp);
-}
+        for (int i = 0; i < W; ++i) {
+            if constexpr (sizeof(Tact) == 4) w[i] = __float_as_uint(f[i]);
+            else w[i] = pack2<Tact>(f[2 * i], f[2 * i + 1]);
+        }
+    }
+};
 
 // Taps of VEC adjacent channels, right-aligned in KV slots (absent taps zero), and bias.
 template <int VEC>
 __device__ __forceinline__ void conv_load_taps(const ConvParams& p, int d, float (*w)[VEC], float* bias) {
     constexpr int KV = kConvKV;
     const int K = p.K;
-    if (VEC % 4 == 0) {
 #pragma unroll
-        for (int v = 0; v + 3 < VEC; v += 4) {
-            const float4 bv = *reinterpret_cast<const float4*>(p.bias + d + v);
-            bias[v] = bv.x; bias[v + 1] = bv.y; bias[v + 2] = bv.z; bias[v + 3] = bv.w;
-        }
-    } else {
-#pragma unroll
-        for (int v = 0; v < VEC; ++v) bias[v] = p.bias[d + v];
-    }
-    if (K == KV) {  // one 16-byte load per channel
-#pragma unroll
-        for (int v = 0; v < VEC; ++v) {
+    for (int v = 0; v < VEC; ++v) {
+        bias[v] = p.bias[d + v];
+        if (K == KV) {  // one 16-byte load per channel
             const float4 wv = *reinterpret_cast<const float4*>(p.w + static_cast<long long>(d + v) * KV);
             w[0][v] = wv.x; w[1][v] = wv.y; w[2][v] = wv.z; w[3][v] = wv.w;
-        }
-    } else {
-#pragma unroll
-        for (int v = 0; v < VEC; ++v)
+        } else {
 #pragma unroll
             for (int k = 0; k < KV; ++k) {
                 const int kk = k - (KV - K);
                 w[k][v] = kk >= 0 ? p.w[static_cast<long long>(d + v) * K + kk] : 0.0f;
             }
+        }
     }
 }
 
 template <typename Tact>
-__global__ void __launch_bounds__(64) conv1d_fwd_vec_kernel(const ConvParams p) {
-    constexpr int VEC = kConvFwdBytes / sizeof(Tact), KV = kConvKV;
-    const int d = (blockIdx.x * blockDim.x + threadIdx.x) * VEC;
-    const int t0 = blockIdx.y * kConvFwdTT, b = blockIdx.z;
-    if (d >= p.D) return;
+__global__ void __launch_bounds__(32 * kConvWarps) conv1d_fwd_rows_kernel(const ConvParams p) {
+    constexpr int VEC = 4, KV = kConvKV, R = kConvRT + KV - 1;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int d = (blockIdx.x * 32 + lane) * VEC, t0 = blockIdx.y * kConvTT + warp * kConvRT, b = blockIdx.z;
+    if (d >= p.D || t0 >= p.T) return;
     const int K = p.K;
     const Tact* xb = static_cast<const Tact*>(p.x) + static_cast<long long>(b) * p.T * p.ld_x + d;
-    Tact* ub = static_cast<Tact*>(p.u) + static_cast<long long>(b) * p.T * p.ld_u + d;
-    // taps right-aligned: w[KV-1] meets x[t], absent taps are zero
-    float w[KV][VEC], win[KV - 1][VEC], bias[VEC];
-    conv_load_taps<VEC>(p, d, w, bias);
-    if (t0 >= KV - 1) {  // history rows lie in x: whole-vector loads (absent taps have zero weight)
+    Tact* ub = static_cast<Tact*>(p.u) + (static_cast<long long>(b) * p.T + t0) * p.ld_u + d;
+    RawVec<Tact, VEC> x[R];  // rows t0 - 3 .. t0 + 7
 #pragma unroll
-        for (int k = 0; k < KV - 1; ++k)
-            load_vec<Tact, VEC>(xb + static_cast<long long>(t0 - (KV - 1) + k) * p.ld_x, win[k]);
-    } else {
-#pragma unroll
-        for (int v = 0; v < VEC; ++v)
-#pragma unroll
-            for (int k = 0; k < KV - 1; ++k)
-                win[k][v] = k - (KV - K) >= 0 ? conv_x_at(p, xb + v, b, d + v, t0 - (KV - 1) + k) : 0.0f;
+    for (int r = 0; r < R; ++r) {
+        const int t = t0 - (KV - 1) + r;
+        x[r].zero();
+        if (t >= 0 && t < p.T) x[r].load(xb + static_cast<long long>(t) * p.ld_x);
     }
-    const int t1 = min(p.T, t0 + kConvFwdTT);
-    for (int tb = t0; tb < t1; tb += kConvUnr) {
-        float cur[kConvUnr][VEC];
+    float w[KV][VEC], bias[VEC];
+    conv_load_taps<VEC>(p, d, w, bias);
+    float pre[KV - 1][VEC];  // first warp of a sequence: the entering window's last inputs
+    const bool first = t0 == 0;
+    if (first) {
 #pragma unroll
-        for (int i = 0; i < kConvUnr; ++i) {
-            if (tb + i < t1) load_vec<Tact, VEC>(xb + static_cast<long long>(tb + i) * p.ld_x, cur[i]);
-        }
+        for (int r = 0; r < KV - 1; ++r)
 #pragma unroll
-        for (int i = 0; i < kConvUnr; ++i) {
-            if (tb + i < t1) {
-                float o[VEC];
-#pragma unroll
-                for (int v = 0; v < VEC; ++v) {
-                    float acc = bias[v];
-#pragma unroll
-                    for (int k = 0; k < KV - 1; ++k) acc = fmaf(win[k][v], w[k][v], acc);
-                    acc = fmaf(cur[i][v], w[KV - 1][v], acc);
-                    o[v] = siluf_fast(acc);
-#pragma unroll
-                    for (int k = 0; k < KV - 2; ++k) win[k][v] = win[k + 1][v];
-                    win[KV - 2][v] = cur[i][v];
-                }
-                store_vec<Tact, VEC>(ub + static_cast<long long>(tb + i) * p.ld_u, o);
+            for (int v = 0; v < VEC; ++v) {
+                const int k = K - (KV - 1) + r;  // slot of step r - 3
+                pre[r][v] = k >= 0 && p.state_in ? p.state_in[(static_cast<long long>(b) * p.D + d + v) * K + k] : 0.0f;
             }
+    }
+    RawVec<Tact, VEC> last[KV];  // and, for the window that it leaves, the sequence's last inputs
+    if (first && p.state_out) {
+#pragma unroll
+        for (int k = 0; k < KV; ++k)
+            if (p.T - KV + k >= 0) last[k].load(xb + static_cast<long long>(p.T - KV + k) * p.ld_x);
+    }
+#pragma unroll
+    for (int i = 0; i < kConvRT; ++i) {
+        float o[VEC];
+#pragma unroll
+        for (int v = 0; v < VEC; ++v) {
+            float acc = bias[v];
+#pragma unroll
+            for (int k = 0; k < KV; ++k) {
+                float xv = x[i + k].get(v);
+                if (i + k < KV - 1 && first) xv = pre[i + k < KV - 1 ? i + k : 0][v];
+                acc = fmaf(xv, w[k][v], acc);
+            }
+            o[v] = siluf_fast(acc);
+        }
+        if (t0 + i < p.T) {
+            RawVec<Tact, VEC> q;
+            q.set(o);
+            q.store(ub + static_cast<long long>(i) * p.ld_u);
+        }
+    }
+    // The window after the sequence: the last K inputs (older slots come from the entering window when
+    // T < K).  The warp that read the entering window replaces it, so in place is safe.
+    if (first && p.state_out) {
+#pragma unroll
+        for (int v = 0; v < VEC; ++v) {
+            float nw[KV];
+            const long long at = (static_cast<long long>(b) * p.D + d + v) * K;
+#pragma unroll
+            for (int k = 0; k < KV; ++k) {
+                const int t = p.T - KV + k;
+                nw[k] = 0.0f;
+                if (t >= 0) nw[k] = last[k].get(v);
+                else if (K + t >= 0 && p.state_in) nw[k] = p.state_in[at + K + t];
+            }
+#pragma unroll
+            for (int k = 0; k < KV; ++k)
+                if (k >= KV - K) p.state_out[at + k - (KV - K)] = nw[k];
         }
     }
 }
 
 template <typename Tact>
-__global__ void __launch_bounds__(64) conv1d_bwd_vec_kernel(const ConvParams p) {
-    constexpr int VEC = sizeof(Tact) == 2 ? 2 : 4, KV = kConvKV;
-    const int d = (blockIdx.x * blockDim.x + threadIdx.x) * VEC;
-    const int chunk = blockIdx.y, t0 = chunk * kConvTT, b = blockIdx.z;
-    if (d >= p.D) return;
-    const int K = p.K, T = p.T;
-    const Tact* xb = static_cast<const Tact*>(p.x) + static_cast<long long>(b) * T * p.ld_x + d;
-    const Tact* gb = static_cast<const Tact*>(p.du) + static_cast<long long>(b) * T * p.ld_du + d;
-    Tact* dxb = static_cast<Tact*>(p.dx) + static_cast<long long>(b) * T * p.ld_dx + d;
-    // right-aligned taps as in the forward; win[k] = x[t - (KV-1) + k]
-    float w[KV][VEC], win[KV][VEC], dco[KV - 1][VEC], dW[KV][VEC], bias[VEC], db[VEC];
-    const int t1 = min(T, t0 + kConvTT);
-    const int t_start = min(T - 1, t1 + K - 2);
-    conv_load_taps<VEC>(p, d, w, bias);
-    if (t_start >= KV - 1) {
-#pragma unroll
-        for (int k = 0; k < KV; ++k)
-            load_vec<Tact, VEC>(xb + static_cast<long long>(t_start - (KV - 1) + k) * p.ld_x, win[k]);
-    } else {
-#pragma unroll
-        for (int v = 0; v < VEC; ++v)
-#pragma unroll
-            for (int k = 0; k < KV; ++k)
-                win[k][v] = k - (KV - K) >= 0 ? conv_x_at(p, xb + v, b, d + v, t_start - (KV - 1) + k) : 0.0f;
-    }
+__global__ void __launch_bounds__(32 * kConvWarps) conv1d_bwd_rows_kernel(const ConvParams p) {
+    constexpr int VEC = 2, KV = kConvKV, H = KV - 1, RG = kConvRT + H, RX = RG + H;
+    __shared__ float red[kConvWarps][KV + 1][32 * VEC];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int d = (blockIdx.x * 32 + lane) * VEC, chunk = blockIdx.y, t0 = chunk * kConvTT + warp * kConvRT, b = blockIdx.z;
+    const int K = p.K;
+    const bool on = d < p.D && t0 < p.T;
+    float dW[KV][VEC], db[VEC];
 #pragma unroll
     for (int v = 0; v < VEC; ++v) {
         db[v] = 0.0f;
 #pragma unroll
-        for (int k = 0; k < KV; ++k) {
-            dW[k][v] = 0.0f;
-            if (k < KV - 1) dco[k][v] = 0.0f;
-        }
+        for (int k = 0; k < KV; ++k) dW[k][v] = 0.0f;
     }
-    for (int tb = t_start; tb >= t0; tb -= kConvUnr) {
-        // loads of four steps: d_u[t] and the input that enters the window when it
-        // slides back past t (x[t - K], from the entering state when negative)
-        float g4[kConvUnr][VEC], xin[kConvUnr][VEC];
+    if (on) {
+        const Tact* xb = static_cast<const Tact*>(p.x) + static_cast<long long>(b) * p.T * p.ld_x + d;
+        const Tact* gb = static_cast<const Tact*>(p.du) + static_cast<long long>(b) * p.T * p.ld_du + d;
+        Tact* dxb = static_cast<Tact*>(p.dx) + (static_cast<long long>(b) * p.T + t0) * p.ld_dx + d;
+        RawVec<Tact, VEC> x[RX], g[RG];  // x rows t0 - 3 .. t0 + 10, d_u rows t0 .. t0 + 10
 #pragma unroll
-        for (int i = 0; i < kConvUnr; ++i) {
-            const int t = tb - i;
-            if (t >= t0) {
-                load_vec<Tact, VEC>(gb + static_cast<long long>(t) * p.ld_du, g4[i]);
-                if (t - K >= 0) {
-                    load_vec<Tact, VEC>(xb + static_cast<long long>(t - K) * p.ld_x, xin[i]);
-                } else {
-#pragma unroll
-                    for (int v = 0; v < VEC; ++v) xin[i][v] = conv_x_at(p, xb + v, b, d + v, t - K);
-                }
-            }
+        for (int r = 0; r < RX; ++r) {
+            const int t = t0 - H + r;
+            x[r].zero();
+            if (t >= 0 && t < p.T) x[r].load(xb + static_cast<long long>(t) * p.ld_x);
         }
 #pragma unroll
-        for (int i = 0; i < kConvUnr; ++i) {
-            const int t = tb - i;
-            if (t >= t0) {
-                float dxv[VEC];
+        for (int r = 0; r < RG; ++r) {
+            g[r].zero();  // past the end: no gradient
+            if (t0 + r < p.T) g[r].load(gb + static_cast<long long>(t0 + r) * p.ld_du);
+        }
+        float w[KV][VEC], bias[VEC], pre[H][VEC];
+        conv_load_taps<VEC>(p, d, w, bias);
+        const bool first = t0 == 0;
+        if (first) {
+#pragma unroll
+            for (int r = 0; r < H; ++r)
 #pragma unroll
                 for (int v = 0; v < VEC; ++v) {
-                    float acc = bias[v];
-#pragma unroll
-                    for (int k = 0; k < KV; ++k) acc = fmaf(win[k][v], w[k][v], acc);
-                    const float sg = sigmoidf_fast(acc);
-                    const float g = g4[i][v] * sg * fmaf(acc, 1.0f - sg, 1.0f);
-                    if (t < t1) {
-                        db[v] += g;
-                        float dx = g * w[KV - 1][v];
-#pragma unroll
-                        for (int k = 0; k < KV; ++k) dW[k][v] = fmaf(g, win[k][v], dW[k][v]);
-                        // future steps: dco[j] = dco[t + 1 + j] meets tap KV-2-j
-#pragma unroll
-                        for (int j = 0; j < KV - 1; ++j) dx = fmaf(dco[j][v], w[KV - 2 - j][v], dx);
-                        dxv[v] = dx;
-                    }
-#pragma unroll
-                    for (int j = KV - 2; j > 0; --j) dco[j][v] = dco[j - 1][v];
-                    dco[0][v] = g;
-#pragma unroll
-                    for (int k = KV - 1; k > 0; --k) win[k][v] = win[k - 1][v];
-                    // x[t - K] enters at the oldest tap that exists (slot KV - K)
-#pragma unroll
-                    for (int k = 0; k < KV; ++k)
-                        if (k == KV - K) win[k][v] = xin[i][v];
+                    const int k = K - H + r;
+                    pre[r][v] = k >= 0 && p.state_in ? p.state_in[(static_cast<long long>(b) * p.D + d + v) * K + k] : 0.0f;
                 }
-                if (t < t1) store_vec<Tact, VEC>(dxb + static_cast<long long>(t) * p.ld_dx, dxv);
-            }
         }
+        float dco[RG][VEC];
+#pragma unroll
+        for (int i = 0; i < RG; ++i)
+#pragma unroll
+            for (int v = 0; v < VEC; ++v) {
+                float xv[KV], acc = bias[v];
+#pragma unroll
+                for (int k = 0; k < KV; ++k) {
+                    xv[k] = x[i + k].get(v);
+                    if (i + k < H && first) xv[k] = pre[i + k < H ? i + k : 0][v];
+                    acc = fmaf(xv[k], w[k][v], acc);
+                }
+                const float sg = sigmoidf_fast(acc);
+                const float gv = g[i].get(v) * sg * fmaf(acc, 1.0f - sg, 1.0f);
+                dco[i][v] = gv;
+                if (i < kConvRT) {
+                    db[v] += gv;
+#pragma unroll
+                    for (int k = 0; k < KV; ++k) dW[k][v] = fmaf(gv, xv[k], dW[k][v]);
+                }
+            }
+#pragma unroll
+        for (int i = 0; i < kConvRT; ++i)
+            if (t0 + i < p.T) {
+                float o[VEC];
+#pragma unroll
+                for (int v = 0; v < VEC; ++v) {
+                    o[v] = 0.0f;
+#pragma unroll
+                    for (int k = 0; k < KV; ++k) o[v] = fmaf(dco[i + H - k][v], w[k][v], o[v]);
+                }
+                RawVec<Tact, VEC> q;
+                q.set(o);
+                q.store(dxb + static_cast<long long>(i) * p.ld_dx);
+            }
     }
-    const int chunks = gridDim.y;
 #pragma unroll
     for (int v = 0; v < VEC; ++v) {
-        float* pt = p.part + ((static_cast<long long>(b) * chunks + chunk) * p.D + d + v) * (K + 1);
 #pragma unroll
-        for (int k = 0; k < KV; ++k) {
-            const int kk = k - (KV - K);
-            if (kk >= 0) pt[kk] = dW[k][v];
-        }
-        pt[K] = db[v];
-    }
-}
-
-// ---------------------------------------------------------------------------
-// conv1d + SiLU backward from shared-memory tiles (16-bit storage, d_conv <= 4, rows on
-// 16-byte boundaries).  The register kernels above are bound by instruction issue and load
-// latency (146 warp-instructions per step of two channels, each thread waiting on its own
-// 4-byte loads); here a CTA of 128 threads first brings the x and d_u rows of its 64 steps
-// (plus the halo) into shared memory with 16-byte loads that are all in flight together, then
-// thread = channel walks the steps out of shared memory with the same arithmetic in the same
-// order, and d_x leaves through a tile and 16-byte stores.
-// ---------------------------------------------------------------------------
-constexpr int kConvTileD = 128;
-constexpr int kConvTileXRows = kConvTT + 2 * kConvKV - 1;  // x[t0 - K .. t1 + K - 2]
-constexpr int kConvTileGRows = kConvTT + kConvKV - 1;      // d_u[t0 .. t1 + K - 2]
-template <typename Tact>
-constexpr size_t conv_tile_smem() {
-    return sizeof(Tact) * kConvTileD * (kConvTileXRows + kConvTileGRows + kConvTT) + sizeof(float) * kConvKV * kConvTileD;
-}
-
-template <typename Tact>
-__global__ void __launch_bounds__(kConvTileD) conv1d_bwd_tile_kernel(const ConvParams p) {
-    static_assert(sizeof(Tact) == 2, "16-bit storage");
-    constexpr int KV = kConvKV, DT = kConvTileD, PIECES = DT / 8;  // 16-byte pieces per row
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    Tact* xs = reinterpret_cast<Tact*>(smem_raw);            // [kConvTileXRows][DT], row r = step xt0 + r
-    Tact* gs = xs + kConvTileXRows * DT;                     // [kConvTileGRows][DT], row r = step t0 + r
-    Tact* dxs = gs + kConvTileGRows * DT;                    // [kConvTT][DT]
-    float* xneg = reinterpret_cast<float*>(dxs + kConvTT * DT);  // [K][DT]: x[-K .. -1] (chunk 0 only)
-    const int d0 = blockIdx.x * DT, chunk = blockIdx.y, t0 = chunk * kConvTT, b = blockIdx.z;
-    const int K = p.K, T = p.T, D = p.D;
-    const int t1 = min(T, t0 + kConvTT), t_start = min(T - 1, t1 + K - 2);
-    // row r of xs is step xt0 + r; rows of negative steps (first chunk) stay unused
-    const int xt0 = t0 - K, nx = t_start - xt0 + 1, ng = t_start - t0 + 1;
-    const Tact* xb = static_cast<const Tact*>(p.x) + static_cast<long long>(b) * T * p.ld_x + d0;
-    const Tact* gb = static_cast<const Tact*>(p.du) + static_cast<long long>(b) * T * p.ld_du + d0;
-    Tact* dxb = static_cast<Tact*>(p.dx) + static_cast<long long>(b) * T * p.ld_dx + d0;
-    const int tid = threadIdx.x;
-    const uint4 z4 = make_uint4(0, 0, 0, 0);
-    for (int i = tid; i < nx * PIECES; i += DT) {
-        const int r = i / PIECES, pc = i - r * PIECES;
-        const bool in = d0 + pc * 8 < D && xt0 + r >= 0;
-        reinterpret_cast<uint4*>(xs)[i] = in ? *reinterpret_cast<const uint4*>(xb + static_cast<long long>(xt0 + r) * p.ld_x + pc * 8) : z4;
-    }
-    for (int i = tid; i < ng * PIECES; i += DT) {
-        const int r = i / PIECES, pc = i - r * PIECES;
-        const bool in = d0 + pc * 8 < D;
-        reinterpret_cast<uint4*>(gs)[i] = in ? *reinterpret_cast<const uint4*>(gb + static_cast<long long>(t0 + r) * p.ld_du + pc * 8) : z4;
-    }
-    const int d = d0 + tid;
-    const bool d_ok = d < D;
-    const bool has_neg = t0 < K;  // only the first chunk reaches the entering window
-    if (has_neg) {
-        for (int k = 0; k < K; ++k)
-            xneg[k * DT + tid] = (p.state_in && d_ok) ? p.state_in[(static_cast<long long>(b) * D + d) * K + k] : 0.0f;
+        for (int k = 0; k < KV; ++k) red[warp][k][lane * VEC + v] = dW[k][v];
+        red[warp][KV][lane * VEC + v] = db[v];
     }
     __syncthreads();
-    // x[t] for t in [-K, T)
-    auto xat = [&](int t) { return (has_neg && t < 0) ? xneg[(K + t) * DT + tid] : to_f(xs[(t - xt0) * DT + tid]); };
-    float w[KV], win[KV], dco[KV - 1], dW[KV], bias = 0.0f, db = 0.0f;
-#pragma unroll
-    for (int k = 0; k < KV; ++k) {
-        const int kk = k - (KV - K);
-        w[k] = (kk >= 0 && d_ok) ? p.w[static_cast<long long>(d) * K + kk] : 0.0f;
-        win[k] = kk >= 0 ? xat(t_start - (KV - 1) + k) : 0.0f;
-        dW[k] = 0.0f;
-        if (k < KV - 1) dco[k] = 0.0f;
-    }
-    if (d_ok) bias = p.bias[d];
-    // One step back in time: gv = d_u[t], xin = x[t - K] (enters the window), OUT: t < t1.
-    auto step = [&](auto out_tag, float gv, float xin, Tact* dst) {
-        float acc = bias;
-#pragma unroll
-        for (int k = 0; k < KV; ++k) acc = fmaf(win[k], w[k], acc);
-        const float sg = sigmoidf_fast(acc);
-        const float g = gv * sg * fmaf(acc, 1.0f - sg, 1.0f);
-        if (decltype(out_tag)::value) {
-            db += g;
-            float dx = g * w[KV - 1];
-#pragma unroll
-            for (int k = 0; k < KV; ++k) dW[k] = fmaf(g, win[k], dW[k]);
-            // future steps: dco[j] = dco[t + 1 + j] meets tap KV-2-j
-#pragma unroll
-            for (int j = 0; j < KV - 1; ++j) dx = fmaf(dco[j], w[KV - 2 - j], dx);
-            *dst = from_f<Tact>(dx);
+    // the chunk's sums in step order, one (tap, channel) per thread and pass
+    for (int i = threadIdx.x; i < (KV + 1) * 32 * VEC; i += blockDim.x) {
+        const int k = i / (32 * VEC), c = i - k * 32 * VEC, dd = blockIdx.x * 32 * VEC + c;
+        const int kk = k == KV ? K : k - (KV - K);
+        if (dd < p.D && kk >= 0) {
+            float s = red[0][k][c];
+            for (int q = 1; q < blockDim.x / 32; ++q) s += red[q][k][c];
+            p.part[((static_cast<long long>(b) * gridDim.y + chunk) * p.D + dd) * (K + 1) + kk] = s;
         }
-#pragma unroll
-        for (int j = KV - 2; j > 0; --j) dco[j] = dco[j - 1];
-        dco[0] = g;
-#pragma unroll
-        for (int k = KV - 1; k > 0; --k) win[k] = win[k - 1];
-        // x[t - K] enters at the oldest tap that exists (slot KV - K)
-#pragma unroll
-        for (int k = 0; k < KV; ++k)
-            if (k == KV - K) win[k] = xin;
-    };
-    // the halo steps after the chunk feed dco only
-    for (int t = t_start; t >= t1; --t) step(std::false_type{}, to_f(gs[(t - t0) * DT + tid]), xat(t - K), dxs);
-    const int n = t1 - t0;
-    const Tact* gp = gs + (n - 1) * DT + tid;
-    Tact* dp = dxs + (n - 1) * DT + tid;
-    if (has_neg) {
-        for (int i = n - 1; i >= 0; --i, gp -= DT, dp -= DT) step(std::true_type{}, to_f(*gp), xat(t0 + i - K), dp);
-    } else {
-        const Tact* xp = xs + (n - 1) * DT + tid;  // x[t - K] sits K rows below x[t]: row (t - K) - xt0 = t - t0
-        int i = n;
-        for (; i >= 8; i -= 8) {
-#pragma unroll
-            for (int u = 0; u < 8; ++u) step(std::true_type{}, to_f(gp[-u * DT]), to_f(xp[-u * DT]), dp - u * DT);
-            gp -= 8 * DT; xp -= 8 * DT; dp -= 8 * DT;
-        }
-        for (; i > 0; --i, gp -= DT, xp -= DT, dp -= DT) step(std::true_type{}, to_f(*gp), to_f(*xp), dp);
     }
-    if (d_ok) {
-        float* pt = p.part + ((static_cast<long long>(b) * gridDim.y + chunk) * D + d) * (K + 1);
-#pragma unroll
-        for (int k = 0; k < KV; ++k) {
-            const int kk = k - (KV - K);
-            if (kk >= 0) pt[kk] = dW[k];
-        }
-        pt[K] = db;
-    }
-    __syncthreads();
-    for (int i = tid; i < (t1 - t0) * PIECES; i += DT) {
-        const int r = i / PIECES, pc = i - r * PIECES;
-        if (d0 + pc * 8 < D)
-            *reinterpret_cast<uint4*>(dxb + static_cast<long long>(t0 + r) * p.ld_dx + pc * 8) = reinterpret_cast<const uint4*>(dxs)[i];
-    }
-}
-
-int conv_configure(Ctx* c) {
-    MB200_CUDA_CHECK(c, cudaFuncSetAttribute(reinterpret_cast<const void*>(conv1d_bwd_tile_kernel<__half>),
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, conv_tile_smem<__half>()));
-    MB200_CUDA_CHECK(c, cudaFuncSetAttribute(reinterpret_cast<const void*>(conv1d_bwd_tile_kernel<__nv_bfloat16>),
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             conv_tile_smem<__nv_bfloat16>()));
-    return MAMBA_B200_OK;
 }
 
 // The vector kernels need d_conv <= 4 and every row start on a vector boundary.
@@ -726,21 +605,20 @@ extern "C" MAMBA_B200_API int mamba_b200_conv1d_fwd(void* handle, void* stream,
     dim3 grid((a.D + 127) / 128, chunks, a.B);
     const unsigned sb = static_cast<unsigned>((static_cast<long long>(a.B) * a.D + 127) / 128);
     const size_t es = a.dtype == MAMBA_B200_F32 ? 4 : 2;
-    const int vec = static_cast<int>(kConvFwdBytes / es);
-    const bool use_vec = conv_vec_ok(a.K, a.D, vec, es, {a.x, a.u}, {a.ld_x, a.ld_u}) &&
-                         reinterpret_cast<uintptr_t>(a.conv_w) % 16 == 0 && reinterpret_cast<uintptr_t>(a.conv_b) % 16 == 0;
-    dim3 vgrid((a.D / vec + 63) / 64, (a.T + kConvFwdTT - 1) / kConvFwdTT, a.B);
-    if (a.dtype == MAMBA_B200_F32) {
-        if (use_vec) conv1d_fwd_vec_kernel<float><<<vgrid, 64, 0, st>>>(p);
-        else conv1d_fwd_kernel<float><<<grid, 128, 0, st>>>(p);
+    if (conv_vec_ok(a.K, a.D, 4, es, {a.x, a.u}, {a.ld_x, a.ld_u}) && reinterpret_cast<uintptr_t>(a.conv_w) % 16 == 0) {
+        dim3 vgrid((a.D / 4 + 31) / 32, chunks, a.B);
+        const int threads = 32 * std::min(kConvWarps, (a.T + kConvRT - 1) / kConvRT);
+        if (a.dtype == MAMBA_B200_F32) conv1d_fwd_rows_kernel<float><<<vgrid, threads, 0, st>>>(p);
+        else if (a.dtype == MAMBA_B200_F16) conv1d_fwd_rows_kernel<__half><<<vgrid, threads, 0, st>>>(p);
+        else conv1d_fwd_rows_kernel<__nv_bfloat16><<<vgrid, threads, 0, st>>>(p);
+    } else if (a.dtype == MAMBA_B200_F32) {
+        conv1d_fwd_kernel<float><<<grid, 128, 0, st>>>(p);
         if (a.conv_state) conv1d_state_kernel<float><<<sb, 128, 0, st>>>(p);
     } else if (a.dtype == MAMBA_B200_F16) {
-        if (use_vec) conv1d_fwd_vec_kernel<__half><<<vgrid, 64, 0, st>>>(p);
-        else conv1d_fwd_kernel<__half><<<grid, 128, 0, st>>>(p);
+        conv1d_fwd_kernel<__half><<<grid, 128, 0, st>>>(p);
         if (a.conv_state) conv1d_state_kernel<__half><<<sb, 128, 0, st>>>(p);
     } else {
-        if (use_vec) conv1d_fwd_vec_kernel<__nv_bfloat16><<<vgrid, 64, 0, st>>>(p);
-        else conv1d_fwd_kernel<__nv_bfloat16><<<grid, 128, 0, st>>>(p);
+        conv1d_fwd_kernel<__nv_bfloat16><<<grid, 128, 0, st>>>(p);
         if (a.conv_state) conv1d_state_kernel<__nv_bfloat16><<<sb, 128, 0, st>>>(p);
     }
     MB200_CUDA_CHECK(c, cudaGetLastError());
@@ -775,27 +653,19 @@ extern "C" MAMBA_B200_API int mamba_b200_conv1d_bwd(void* handle, void* stream,
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     dim3 grid((a.D + 127) / 128, chunks, a.B);
     const size_t es = a.dtype == MAMBA_B200_F32 ? 4 : 2;
-    const int bvec = es == 2 ? 2 : 4;
-    const bool use_vec = conv_vec_ok(a.K, a.D, bvec, es, {a.x, a.d_u, a.d_x}, {a.ld_x, a.ld_du, a.ld_dx}) &&
-                         reinterpret_cast<uintptr_t>(a.conv_w) % 16 == 0 && reinterpret_cast<uintptr_t>(a.conv_b) % 16 == 0;
-    dim3 vgrid((a.D / bvec + 63) / 64, chunks, a.B);
-    // 16-bit storage with rows on 16-byte boundaries: the shared-memory tile kernel
-    const bool use_tile = es == 2 && conv_vec_ok(a.K, a.D, 8, es, {a.x, a.d_u, a.d_x}, {a.ld_x, a.ld_du, a.ld_dx});
-    if (use_tile) {
-        dim3 tgrid((a.D + kConvTileD - 1) / kConvTileD, chunks, a.B);
-        if (a.dtype == MAMBA_B200_F16)
-            conv1d_bwd_tile_kernel<__half><<<tgrid, kConvTileD, conv_tile_smem<__half>(), st>>>(p);
-        else
-            conv1d_bwd_tile_kernel<__nv_bfloat16><<<tgrid, kConvTileD, conv_tile_smem<__nv_bfloat16>(), st>>>(p);
+    if (conv_vec_ok(a.K, a.D, 2, es, {a.x, a.d_u, a.d_x}, {a.ld_x, a.ld_du, a.ld_dx}) &&
+        reinterpret_cast<uintptr_t>(a.conv_w) % 16 == 0) {
+        dim3 vgrid((a.D / 2 + 31) / 32, chunks, a.B);
+        const int threads = 32 * std::min(kConvWarps, (a.T + kConvRT - 1) / kConvRT);
+        if (a.dtype == MAMBA_B200_F32) conv1d_bwd_rows_kernel<float><<<vgrid, threads, 0, st>>>(p);
+        else if (a.dtype == MAMBA_B200_F16) conv1d_bwd_rows_kernel<__half><<<vgrid, threads, 0, st>>>(p);
+        else conv1d_bwd_rows_kernel<__nv_bfloat16><<<vgrid, threads, 0, st>>>(p);
     } else if (a.dtype == MAMBA_B200_F32) {
-        if (use_vec) conv1d_bwd_vec_kernel<float><<<vgrid, 64, 0, st>>>(p);
-        else conv1d_bwd_kernel<float><<<grid, 128, 0, st>>>(p);
+        conv1d_bwd_kernel<float><<<grid, 128, 0, st>>>(p);
     } else if (a.dtype == MAMBA_B200_F16) {
-        if (use_vec) conv1d_bwd_vec_kernel<__half><<<vgrid, 64, 0, st>>>(p);
-        else conv1d_bwd_kernel<__half><<<grid, 128, 0, st>>>(p);
+        conv1d_bwd_kernel<__half><<<grid, 128, 0, st>>>(p);
     } else {
-        if (use_vec) conv1d_bwd_vec_kernel<__nv_bfloat16><<<vgrid, 64, 0, st>>>(p);
-        else conv1d_bwd_kernel<__nv_bfloat16><<<grid, 128, 0, st>>>(p);
+        conv1d_bwd_kernel<__nv_bfloat16><<<grid, 128, 0, st>>>(p);
     }
     MB200_CUDA_CHECK(c, cudaGetLastError());
     const int n = a.D * (a.K + 1);

@@ -102,6 +102,14 @@ def test_conv1d_forward_and_backward_match_oracle(cuda_dev, shape, dt):
     assert rel_err(g["dconv_b"].cpu().numpy(), ref_b["dconv_b"]) <= max(tol, 2e-4)
 
 
+@pytest.mark.parametrize("dt", ["f32", "bf16", "f16"])
+@pytest.mark.parametrize("T", [1, 2, 3, 4, 8, 9, 63, 64, 67, 130])
+def test_conv1d_rows_kernel_edges(cuda_dev, T, dt):
+    """K = 4 with aligned channels: steps around a warp's 8 and a block's 64, fewer steps than the window,
+    a last warp with part of its channels."""
+    test_conv1d_forward_and_backward_match_oracle(cuda_dev, (2, T, 132, 4), dt)
+
+
 def test_conv_then_scan_equals_fused_conv_scan(cuda_dev):
     """conv1d_fwd followed by the scan on u == the scan with the conv fused in."""
     import torch
