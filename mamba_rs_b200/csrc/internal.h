@@ -53,6 +53,11 @@ bool make_tmap_stack(Ctx* c, CUtensorMap* map, int dtype, const void* base, int 
 bool make_tmap_head_tile(Ctx* c, CUtensorMap* map, int dtype, const void* base, int cols, int heads, int T,
                          int B);
 
+// CTAs of a cluster that share one (sample, head) of the Mamba-3 tensor-core kernels (1: no cluster), and the
+// launch of a kernel in clusters of `ranks` CTAs along x.
+int m3_cluster_ranks(int heads, int nchunks, double full, double pair, double many, double fixed);
+cudaError_t launch_cluster(const void* fn, dim3 grid, dim3 block, size_t smem, cudaStream_t st, int ranks, void** args);
+
 #define MB200_CUDA_CHECK(ctx, expr)                                                          \
     do {                                                                                     \
         cudaError_t _e = (expr);                                                             \

@@ -217,7 +217,9 @@ constexpr uint32_t kCarry = kVec + 2 * kVecSet * 4, kBias = kCarry + 64 * 8;
 constexpr uint32_t kStage = kBias + 2 * 128 * 4, kStageArr = 17 * 128;
 static_assert(kStage % 128 == 0 && kStageArr >= 129 * 16, "scalar staging");
 constexpr uint32_t kBar = kStage + 3 * kStageArr + 16, kTmemSlot = kBar + 48;
+constexpr uint32_t kTot = kTmemSlot + 8;  // SEG: log2 of the decay over this CTA's chunks
 constexpr uint32_t kSmem = kTmemSlot + 16;
+constexpr uint32_t kLoc = kM;             // SEG: f32 local state [128 n][64 p], before M is used
 // TMEM columns: G; Y1; Y2; S^T.
 constexpr uint32_t cG = 0, cY1 = 256, cY2 = 320, cS = 384, kTmemCols = 512;
 
@@ -237,14 +239,21 @@ constexpr uint32_t cG = 0, cY1 = 256, cY2 = 320, cS = 384, kTmemCols = 512;
 // V buffers: Q of the next chunk is requested when the first MMA group has read it, K and V when
 // the second has.  8 x 256 steps x 32 heads of 64 x 128, bf16: 43 us (2050 us sequentially), the
 // state within 3e-6 of the sequential kernel's.
-template <typename Th, bool GEN, bool CARRY>
+//
+// SEG: the chunks of a (sample, head) are divided over the CTAs of a thread-block cluster, for shapes
+// with fewer (sample, head) pairs than SMs.  Every CTA but the last first walks its chunks for the state
+// alone (K, V, one product a chunk) from zero; the CTAs then read one another's local states and decays
+// through distributed shared memory, which gives each the exact state entering its chunks, and walk them
+// in full.
+template <typename Th, bool GEN, bool CARRY, bool SEG>
 __global__ void __launch_bounds__(256, 1) m3_ssd_fwd_tc_kernel(const __grid_constant__ M3Params p) {
     extern __shared__ __align__(1024) unsigned char smem[];
     // two threads per step: thread (row, half) owns row `row` of the chunk (TMEM lane
     // `row`) and half of that row's columns in every elementwise stage
     const int tid = threadIdx.x & 127, half = threadIdx.x >> 7, warp = (threadIdx.x >> 5) & 3;
     const int lane = threadIdx.x & 31, wfull = threadIdx.x >> 5;
-    const int h = blockIdx.x, b = blockIdx.y;
+    const int nrank = SEG ? static_cast<int>(gridDim.x) / p.nh : 1, rank = SEG ? blockIdx.x % nrank : 0;
+    const int h = SEG ? blockIdx.x / nrank : blockIdx.x, b = blockIdx.y;
     const int T = p.T, nh = p.nh;
     // headdim <= 64 and d_state <= 128 (multiples of 8): the tiles keep their full
     // size and the missing columns are zero-filled, so every product is unchanged.
@@ -293,6 +302,12 @@ __global__ void __launch_bounds__(256, 1) m3_ssd_fwd_tc_kernel(const __grid_cons
     const Th* Kg = static_cast<const Th*>(p.K);
     const float Dv = p.Dh[h];
     const int nchunks = (T + CS - 1) / CS;
+    // this CTA's chunks; every chunk walked (in either pass) has a number j of its own, which the two-deep
+    // buffers and barrier phases go by: j0 is that of chunk c_lo in the full pass
+    const int per_rank = SEG ? (nchunks + nrank - 1) / nrank : nchunks;
+    const int c_lo = SEG ? min(nchunks, rank * per_rank) : 0, c_hi = SEG ? min(nchunks, c_lo + per_rank) : nchunks;
+    const bool state_pass = SEG && c_lo < c_hi && c_hi < nchunks;
+    const int j0 = state_pass ? c_hi - c_lo : 0;
     bool ok = true;
 
     // Per-row scalars of chunk c into stage `st`: inclusive cumsum of adt, scale, gamma.
@@ -305,7 +320,7 @@ __global__ void __launch_bounds__(256, 1) m3_ssd_fwd_tc_kernel(const __grid_cons
     uint64_t* scf = bars + 4;
     const int hcol = h & 3;
     auto stage_scalars = [&](int c) {
-        if (c >= nchunks) return;
+        if (c >= c_hi) return;
         if (p.sc_tma) {
             if (threadIdx.x == 0) {
                 mbar_expect_tx(scf, 3 * 129 * 16);
@@ -329,12 +344,13 @@ __global__ void __launch_bounds__(256, 1) m3_ssd_fwd_tc_kernel(const __grid_cons
             asm volatile("cp.async.commit_group;" ::: "memory");
         }
     };
-    auto scalars = [&](int c, int st) {
+    auto scalars = [&](int j) {
+        const int st = j & 1;
         float* dA = vec + st * kVecSet;
         float* scl = dA + 128;
         float* gam = dA + 256;
         if (p.sc_tma) {
-            ok = mbar_wait(scf, c & 1, p.status) && ok;
+            ok = mbar_wait(scf, j & 1, p.status) && ok;
         } else {
             asm volatile("cp.async.wait_group 0;" ::: "memory");
             __syncthreads();  // every thread's staged words of this chunk are in shared memory
@@ -506,9 +522,19 @@ __global__ void __launch_bounds__(256, 1) m3_ssd_fwd_tc_kernel(const __grid_cons
             tma_load_4d(smem + kCarryV, &p.tm_v, &full[1], 0, h, c * CS, b);
         }
     };
-    auto issue_tiles = [&](int c) {
+    auto issue_kv = [&](int c, int j) {  // state pass
         if (threadIdx.x == 0) {
-            const int buf = c & 1, t0 = c * CS;
+            const int buf = j & 1, t0 = c * CS;
+            mbar_expect_tx(&full[buf], kQKStride + kVStride);
+#pragma unroll
+            for (int sub = 0; sub < 2; ++sub)
+                tma_load_4d(smem + kK0 + buf * kQKStride + sub * kSwSub, &p.tm_k, &full[buf], 64 * sub, h, t0, b);
+            tma_load_4d(smem + kV0 + buf * kVStride, &p.tm_v, &full[buf], 0, h, t0, b);
+        }
+    };
+    auto issue_tiles = [&](int c, int j) {
+        if (threadIdx.x == 0) {
+            const int buf = j & 1, t0 = c * CS;
             const int hq = GEN ? h / (nh / p.ng) : h;
             mbar_expect_tx(&full[buf], 2 * kQKStride + kVStride);
 #pragma unroll
@@ -519,14 +545,6 @@ __global__ void __launch_bounds__(256, 1) m3_ssd_fwd_tc_kernel(const __grid_cons
             tma_load_4d(smem + kV0 + buf * kVStride, &p.tm_v, &full[buf], 0, h, t0, b);
         }
     };
-    if (CARRY) {
-        issue_carry_q(0);
-        issue_carry_kv(0);
-    } else {
-        issue_tiles(0);
-    }
-    stage_scalars(0);
-    if (GEN) load_vel(0);
     // 16-bit copy of this thread's state row (and the remainders): the B operand of Y2
     auto copy_state = [&](const float* sv) {
 #pragma unroll
@@ -546,39 +564,175 @@ __global__ void __launch_bounds__(256, 1) m3_ssd_fwd_tc_kernel(const __grid_cons
                     make_uint4(lo[0], lo[1], lo[2], lo[3]);
         }
     };
-    if (CARRY) {
+    // the carried state as this thread's row: h + dt_0 (1 - trap_0) k_prev v_prev^T
+    auto carried_state = [&](float* sv) {
         const long long bh = static_cast<long long>(b) * nh + h, th0 = static_cast<long long>(b) * T * nh + h;
         const float kc = tid < nsv ? p.dt[th0] * (1.0f - p.trap[th0]) * p.k_state[bh * nsv + tid] : 0.0f;
-        float sv[32];
 #pragma unroll
         for (int i = 0; i < 32; ++i) {
             const int pp = half * 32 + i;
             sv[i] = pp < hdv && tid < nsv ? fmaf(kc, p.v_state[bh * hdv + pp], p.ssm_state[(bh * hdv + pp) * nsv + tid])
                                           : 0.0f;
         }
+    };
+    // w o V of chunk j (and its remainders): the B operand of the state update
+    auto weigh_v = [&](const float* dA, const float* scl, int nv, uint32_t tV) {
+        const float wt = tid < nv ? ex2((dA[nv - 1] - dA[tid]) * kLog2e) * scl[tid] : 0.0f;
+#pragma unroll
+        for (int jj = half * (HD / 16); jj < (half + 1) * (HD / 16); ++jj) {
+            const uint4 v = *reinterpret_cast<const uint4*>(smem + tV + sw_chunk(tid, jj));
+            uint32_t w4[4] = {v.x, v.y, v.z, v.w}, lo[4];
+#pragma unroll
+            for (int q4 = 0; q4 < 4; ++q4) {
+                const float2 f = unpack2<Th>(w4[q4]);
+                w4[q4] = pack2<Th>(f.x * wt, f.y * wt);
+                if (CARRY) {
+                    const float2 r = unpack2<Th>(w4[q4]);
+                    lo[q4] = pack2<Th>(f.x * wt - r.x, f.y * wt - r.y);
+                }
+            }
+            *reinterpret_cast<uint4*>(smem + kVw + sw_chunk(tid, jj)) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
+            if (CARRY)
+                *reinterpret_cast<uint4*>(smem + kVwLo + sw_chunk(tid, jj)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+        }
+    };
+    auto decay_state = [&](float e_end) {  // S^T row `tid` (state index n = tid) *= exp(dA_end)
+        float sv[32];
+        tmem_ld32(lane_addr + cS + half * 32, sv);
+#pragma unroll
+        for (int i = 0; i < 32; ++i) sv[i] *= e_end;
+        tmem_st32(lane_addr + cS + half * 32, sv);
+    };
+    auto update_state = [&](uint32_t tK, bool accumulate) {  // S^T += K^T (w o V); one thread
+        const uint32_t idS = instr_desc(fmt, 1, 1, 64);
+#pragma unroll
+        for (int k = 0; k < CS / 16; ++k)  // M = n, N = p, K = t
+            mma(tmem + cS, desc_sw_mn(sbase + tK, k), desc_sw_mn(sbase + kVw, k), idS, accumulate || k > 0);
+        if (CARRY) {
+#pragma unroll
+            for (int k = 0; k < CS / 16; ++k)
+                mma(tmem + cS, desc_sw_mn(sbase + tK, k), desc_sw_mn(sbase + kVwLo, k), idS, true);
+        }
+    };
+
+    if constexpr (SEG) {
+        float tot = 0.0f;  // sum of dA over this CTA's chunks
+        if (state_pass) {
+            if (CARRY && rank == 0) {
+                float sv[32];
+                carried_state(sv);
+                tmem_st32(lane_addr + cS + half * 32, sv);
+            }
+            if (CARRY) issue_carry_kv(c_lo);
+            else issue_kv(c_lo, 0);
+            stage_scalars(c_lo);
+            for (int c = c_lo; c < c_hi; ++c) {
+                const int j = c - c_lo, nv = min(CS, T - c * CS);
+                const uint32_t tK = CARRY ? kCarryK : kK0 + (j & 1) * kQKStride;
+                const uint32_t tV = CARRY ? kCarryV : kV0 + (j & 1) * kVStride;
+                const float* dA = vec + (j & 1) * kVecSet;
+                if (!CARRY && c + 1 < c_hi) issue_kv(c + 1, j + 1);
+                scalars(j);
+                ok = mbar_wait(CARRY ? &full[1] : &full[j & 1], CARRY ? j & 1 : (j >> 1) & 1, p.status) && ok;
+                __syncthreads();  // the per-row vectors of every row
+                stage_scalars(c + 1);
+                weigh_v(dA, dA + 128, nv, tV);
+                const bool have = c > c_lo || (CARRY && rank == 0);
+                if (have) decay_state(ex2(dA[nv - 1] * kLog2e));
+                tot += dA[nv - 1];
+                fence_proxy_async();
+                fence_before();
+                __syncthreads();
+                if (threadIdx.x == 0) {
+                    fence_after();
+                    update_state(tK, have);
+                    commit(&bars[1]);
+                }
+                ok = mbar_wait(&bars[1], j & 1, p.status) && ok;
+                fence_after();
+                if (CARRY && c + 1 < c_hi) issue_carry_kv(c + 1);
+            }
+        }
+        // the full pass's first tiles travel while the states are exchanged
+        if (c_lo < c_hi) {
+            if (CARRY) {
+                issue_carry_q(c_lo);
+                issue_carry_kv(c_lo);
+            } else {
+                issue_tiles(c_lo, j0);
+            }
+            stage_scalars(c_lo);
+        }
+        if (state_pass) {
+            float sv[32];
+            tmem_ld32(lane_addr + cS + half * 32, sv);
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                *reinterpret_cast<float4*>(smem + kLoc + tid * 256 + half * 128 + i * 16) =
+                    make_float4(sv[4 * i], sv[4 * i + 1], sv[4 * i + 2], sv[4 * i + 3]);
+            if (threadIdx.x == 0) *reinterpret_cast<float*>(smem + kTot) = tot * kLog2e;
+        }
+        cluster_sync();
+        if (c_lo < c_hi && rank > 0) {
+            float sv[32];
+#pragma unroll
+            for (int i = 0; i < 32; ++i) sv[i] = 0.0f;
+            float between = 0.0f;  // log2 of the decay of the CTAs between q and this one
+            for (int q = rank - 1; q >= 0; --q) {
+                const float f = ex2(between);
+                const uint32_t src = cluster_addr(sbase + kLoc + tid * 256 + half * 128, q);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const float4 v = ld_cluster4(src + i * 16);
+                    sv[4 * i] = fmaf(f, v.x, sv[4 * i]);
+                    sv[4 * i + 1] = fmaf(f, v.y, sv[4 * i + 1]);
+                    sv[4 * i + 2] = fmaf(f, v.z, sv[4 * i + 2]);
+                    sv[4 * i + 3] = fmaf(f, v.w, sv[4 * i + 3]);
+                }
+                between += ld_cluster1(cluster_addr(sbase + kTot, q));
+            }
+            tmem_st32(lane_addr + cS + half * 32, sv);
+            copy_state(sv);
+            fence_proxy_async();  // (published by the barriers ahead of the first MMA group)
+        }
+        cluster_sync();  // nobody reads this CTA's shared memory any more
+    } else {
+        if (CARRY) {
+            issue_carry_q(0);
+            issue_carry_kv(0);
+        } else {
+            issue_tiles(0, 0);
+        }
+        stage_scalars(0);
+        if (GEN) load_vel(0);
+    }
+    if (CARRY && rank == 0) {
+        float sv[32];
+        carried_state(sv);
         tmem_st32(lane_addr + cS + half * 32, sv);
         copy_state(sv);
-        fence_proxy_async();  // (published by the barriers ahead of the first MMA group)
+        fence_proxy_async();
     }
 
-    for (int c = 0; c < nchunks; ++c) {
+    for (int c = c_lo; c < c_hi; ++c) {
+        const int i0 = c - c_lo, j = j0 + i0;
         const int t0 = c * CS, nv = min(CS, T - t0);
         const bool row_ok = tid < nv;
-        const float* dA = vec + (c & 1) * kVecSet;
+        const float* dA = vec + (j & 1) * kVecSet;
         const float* scl = dA + 128;
         const float* gam = dA + 256;
-        const uint32_t tQ = kQ0 + (CARRY ? 0u : (c & 1) * kQKStride);
-        const uint32_t tK = CARRY ? kCarryK : kK0 + (c & 1) * kQKStride;
-        const uint32_t tV = CARRY ? kCarryV : kV0 + (c & 1) * kVStride;
+        const uint32_t tQ = kQ0 + (CARRY ? 0u : (j & 1) * kQKStride);
+        const uint32_t tK = CARRY ? kCarryK : kK0 + (j & 1) * kQKStride;
+        const uint32_t tV = CARRY ? kCarryV : kV0 + (j & 1) * kVStride;
         // ---- 1. copies of the next chunk's tiles into the other buffers (their last readers,
         //         the MMAs of chunk c - 1, have completed); per-row scalars; this chunk's tiles ----
-        if (!CARRY && c + 1 < nchunks) issue_tiles(c + 1);
-        scalars(c, c & 1);
+        if (!CARRY && c + 1 < c_hi) issue_tiles(c + 1, j + 1);
+        scalars(j);
         if (CARRY) {
-            ok = mbar_wait(&full[0], c & 1, p.status) && ok;
-            ok = mbar_wait(&full[1], c & 1, p.status) && ok;
+            ok = mbar_wait(&full[0], i0 & 1, p.status) && ok;
+            ok = mbar_wait(&full[1], j & 1, p.status) && ok;
         } else {
-            ok = mbar_wait(&full[c & 1], (c >> 1) & 1, p.status) && ok;
+            ok = mbar_wait(&full[j & 1], (j >> 1) & 1, p.status) && ok;
         }
         if (GEN) {
             gen_apply(c, c & 1);
@@ -609,33 +763,13 @@ __global__ void __launch_bounds__(256, 1) m3_ssd_fwd_tc_kernel(const __grid_cons
             }
             commit(&bars[0]);
         }
-        ok = mbar_wait(&bars[0], c & 1, p.status) && ok;
+        ok = mbar_wait(&bars[0], i0 & 1, p.status) && ok;
         fence_after();
-        if (CARRY && c + 1 < nchunks) issue_carry_q(c + 1);
+        if (CARRY && c + 1 < c_hi) issue_carry_q(c + 1);
         // ---- 3. decay / causal mask -> M (over the Q tile); w o V (over the old state
         //         copy); rescale the running state ----
         {
-            {
-                const float wt = row_ok ? ex2((dA[nv - 1] - dA[tid]) * kLog2e) * scl[tid] : 0.0f;
-#pragma unroll
-                for (int j = half * (HD / 16); j < (half + 1) * (HD / 16); ++j) {
-                    const uint4 v = *reinterpret_cast<const uint4*>(smem + tV + sw_chunk(tid, j));
-                    uint32_t w4[4] = {v.x, v.y, v.z, v.w}, lo[4];
-#pragma unroll
-                    for (int q4 = 0; q4 < 4; ++q4) {
-                        const float2 f = unpack2<Th>(w4[q4]);
-                        w4[q4] = pack2<Th>(f.x * wt, f.y * wt);
-                        if (CARRY) {
-                            const float2 r = unpack2<Th>(w4[q4]);
-                            lo[q4] = pack2<Th>(f.x * wt - r.x, f.y * wt - r.y);
-                        }
-                    }
-                    *reinterpret_cast<uint4*>(smem + kVw + sw_chunk(tid, j)) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
-                    if (CARRY)
-                        *reinterpret_cast<uint4*>(smem + kVwLo + sw_chunk(tid, j)) =
-                            make_uint4(lo[0], lo[1], lo[2], lo[3]);
-                }
-            }
+            weigh_v(dA, scl, nv, tV);
             const float* dAl = dA + 384;  // dA * log2(e)
             const float dAlt = dAl[tid], gt = gam[tid];
             // One 32-column block of row `tid`.  Blocks left of the diagonal block need no
@@ -694,14 +828,7 @@ __global__ void __launch_bounds__(256, 1) m3_ssd_fwd_tc_kernel(const __grid_cons
                     mask_block(std::false_type{}, q4);
                 }
             }
-            if (CARRY || c > 0) {  // S^T row `tid` (state index n = tid) *= exp(dA_end)
-                const float e_end = ex2(dA[nv - 1] * kLog2e);
-                float sv[32];
-                tmem_ld32(lane_addr + cS + half * 32, sv);
-#pragma unroll
-                for (int i = 0; i < 32; ++i) sv[i] *= e_end;
-                tmem_st32(lane_addr + cS + half * 32, sv);
-            }
+            if (CARRY || c > 0) decay_state(ex2(dA[nv - 1] * kLog2e));
         }
         fence_proxy_async();
         fence_before();
@@ -711,26 +838,21 @@ __global__ void __launch_bounds__(256, 1) m3_ssd_fwd_tc_kernel(const __grid_cons
         // ---- 4. Y1 = M V ;  S^T += K^T (w o V) ----
         if (threadIdx.x == 0) {
             fence_after();
-            const uint32_t idY = instr_desc(fmt, 0, 1, 64), idS = instr_desc(fmt, 1, 1, 64);
+            const uint32_t idY = instr_desc(fmt, 0, 1, 64);
 #pragma unroll
             for (int k = 0; k < CS / 16; ++k)  // N = p, K = s
                 mma(tmem + cY1, desc_sw_k(sbase + kM, k), desc_sw_mn(sbase + tV, k), idY, k > 0);
-#pragma unroll
-            for (int k = 0; k < CS / 16; ++k)  // M = n, N = p, K = t
-                mma(tmem + cS, desc_sw_mn(sbase + tK, k), desc_sw_mn(sbase + kVw, k), idS, CARRY || c > 0 || k > 0);
             if (CARRY) {
 #pragma unroll
                 for (int k = 0; k < CS / 16; ++k)
                     mma(tmem + cY1, desc_sw_k(sbase + kMlo, k), desc_sw_mn(sbase + tV, k), idY, true);
-#pragma unroll
-                for (int k = 0; k < CS / 16; ++k)
-                    mma(tmem + cS, desc_sw_mn(sbase + tK, k), desc_sw_mn(sbase + kVwLo, k), idS, true);
             }
+            update_state(tK, CARRY || c > 0);
             commit(&bars[1]);
         }
-        ok = mbar_wait(&bars[1], c & 1, p.status) && ok;
+        ok = mbar_wait(&bars[1], j & 1, p.status) && ok;
         fence_after();
-        if (CARRY && c + 1 < nchunks) issue_carry_kv(c + 1);
+        if (CARRY && c + 1 < c_hi) issue_carry_kv(c + 1);
         // ---- 5. epilogue: y row; 16-bit copy of the new state for the next chunk ----
         {
             const float e_t = ex2(dA[tid] * kLog2e);
@@ -750,9 +872,9 @@ __global__ void __launch_bounds__(256, 1) m3_ssd_fwd_tc_kernel(const __grid_cons
                                    pack2<Th>(y1[8 * j + 4], y1[8 * j + 5]), pack2<Th>(y1[8 * j + 6], y1[8 * j + 7]));
             float sv[32];
             tmem_ld32(lane_addr + cS + q2 * 32, sv);
-            if (c + 1 < nchunks) {
+            if (c + 1 < c_hi) {
                 copy_state(sv);
-            } else if (p.ssm_state) {  // final state [b, h, p, n], n = tid
+            } else if (c + 1 == nchunks && p.ssm_state) {  // final state [b, h, p, n], n = tid
 #pragma unroll
                 for (int i = 0; i < 32; ++i)
                     if (q2 * 32 + i < hdv && tid < nsv)
@@ -781,7 +903,7 @@ __global__ void __launch_bounds__(256, 1) m3_ssd_fwd_tc_kernel(const __grid_cons
     __syncthreads();
     fence_after();
     // last inputs of the window (kernels/mamba3_chunked.cu:289-330)
-    if (T > 0) {
+    if (c_lo < c_hi && c_hi == nchunks) {
         const long long last = static_cast<long long>(b) * T + (T - 1);
         if (GEN) {
             // the last K row is still in its tile; fold the last chunk's sums into the angle
@@ -806,13 +928,54 @@ __global__ void __launch_bounds__(256, 1) m3_ssd_fwd_tc_kernel(const __grid_cons
 
 }  // namespace tc
 
+// CTAs of a cluster that share one (sample, head), by estimated time: a chunk takes one CTA `full` us
+// undivided, `pair` in a cluster of two and `many` in a larger one; the exchange takes `fixed` a rank.  A wave
+// is one CTA per SM, less what clusters of 4 and 8 cannot place.  A division that gains less than 5 % is not
+// taken.
+int m3_cluster_ranks(int heads, int nchunks, double full, double pair, double many, double fixed) {
+    int best = 1;
+    double cost = static_cast<double>((heads + 147) / 148) * nchunks * full;
+    const int cap[4] = {148, 148, 144, 128};
+    for (int i = 1; i < 4; ++i) {
+        const int r = 1 << i, per = (nchunks + r - 1) / r;
+        if (r > nchunks) break;
+        const double c = static_cast<double>((heads * r + cap[i] - 1) / cap[i]) * (per * (r == 2 ? pair : many) + r * fixed);
+        if (c < 0.95 * cost) {
+            cost = c;
+            best = r;
+        }
+    }
+    return best;
+}
+
+cudaError_t launch_cluster(const void* fn, dim3 grid, dim3 block, size_t smem, cudaStream_t st, int ranks, void** args) {
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at;
+    memset(&at, 0, sizeof(at));
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = ranks;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelExC(&cfg, fn, args);
+}
+
 int m3_configure(Ctx* c) {
-    const void* fns[6] = {reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, false>),
-                          reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__half, false, false>),
-                          reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, true, false>),
-                          reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__half, true, false>),
-                          reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, true>),
-                          reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__half, false, true>)};
+    const void* fns[10] = {reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, false, false>),
+                          reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__half, false, false, false>),
+                          reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, true, false, false>),
+                          reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__half, true, false, false>),
+                          reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, true, false>),
+                          reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__half, false, true, false>),
+                          reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, false, true>),
+                          reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__half, false, false, true>),
+                          reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, true, true>),
+                          reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__half, false, true, true>)};
     for (const void* fn : fns)
         MB200_CUDA_CHECK(c, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::kSmem));
     return MAMBA_B200_OK;
@@ -903,14 +1066,27 @@ extern "C" MAMBA_B200_API int mamba_b200_m3_ssd_fwd(void* handle, void* stream,
                    make_tmap_3d(c, &p.tm_dt, MAMBA_B200_F32, a.dt, a.nh, a.nh, a.T, a.B, 4, 129) &&
                    make_tmap_3d(c, &p.tm_trap, MAMBA_B200_F32, a.trap, a.nh, a.nh, a.T, a.B, 4, 129);
         dim3 grid(a.nh, a.B);
-        if (a.dtype == MAMBA_B200_BF16) {
-            if (gen) tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, true, false><<<grid, 256, tc::kSmem, st>>>(p);
-            else if (a.carry_in) tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, true><<<grid, 256, tc::kSmem, st>>>(p);
-            else tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, false><<<grid, 256, tc::kSmem, st>>>(p);
+        const bool bf = a.dtype == MAMBA_B200_BF16;
+        // bf16, 64 x 128: 4 heads x 4096 steps 44 us (one CTA each: 123), 24 x 2048 34 (63), 64 x 4096 91 (124);
+        // continued from a state 4 x 4096 62 us
+        const int nchunks = (a.T + tc::CS - 1) / tc::CS;
+        const int ranks = gen ? 1 : a.carry_in ? m3_cluster_ranks(a.B * a.nh, nchunks, 5.5, 6.6, 6.6, 3.2)
+                                               : m3_cluster_ranks(a.B * a.nh, nchunks, 3.7, 5.15, 5.15, 2.6);
+        if (ranks > 1) {
+            const void* fn = bf ? (a.carry_in ? reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, true, true>)
+                                              : reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, false, true>))
+                                : (a.carry_in ? reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__half, false, true, true>)
+                                              : reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__half, false, false, true>));
+            void* args[1] = {&p};
+            MB200_CUDA_CHECK(c, launch_cluster(fn, dim3(a.nh * ranks, a.B), dim3(256), tc::kSmem, st, ranks, args));
+        } else if (bf) {
+            if (gen) tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, true, false, false><<<grid, 256, tc::kSmem, st>>>(p);
+            else if (a.carry_in) tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, true, false><<<grid, 256, tc::kSmem, st>>>(p);
+            else tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, false, false><<<grid, 256, tc::kSmem, st>>>(p);
         } else {
-            if (gen) tc::m3_ssd_fwd_tc_kernel<__half, true, false><<<grid, 256, tc::kSmem, st>>>(p);
-            else if (a.carry_in) tc::m3_ssd_fwd_tc_kernel<__half, false, true><<<grid, 256, tc::kSmem, st>>>(p);
-            else tc::m3_ssd_fwd_tc_kernel<__half, false, false><<<grid, 256, tc::kSmem, st>>>(p);
+            if (gen) tc::m3_ssd_fwd_tc_kernel<__half, true, false, false><<<grid, 256, tc::kSmem, st>>>(p);
+            else if (a.carry_in) tc::m3_ssd_fwd_tc_kernel<__half, false, true, false><<<grid, 256, tc::kSmem, st>>>(p);
+            else tc::m3_ssd_fwd_tc_kernel<__half, false, false, false><<<grid, 256, tc::kSmem, st>>>(p);
         }
     } else {
         if (a.dtype == MAMBA_B200_F32) launch_seq<float>(p, c->sm_count, st);

@@ -325,6 +325,12 @@ __global__ void m3_bwd_finish_kernel(const M3BwdParams p) {
 //      3. dK = M1^T Q, U = V dS, dS += Q^T (E o dY)
 // Operands are rounded to the storage dtype (M1, M2, E o dY, the state copies),
 // so results carry 16-bit rounding like the forward's tensor-core path.
+//
+// SEG: the chunks of a (sample, head) are divided over the CTAs of a thread-block cluster, for shapes
+// with fewer (sample, head) pairs than SMs.  Every CTA first walks its chunks twice for the recurrences
+// alone, from zero: forward for the state (K, V), backward for its gradient (Q, dY), one product a chunk.
+// The CTAs then read one another's sums and decays through distributed shared memory, which gives each
+// the exact state entering its chunks and the exact gradient entering them from behind, and run A and B.
 namespace tcb {
 using namespace tc;
 
@@ -353,13 +359,16 @@ constexpr uint32_t kBar = kStage + 3 * kStageArr, kTmemSlot = kBar + 64, kSmem =
 static_assert(kSmem <= 227 * 1024, "shared memory");
 constexpr uint32_t c0 = 0, c1 = 128, c2 = 256, c3 = 384, cDS = 448, kTmemCols = 512;
 constexpr uint32_t kStateTile = NS * HD * 2;  // bytes of one 16-bit state copy
+// SEG: what a CTA leaves for the others, f32 [128 n][64 p] each, and log2 of the decay over its chunks
+constexpr uint32_t kLocS = kQ, kLocD = kM2, kTot = kTmemSlot + 8;
 
-template <typename Th>
+template <typename Th, bool SEG>
 __global__ void __launch_bounds__(256) m3_ssd_bwd_tc_kernel(const __grid_constant__ M3BwdParams p) {
     extern __shared__ __align__(1024) unsigned char smem[];
     // two threads per step: (row tid, half) share TMEM lane tid and split its columns
     const int tid = threadIdx.x & 127, half = threadIdx.x >> 7, warp = (threadIdx.x >> 5) & 3, lane = tid & 31;
-    const int h = blockIdx.x, b = blockIdx.y;
+    const int nrank = SEG ? static_cast<int>(gridDim.x) / p.nh : 1, rank = SEG ? blockIdx.x % nrank : 0;
+    const int h = SEG ? blockIdx.x / nrank : blockIdx.x, b = blockIdx.y;
     const int T = p.T, nh = p.nh;
     // headdim <= 64, d_state <= 128 (multiples of 8): full-size tiles, missing columns zero-filled
     const int hdv = p.hd, nsv = p.N;
@@ -399,6 +408,8 @@ __global__ void __launch_bounds__(256) m3_ssd_bwd_tc_kernel(const __grid_constan
     Th* dxg = static_cast<Th*>(p.dx);
     const float Dv = p.Dh[h];
     const int nc = (T + CS - 1) / CS;
+    const int per_rank = SEG ? (nc + nrank - 1) / nrank : nc;  // this CTA's chunks: c_lo .. c_hi - 1
+    const int c_lo = SEG ? min(nc, rank * per_rank) : 0, c_hi = SEG ? min(nc, c_lo + per_rank) : nc;
     unsigned char* ws_st = reinterpret_cast<unsigned char*>(p.ws_states) +
                            (static_cast<size_t>(b) * nh + h) * nc * kStateTile;
     uint32_t ph[4] = {0, 0, 0, 0};
@@ -489,59 +500,161 @@ __global__ void __launch_bounds__(256) m3_ssd_bwd_tc_kernel(const __grid_constan
         tfph[bi] ^= 1;
     };
 
-    // ---------------- A. forward: 16-bit copies of the entering states ----------------
-    // K and V of chunk c + 1 are requested while chunk c is worked on; the pass needs few tiles,
-    // so odd chunks simply use the tiles the backward pass calls M1 and S_in.
-    auto request_kv = [&](int c) {  // one thread
-        const int t0 = c * CS;
-        mbar_expect_tx(&bars[5 + (c & 1)], 2 * kSwSub + kSwSub);
-        load_qk((c & 1) ? kM1 : kK, &p.tm_k, t0, c & 1);
-        tma_load_4d(smem + ((c & 1) ? kSin : kV), &p.tm_x, &bars[5 + (c & 1)], 0, h, t0, b);
+    // weights (0 past the end) times this thread's half row of the tile at tV -> the tile at kDY
+    auto weigh = [&](uint32_t tV, uint32_t dst, float wt) {
+#pragma unroll
+        for (int j = half * (HD / 16); j < (half + 1) * (HD / 16); ++j) {
+            const uint4 v = *reinterpret_cast<const uint4*>(smem + tV + sw_chunk(tid, j));
+            uint32_t w4[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int q4 = 0; q4 < 4; ++q4) {
+                const float2 f = unpack2<Th>(w4[q4]);
+                w4[q4] = pack2<Th>(f.x * wt, f.y * wt);
+            }
+            *reinterpret_cast<uint4*>(smem + dst + sw_chunk(tid, j)) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
+        }
     };
-    if (threadIdx.x == 0 && nc > 1) {
-        issue_scalars_now(0);
-        request_kv(0);
+    auto copy16 = [&](unsigned char* dst, const float* sv) {  // this thread's half row of a state, rounded
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            *reinterpret_cast<uint4*>(dst + sw_chunk(tid, half * 4 + j)) =
+                make_uint4(pack2<Th>(sv[8 * j], sv[8 * j + 1]), pack2<Th>(sv[8 * j + 2], sv[8 * j + 3]),
+                           pack2<Th>(sv[8 * j + 4], sv[8 * j + 5]), pack2<Th>(sv[8 * j + 6], sv[8 * j + 7]));
+    };
+    // [n][p] (+)= sum_t A[t][n] (weighted)[t][p], the weighted rows at kDY; one thread
+    auto accumulate = [&](uint32_t tA, bool more) {
+        const uint32_t idS = instr_desc(fmt, 1, 1, 64);
+#pragma unroll
+        for (int k = 0; k < CS / 16; ++k)
+            mma(tmem + cDS, desc_sw_mn(sbase + tA, k), desc_sw_mn(sbase + kDY, k), idS, more || k > 0);
+        commit(&bars[3]);
+    };
+    // The tiles of the state passes: those of the next chunk are requested while a chunk is worked on; the
+    // passes need few tiles, so every second chunk simply uses the tiles the backward pass calls M1 and S_in.
+    auto request_pair = [&](int c, int j, const CUtensorMap* ma, const CUtensorMap* mv) {  // one thread
+        const int t0 = c * CS;
+        mbar_expect_tx(&bars[5 + (j & 1)], 2 * kSwSub + kSwSub);
+        load_qk((j & 1) ? kM1 : kK, ma, t0, j & 1);
+        tma_load_4d(smem + ((j & 1) ? kSin : kV), mv, &bars[5 + (j & 1)], 0, h, t0, b);
+    };
+
+    if constexpr (SEG) {
+        float tot = 0.0f;  // sum of dA over this CTA's chunks
+        // one recurrence over this CTA's chunks from zero, left in f32 at `dst`
+        auto local_pass = [&](auto back_tag, uint32_t dst) {
+            constexpr bool BACK = decltype(back_tag)::value;
+            const int n = c_hi - c_lo;
+            const CUtensorMap* ma = BACK ? &p.tm_q : &p.tm_k;
+            const CUtensorMap* mv = BACK ? &p.tm_dy : &p.tm_x;
+            auto chunk = [&](int j) { return BACK ? c_hi - 1 - j : c_lo + j; };
+            if (threadIdx.x == 0) {
+                issue_scalars_now(chunk(0) * CS);
+                request_pair(chunk(0), 0, ma, mv);
+            }
+            tot = 0.0f;
+            for (int j = 0; j < n; ++j) {
+                const int t0 = chunk(j) * CS, nv = min(CS, T - t0);
+                if (threadIdx.x == 0 && j + 1 < n) request_pair(chunk(j + 1), j + 1, ma, mv);
+                float run, g, sc;
+                load_scalars(t0, nv, run, g, sc);
+                if (threadIdx.x == 0 && j + 1 < n) issue_scalars_now(chunk(j + 1) * CS);
+                const float dA_end = dA[nv - 1];
+                const float wt = tid >= nv ? 0.0f : BACK ? ex2(run * kLog2e) : ex2((dA_end - run) * kLog2e) * sc;
+                tot += dA_end;
+                wait_tiles(j & 1);
+                weigh((j & 1) ? kSin : kV, kDY, wt);
+                if (j > 0) {
+                    const float e_end = ex2(dA_end * kLog2e);
+                    float sv[32];
+                    tmem_ld32(lane_addr + cDS + half * 32, sv);
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) sv[i] *= e_end;
+                    tmem_st32(lane_addr + cDS + half * 32, sv);
+                }
+                fence_proxy_async();
+                fence_before();
+                __syncthreads();
+                if (threadIdx.x == 0) {
+                    fence_after();
+                    accumulate((j & 1) ? kM1 : kK, j > 0);
+                }
+                wait_bar(3);
+            }
+            float sv[32];
+            tmem_ld32(lane_addr + cDS + half * 32, sv);
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                *reinterpret_cast<float4*>(smem + dst + tid * 256 + half * 128 + i * 16) =
+                    make_float4(sv[4 * i], sv[4 * i + 1], sv[4 * i + 2], sv[4 * i + 3]);
+            fence_before();
+            __syncthreads();  // read before the next product writes it
+            fence_after();
+        };
+        const bool some = c_lo < c_hi;
+        if (some && c_hi < nc) local_pass(std::false_type{}, kLocS);
+        if (some && c_lo > 0) local_pass(std::true_type{}, kLocD);
+        if (threadIdx.x == 0) *reinterpret_cast<float*>(smem + kTot) = tot * kLog2e;
+        cluster_sync();
+        // sum over the CTAs before (dir -1) or behind (dir 1) this one, each decayed by those in between
+        auto gather = [&](uint32_t loc, int dir, float* sv) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) sv[i] = 0.0f;
+            float between = 0.0f;
+            for (int q = rank + dir; q >= 0 && q * per_rank < nc && q < nrank; q += dir) {
+                const float f = ex2(between);
+                const uint32_t src = cluster_addr(sbase + loc + tid * 256 + half * 128, q);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const float4 v = ld_cluster4(src + i * 16);
+                    sv[4 * i] = fmaf(f, v.x, sv[4 * i]);
+                    sv[4 * i + 1] = fmaf(f, v.y, sv[4 * i + 1]);
+                    sv[4 * i + 2] = fmaf(f, v.z, sv[4 * i + 2]);
+                    sv[4 * i + 3] = fmaf(f, v.w, sv[4 * i + 3]);
+                }
+                between += ld_cluster1(cluster_addr(sbase + kTot, q));
+            }
+        };
+        if (some) {
+            float sv[32];
+            if (c_lo > 0) {
+                gather(kLocS, -1, sv);
+                tmem_st32(lane_addr + cDS + half * 32, sv);
+            }
+            if (c_hi < nc) {  // waits in columns that pass A leaves alone
+                gather(kLocD, 1, sv);
+                tmem_st32(lane_addr + c0 + half * 32, sv);
+            }
+        }
+        cluster_sync();  // nobody reads this CTA's shared memory any more
     }
-    for (int c = 0; c < nc; ++c) {
-        const int t0 = c * CS, nv = min(CS, T - t0);
-        const bool last = c + 1 == nc;
-        const uint32_t tKa = (c & 1) ? kM1 : kK, tVa = (c & 1) ? kSin : kV;
+
+    // ---------------- A. forward: 16-bit copies of the entering states ----------------
+    if (threadIdx.x == 0 && c_hi - c_lo > 1) {
+        issue_scalars_now(c_lo * CS);
+        request_pair(c_lo, 0, &p.tm_k, &p.tm_x);
+    }
+    for (int c = c_lo; c < c_hi; ++c) {
+        const int t0 = c * CS, nv = min(CS, T - t0), i0 = c - c_lo;
+        const bool last = c + 1 == c_hi;
         float run = 0.0f, g = 0.0f, s = 0.0f;
         if (!last) {
-            if (threadIdx.x == 0 && c + 2 < nc) request_kv(c + 1);  // its tiles were last read by chunk c - 1
+            // (tiles of chunk c + 1: last read by chunk c - 1)
+            if (threadIdx.x == 0 && c + 2 < c_hi) request_pair(c + 1, i0 + 1, &p.tm_k, &p.tm_x);
             load_scalars(t0, nv, run, g, s);
-            if (threadIdx.x == 0 && c + 2 < nc) issue_scalars_now(t0 + CS);  // the staging was read just above
-            const float dA_end = dA[nv - 1];
-            const float wt = tid < nv ? ex2((dA_end - run) * kLog2e) * s : 0.0f;
-            wait_tiles(c & 1);
-#pragma unroll
-            for (int j = half * (HD / 16); j < (half + 1) * (HD / 16); ++j) {
-                const uint4 v = *reinterpret_cast<const uint4*>(smem + tVa + sw_chunk(tid, j));
-                uint32_t w4[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-                for (int q4 = 0; q4 < 4; ++q4) {
-                    const float2 f = unpack2<Th>(w4[q4]);
-                    w4[q4] = pack2<Th>(f.x * wt, f.y * wt);
-                }
-                *reinterpret_cast<uint4*>(smem + kDY + sw_chunk(tid, j)) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
-            }
+            if (threadIdx.x == 0 && c + 2 < c_hi) issue_scalars_now(t0 + CS);  // the staging was read just above
+            const float wt = tid < nv ? ex2((dA[nv - 1] - run) * kLog2e) * s : 0.0f;
+            wait_tiles(i0 & 1);
+            weigh((i0 & 1) ? kSin : kV, kDY, wt);
         }
         if (c > 0) {  // state entering chunk c: copy out, then decay for the update
             const float e_end = last ? 0.0f : ex2(dA[nv - 1] * kLog2e);
-            {
-                const int q2 = half;
-                float sv[32];
-                tmem_ld32(lane_addr + cDS + q2 * 32, sv);
+            float sv[32];
+            tmem_ld32(lane_addr + cDS + half * 32, sv);
+            copy16(ws_st + static_cast<size_t>(c) * kStateTile, sv);
+            if (!last) {
 #pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    *reinterpret_cast<uint4*>(ws_st + static_cast<size_t>(c) * kStateTile + sw_chunk(tid, q2 * 4 + j)) =
-                        make_uint4(pack2<Th>(sv[8 * j], sv[8 * j + 1]), pack2<Th>(sv[8 * j + 2], sv[8 * j + 3]),
-                                   pack2<Th>(sv[8 * j + 4], sv[8 * j + 5]), pack2<Th>(sv[8 * j + 6], sv[8 * j + 7]));
-                if (!last) {
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) sv[i] *= e_end;
-                    tmem_st32(lane_addr + cDS + q2 * 32, sv);
-                }
+                for (int i = 0; i < 32; ++i) sv[i] *= e_end;
+                tmem_st32(lane_addr + cDS + half * 32, sv);
             }
         }
         if (last) break;
@@ -550,11 +663,7 @@ __global__ void __launch_bounds__(256) m3_ssd_bwd_tc_kernel(const __grid_constan
         __syncthreads();
         if (threadIdx.x == 0) {
             fence_after();
-            const uint32_t idS = instr_desc(fmt, 1, 1, 64);
-#pragma unroll
-            for (int k = 0; k < CS / 16; ++k)  // S^T[n][p] += sum_t K[t][n] (w V)[t][p]
-                mma(tmem + cDS, desc_sw_mn(sbase + tKa, k), desc_sw_mn(sbase + kDY, k), idS, c > 0 || k > 0);
-            commit(&bars[3]);
+            accumulate((i0 & 1) ? kM1 : kK, c > 0);  // S^T[n][p] += sum_t K[t][n] (w V)[t][p]
         }
         wait_bar(3);
     }
@@ -567,6 +676,13 @@ __global__ void __launch_bounds__(256) m3_ssd_bwd_tc_kernel(const __grid_constan
     // ---------------- B. backward over the chunks ----------------
     bool has_ds = false;
     float dD_acc = 0.0f;
+    if (SEG && c_lo < c_hi && c_hi < nc) {  // the gradient from the CTAs behind this one
+        float sv[32];
+        tmem_ld32(lane_addr + c0 + half * 32, sv);
+        tmem_st32(lane_addr + cDS + half * 32, sv);
+        copy16(smem + kDS, sv);  // (published by the fence and barrier ahead of the first products)
+        has_ds = true;
+    }
     // The tiles of a chunk are requested while the previous chunk's last epilogue runs: as soon
     // as its last MMA group is done, Q and K of the next chunk go where this chunk's M1 and M2
     // were (the two pairs of tiles swap places every chunk, so nothing is double-buffered), V, dY
@@ -581,8 +697,8 @@ __global__ void __launch_bounds__(256) m3_ssd_bwd_tc_kernel(const __grid_constan
         tma_load_4d(smem + kDY, &p.tm_dy, &bars[5], 0, h, t0, b);
         if (c > 0) bulk_load(smem + kSin, ws_st + static_cast<size_t>(c) * kStateTile, kStateTile, &bars[5]);
     };
-    if (threadIdx.x == 0 && nc > 0) request_tiles(nc - 1, kQ, kK);
-    for (int c = nc - 1, it = 0; c >= 0; --c, ++it) {
+    if (threadIdx.x == 0 && c_lo < c_hi) request_tiles(c_hi - 1, kQ, kK);
+    for (int c = c_hi - 1, it = 0; c >= c_lo; --c, ++it) {
         const bool par = (it & 1) != 0;
         const uint32_t tQ = par ? kM1 : kQ, tK = par ? kM2 : kK, tM1 = par ? kQ : kM1, tM2 = par ? kK : kM2;
         const int t0 = c * CS, nv = min(CS, T - t0);
@@ -598,18 +714,7 @@ __global__ void __launch_bounds__(256) m3_ssd_bwd_tc_kernel(const __grid_constan
         const long long qk_row = ((static_cast<long long>(b) * T + t) * nh + h) * nsv;
         const long long x_row = (static_cast<long long>(b) * T + t) * nh * hdv + h * hdv;
         wait_tiles(0);
-        // E o dY from the landed dY tile (own row, own half of the columns)
-#pragma unroll
-        for (int j = half * (HD / 16); j < (half + 1) * (HD / 16); ++j) {
-            const uint4 dyv = *reinterpret_cast<const uint4*>(smem + kDY + sw_chunk(tid, j));
-            uint32_t w4[4] = {dyv.x, dyv.y, dyv.z, dyv.w};
-#pragma unroll
-            for (int q4 = 0; q4 < 4; ++q4) {
-                const float2 f = unpack2<Th>(w4[q4]);
-                w4[q4] = pack2<Th>(f.x * e_t, f.y * e_t);
-            }
-            *reinterpret_cast<uint4*>(smem + kEdY + sw_chunk(tid, j)) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
-        }
+        weigh(kDY, kEdY, e_t);  // E o dY
         fence_proxy_async();
         fence_before();
         __syncthreads();
@@ -862,20 +967,13 @@ __global__ void __launch_bounds__(256) m3_ssd_bwd_tc_kernel(const __grid_constan
             commit(&bars[2]);
         }
         wait_bar(2);
-        if (threadIdx.x == 0 && c > 0) request_tiles(c - 1, tM1, tM2);
+        if (threadIdx.x == 0 && c > c_lo) request_tiles(c - 1, tM1, tM2);
         // ---- epilogue 3 ----
         // 16-bit copy of the new dS for the next (earlier) chunk
-        if (c > 0) {
-            {
-                const int q2 = half;
-                float sv[32];
-                tmem_ld32(lane_addr + cDS + q2 * 32, sv);
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    *reinterpret_cast<uint4*>(smem + kDS + sw_chunk(tid, q2 * 4 + j)) =
-                        make_uint4(pack2<Th>(sv[8 * j], sv[8 * j + 1]), pack2<Th>(sv[8 * j + 2], sv[8 * j + 3]),
-                                   pack2<Th>(sv[8 * j + 4], sv[8 * j + 5]), pack2<Th>(sv[8 * j + 6], sv[8 * j + 7]));
-            }
+        if (c > c_lo) {
+            float sv[32];
+            tmem_ld32(lane_addr + cDS + half * 32, sv);
+            copy16(smem + kDS, sv);
         }
         // The proxy fence this copy needs comes before the dK rows are stored: a fence waits for
         // the thread's outstanding global stores, and stored after it the 64 KB of dK drain
@@ -952,8 +1050,15 @@ __global__ void __launch_bounds__(256) m3_ssd_bwd_tc_kernel(const __grid_constan
         fence_after();
     }
     {
-        const float tot = block_sum(half == 0 ? dD_acc : 0.0f);
-        if (threadIdx.x == 0) p.ws_dD[static_cast<long long>(b) * nh + h] = tot;
+        float tot = block_sum(half == 0 ? dD_acc : 0.0f);
+        if constexpr (SEG) {
+            if (threadIdx.x == 0) *reinterpret_cast<float*>(smem + kTot) = tot;
+            cluster_sync();
+            if (rank == 0)
+                for (int q = 1; q < nrank; ++q) tot += ld_cluster1(cluster_addr(sbase + kTot, q));
+            cluster_sync();
+        }
+        if (threadIdx.x == 0 && rank == 0) p.ws_dD[static_cast<long long>(b) * nh + h] = tot;
     }
     __syncthreads();
     if (threadIdx.x < 32)
@@ -994,10 +1099,12 @@ int m3_bwd_configure(Ctx* c) {
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     MB200_CUDA_CHECK(c, cudaFuncSetAttribute(reinterpret_cast<const void*>(m3_ssd_bwd_kernel<__nv_bfloat16>),
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    MB200_CUDA_CHECK(c, cudaFuncSetAttribute(reinterpret_cast<const void*>(tcb::m3_ssd_bwd_tc_kernel<__half>),
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, tcb::kSmem));
-    MB200_CUDA_CHECK(c, cudaFuncSetAttribute(reinterpret_cast<const void*>(tcb::m3_ssd_bwd_tc_kernel<__nv_bfloat16>),
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, tcb::kSmem));
+    const void* tc_fns[4] = {reinterpret_cast<const void*>(tcb::m3_ssd_bwd_tc_kernel<__half, false>),
+                             reinterpret_cast<const void*>(tcb::m3_ssd_bwd_tc_kernel<__nv_bfloat16, false>),
+                             reinterpret_cast<const void*>(tcb::m3_ssd_bwd_tc_kernel<__half, true>),
+                             reinterpret_cast<const void*>(tcb::m3_ssd_bwd_tc_kernel<__nv_bfloat16, true>)};
+    for (const void* fn : tc_fns)
+        MB200_CUDA_CHECK(c, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, tcb::kSmem));
     return MAMBA_B200_OK;
 }
 
@@ -1073,8 +1180,20 @@ extern "C" MAMBA_B200_API int mamba_b200_m3_ssd_bwd(void* handle, void* stream,
                    make_tmap_3d(c, &p.tm_adt, MAMBA_B200_F32, a.adt, a.nh, a.nh, a.T, a.B, 4, 129) &&
                    make_tmap_3d(c, &p.tm_dt, MAMBA_B200_F32, a.dt, a.nh, a.nh, a.T, a.B, 4, 129) &&
                    make_tmap_3d(c, &p.tm_trap, MAMBA_B200_F32, a.trap, a.nh, a.nh, a.T, a.B, 4, 129);
-        if (a.dtype == MAMBA_B200_F16) tcb::m3_ssd_bwd_tc_kernel<__half><<<grid, 256, tcb::kSmem, st>>>(p);
-        else tcb::m3_ssd_bwd_tc_kernel<__nv_bfloat16><<<grid, 256, tcb::kSmem, st>>>(p);
+        const bool f16 = a.dtype == MAMBA_B200_F16;
+        // (the outer CTAs of a cluster have one pass more than an undivided one, those between them two.)  bf16,
+        // 64 x 128: 4 heads x 4096 steps 114 us (one CTA each: 446), 24 x 2048 104 (224), 64 x 4096 285 (450)
+        const int ranks = m3_cluster_ranks(a.B * a.nh, (a.T + tcb::CS - 1) / tcb::CS, 14.1, 17.0, 19.5, 5.0);
+        if (ranks > 1) {
+            const void* fn = f16 ? reinterpret_cast<const void*>(tcb::m3_ssd_bwd_tc_kernel<__half, true>)
+                                 : reinterpret_cast<const void*>(tcb::m3_ssd_bwd_tc_kernel<__nv_bfloat16, true>);
+            void* args[1] = {&p};
+            MB200_CUDA_CHECK(c, launch_cluster(fn, dim3(a.nh * ranks, a.B), dim3(256), tcb::kSmem, st, ranks, args));
+        } else if (f16) {
+            tcb::m3_ssd_bwd_tc_kernel<__half, false><<<grid, 256, tcb::kSmem, st>>>(p);
+        } else {
+            tcb::m3_ssd_bwd_tc_kernel<__nv_bfloat16, false><<<grid, 256, tcb::kSmem, st>>>(p);
+        }
     } else if (a.dtype == MAMBA_B200_F32) m3_ssd_bwd_kernel<float><<<grid, 256, smem, st>>>(p);
     else if (a.dtype == MAMBA_B200_F16) m3_ssd_bwd_kernel<__half><<<grid, 256, smem, st>>>(p);
     else m3_ssd_bwd_kernel<__nv_bfloat16><<<grid, 256, smem, st>>>(p);

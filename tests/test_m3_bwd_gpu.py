@@ -71,6 +71,18 @@ def test_tensor_core_path_matches_cuda_core_path_at_model_size(cuda_dev):
         assert rel_err(tcg[k], ccg[k]) <= TOL["bf16"], k
 
 
+# few (sample, head) pairs: the chunks are divided over the CTAs of a cluster; ranks left without chunks, a last
+# chunk of one step, ranks of one and of several chunks
+@pytest.mark.parametrize("dt", ["bf16", "f16"])
+@pytest.mark.parametrize("shape", [(1, 640, 3, 64, 128), (2, 1153, 2, 32, 64), (1, 1290, 4, 64, 128), (2, 2048, 18, 64, 128)],
+                         ids=lambda s: "B%dT%dnh%dhd%dN%d" % s)
+def test_chunks_divided_over_a_cluster_match_cuda_core_path(cuda_dev, shape, dt):
+    i, dy = case(shape, dt, seed=shape[1])
+    got, ref = run_gpu(i, dy, dt, cuda_dev), run_gpu(i, dy, "f32", cuda_dev)
+    for k in ("dx",) + F32_OUT:
+        assert rel_err(got[k], ref[k]) <= TOL[dt], k
+
+
 def test_dD_accumulates_and_rerun_is_identical(cuda_dev):
     import torch
     i, dy = case((2, 70, 2, 16, 32), "f32", seed=9)

@@ -186,3 +186,32 @@ def test_windows_of_a_stream_carry_state(cuda_dev, shape, dt):
     assert rel_err(ssm.cpu().numpy(), whole["ssm_state"]) <= 1e-4
     np.testing.assert_array_equal(ks.cpu().numpy(), whole["k_state"])
     np.testing.assert_array_equal(vs.cpu().numpy(), whole["v_state"])
+
+
+# few (sample, head) pairs: the chunks are divided over the CTAs of a cluster; fewer chunks than ranks, ranks
+# left without chunks, a last chunk of one step
+CLUSTER_SHAPES = [(1, 257, 1, 64, 128), (1, 640, 3, 64, 128), (2, 1153, 2, 32, 64), (1, 1290, 4, 64, 128),
+                  (2, 2048, 37, 64, 128)]
+
+
+@pytest.mark.parametrize("carry", [False, True])
+@pytest.mark.parametrize("shape", CLUSTER_SHAPES, ids=lambda s: "B%dT%dnh%dhd%dN%d" % s)
+def test_chunks_divided_over_a_cluster_match_sequential(cuda_dev, shape, carry):
+    import torch
+
+    import mamba_rs_b200 as mb
+    i = rounded(synth.m3_ssd_inputs(*shape, seed=shape[1]), "bf16")
+    B, T, nh, hd, N = shape
+    g = torch.Generator().manual_seed(T)
+    st0 = [torch.randn(*s, generator=g).to(cuda_dev) for s in ((B, nh, hd, N), (B, nh, N), (B, nh, hd))]
+    args = [to_dev(i[k], cuda_dev, torch.bfloat16 if k in ("x", "K", "Q") else None) for k in ARGS]
+    out = []
+    for seq in (False, True):
+        ssm, ks, vs = (t.clone() for t in st0)
+        y = mb.m3_ssd_fwd(*args, ssm_state=ssm, k_state=ks, v_state=vs, carry_in=carry, force_sequential=seq)
+        out.append([t.float().cpu().numpy() for t in (y, ssm, ks, vs)])
+    mb.ffi.default_handle(0).check_status()
+    assert rel_err(out[0][0], out[1][0]) <= TOL["bf16"]
+    assert rel_err(out[0][1], out[1][1]) <= (1e-4 if carry else TOL["bf16"])
+    np.testing.assert_array_equal(out[0][2], out[1][2])
+    np.testing.assert_array_equal(out[0][3], out[1][3])
