@@ -28,8 +28,8 @@
 //   take the weights as the M side of mma.sync m16n8k16 (a tile of x beside its tile of z) with eight
 //   sequences as N, so a warp issues about 900 instructions a layer where it issued 2,800.
 // Loops stay rolled: code that outgrows the instruction cache takes longer than it saves.  Measured
-// (before: the same split with four barriers): 0.295 ms a token of the 130m architecture at batch 8
-// (0.336), of which 0.025 are the head; 33 us a step of three layers of d_model 128 (38).
+// (before: the same split with four barriers): 0.286 ms a token of the 130m architecture at batch 8
+// (0.336), of which 0.025 are the head; 30 us a step of three layers of d_model 128 (38).
 // Arithmetic: mma.sync for 16-bit storage (tcgen05's 128-row tiles would be mostly padding at these
 // batch sizes and the products are not what takes the time), FMA for f32.  Sums are f32 in a fixed
 // order: two runs are bit-identical.
@@ -45,7 +45,7 @@ namespace dec {
 
 constexpr int kThreads = 512, kWarps = 16;  // compute threads; one more warp asks for the operands
 constexpr int kN = 16, kK = 4;          // d_state and d_conv of this kernel
-constexpr int kMaxDm = 1024, kMaxB = 64, kMaxKSlice = 192, kMaxKs = 8;
+constexpr int kMaxDm = 1024, kMaxB = 64, kMaxKSlice = 384, kMaxKs = 4;
 constexpr int kMaxPolls = 1 << 21;      // a poll is about a microsecond's L2 round trip
 
 struct Params {
@@ -73,8 +73,8 @@ struct Params {
     int t1, c1, kp1, ka1, br1;
     int t4, c4, kp4, ka4, br4;
     int ncg, ks, kslice, nch;           // x_proj: column groups, K slices; channels per CTA
-    int brd, x_tma, dt_tma;             // rows of a W_dt box; whether W_x, W_dt come by TMA
-    uint32_t s_w1, s_w4, s_act, s_red, s_wx, s_wd, s_norm, s_conv, s_uz;
+    int brx, brd, x_tma, dt_tma;        // rows of a W_x and a W_dt box; whether the two come by TMA
+    uint32_t s_w1, s_w4, s_act, s_red, s_wx, s_wd, s_norm, s_conv, s_uz, s_a;
     int* status;
 };
 
@@ -85,7 +85,6 @@ __device__ __forceinline__ void cp4(uint32_t dst, const void* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-__device__ __forceinline__ void l2_prefetch(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 __device__ __forceinline__ void ldmatrix_x4(uint32_t addr, uint32_t* r) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
@@ -236,34 +235,36 @@ struct Step {
     __device__ void ask_x(int l) {
         if (lane == 0) {
             mbar_expect_tx(&bars[kWX], static_cast<uint32_t>(p.kslice) * 8 * sizeof(Tact));
-            tma_load_3d(sm + p.s_wx, &p.tm_x, &bars[kWX], unit0() % p.ncg * 8, unit0() / p.ncg * p.kslice, l);
+            for (int k = 0; k < p.kslice; k += p.brx)
+                tma_load_3d(sm + p.s_wx + k * 8 * sizeof(Tact), &p.tm_x, &bars[kWX], unit0() % p.ncg * 8, unit0() / p.ncg * p.kslice + k, l);
         }
     }
-    // norm weights; conv windows [B][channels], taps and bias; W_dt's columns
+    // norm weights; conv windows [B][channels], taps and bias; W_dt's columns; A, D and dt's bias of the channels
     __device__ void ask_small(int l) {
         const int n = channels(), d0 = cta * p.nch, db = (p.dr + p.brd - 1) / p.brd;
         unsigned char* cv = sm + p.s_conv;
         if (lane == 0)
-            mbar_expect_tx(&bars[kSmall], p.dm * 4 + (p.B + 1) * n * 16 + n * 4 +
+            mbar_expect_tx(&bars[kSmall], p.dm * 4 + (p.B + 1) * n * 16 + n * (4 + kN * 4 + 4 + static_cast<int>(sizeof(Tact))) +
                                               (p.dt_tma ? db * p.brd * p.nch * static_cast<int>(sizeof(Tact)) : 0));
         __syncwarp();
         if (lane == 0) bulk_load(sm + p.s_norm, mf(l, 0), p.dm * 4, &bars[kSmall]);
         if (lane == 1) bulk_load(cv + p.B * p.nch * 16, mf(l, p.o_cw) + d0 * kK, n * 16, &bars[kSmall]);
         if (lane == 2) bulk_load(cv + (p.B + 1) * p.nch * 16, mf(l, p.o_cb) + d0, n * 4, &bars[kSmall]);
+        unsigned char* am = sm + p.s_a;
+        if (lane == 3) bulk_load(am, p.a_neg + (static_cast<long long>(l) * p.di + d0) * kN, n * kN * 4, &bars[kSmall]);
+        if (lane == 4) bulk_load(am + p.nch * kN * 4, mf(l, p.o_D) + d0, n * 4, &bars[kSmall]);
+        if (lane == 5) bulk_load(am + p.nch * (kN + 1) * 4, lp(l, p.o_dtb) + d0, n * sizeof(Tact), &bars[kSmall]);
         for (int b = lane; b < p.B; b += 32)
             bulk_load(cv + b * p.nch * 16, p.conv + ((static_cast<long long>(l) * p.Bcap + b) * p.di + d0) * kK, n * 16, &bars[kSmall]);
         if (p.dt_tma && lane < db)
             tma_load_3d(sm + p.s_wd + lane * p.brd * p.nch * sizeof(Tact), &p.tm_dt, &bars[kSmall], d0, lane * p.brd, l);
     }
-    // what the scan of layer l loads itself, into L2
+    // the states of layer l, which the scan loads itself, into L2
     __device__ void hint(int l) {
         const int ch0 = cta * p.nch, n = channels();
         if (l >= p.L || n <= 0) return;
         for (int b = lane; b < p.B; b += 32)
             l2_prefetch_bulk(p.ssm + ((static_cast<long long>(l) * p.Bcap + b) * p.di + ch0) * kN, n * kN * 4);
-        if (lane == 0) l2_prefetch_bulk(p.a_neg + (static_cast<long long>(l) * p.di + ch0) * kN, n * kN * 4);
-        if (lane == 1) l2_prefetch(mf(l, p.o_D) + ch0);
-        if (lane == 2) l2_prefetch(lp(l, p.o_dtb) + ch0);
     }
     __device__ void ask_in(int l) { ask_tiles(&p.tm_in, kWIn, p.s_w1, l, cta * p.t1, p.t1, 2, p.c1, p.ka1, p.br1); }
     __device__ void ask_out(int l) { ask_tiles(&p.tm_out, kWOut, p.s_w4, l, out_tile(), p.t4, 1, p.c4, p.ka4, p.br4); }
@@ -388,7 +389,7 @@ struct Step {
     // ---- out[b][column] = act W for n <= PP pairs of column tiles; pair i is tile a0 + i * da and tile b0 + i * db
     //      of the CTA's (the second clamped to the last one there is).  The warps split K; partials in s_red. ----
     static constexpr int RP = H ? 160 : 32;  // floats of a part: [8 rows, 20 apart][16 columns] / [8 rows][4 columns]
-    __device__ static int parts_log(int n) { return H ? (n > 2 ? 2 : n > 1 ? 3 : 4) : 4; }  // log2 of the K parts
+    __device__ static int parts_log(int n) { return H ? (n > 2 ? 2 : n > 1 ? 3 : 4) : n > 1 ? 2 : 3; }  // log2 of the K parts
     __device__ void project(uint32_t wofs, int kp, int ka, int cw, int ta, int da, int tb, int db, int last, int n, int rows) {
         float* red = reinterpret_cast<float*>(sm + p.s_red);
         const int ld = kp + TW;
@@ -401,67 +402,79 @@ struct Step {
             uint32_t arow = smem_u32(sm + wofs) + static_cast<uint32_t>((q * ka + kr + part * 32) * cw + tile - q * cw) * 16;
             uint32_t brow = smem_u32(sm + p.s_act) + (min(lane & 7, rows - 1) * ld + (lane >> 3) * 8 + part * 32) * 2;
             const uint32_t brow2 = (min(8 + (lane & 7), rows - 1) - min(lane & 7, rows - 1)) * ld * 2;
-            float c[2][4];
+            float c[4][4];  // two accumulators for each group of eight rows
 #pragma unroll
-            for (int e = 0; e < 4; ++e) c[0][e] = c[1][e] = 0.0f;
+            for (int e = 0; e < 4; ++e) c[0][e] = c[1][e] = c[2][e] = c[3][e] = 0.0f;
             const uint32_t ahalf = 256 * cw, astep = (512u * cw) << lg, bstep = 64u << lg;
-#pragma unroll 2
-            for (int u = part; u < kp / 32; u += 1 << lg, arow += astep, brow += bstep) {
-                uint32_t a0[4], a1[4], b[4];
-                ldmatrix_x4_trans(arow, a0);
-                ldmatrix_x4_trans(arow + ahalf, a1);
-                ldmatrix_x4(brow, b);
-                mma16816<Tact>(c[0], a0[0], a0[1], a0[2], a0[3], b[0], b[1]);
-                mma16816<Tact>(c[0], a1[0], a1[1], a1[2], a1[3], b[2], b[3]);
+            const int units = kp / 32;
+            // three units of 32 at a time, all their loads ahead of the products
+#pragma unroll 1
+            for (int u = part; u < units; u += 3 << lg, arow += 3 * astep, brow += 3 * bstep) {
+                uint32_t a[3][8], b[3][4];
+                const int m = min(3, (units - u + (1 << lg) - 1) >> lg);
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    const uint32_t o = k < m ? k : 0;
+                    ldmatrix_x4_trans(arow + o * astep, a[k]);
+                    ldmatrix_x4_trans(arow + o * astep + ahalf, a[k] + 4);
+                    ldmatrix_x4(brow + o * bstep, b[k]);
+                }
+#pragma unroll
+                for (int k = 0; k < 3; ++k)
+                    if (k < m) {
+                        mma16816<Tact>(c[0], a[k][0], a[k][1], a[k][2], a[k][3], b[k][0], b[k][1]);
+                        mma16816<Tact>(c[1], a[k][4], a[k][5], a[k][6], a[k][7], b[k][2], b[k][3]);
+                    }
                 if (groups == 2) {
-                    ldmatrix_x4(brow + brow2, b);
-                    mma16816<Tact>(c[1], a0[0], a0[1], a0[2], a0[3], b[0], b[1]);
-                    mma16816<Tact>(c[1], a1[0], a1[1], a1[2], a1[3], b[2], b[3]);
+#pragma unroll
+                    for (int k = 0; k < 3; ++k)
+                        if (k < m) {
+                            ldmatrix_x4(brow + brow2 + k * bstep, b[k]);
+                            mma16816<Tact>(c[2], a[k][0], a[k][1], a[k][2], a[k][3], b[k][0], b[k][1]);
+                            mma16816<Tact>(c[3], a[k][4], a[k][5], a[k][6], a[k][7], b[k][2], b[k][3]);
+                        }
                 }
             }
             float* o = red + warp * (2 * RP) + (lane & 3) * 40 + (lane >> 2);
-            o[0] = c[0][0]; o[20] = c[0][1]; o[8] = c[0][2]; o[28] = c[0][3];
-            if (groups == 2) { o[RP] = c[1][0]; o[RP + 20] = c[1][1]; o[RP + 8] = c[1][2]; o[RP + 28] = c[1][3]; }
+            o[0] = c[0][0] + c[1][0]; o[20] = c[0][1] + c[1][1]; o[8] = c[0][2] + c[1][2]; o[28] = c[0][3] + c[1][3];
+            if (groups == 2) {
+                o += RP;
+                o[0] = c[2][0] + c[3][0]; o[20] = c[2][1] + c[3][1]; o[8] = c[2][2] + c[3][2]; o[28] = c[2][3] + c[3][3];
+            }
         } else {
             const float* act = reinterpret_cast<const float*>(sm + p.s_act);
-#pragma unroll 1
-            for (int t = 0; t < 2 * n; ++t) {
-                float acc[32];
+            // a warp has one tile and a part of K
+            const int lg = parts_log(n), t = warp >> lg, part = warp & ((1 << lg) - 1);
+            float acc[32];
 #pragma unroll
-                for (int i = 0; i < 32; ++i) acc[i] = 0.0f;
-                const int tile = (t & 1) ? min(tb + (t >> 1) * db, last) : ta + (t >> 1) * da, q = tile / cw;
-                const float4* w = reinterpret_cast<const float4*>(sm + wofs) + q * ka * cw + (tile - q * cw);
+            for (int i = 0; i < 32; ++i) acc[i] = 0.0f;
+            const int tile = (t & 1) ? min(tb + (t >> 1) * db, last) : ta + (t >> 1) * da, q = tile / cw;
+            const float4* w = reinterpret_cast<const float4*>(sm + wofs) + q * ka * cw + (tile - q * cw);
 #pragma unroll 1
-                for (int k = tid; k < kp; k += kThreads) {
-                    const float4 wv = w[k * cw];
+            for (int k = part * 32 + lane; k < kp; k += 32 << lg) {
+                const float4 wv = w[k * cw];
 #pragma unroll
-                    for (int b = 0; b < 8; ++b) {
-                        if (b >= rows) break;
-                        const float a = act[b * ld + k];
-                        acc[4 * b] = fmaf(a, wv.x, acc[4 * b]);
-                        acc[4 * b + 1] = fmaf(a, wv.y, acc[4 * b + 1]);
-                        acc[4 * b + 2] = fmaf(a, wv.z, acc[4 * b + 2]);
-                        acc[4 * b + 3] = fmaf(a, wv.w, acc[4 * b + 3]);
-                    }
+                for (int b = 0; b < 8; ++b) {
+                    const float a = act[min(b, rows - 1) * ld + k];
+                    acc[4 * b] = fmaf(a, wv.x, acc[4 * b]);
+                    acc[4 * b + 1] = fmaf(a, wv.y, acc[4 * b + 1]);
+                    acc[4 * b + 2] = fmaf(a, wv.z, acc[4 * b + 2]);
+                    acc[4 * b + 3] = fmaf(a, wv.w, acc[4 * b + 3]);
                 }
-                red[(warp * 4 + t) * RP + lane] = sum32(acc, lane);
             }
+            red[warp * RP + lane] = sum32(acc, lane);
         }
     }
     // the sum of output (pair i, second: column c of its second tile, row b)
     __device__ float total(int n, int i, bool second, int b, int c) const {
         const float* o = reinterpret_cast<const float*>(sm + p.s_red);
-        float s = 0.0f;
-        if constexpr (H) {
-            const int lg = parts_log(n);
-            o += (i << lg) * (2 * RP) + (b >> 3) * RP + (b & 7) * 20 + (second ? 8 : 0) + c;
-#pragma unroll 1
-            for (int q = 0; q < 1 << lg; q += 4, o += 8 * RP) s = (((s + o[0]) + o[2 * RP]) + o[4 * RP]) + o[6 * RP];
-        } else {
-            o += (2 * i + (second ? 1 : 0)) * RP + b * 4 + c;
-#pragma unroll
-            for (int q = 0; q < kWarps; ++q) s += o[q * 4 * RP];
-        }
+        const int lg = parts_log(n);
+        constexpr int D = H ? 2 * RP : RP;  // from part to part
+        if constexpr (H) o += (i << lg) * D + (b >> 3) * RP + (b & 7) * 20 + (second ? 8 : 0) + c;
+        else o += ((2 * i + (second ? 1 : 0)) << lg) * D + b * 4 + c;
+        float s = (o[0] + o[D]) + (o[2 * D] + o[3 * D]);
+        if (lg >= 3) s += (o[4 * D] + o[5 * D]) + (o[6 * D] + o[7 * D]);
+        if (lg >= 4) s += ((o[8 * D] + o[9 * D]) + (o[10 * D] + o[11 * D])) + ((o[12 * D] + o[13 * D]) + (o[14 * D] + o[15 * D]));
         return s;
     }
     // rows of a pass as a power of two: 8 or 16
@@ -549,7 +562,7 @@ struct Step {
 #pragma unroll 1
             for (int b0 = 0; b0 < p.B; b0 += BT) {
                 const int bt = min(BT, p.B - b0);
-                constexpr int CH = H ? 32 : 64, N = H ? 2 : 2;  // threads a row, packets a thread
+                constexpr int CH = H ? 32 : 64, N = 3;  // threads a row, packets a thread
                 static_assert(CH * N * 2 * E >= kMaxKSlice && kThreads / CH >= (H ? 16 : 8), "slice");
                 const int b = tid / CH, j = tid % CH, nj = p.kslice / (2 * E), have = min(nj, (p.di - k0) / (2 * E));
                 if (b < bt) {
@@ -568,18 +581,23 @@ struct Step {
                 float* red = reinterpret_cast<float*>(sm + p.s_red);
                 if constexpr (H) {
                     const int steps = p.kslice / 16, groups = bt > 8 ? 2 : 1;
-                    static_assert(kMaxKSlice / 16 <= kWarps, "a K step per warp");
+                    static_assert(kMaxKSlice / 16 <= 2 * kWarps, "two K steps a warp");
                     if (warp < steps) {
-                        uint32_t a[4], bb[4];
                         float c[2][4];
 #pragma unroll
                         for (int e = 0; e < 4; ++e) c[0][e] = c[1][e] = 0.0f;
                         // (the second tile of the pair is the first one again, its sums go nowhere)
-                        ldmatrix_x4_trans(smem_u32(sm + p.s_wx) + (warp * 16 + (lane & 7) + ((lane & 16) >> 1)) * 16, a);
+                        uint32_t arow = smem_u32(sm + p.s_wx) + (warp * 16 + (lane & 7) + ((lane & 16) >> 1)) * 16;
                         // matrices: rows 0-7 of K 0-7, 8-15, then rows 8-15
-                        ldmatrix_x4(smem_u32(us) + (min((lane & 7) + ((lane & 16) >> 1), bt - 1) * uld + warp * 16 + (lane & 8)) * 2, bb);
-                        mma16816<Tact>(c[0], a[0], a[1], a[2], a[3], bb[0], bb[1]);
-                        if (groups == 2) mma16816<Tact>(c[1], a[0], a[1], a[2], a[3], bb[2], bb[3]);
+                        uint32_t brow = smem_u32(us) + (min((lane & 7) + ((lane & 16) >> 1), bt - 1) * uld + warp * 16 + (lane & 8)) * 2;
+#pragma unroll 1
+                        for (int k = warp; k < steps; k += kWarps, arow += kWarps * 256, brow += kWarps * 32) {
+                            uint32_t a[4], bb[4];
+                            ldmatrix_x4_trans(arow, a);
+                            ldmatrix_x4(brow, bb);
+                            mma16816<Tact>(c[0], a[0], a[1], a[2], a[3], bb[0], bb[1]);
+                            if (groups == 2) mma16816<Tact>(c[1], a[0], a[1], a[2], a[3], bb[2], bb[3]);
+                        }
                         float* o = red + warp * 128 + (lane & 3) * 16 + (lane >> 2);
                         o[0] = c[0][0]; o[8] = c[0][1];
                         if (groups == 2) { o[64] = c[1][0]; o[72] = c[1][1]; }
@@ -587,9 +605,11 @@ struct Step {
                     sync();
                     if (b0 + BT >= p.B && unit == unit0()) release(kWX);
                     if (tid < 8 * bt) {
-                        float sum = red[tid];
-#pragma unroll 1
-                        for (int w = 1; w < steps; ++w) sum += red[w * 128 + tid];
+                        float sum = red[tid], sum2 = 0.0f;
+#pragma unroll
+                        for (int w = 1; w < kWarps; ++w)
+                            if (w < steps) (w & 1 ? sum2 : sum) += red[w * 128 + tid];
+                        sum += sum2;
                         put(out + (tid >> 3) * p.ncg * 8 + (tid & 7), __float_as_uint(sum), tag_of(l));
                     }
                 } else {
@@ -628,42 +648,35 @@ struct Step {
             wd[r * p.nch + c] = w[static_cast<long long>(r) * p.di + c];
         }
     }
-    // what a quad needs of its (sequence, channel) that is ready before the x_proj sums are
-    struct Task {
-        float4 h, a;
-        float D;
-        Tact dtb;  // as loaded: a conversion here would wait for the load
-    };
-    __device__ void load_task(int l, int b, int c, Task& t) {
-        const int d = cta * p.nch + c, j = tid & 3;
-        t.h = ldcg4(p.ssm + ((static_cast<long long>(l) * p.Bcap + b) * p.di + d) * kN + 4 * j);
-        t.a = __ldg(reinterpret_cast<const float4*>(p.a_neg + (static_cast<long long>(l) * p.di + d) * kN) + j);
-        t.dtb = lp(l, p.o_dtb)[d];
-        t.D = __ldg(mf(l, p.o_D) + d);
+    __device__ float4 load_state(int l, int b, int c) const {
+        return ldcg4(p.ssm + ((static_cast<long long>(l) * p.Bcap + b) * p.di + cta * p.nch + c) * kN + 4 * (tid & 3));
     }
-    __device__ void do_task(int l, int b, int c, bool on, const Task& t) {
+    __device__ void do_task(int l, int b, int c, bool on, float4 h0) {
         const Tact* wd = reinterpret_cast<const Tact*>(sm + p.s_wd) + c;
         const int j = tid & 3, d = cta * p.nch + c;
         const float* xr = reinterpret_cast<const float*>(sm + p.s_act) + b * p.xd;
+        const float* am = reinterpret_cast<const float*>(sm + p.s_a);
+        const float4 a = *reinterpret_cast<const float4*>(am + c * kN + 4 * j);
+        const float D = am[p.nch * kN + c], dtb = to_f(reinterpret_cast<const Tact*>(am + p.nch * (kN + 1))[c]);
         float dl = 0.0f;
 #pragma unroll 4
         for (int r = j; r < p.dr; r += 4) dl = fmaf(xr[r], to_f(wd[r * p.nch]), dl);
         dl += __shfl_xor_sync(0xffffffffu, dl, 1);
         dl += __shfl_xor_sync(0xffffffffu, dl, 2);
-        dl = softplusf_fast(dl + to_f(t.dtb));
+        dl = softplusf_fast(dl + dtb);
         const float2 uz = reinterpret_cast<const float2*>(sm + p.s_uz)[b * p.nch + c];
         const float du = dl * uz.x, dk = dl * kLog2e;
         const float* Bv = xr + p.dr + 4 * j;
         const float* Cv = Bv + kN;
         float4 h;
-        h.x = fmaf(ex2(dk * t.a.x), t.h.x, du * Bv[0]);
-        h.y = fmaf(ex2(dk * t.a.y), t.h.y, du * Bv[1]);
-        h.z = fmaf(ex2(dk * t.a.z), t.h.z, du * Bv[2]);
-        h.w = fmaf(ex2(dk * t.a.w), t.h.w, du * Bv[3]);
+        h.x = fmaf(ex2(dk * a.x), h0.x, du * Bv[0]);
+        h.y = fmaf(ex2(dk * a.y), h0.y, du * Bv[1]);
+        h.z = fmaf(ex2(dk * a.z), h0.z, du * Bv[2]);
+        h.w = fmaf(ex2(dk * a.w), h0.w, du * Bv[3]);
         float y = fmaf(h.x, Cv[0], fmaf(h.y, Cv[1], fmaf(h.z, Cv[2], h.w * Cv[3])));
         y += __shfl_xor_sync(0xffffffffu, y, 1);
         y += __shfl_xor_sync(0xffffffffu, y, 2);
-        publish<4>(p.y_x, b * p.di + d, from_f<Tact>(fmaf(t.D, uz.x, y) * siluf_fast(uz.y)), on && j == 0, tag_of(l));
+        publish<4>(p.y_x, b * p.di + d, from_f<Tact>(fmaf(D, uz.x, y) * siluf_fast(uz.y)), on && j == 0, tag_of(l));
         if (on) *reinterpret_cast<float4*>(p.ssm + ((static_cast<long long>(l) * p.Bcap + b) * p.di + d) * kN + 4 * j) = h;
     }
     // (b, c) of this thread's first task and first pair of x_proj columns: the same in every layer
@@ -672,8 +685,8 @@ struct Step {
         const int n = channels();
         if (n <= 0) return;
         const int tasks = p.B * n, q0 = tid >> 2;
-        Task t;
-        if (q0 < tasks) load_task(l, at.b, at.c, t);
+        float4 h = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (q0 < tasks) h = load_state(l, at.b, at.c);
         float* xs = reinterpret_cast<float*>(sm + p.s_act);
         const int per = p.ncg * 4, pairs = p.B * per;  // pairs of columns of all rows
         int row = at.row, col = at.col;
@@ -707,9 +720,9 @@ struct Step {
             if (r > 0) {
                 b = q < tasks ? q / n : 0;
                 c = q < tasks ? q - b * n : 0;
-                if (q < tasks) load_task(l, b, c, t);
+                if (q < tasks) h = load_state(l, b, c);
             }
-            if (q - lane / 4 < tasks) do_task(l, b, c, q < tasks, t);  // whole warps
+            if (q - lane / 4 < tasks) do_task(l, b, c, q < tasks, h);  // whole warps
         }
     }
 
@@ -1067,7 +1080,7 @@ static int plan(int sms, const mamba_b200_decode_args& a, dec::Params& p, long l
     p.kp4 = (p.di + 31) / 32 * 32;
     p.ncg = (p.xd + 7) / 8;
     const int tiles1 = p.di / tw, tiles4 = p.dm / tw;
-    int grid = tiles1 > 8 * p.ncg ? tiles1 : 8 * p.ncg;
+    int grid = tiles1 > kMaxKs * p.ncg ? tiles1 : kMaxKs * p.ncg;
     if (grid > sms || a.vocab > 0) grid = sms;
     auto tiles = [](int n, int g, int kp, int& per, int& c, int& ka, int& br) {
         per = (n + g - 1) / g;
@@ -1083,11 +1096,12 @@ static int plan(int sms, const mamba_b200_decode_args& a, dec::Params& p, long l
     if (p.nch > 256) return 0;
     // enough slices to use the CTAs, few enough that adding them up stays short
     int ks = grid / p.ncg;
-    ks = ks < 1 ? 1 : ks > 8 ? 8 : ks;
+    ks = ks < 1 ? 1 : ks > kMaxKs ? kMaxKs : ks;
     int sl = ((p.di + ks - 1) / ks + 15) / 16 * 16;
     if (sl > kMaxKSlice) sl = kMaxKSlice;
     p.kslice = sl;
     p.ks = (p.di + sl - 1) / sl;
+    p.brx = sl > 256 ? sl / 2 : sl;
     const int dboxes = (p.dr + 255) / 256;
     p.brd = ((p.dr + dboxes - 1) / dboxes + 7) / 8 * 8;
     auto up = [](long long v) { return (v + 15) / 16 * 16; };
@@ -1107,10 +1121,11 @@ static int plan(int sms, const mamba_b200_decode_args& a, dec::Params& p, long l
     p.s_wx = o; o += up128(static_cast<long long>(p.kslice) * 8 * es);
     p.s_wd = o; o += up128(static_cast<long long>(dboxes) * p.brd * p.nch * es);
     p.s_act = o; o += up(act);
-    p.s_red = o; o += up(half ? kWarps * 2 * 160 * 4 : kWarps * 4 * 32 * 4);
+    p.s_red = o; o += up(half ? kWarps * 2 * 160 * 4 : kWarps * 2 * 32 * 4);
     p.s_norm = o; o += up(static_cast<long long>(p.dm) * 4);
     p.s_conv = o; o += up(static_cast<long long>(p.nch) * (16LL * (p.B + 1) + 4));
     p.s_uz = o; o += up(8LL * p.B * p.nch);
+    p.s_a = o; o += up(p.nch * (kN * 4 + 4 + es));
     if (o > 227 * 1024 - 1024) return 0;
     *smem = static_cast<uint32_t>(o);
     const long long Bl = p.B;
@@ -1153,7 +1168,7 @@ extern "C" MAMBA_B200_API int mamba_b200_decode_step(void* handle, void* stream,
     const void* al[8] = {a.lp, a.master, a.a_neg, a.conv_state, a.ssm_state, a.residual, a.workspace, lm ? a.logits : a.out};
     for (int i = 0; i < 7; ++i)
         if (reinterpret_cast<uintptr_t>(al[i]) & 15) return fail(c, MAMBA_B200_ERR_ARG, "decode_step: pointer %d is not 16-byte aligned", i);
-    const long long offs[] = {a.layer_stride, a.o_in_proj, a.o_conv_w, a.o_conv_b, a.o_out_proj, a.o_norm_f, lm ? a.o_embedding : 0};
+    const long long offs[] = {a.layer_stride, a.o_in_proj, a.o_conv_w, a.o_conv_b, a.o_dt_proj_b, a.o_d_param, a.o_out_proj, a.o_norm_f, lm ? a.o_embedding : 0};
     for (long long v : offs)
         if (v % 8 != 0) return fail(c, MAMBA_B200_ERR_ARG, "decode_step: arena offsets must be multiples of 8 elements");
     p.lp = a.lp; p.master = a.master; p.a_neg = a.a_neg; p.lstride = a.layer_stride;
@@ -1180,7 +1195,7 @@ extern "C" MAMBA_B200_API int mamba_b200_decode_step(void* handle, void* stream,
         !make_tmap_stack(c, &p.tm_out, a.dtype, lp8 + p.o_out * es, p.dm, p.di, p.L, p.lstride, p.c4 * tw, p.br4))
         return fail(c, MAMBA_B200_ERR_CUDA, "decode_step: the weight tensor maps were refused");
     // rows of W_x or W_dt that do not start on 16 bytes are copied by the compute warps
-    p.x_tma = p.ncg * p.ks <= grid && make_tmap_stack(c, &p.tm_x, a.dtype, lp8 + p.o_x * es, p.xd, p.di, p.L, p.lstride, 8, p.kslice);
+    p.x_tma = p.ncg * p.ks <= grid && make_tmap_stack(c, &p.tm_x, a.dtype, lp8 + p.o_x * es, p.xd, p.di, p.L, p.lstride, 8, p.brx);
     p.dt_tma = make_tmap_stack(c, &p.tm_dt, a.dtype, lp8 + p.o_dtw * es, p.di, p.dr, p.L, p.lstride, p.nch, p.brd);
     int steps = lm && a.steps > 1 ? a.steps : 1;
     const void* fn = a.dtype == MAMBA_B200_F32   ? reinterpret_cast<const void*>(dec::decode_step_kernel<float>)
