@@ -46,6 +46,7 @@ namespace dec {
 constexpr int kThreads = 512, kWarps = 16;  // compute threads; one more warp asks for the operands
 constexpr int kN = 16, kK = 4;          // d_state and d_conv of this kernel
 constexpr int kMaxDm = 1024, kMaxB = 64, kMaxKSlice = 384, kMaxKs = 4;
+constexpr long long kHeadAhead = 64ll << 20;  // bytes of the head's table asked for ahead of it
 constexpr int kMaxPolls = 1 << 21;      // a poll is about a microsecond's L2 round trip
 
 struct Params {
@@ -276,6 +277,20 @@ struct Step {
         }
         return false;
     }
+    // A quarter of this CTA's tiles of the head, into L2 under each of the last four layers, whose weights leave
+    // HBM nine tenths idle.  Beyond kHeadAhead they would only push one another out.
+    static constexpr int kHeadRows = H ? 16 : 4;  // of a tile
+    __device__ void hint_head(int l) {
+        const int quarter = l - (p.L - 4);
+        if (!p.next_ids || quarter < 0) return;
+        const long long row = static_cast<long long>(p.dm) * sizeof(Tact);
+        for (int t = lane;; t += 32) {
+            const long long r = (static_cast<long long>(t) * ncta + cta) * kHeadRows + quarter * (kHeadRows / 4);
+            if (r >= p.V || r * row > kHeadAhead) return;
+            l2_prefetch_bulk(static_cast<const Tact*>(p.lp) + p.o_emb + r * p.dm,
+                             static_cast<uint32_t>(min(static_cast<long long>(kHeadRows / 4), p.V - r) * row));
+        }
+    }
     __device__ void feed() {
         const bool in = channels() > 0, x = has_unit() && p.x_tma, out = out_tiles() > 0;
         if (in) ask_in(0);
@@ -297,6 +312,7 @@ struct Step {
                 ++n_x;
             }
             hint(l + 2);
+            hint_head(l + 1);
             if (in) {
                 if (!freed(kSmall, l)) break;
                 ask_small(l + 1);
@@ -825,7 +841,7 @@ struct Step {
                 // the walk goes on into the warp's next tile, so 2 U to 4 U loads a lane are always in flight
                 constexpr int U = 3;
                 const int stride = ncta * kWarps;
-                int lt = cta * kWarps + warp, lk = 0;  // what is requested next
+                int lt = warp * ncta + cta, lk = 0;  // what is requested next (a round's tiles go around the CTAs first)
                 auto request = [&](uint4 (*x)[2]) {
                     if (lt * 16 < p.V) {
                         const Tact* w0 = emb + static_cast<long long>(min(lt * 16 + g, p.V - 1)) * p.dm + 8 * q;
@@ -859,7 +875,7 @@ struct Step {
                 uint4 xa[U][2], xb[U][2];
                 bool first = true;
                 request(xa);
-                for (int tile = cta * kWarps + warp; tile * 16 < p.V; tile += stride) {
+                for (int tile = warp * ncta + cta; tile * 16 < p.V; tile += stride) {
                     const int v0 = tile * 16 + g, v1 = v0 + 8;
 #pragma unroll
                     for (int t = 0; t < 4; ++t)
@@ -898,7 +914,7 @@ struct Step {
                 const float* act = reinterpret_cast<const float*>(sm + p.s_act);
                 float bv = -INFINITY;
                 int bi = 0x7fffffff;
-                for (int tile = cta * kWarps + warp; tile * 4 < p.V; tile += ncta * kWarps) {
+                for (int tile = warp * ncta + cta; tile * 4 < p.V; tile += ncta * kWarps) {
                     float acc[32];
 #pragma unroll
                     for (int i = 0; i < 32; ++i) acc[i] = 0.0f;
