@@ -171,3 +171,46 @@ def test_greedy_decode_from_a_captured_graph_equals_eager_decode(cuda_dev):
         outs.append(lm.generate_greedy(n, use_graph=use_graph).cpu().numpy())
     np.testing.assert_array_equal(outs[0], outs[1])
     assert outs[0].min() >= 0 and outs[0].max() < V
+
+
+@pytest.mark.parametrize("dt", ["bf16", "f32"])
+@pytest.mark.parametrize("shape", [(1, 1, 1), (2, 33, 2), (3, 130, 2)], ids=lambda s: "b%dt%dl%d" % s)
+def test_passes_that_come_again_equal_the_first_ones(cuda_dev, shape, dt):
+    """From the third call with the same addresses on a pass is a replay; other ids, other lengths in
+    between, a result that the caller keeps and changed hyperparameters give what single launches give."""
+    import torch
+
+    import mamba_rs_b200 as mb
+    B, T, L = shape
+    td = {"bf16": torch.bfloat16, "f32": torch.float32}[dt]
+    make = lambda: mb.MambaWeights(mb.MambaConfig(d_model=64, n_layers=L), cuda_dev, dtype=td, vocab=300).init_random(3)  # noqa: E731
+    g = torch.Generator(device=cuda_dev).manual_seed(T)
+    ids = [torch.randint(0, 300, (B, T + 1), device=cuda_dev, dtype=torch.int32, generator=g) for _ in range(6)]
+    x = torch.randn(B, T, 64, device=cuda_dev, generator=g)
+    runs = []
+    for replay in (False, True):
+        w, got = make(), []
+        lm = mb.GpuMambaLM(w, B)
+        for (n, i) in ((T, 0), (T, 1), (T, 2), (T + 1, 3), (T, 4), (T, 5)):
+            lm.backbone._prefill_plan(B, n).launch_bound = replay
+            lm.backbone.reset()
+            got += [lm.prefill(ids[i][:, :n]).clone(), lm.next_ids.clone(), lm.backbone.ssm.clone(), lm.backbone.conv.clone()]
+        buf, kept = torch.empty_like(x), []
+        for i in range(5):
+            lm.backbone.reset()
+            buf.copy_(x * (i + 1))
+            kept.append(lm.backbone.prefill_sequence(buf))
+            got.append(buf.clone())
+        got += kept
+        tr = mb.MambaLMTrainer(w, lr=1e-3)
+        tr._plan(B, T).launch_bound = replay
+        for i in range(6):
+            if i == 4:
+                tr.lr = 2e-3
+            got.append(tr.step(ids[i]))
+        got += [w.master.clone(), w.lp.clone(), tr.m, tr.v]
+        assert bool(lm.backbone._prefill_plan(B, T).replay.kept) == replay == bool(tr._plan(B, T).replay.kept)
+        runs.append(got)
+    for a, b in zip(*runs):
+        assert rel_err(b.float().cpu().numpy(), a.float().cpu().numpy()) <= (1e-5 if dt == "f32" else 2e-2)
+    mb.ffi.default_handle(0).check_status()
