@@ -364,21 +364,30 @@ __global__ void __launch_bounds__(32) sscan_bwd_kernel(const __grid_constant__ B
 
 // dB / dC: add the channel tiles in index order.  part [B][tiles][T][2N] -> dB, dC [B,T,N].
 // A thread owns four adjacent values of one (sample, step) and keeps eight 16-byte
-// loads in flight; the sum still runs in tile order.
-__global__ void __launch_bounds__(256) bwd_reduce_bc_kernel(const float* __restrict__ part, float* __restrict__ dB,
+// loads in flight; the sum runs in tile order.  PARTS > 1, for calls too small to fill the chip that
+// way (reduce_bc): the tiles of a value are divided over PARTS warps, whose sums are added in order
+// (1 x 32 steps x 96 tiles: 3 us, 9.1 with one thread a value).
+template <int PARTS>
+__global__ void __launch_bounds__(256) bwd_reduce_bc_kernel(const float* __restrict__ parts, float* __restrict__ dB,
                                                             float* __restrict__ dC, int B, int T, int N, int NSv,
                                                             int tiles, int vec_out) {
-    const long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
+    constexpr int OUT = 256 / PARTS;  // values (of four) a CTA
+    __shared__ float4 sums[PARTS > 1 ? 256 : 1];
+    const int part = PARTS > 1 ? threadIdx.x / OUT : 0;
+    const long long i = blockIdx.x * static_cast<long long>(OUT) + threadIdx.x % OUT;
     const int V = 2 * NSv, V4 = V / 4;
-    if (i >= static_cast<long long>(B) * T * V4) return;
+    const bool on = i < static_cast<long long>(B) * T * V4;
+    if (PARTS == 1 && !on) return;
     const int v = static_cast<int>(i % V4) * 4;
     const long long bt = i / V4;
     const long long bb = bt / T, t = bt % T;
     const long long stride = static_cast<long long>(T) * V;
-    const float* src = part + (bb * tiles * T + t) * V + v;
+    const float* src = parts + (bb * tiles * T + t) * V + v;
     float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    int k = 0;
-    for (; k + 8 <= tiles; k += 8) {
+    const int per = (tiles + PARTS - 1) / PARTS;
+    int k = part * per;
+    const int end = on ? min(tiles, k + per) : 0;
+    for (; k + 8 <= end; k += 8) {
         float4 q[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) q[j] = __ldcs(reinterpret_cast<const float4*>(src + (k + j) * stride));
@@ -387,9 +396,19 @@ __global__ void __launch_bounds__(256) bwd_reduce_bc_kernel(const float* __restr
             acc.x += q[j].x; acc.y += q[j].y; acc.z += q[j].z; acc.w += q[j].w;
         }
     }
-    for (; k < tiles; ++k) {
+    for (; k < end; ++k) {
         const float4 q = __ldcs(reinterpret_cast<const float4*>(src + k * stride));
         acc.x += q.x; acc.y += q.y; acc.z += q.z; acc.w += q.w;
+    }
+    if (PARTS > 1) {
+        sums[threadIdx.x] = acc;
+        __syncthreads();
+        if (part != 0 || !on) return;
+#pragma unroll
+        for (int j = 1; j < PARTS; ++j) {
+            const float4 q = sums[j * OUT + threadIdx.x];
+            acc.x += q.x; acc.y += q.y; acc.z += q.z; acc.w += q.w;
+        }
     }
     float* dst = v < NSv ? dB : dC;
     const int n = v % NSv;
@@ -403,6 +422,16 @@ __global__ void __launch_bounds__(256) bwd_reduce_bc_kernel(const float* __restr
     }
 }
 
+// One thread a value from two CTAs per SM on (the tiles' loads of a warp then overlap the others'); eight
+// warps a value below.
+static void reduce_bc(const float* parts, float* dB, float* dC, int B, int T, int N, int NSv, int tiles, int vec_out, cudaStream_t st) {
+    const long long n = static_cast<long long>(B) * T * 2 * NSv / 4;
+    if (n >= 2LL * 148 * 256)
+        bwd_reduce_bc_kernel<1><<<static_cast<unsigned>((n + 255) / 256), 256, 0, st>>>(parts, dB, dC, B, T, N, NSv, tiles, vec_out);
+    else
+        bwd_reduce_bc_kernel<8><<<static_cast<unsigned>((n + 31) / 32), 256, 0, st>>>(parts, dB, dC, B, T, N, NSv, tiles, vec_out);
+}
+
 // Segment hand-over of the two-lane backward: slot s of seg_dh arrives holding the dh segment s leaves
 // where it begins when started from zero and leaves holding the true one, which segment s - 1 starts
 // from.  (Slot 0 is not used: nothing precedes segment 0.)
@@ -412,11 +441,23 @@ __global__ void sscan_bwd_carry_kernel(float* seg_dh, const float* seg_sum, cons
     if (i >= B * DN) return;
     const long long b = i / DN, dn = i - b * DN, d = dn / N;
     const float a2 = a_neg[dn] * kLog2e;
+    float* st = seg_dh + b * S * DN + dn;
+    const float* sums = seg_sum + b * S * D + d;
     float run = 0.0f;
-    for (int s = S - 1; s >= 1; --s) {
-        const long long at = (b * S + s) * DN + dn;
-        run = fmaf(ex2(a2 * seg_sum[(b * S + s) * D + d]), run, seg_dh[at]);
-        seg_dh[at] = run;
+    for (int s0 = S - 1; s0 >= 1; s0 -= 8) {  // eight segments' loads at once: their latency is what takes the time
+        float h[8], q[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const int s = s0 - k >= 1 ? s0 - k : s0;
+            h[k] = st[s * DN];
+            q[k] = sums[static_cast<long long>(s) * D];
+        }
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            if (s0 - k >= 1) {
+                run = fmaf(ex2(a2 * q[k]), run, h[k]);
+                st[(s0 - k) * DN] = run;
+            }
     }
 }
 
@@ -700,9 +741,7 @@ static int launch_bwd(Ctx* c, void* stream, const mamba_b200_sscan_bwd_args& a, 
         cudaError_t e = launch_bwd_wide(p, a.dtype, a.delta_softplus, stw, &wtiles);
         if (e != cudaSuccess) return fail(c, MAMBA_B200_ERR_CUDA, "sscan_bwd (wide): %s", cudaGetErrorString(e));
         const int np = 8 * bwd_wide_lpc(a.N);
-        const long long nbcw = static_cast<long long>(a.B) * a.T * 2 * np / 4;
-        bwd_reduce_bc_kernel<<<static_cast<unsigned>((nbcw + 255) / 256), 256, 0, stw>>>(
-            p.part_bc, a.dBm, a.dCm, a.B, a.T, a.N, np, wtiles, bc_vec);
+        reduce_bc(p.part_bc, a.dBm, a.dCm, a.B, a.T, a.N, np, wtiles, bc_vec, stw);
         MB200_CUDA_CHECK(c, cudaGetLastError());
         const int npar = a.D * a.N;
         bwd_reduce_params_kernel<<<(npar + 255) / 256, 256, 0, stw>>>(p.part_a, p.part_d, a.dA_log, a.dD, a.B, a.D,
@@ -776,9 +815,7 @@ static int launch_bwd(Ctx* c, void* stream, const mamba_b200_sscan_bwd_args& a, 
         t.fn[a.dtype][vi][flags]<<<grid, 32, t.smem[a.dtype][vi], st>>>(p);
     }
     MB200_CUDA_CHECK(c, cudaGetLastError());
-    const long long nbc = static_cast<long long>(a.B) * a.T * 2 * ns / 4;
-    bwd_reduce_bc_kernel<<<static_cast<unsigned>((nbc + 255) / 256), 256, 0, st>>>(
-        p.part_bc, a.dBm, a.dCm, a.B, a.T, a.N, ns, tiles, bc_vec);
+    reduce_bc(p.part_bc, a.dBm, a.dCm, a.B, a.T, a.N, ns, tiles, bc_vec, st);
     MB200_CUDA_CHECK(c, cudaGetLastError());
     const int np = a.D * a.N;
     bwd_reduce_params_kernel<<<(np + 255) / 256, 256, 0, st>>>(p.part_a, p.part_d, a.dA_log, a.dD, a.B * segs,

