@@ -455,6 +455,15 @@ MAMBA_B200_API int mamba_b200_residual_rmsnorm_fwd(void* handle, void* stream, i
 MAMBA_B200_API int mamba_b200_residual_rmsnorm_fwd_to(void* handle, void* stream, int dtype, const float* residual,
                                        const void* branch, const float* scale, float* residual_out, void* y,
                                        float* rms_out, int rows, int dim, float eps);
+
+/* f32 products of a few rows of activations with a weight matrix, and its gradient; any sizes and row
+ * strides (in elements), made for up to a few dozen rows.
+ *   op 0  C[M,N] = A[M,K] B[K,N] (+ bias[N], may be NULL)
+ *   op 1  C[M,N] = A[M,K] B[N,K]^T (+ bias)
+ *   op 2  C[M,N] += A[K,M]^T B[K,N] */
+MAMBA_B200_API int mamba_b200_sgemm_rows(void* handle, void* stream, int op, const float* a, long long lda,
+                                         const float* b, long long ldb, const float* bias, float* c, long long ldc,
+                                         int M, int N, int K);
 MAMBA_B200_API long long mamba_b200_residual_rmsnorm_bwd_workspace_bytes(int rows, int dim);
 MAMBA_B200_API int mamba_b200_residual_rmsnorm_bwd(void* handle, void* stream, int dtype, const void* dy,
                                     const float* x, const float* scale, const float* rms_saved,

@@ -168,6 +168,7 @@ def lib() -> C.CDLL:
         ll, fl, it = C.c_longlong, C.c_float, C.c_int
         bind("mamba_b200_residual_rmsnorm_fwd", [vp, vp, it, vp, vp, vp, vp, vp, it, it, fl])
         bind("mamba_b200_residual_rmsnorm_fwd_to", [vp, vp, it, vp, vp, vp, vp, vp, vp, it, it, fl])
+        bind("mamba_b200_sgemm_rows", [vp, vp, it, vp, ll, vp, ll, vp, vp, ll, it, it, it])
         bind("mamba_b200_residual_rmsnorm_bwd_workspace_bytes", [it, it], ll)
         bind("mamba_b200_residual_rmsnorm_bwd", [vp, vp, it, vp, vp, vp, vp, vp, vp, it, it, vp, ll])
         bind("mamba_b200_embedding_gather", [vp, vp, it, vp, vp, vp, ll, it, it])

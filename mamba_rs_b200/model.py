@@ -204,6 +204,20 @@ class _Launcher:
             self.handle.check(rc, getattr(fn, "__name__", "kernel call"))
 
 
+def _product(go, op, a, b, out):
+    """out = a b (op 0) or a b^T (op 1), inside go.begin().  In f32 with few output tiles and a long
+    contraction the rows kernel has the parts of K that the library's tiles leave to one SM (32 rows,
+    768 x 3072: 8.6 us for 14.5; 1536 x 768: 7.9 for 18.1); from 64 tiles of 32 x 64 on, or under a
+    dozen rows or 512 steps of K, the library is as fast."""
+    M, K = a.shape
+    N = out.shape[1]
+    if a.dtype == torch.float32 and M >= 12 and K >= 512 and ((M + 31) // 32) * ((N + 63) // 64) <= 64:
+        go.call(go.lib.mamba_b200_sgemm_rows, op, a.data_ptr(), a.stride(0), b.data_ptr(), b.stride(0), None, out.data_ptr(),
+                out.stride(0), M, N, K)
+    else:
+        torch.mm(a, b if op == 0 else b.t(), out=out)
+
+
 class _Replay:
     """Sequences of launches that come again with the same addresses, as CUDA graphs.  A model small
     enough for its launches to cost more than its work spends a fifth to a half of a pass between
@@ -308,19 +322,19 @@ class _PrefillPlan:
         go, lib = self.run_on, self.run_on.lib
         norm, conv, scan = lib.mamba_b200_residual_rmsnorm_fwd, lib.mamba_b200_conv1d_fwd, lib.mamba_b200_sscan_fwd
         res_p, post_p = temporal.data_ptr(), post.data_ptr()
-        mm, addmm = torch.mm, torch.addmm
+        addmm = torch.addmm
         with go.begin():
             br = None
             for norm_w, w_in, cv, w_x, b_dt, w_dt, sc, w_out, *_ in self.layers:
                 go.call(norm, self.dt, res_p, br, norm_w, post_p, None, BT, dm, c.rms_norm_eps)
-                mm(post, w_in, out=proj)                                    # [BT, 2 di]: x | z in place
+                _product(go, 0, post, w_in, proj)                           # [BT, 2 di]: x | z in place
                 go.call(conv, cv)
-                mm(u, w_x, out=xdbl)                                        # [BT, dr + 2N]: dt | B | C in place
+                _product(go, 0, u, w_x, xdbl)                               # [BT, dr + 2N]: dt | B | C in place
                 addmm(b_dt, dtx, w_dt, out=delta)
                 go.call(scan, sc)
                 if last_only and w_out is self.layers[-1][7]:
                     break
-                mm(y, w_out, out=branch)
+                _product(go, 0, y, w_out, branch)
                 br = post_p
             if last_only:
                 return temporal.view(B, T, dm)[:, -1].contiguous(), y.view(B, T, di)[:, -1] @ self.layers[-1][7]
@@ -571,7 +585,7 @@ class _TrainPlan:
     the caching allocator in each step; the structs are pointed at them when their addresses changed."""
 
     class Layer:
-        __slots__ = ("norm_w", "g_norm", "w_in", "w_in_t", "w_x", "w_x_t", "b_dt", "w_dt", "w_dt_t", "w_out", "w_out_t",
+        __slots__ = ("norm_w", "g_norm", "w_in", "w_x", "w_x_t", "b_dt", "w_dt", "w_out",
                      "conv", "scan", "conv_b", "scan_b", "structs")
 
     def __init__(self, w: MambaWeights, B: int, T: int, save: int):
@@ -597,7 +611,7 @@ class _TrainPlan:
             p, pm, g, lay = w.layer(l), w.layer(l, "master"), w.layer(l, "grad"), self.Layer()
             lay.norm_w, lay.g_norm = pm["norm_w"].data_ptr(), g["norm_w"].data_ptr()
             lay.w_in, lay.w_x, lay.b_dt, lay.w_dt, lay.w_out = (p[k] for k in ("in_proj_w", "x_proj_w", "dt_proj_b", "dt_proj_w", "out_proj_w"))
-            lay.w_in_t, lay.w_x_t, lay.w_dt_t, lay.w_out_t = (t.t() for t in (lay.w_in, lay.w_x, lay.w_dt, lay.w_out))
+            lay.w_x_t = lay.w_x.t()
             cv, sc, cb, sb = ffi.Conv1dArgs(), ffi.SscanFwdArgs(), ffi.Conv1dArgs(), ffi.SscanBwdArgs()
             for q in (cv, cb):
                 q.dtype, q.B, q.T, q.D, q.K, q.ld_x = self.dt, B, T, di, K, 2 * di
@@ -702,7 +716,7 @@ class MambaLMTrainer:
         plan.point_forward(proj, u, xdbl, delta, y, cs, ws)
         norm, conv, scan = lib.mamba_b200_residual_rmsnorm_fwd_to, lib.mamba_b200_conv1d_fwd, lib.mamba_b200_sscan_fwd
         ops.embedding_gather(emb, inp, res[0])
-        mm, addmm, dr = torch.mm, torch.addmm, c.dt_rank
+        addmm, dr = torch.addmm, c.dt_rank
         res_p, rms_p, post_p, branch_p = res.data_ptr(), rms.data_ptr(), post.data_ptr(), branch.data_ptr()
         with go.begin():
             acts = list(zip(post.unbind(), proj.unbind(), u.unbind(), xdbl.unbind(), delta.unbind(), y.unbind()))
@@ -710,12 +724,12 @@ class MambaLMTrainer:
                 # the stream this layer's norm saw is kept in res[l]; the embedding is there already
                 go.call(norm, plan.dt, res_p + 4 * BT * dm * max(l - 1, 0), branch_p if l else None, lay.norm_w,
                         res_p + 4 * BT * dm * l, post_p + plan.es * BT * dm * l, rms_p + 4 * BT * l, BT, dm, c.rms_norm_eps)
-                mm(post_l, lay.w_in, out=proj_l)
+                _product(go, 0, post_l, lay.w_in, proj_l)
                 go.call(conv, lay.conv)
-                mm(u_l, lay.w_x, out=xdbl_l)
+                _product(go, 0, u_l, lay.w_x, xdbl_l)
                 addmm(lay.b_dt, xdbl_l[:, :dr], lay.w_dt, out=delta_l)
                 go.call(scan, lay.scan)
-                mm(y_l, lay.w_out, out=branch)
+                _product(go, 0, y_l, lay.w_out, branch)
             go.call(norm, plan.dt, res_p + 4 * BT * dm * (L - 1), branch_p, plan.norm_f, res_p + 4 * BT * dm * L,
                     hidden.data_ptr(), rms_p + 4 * BT * L, BT, dm, c.rms_norm_eps)
         logits = hidden @ emb.t()                                  # tied head, [BT, V]
@@ -736,7 +750,12 @@ class MambaLMTrainer:
 
     def _accumulate(self, g, a, b):
         """g (f32) += a.T @ b, the product accumulated into g by the GEMM itself."""
-        if a.dtype == torch.float32:
+        if a.dtype == torch.float32 and a.shape[0] <= 32:  # (32 tokens, 768 x 3072: 6.3 us for the library's 8.8)
+            go = self._acts["plan"].run_on
+            with go.begin():
+                go.call(go.lib.mamba_b200_sgemm_rows, 2, a.data_ptr(), a.stride(0), b.data_ptr(), b.stride(0), None,
+                        g.data_ptr(), g.stride(0), g.shape[0], g.shape[1], a.shape[0])
+        elif a.dtype == torch.float32:
             g.addmm_(a.t(), b)
         else:
             torch.addmm(g, a.t(), b, out_dtype=torch.float32, out=g)
@@ -757,7 +776,9 @@ class MambaLMTrainer:
         gt = w.tail("grad")
         dl, acc = a["dlogits"], self._accumulate
         acc(gt["embedding"], dl, a["hidden"])                       # head weight gradient
-        d_post = dl @ emb                                           # [BT, dm], here of the final norm
+        d_post = torch.empty(BT, dm, dtype=dt, device=dev)          # here of the final norm
+        with plan.run_on.begin():
+            _product(plan.run_on, 0, dl, emb, d_post)
         a["dlogits"] = dl = None
         new = lambda *shape: torch.empty(shape, dtype=dt, device=dev)  # noqa: E731
         d_res = torch.zeros(BT, dm, device=dev)
@@ -770,7 +791,7 @@ class MambaLMTrainer:
         norm, conv, scan = lib.mamba_b200_residual_rmsnorm_bwd, lib.mamba_b200_conv1d_bwd, lib.mamba_b200_sscan_bwd
         res_p, rms_p, dres_p, ws_p = a["res"].data_ptr(), a["rms"].data_ptr(), d_res.data_ptr(), ws.data_ptr()
         d_dt_in, d_bc_out, d_bc_in = d_xdbl[:, :dr], d_xdbl[:, dr:].view(BT, 2, N), d_bc.transpose(0, 1)
-        mm, addmm = torch.mm, torch.addmm
+        addmm = torch.addmm
         with go.begin():
             dp = d_post.data_ptr()
             go.call(norm, plan.dt, dp, res_p + 4 * BT * dm * L, plan.norm_f, rms_p + 4 * BT * L, dres_p, gt["norm_f"].data_ptr(),
@@ -781,17 +802,17 @@ class MambaLMTrainer:
                 if d_out is not d_res:
                     d_out.copy_(d_res)                              # gradient of this layer's branch output
                 acc(g["out_proj_w"], y, d_out)
-                mm(d_out, lay.w_out_t, out=d_y)
+                _product(go, 1, d_out, lay.w_out, d_y)
                 go.call(scan, lay.scan_b)
                 g["dt_proj_b"].add_(torch.sum(d_delta, 0, dtype=torch.float32))
                 acc(g["dt_proj_w"], xdbl[:, :dr], d_delta)
-                mm(d_delta, lay.w_dt_t, out=d_dt_in)
+                _product(go, 1, d_delta, lay.w_dt, d_dt_in)
                 d_bc_out.copy_(d_bc_in)
                 acc(g["x_proj_w"], u, d_xdbl)
                 addmm(d_u, d_xdbl, lay.w_x_t, out=d_u)              # backward_mixed.rs:350-580
                 go.call(conv, lay.conv_b)
                 acc(g["in_proj_w"], post, d_proj)
-                mm(d_proj, lay.w_in_t, out=d_post)
+                _product(go, 1, d_proj, lay.w_in, d_post)
                 go.call(norm, plan.dt, dp, res_p + 4 * BT * dm * l, lay.norm_w, rms_p + 4 * BT * l, dres_p, lay.g_norm,
                         BT, dm, ws_p, plan.bwd_ws)
                 if red is not None:

@@ -116,3 +116,29 @@ def test_adamw_matches_the_reference_update_rule(cuda_dev, lp):
     assert rel_err(host(v), v_ref) <= 1e-6
     if lp is not None:
         np.testing.assert_array_equal(host(lp_t), synth.round_to(host(p), lp))
+
+
+@pytest.mark.parametrize("op", [0, 1, 2])
+@pytest.mark.parametrize("size", [(1, 1, 1), (32, 64, 600), (33, 65, 33), (5, 100, 37), (64, 63, 1536), (31, 80, 520), (32, 768, 2050)],
+                         ids=lambda s: "m%dn%dk%d" % s)
+def test_sgemm_rows_matches_f64(cuda_dev, size, op):
+    """Edges of the 32 x 64 tiles and of the parts of K, rows on and off 16 bytes, with and without a bias."""
+    import torch
+
+    from mamba_rs_b200 import ffi
+    M, N, K = size
+    h, lib = ffi.default_handle(0), ffi.lib()
+    g = torch.Generator(device=cuda_dev).manual_seed(M + N + K)
+    for pad in (0, 4, 3):
+        new = lambda r, c: torch.randn(r, c + pad, device=cuda_dev, generator=g)[:, :c]  # noqa: E731
+        a = new(K, M) if op == 2 else new(M, K)
+        b = new(N, K) if op == 1 else new(K, N)
+        c, bias = new(M, N), (torch.randn(N, device=cuda_dev, generator=g) if op != 2 and pad else None)
+        ad, bd = a.double(), b.double()
+        ref = ad @ bd if op == 0 else ad @ bd.t() if op == 1 else c.double() + ad.t() @ bd
+        ref = ref if bias is None else ref + bias.double()
+        rc = lib.mamba_b200_sgemm_rows(h.ptr, torch.cuda.current_stream().cuda_stream, op, a.data_ptr(), a.stride(0), b.data_ptr(),
+                                       b.stride(0), None if bias is None else bias.data_ptr(), c.data_ptr(), c.stride(0), M, N, K)
+        h.check(rc, "sgemm_rows")
+        torch.cuda.synchronize()
+        assert float((c.double() - ref).abs().max()) <= 3e-6 * K ** 0.5 * max(1.0, float(ref.abs().max()) / K ** 0.5)
