@@ -388,6 +388,7 @@ class _DecodePlan:
         whole = all(t.data_ptr() == w._a_neg_all[l].data_ptr() for l, t in enumerate(w.a_neg))
         a.workspace_bytes = lib.mamba_b200_decode_workspace_bytes(self.handle.ptr, C.byref(a)) if whole else 0
         self.ok = a.workspace_bytes > 0
+        self.replay = _Replay(w.device)  # of the operators' launches where the kernel does not take the model
         if self.ok:
             self.ws = torch.zeros(a.workspace_bytes, dtype=torch.uint8, device=w.device)
             a.workspace = self.ws.data_ptr()
@@ -474,8 +475,18 @@ class GpuMambaBackbone:
             plan.args.residual, plan.args.out = temporal.data_ptr(), out.data_ptr()
             plan.launch()
             return out
+        if (B <= self.batch and temporal.is_cuda and temporal.dtype == torch.float32 and temporal.is_contiguous()
+                and not torch.cuda.is_current_stream_capturing()):
+            branch = plan.replay.run(temporal.data_ptr(), lambda: self._step_layers(temporal))
+        else:
+            branch = self._step_layers(temporal)
+        # (the caller keeps the result, so the norm that writes it is no part of a replay)
+        out, _ = ops.residual_rmsnorm_fwd(temporal, branch, w.tail("master")["norm_f"], eps=c.rms_norm_eps, out_dtype=w.dtype)
+        return out
+
+    def _step_layers(self, res):
+        c, w, B = self.cfg, self.w, res.shape[0]
         di, N, dr = c.d_inner, c.d_state, c.dt_rank
-        res = temporal
         branch = None
         for l in range(c.n_layers):
             p, pm = w.layer(l), w.layer(l, "master")
@@ -491,8 +502,7 @@ class GpuMambaBackbone:
             y = ops.selective_scan_step(u, delta, xdbl[:, dr:dr + N], xdbl[:, dr + N:], w.a_neg[l], pm["d_param"],
                                         self.ssm[l], proj[:, di:])
             branch = y @ p["out_proj_w"]
-        out, _ = ops.residual_rmsnorm_fwd(res, branch, w.tail("master")["norm_f"], eps=c.rms_norm_eps, out_dtype=w.dtype)
-        return out
+        return branch
 
 
 class GpuMambaLM:

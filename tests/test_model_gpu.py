@@ -214,3 +214,25 @@ def test_passes_that_come_again_equal_the_first_ones(cuda_dev, shape, dt):
     for a, b in zip(*runs):
         assert rel_err(b.float().cpu().numpy(), a.float().cpu().numpy()) <= (1e-5 if dt == "f32" else 2e-2)
     mb.ffi.default_handle(0).check_status()
+
+
+def test_steps_by_operators_that_come_again_equal_the_first_ones(cuda_dev):
+    """A model the one-launch step does not take (d_state 8): the third step with the same rows is a replay."""
+    import torch
+
+    import mamba_rs_b200 as mb
+    w = mb.MambaWeights(mb.MambaConfig(d_model=64, n_layers=2, d_state=8), cuda_dev, dtype=torch.float32).init_random(3)
+    again, once = mb.GpuMambaBackbone(w, 3), mb.GpuMambaBackbone(w, 3)
+    assert not again._plan(3).ok
+    buf, xs = torch.empty(3, 64, device=cuda_dev), torch.randn(6, 3, 64, device=cuda_dev)
+    got = []
+    for x in xs:
+        buf.copy_(x)
+        got.append((again.step(buf), buf.clone()))
+    assert again._plan(3).replay.kept
+    for x, (out, res) in zip(xs, got):
+        once._plan(3).replay.seen.clear()
+        y = x.clone()
+        ref = once.step(y)
+        assert rel_err(out.cpu().numpy(), ref.cpu().numpy()) <= 1e-6 and rel_err(res.cpu().numpy(), y.cpu().numpy()) <= 1e-6
+    assert not once._plan(3).replay.kept and torch.equal(again.ssm, once.ssm) and torch.equal(again.conv, once.conv)
