@@ -47,6 +47,8 @@ struct M3BwdParams {
     float *ws_dgam;    // [B,T,nh] dgamma (diagonal part)
     float *ws_dscl;    // [B,T,nh] dscale
     float *ws_dD;      // [B,nh]
+    float* ws_hand;     // WRAP: per boundary, a state (or its gradient) in f32 and a part of dD
+    unsigned* ws_flag;  // WRAP: per boundary, 1 once it is there
     int B, T, nh, hd, N;
     int* status;
 };
@@ -362,13 +364,40 @@ constexpr uint32_t kStateTile = NS * HD * 2;  // bytes of one 16-bit state copy
 // SEG: what a CTA leaves for the others, f32 [128 n][64 p] each, and log2 of the decay over its chunks
 constexpr uint32_t kLocS = kQ, kLocD = kM2, kTot = kTmemSlot + 8;
 
-template <typename Th, bool SEG>
+//
+// WRAP: more pairs than SMs that do not fill whole waves (256 on 148 leave a quarter of two waves idle).
+// The pairs' work is laid out on a line, measured in time (5 for a chunk of A, 21 for one of B), and cut
+// into one equal length per CTA.  A pair that a cut divides is begun by the CTA behind the cut, first
+// thing, and finished by the CTA ahead of it, last thing, which takes the state (or dS, if the cut lies
+// in B) over through memory; as a pair is shorter than a CTA's length, it is there by then.
+enum Mode { kOne, kSeg, kWrap };
+constexpr int kCostA = 5, kCostB = 21, kHand = NS * HD + 64;  // floats of a hand-over
+
+struct Cut {  // what a cut makes of the pair it falls into
+    int head, steps_a, chunks_b;  // begun: steps_a products of A (nc: all of it), chunks_b chunks of B
+    bool any, ahead, behind;      // divided; wholly ahead of the cut; wholly behind it
+};
+__device__ __forceinline__ Cut cut_at(long long x, int nc, int heads) {
+    const long long cost_a = static_cast<long long>(kCostA) * (nc - 1), u = cost_a + static_cast<long long>(kCostB) * nc;
+    Cut c;
+    c.head = static_cast<int>(x / u);
+    const long long before = x - c.head * u, r = u - before;  // r: what the CTA behind the cut should do of it
+    c.any = before > 0 && c.head < heads;
+    c.steps_a = r <= cost_a ? static_cast<int>((r + kCostA / 2) / kCostA) : nc;
+    c.chunks_b = r <= cost_a ? 0 : static_cast<int>((r - cost_a + kCostB / 2) / kCostB);
+    if (c.chunks_b == 0) c.steps_a = min(c.steps_a, nc - 1);  // nothing of B: what is handed over is the state
+    c.ahead = c.any && c.steps_a == 0;
+    c.behind = c.any && c.chunks_b >= nc;
+    return c;
+}
+
+template <typename Th, int MODE>
 __global__ void __launch_bounds__(256) m3_ssd_bwd_tc_kernel(const __grid_constant__ M3BwdParams p) {
     extern __shared__ __align__(1024) unsigned char smem[];
     // two threads per step: (row tid, half) share TMEM lane tid and split its columns
     const int tid = threadIdx.x & 127, half = threadIdx.x >> 7, warp = (threadIdx.x >> 5) & 3, lane = tid & 31;
+    constexpr bool SEG = MODE == kSeg;
     const int nrank = SEG ? static_cast<int>(gridDim.x) / p.nh : 1, rank = SEG ? blockIdx.x % nrank : 0;
-    const int h = SEG ? blockIdx.x / nrank : blockIdx.x, b = blockIdx.y;
     const int T = p.T, nh = p.nh;
     // headdim <= 64, d_state <= 128 (multiples of 8): full-size tiles, missing columns zero-filled
     const int hdv = p.hd, nsv = p.N;
@@ -406,20 +435,46 @@ __global__ void __launch_bounds__(256) m3_ssd_bwd_tc_kernel(const __grid_constan
     const Th* Qg = static_cast<const Th*>(p.Q);
     const Th* dyg = static_cast<const Th*>(p.dy);
     Th* dxg = static_cast<Th*>(p.dx);
-    const float Dv = p.Dh[h];
     const int nc = (T + CS - 1) / CS;
     const int per_rank = SEG ? (nc + nrank - 1) / nrank : nc;  // this CTA's chunks: c_lo .. c_hi - 1
     const int c_lo = SEG ? min(nc, rank * per_rank) : 0, c_hi = SEG ? min(nc, c_lo + per_rank) : nc;
+    uint32_t ph[4] = {0, 0, 0, 0}, scph = 0, tfph[2] = {0, 0};
+    bool ok = true;
+    // WRAP: this CTA's stretch of the line
+    const long long unit = static_cast<long long>(kCostA) * (nc - 1) + static_cast<long long>(kCostB) * nc;
+    const long long line = (unit * nh * p.B + gridDim.x - 1) / gridDim.x, x0 = line * blockIdx.x, x1 = x0 + line;
+    for (int j = MODE == kWrap ? static_cast<int>(x0 / unit) : 0; MODE != kWrap || (j < nh * p.B && j * unit < x1); ++j) {
+    const int h = MODE == kWrap ? j % nh : SEG ? blockIdx.x / nrank : blockIdx.x, b = MODE == kWrap ? j / nh : blockIdx.y;
+    // chunks whose entering states are walked (the last one's needs no product), chunks of B; the cut at
+    // which the pair is handed over by this CTA, or to it
+    int a_lo = c_lo, a_hi = c_hi, b_lo = c_lo, b_hi = c_hi, give = -1, get = -1;
+    if constexpr (MODE == kWrap) {
+        if (j * unit < x0) {
+            const Cut c = cut_at(x0, nc, nh * p.B);
+            if (c.ahead) continue;
+            if (!c.behind) {
+                give = blockIdx.x;
+                a_hi = c.steps_a;
+                b_lo = nc - c.chunks_b;
+            }
+        } else if ((j + 1) * unit > x1) {
+            const Cut c = cut_at(x1, nc, nh * p.B);
+            if (c.behind) continue;
+            if (!c.ahead) {
+                get = blockIdx.x + 1;
+                a_lo = c.steps_a;
+                b_hi = nc - c.chunks_b;
+            }
+        }
+    }
+    const float Dv = p.Dh[h];
     unsigned char* ws_st = reinterpret_cast<unsigned char*>(p.ws_states) +
                            (static_cast<size_t>(b) * nh + h) * nc * kStateTile;
-    uint32_t ph[4] = {0, 0, 0, 0};
-    bool ok = true;
     const uint4 zero4 = make_uint4(0, 0, 0, 0);
 
     // The per-row adt, dt, trap of a chunk come as three TMA boxes issued before the tile
     // copies (so they land while those are being issued) instead of 128-byte-strided register
     // loads with their latency exposed; without the maps (nheads % 4 != 0) the loads remain.
-    uint32_t scph = 0;
     const int hcol = h & 3;
     auto issue_scalars_now = [&](int t0) {  // one thread
         if (p.sc_tma) {
@@ -489,7 +544,6 @@ __global__ void __launch_bounds__(256) m3_ssd_bwd_tc_kernel(const __grid_constan
     // zeros), the 16-bit state copy of a chunk by one contiguous bulk copy.
     // barrier 5 for the backward pass and the even chunks of the state pass, 6 for its odd
     // chunks (two requests are in flight there)
-    uint32_t tfph[2] = {0, 0};
     auto load_qk = [&](uint32_t tile, const CUtensorMap* map, int t0, int bi) {
 #pragma unroll
         for (int sub = 0; sub < 2; ++sub)
@@ -628,20 +682,42 @@ __global__ void __launch_bounds__(256) m3_ssd_bwd_tc_kernel(const __grid_constan
         cluster_sync();  // nobody reads this CTA's shared memory any more
     }
 
-    // ---------------- A. forward: 16-bit copies of the entering states ----------------
-    if (threadIdx.x == 0 && c_hi - c_lo > 1) {
-        issue_scalars_now(c_lo * CS);
-        request_pair(c_lo, 0, &p.tm_k, &p.tm_x);
+    if constexpr (MODE == kWrap) {
+        if (get >= 0) {
+            if (threadIdx.x == 0) {
+                unsigned v = 0;
+                for (int it = 0; it < (1 << 21) && v == 0; ++it)
+                    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p.ws_flag + get) : "memory");
+                if (v == 0) atomicCAS(p.status, kStatusOk, kStatusBarrierTimeout);
+            }
+            __syncthreads();
+            const float* src = p.ws_hand + static_cast<long long>(get) * kHand + tid * HD + half * 32;
+            float sv[32];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const float4 v = __ldcg(reinterpret_cast<const float4*>(src) + i);
+                sv[4 * i] = v.x; sv[4 * i + 1] = v.y; sv[4 * i + 2] = v.z; sv[4 * i + 3] = v.w;
+            }
+            tmem_st32(lane_addr + cDS + half * 32, sv);
+            if (a_lo == nc) copy16(smem + kDS, sv);  // (published by the fence and barrier ahead of the first products)
+        }
     }
-    for (int c = c_lo; c < c_hi; ++c) {
-        const int t0 = c * CS, nv = min(CS, T - t0), i0 = c - c_lo;
+
+    // ---------------- A. forward: 16-bit copies of the entering states ----------------
+    const int a_top = min(a_hi, c_hi - 1);  // products end here
+    if (threadIdx.x == 0 && a_lo < a_top) {
+        issue_scalars_now(a_lo * CS);
+        request_pair(a_lo, 0, &p.tm_k, &p.tm_x);
+    }
+    for (int c = a_lo; c < a_hi; ++c) {
+        const int t0 = c * CS, nv = min(CS, T - t0), i0 = c - a_lo;
         const bool last = c + 1 == c_hi;
         float run = 0.0f, g = 0.0f, s = 0.0f;
         if (!last) {
             // (tiles of chunk c + 1: last read by chunk c - 1)
-            if (threadIdx.x == 0 && c + 2 < c_hi) request_pair(c + 1, i0 + 1, &p.tm_k, &p.tm_x);
+            if (threadIdx.x == 0 && c + 1 < a_top) request_pair(c + 1, i0 + 1, &p.tm_k, &p.tm_x);
             load_scalars(t0, nv, run, g, s);
-            if (threadIdx.x == 0 && c + 2 < c_hi) issue_scalars_now(t0 + CS);  // the staging was read just above
+            if (threadIdx.x == 0 && c + 1 < a_top) issue_scalars_now(t0 + CS);  // the staging was read just above
             const float wt = tid < nv ? ex2((dA[nv - 1] - run) * kLog2e) * s : 0.0f;
             wait_tiles(i0 & 1);
             weigh((i0 & 1) ? kSin : kV, kDY, wt);
@@ -674,7 +750,7 @@ __global__ void __launch_bounds__(256) m3_ssd_bwd_tc_kernel(const __grid_constan
     fence_after();
 
     // ---------------- B. backward over the chunks ----------------
-    bool has_ds = false;
+    bool has_ds = MODE == kWrap && get >= 0 && a_lo == nc;
     float dD_acc = 0.0f;
     if (SEG && c_lo < c_hi && c_hi < nc) {  // the gradient from the CTAs behind this one
         float sv[32];
@@ -697,8 +773,8 @@ __global__ void __launch_bounds__(256) m3_ssd_bwd_tc_kernel(const __grid_constan
         tma_load_4d(smem + kDY, &p.tm_dy, &bars[5], 0, h, t0, b);
         if (c > 0) bulk_load(smem + kSin, ws_st + static_cast<size_t>(c) * kStateTile, kStateTile, &bars[5]);
     };
-    if (threadIdx.x == 0 && c_lo < c_hi) request_tiles(c_hi - 1, kQ, kK);
-    for (int c = c_hi - 1, it = 0; c >= c_lo; --c, ++it) {
+    if (threadIdx.x == 0 && b_lo < b_hi) request_tiles(b_hi - 1, kQ, kK);
+    for (int c = b_hi - 1, it = 0; c >= b_lo; --c, ++it) {
         const bool par = (it & 1) != 0;
         const uint32_t tQ = par ? kM1 : kQ, tK = par ? kM2 : kK, tM1 = par ? kQ : kM1, tM2 = par ? kK : kM2;
         const int t0 = c * CS, nv = min(CS, T - t0);
@@ -967,10 +1043,10 @@ __global__ void __launch_bounds__(256) m3_ssd_bwd_tc_kernel(const __grid_constan
             commit(&bars[2]);
         }
         wait_bar(2);
-        if (threadIdx.x == 0 && c > c_lo) request_tiles(c - 1, tM1, tM2);
+        if (threadIdx.x == 0 && c > b_lo) request_tiles(c - 1, tM1, tM2);
         // ---- epilogue 3 ----
         // 16-bit copy of the new dS for the next (earlier) chunk
-        if (c > c_lo) {
+        if (c > b_lo) {
             float sv[32];
             tmem_ld32(lane_addr + cDS + half * 32, sv);
             copy16(smem + kDS, sv);
@@ -1058,7 +1134,29 @@ __global__ void __launch_bounds__(256) m3_ssd_bwd_tc_kernel(const __grid_constan
                 for (int q = 1; q < nrank; ++q) tot += ld_cluster1(cluster_addr(sbase + kTot, q));
             cluster_sync();
         }
+        if constexpr (MODE == kWrap) {
+            if (give >= 0) {
+                float* dst = p.ws_hand + static_cast<long long>(give) * kHand;
+                float sv[32];
+                tmem_ld32(lane_addr + cDS + half * 32, sv);
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    reinterpret_cast<float4*>(dst + tid * HD + half * 32)[i] = make_float4(sv[4 * i], sv[4 * i + 1], sv[4 * i + 2], sv[4 * i + 3]);
+                if (threadIdx.x == 0) dst[NS * HD] = tot;
+                fence_before();
+                __syncthreads();
+                fence_after();
+                if (threadIdx.x == 0) {  // the release covers what the other threads wrote before the barrier
+                    __threadfence();
+                    asm volatile("st.release.gpu.global.u32 [%0], 1;" ::"l"(p.ws_flag + give) : "memory");
+                }
+                continue;
+            }
+            if (get >= 0) tot += __ldcg(p.ws_hand + static_cast<long long>(get) * kHand + NS * HD);
+        }
         if (threadIdx.x == 0 && rank == 0) p.ws_dD[static_cast<long long>(b) * nh + h] = tot;
+    }
+    if (MODE != kWrap) break;
     }
     __syncthreads();
     if (threadIdx.x < 32)
@@ -1091,6 +1189,15 @@ static void m3_bwd_ws(bool tc, int B, int T, int nh, int hd, int N, size_t* o_g,
     *total = st + 2 * v + al(sizeof(float) * static_cast<size_t>(B) * nh);
 }
 
+// The line of pairs cut into one length per SM (WRAP): from one pair per SM on, where whole waves would
+// leave more than 4 % of the SMs' time idle.
+constexpr int kWrapSms = 160;  // hand-overs the workspace has room for
+static bool m3_bwd_wraps(long long heads, int sms) {
+    const long long waves = (heads + sms - 1) / sms;
+    return heads > sms && sms < kWrapSms && heads * 100 < waves * sms * 96;
+}
+static size_t m3_bwd_wrap_bytes() { return 1024 + sizeof(float) * kWrapSms * tcb::kHand; }
+
 int m3_bwd_configure(Ctx* c) {
     const int smem = static_cast<int>(m3_bwd_smem(64, 128));
     MB200_CUDA_CHECK(c, cudaFuncSetAttribute(reinterpret_cast<const void*>(m3_ssd_bwd_kernel<float>),
@@ -1099,10 +1206,12 @@ int m3_bwd_configure(Ctx* c) {
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     MB200_CUDA_CHECK(c, cudaFuncSetAttribute(reinterpret_cast<const void*>(m3_ssd_bwd_kernel<__nv_bfloat16>),
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    const void* tc_fns[4] = {reinterpret_cast<const void*>(tcb::m3_ssd_bwd_tc_kernel<__half, false>),
-                             reinterpret_cast<const void*>(tcb::m3_ssd_bwd_tc_kernel<__nv_bfloat16, false>),
-                             reinterpret_cast<const void*>(tcb::m3_ssd_bwd_tc_kernel<__half, true>),
-                             reinterpret_cast<const void*>(tcb::m3_ssd_bwd_tc_kernel<__nv_bfloat16, true>)};
+    const void* tc_fns[6] = {reinterpret_cast<const void*>(tcb::m3_ssd_bwd_tc_kernel<__half, tcb::kOne>),
+                             reinterpret_cast<const void*>(tcb::m3_ssd_bwd_tc_kernel<__nv_bfloat16, tcb::kOne>),
+                             reinterpret_cast<const void*>(tcb::m3_ssd_bwd_tc_kernel<__half, tcb::kSeg>),
+                             reinterpret_cast<const void*>(tcb::m3_ssd_bwd_tc_kernel<__nv_bfloat16, tcb::kSeg>),
+                             reinterpret_cast<const void*>(tcb::m3_ssd_bwd_tc_kernel<__half, tcb::kWrap>),
+                             reinterpret_cast<const void*>(tcb::m3_ssd_bwd_tc_kernel<__nv_bfloat16, tcb::kWrap>)};
     for (const void* fn : tc_fns)
         MB200_CUDA_CHECK(c, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, tcb::kSmem));
     return MAMBA_B200_OK;
@@ -1124,6 +1233,7 @@ extern "C" MAMBA_B200_API long long mamba_b200_m3_ssd_bwd_workspace_bytes_for(in
     if (B <= 0 || T <= 0 || nh <= 0 || hd <= 0 || N <= 0) return 0;
     size_t a, b2, d, total;
     m3_bwd_ws(m3_bwd_tc_shape(dtype, hd, N), B, T, nh, hd, N, &a, &b2, &d, &total);
+    if (m3_bwd_tc_shape(dtype, hd, N) && static_cast<long long>(B) * nh > 128) total += m3_bwd_wrap_bytes();
     return static_cast<long long>(total);
 }
 
@@ -1183,16 +1293,32 @@ extern "C" MAMBA_B200_API int mamba_b200_m3_ssd_bwd(void* handle, void* stream,
         const bool f16 = a.dtype == MAMBA_B200_F16;
         // (the outer CTAs of a cluster have one pass more than an undivided one, those between them two.)  bf16,
         // 64 x 128: 4 heads x 4096 steps 114 us (one CTA each: 446), 24 x 2048 104 (224), 64 x 4096 285 (450)
+        const bool wrap = m3_bwd_wraps(static_cast<long long>(a.B) * a.nh, c->sm_count) &&
+                          a.workspace_bytes >= static_cast<long long>(total + m3_bwd_wrap_bytes());
+        // 8 x 4096 steps x 32 heads of 64 x 128, bf16: 861 us (931 in two waves).  False: plain launch.
+        auto wrap_launch = [&]() {
+            p.ws_flag = reinterpret_cast<unsigned*>(ws + total);
+            p.ws_hand = reinterpret_cast<float*>(ws + total + 1024);
+            if (cudaMemsetAsync(p.ws_flag, 0, 1024, st) != cudaSuccess) return false;
+            void* args[1] = {&p};
+            const void* fn = f16 ? reinterpret_cast<const void*>(tcb::m3_ssd_bwd_tc_kernel<__half, tcb::kWrap>)
+                                 : reinterpret_cast<const void*>(tcb::m3_ssd_bwd_tc_kernel<__nv_bfloat16, tcb::kWrap>);
+            // cooperative: a CTA may wait for another one, so all of them have to be resident
+            if (cudaLaunchCooperativeKernel(fn, dim3(c->sm_count), dim3(256), args, tcb::kSmem, st) == cudaSuccess) return true;
+            cudaGetLastError();
+            return false;
+        };
         const int ranks = m3_cluster_ranks(a.B * a.nh, (a.T + tcb::CS - 1) / tcb::CS, 14.1, 17.0, 19.5, 5.0);
-        if (ranks > 1) {
-            const void* fn = f16 ? reinterpret_cast<const void*>(tcb::m3_ssd_bwd_tc_kernel<__half, true>)
-                                 : reinterpret_cast<const void*>(tcb::m3_ssd_bwd_tc_kernel<__nv_bfloat16, true>);
+        if (wrap && wrap_launch()) {
+        } else if (ranks > 1) {
+            const void* fn = f16 ? reinterpret_cast<const void*>(tcb::m3_ssd_bwd_tc_kernel<__half, tcb::kSeg>)
+                                 : reinterpret_cast<const void*>(tcb::m3_ssd_bwd_tc_kernel<__nv_bfloat16, tcb::kSeg>);
             void* args[1] = {&p};
             MB200_CUDA_CHECK(c, launch_cluster(fn, dim3(a.nh * ranks, a.B), dim3(256), tcb::kSmem, st, ranks, args));
         } else if (f16) {
-            tcb::m3_ssd_bwd_tc_kernel<__half, false><<<grid, 256, tcb::kSmem, st>>>(p);
+            tcb::m3_ssd_bwd_tc_kernel<__half, tcb::kOne><<<grid, 256, tcb::kSmem, st>>>(p);
         } else {
-            tcb::m3_ssd_bwd_tc_kernel<__nv_bfloat16, false><<<grid, 256, tcb::kSmem, st>>>(p);
+            tcb::m3_ssd_bwd_tc_kernel<__nv_bfloat16, tcb::kOne><<<grid, 256, tcb::kSmem, st>>>(p);
         }
     } else if (a.dtype == MAMBA_B200_F32) m3_ssd_bwd_kernel<float><<<grid, 256, smem, st>>>(p);
     else if (a.dtype == MAMBA_B200_F16) m3_ssd_bwd_kernel<__half><<<grid, 256, smem, st>>>(p);

@@ -83,6 +83,19 @@ def test_chunks_divided_over_a_cluster_match_cuda_core_path(cuda_dev, shape, dt)
         assert rel_err(got[k], ref[k]) <= TOL[dt], k
 
 
+# more pairs than SMs, not in whole waves: pairs cut in the state pass and in the backward, of one, a few and
+# several chunks, with a ragged last one
+@pytest.mark.parametrize("dt", ["bf16", "f16"])
+@pytest.mark.parametrize("shape", [(5, 100, 37, 64, 128), (2, 300, 80, 32, 64), (3, 1100, 64, 64, 128), (8, 260, 32, 64, 128)],
+                         ids=lambda s: "B%dT%dnh%dhd%dN%d" % s)
+def test_pairs_cut_between_ctas_match_cuda_core_path(cuda_dev, shape, dt):
+    i, dy = case(shape, dt, seed=shape[1])
+    got, again, ref = run_gpu(i, dy, dt, cuda_dev), run_gpu(i, dy, dt, cuda_dev), run_gpu(i, dy, "f32", cuda_dev)
+    for k in ("dx",) + F32_OUT:
+        assert rel_err(got[k], ref[k]) <= TOL[dt], k
+        np.testing.assert_array_equal(got[k], again[k])
+
+
 def test_dD_accumulates_and_rerun_is_identical(cuda_dev):
     import torch
     i, dy = case((2, 70, 2, 16, 32), "f32", seed=9)
