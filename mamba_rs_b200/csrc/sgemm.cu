@@ -233,9 +233,10 @@ extern "C" MAMBA_B200_API int mamba_b200_sgemm_rows(void* handle, void* stream, 
     }
     const int tiles = (N + sg::BN - 1) / sg::BN, rows = (M + sg::BM - 1) / sg::BM;
     if (rows > 65535) return fail(c, MAMBA_B200_ERR_SHAPE, "sgemm_rows: %d rows", M);
-    // parts of K until there are four CTAs for every SM, none shorter than two tiles
+    // parts of K until there are two CTAs for every SM (more only adds to the sums: 64 rows, 768 x 3072 took
+    // 15.3 us with four, 13.4 with two, 18.5 with one), none shorter than two tiles
     int parts = 1;
-    while (parts < 8 && static_cast<long long>(tiles) * rows * parts < 4 * 148 && K >= parts * 4 * sg::BK) parts *= 2;
+    while (parts < 8 && static_cast<long long>(tiles) * rows * parts < 2 * 148 && K >= parts * 4 * sg::BK) parts *= 2;
     p.kper = ((K + parts - 1) / parts + sg::BK - 1) / sg::BK * sg::BK;
     const bool vec = al(a, lda) && al(b, ldb) && K % 4 == 0 && (op == 1 || N % 4 == 0);
     const void* fns[4] = {reinterpret_cast<const void*>(sg::rows_kernel<0, false>), reinterpret_cast<const void*>(sg::rows_kernel<0, true>),

@@ -207,11 +207,11 @@ class _Launcher:
 def _product(go, op, a, b, out):
     """out = a b (op 0) or a b^T (op 1), inside go.begin().  In f32 with few output tiles and a long
     contraction the rows kernel has the parts of K that the library's tiles leave to one SM (32 rows,
-    768 x 3072: 8.6 us for 14.5; 1536 x 768: 7.9 for 18.1); from 64 tiles of 32 x 64 on, or under a
+    768 x 3072: 8.6 us for 14.5; 1536 x 768: 7.9 for 18.1); beyond 96 tiles of 32 x 64, or under a
     dozen rows or 512 steps of K, the library is as fast."""
     M, K = a.shape
     N = out.shape[1]
-    if a.dtype == torch.float32 and M >= 12 and K >= 512 and ((M + 31) // 32) * ((N + 63) // 64) <= 64:
+    if a.dtype == torch.float32 and M >= 12 and K >= 512 and ((M + 31) // 32) * ((N + 63) // 64) <= 96:
         go.call(go.lib.mamba_b200_sgemm_rows, op, a.data_ptr(), a.stride(0), b.data_ptr(), b.stride(0), None, out.data_ptr(),
                 out.stride(0), M, N, K)
     else:
@@ -613,6 +613,8 @@ class _TrainPlan:
         self.norm_f = w.tail("master")["norm_f"].data_ptr()
         self.fwd_at = self.bwd_at = None
         self.replay, self.ids = _Replay(w.device), None
+        # few f32 rows: their sum is one more product (of the rows kernel)
+        self.ones = torch.ones(B * T, 1, device=w.device) if w.dtype == torch.float32 and B * T <= 32 else None
         a_layer = B * T * (4 * (c.d_model + 1) + self.es * (c.d_model + 5 * di + xd)) + 4 * B * self.blocks * di * N
         written = c.n_layers * a_layer + B * T * self.es * (w.vocab or 0) + self.fwd_ws + self.bwd_ws
         self.launch_bound = w.device.type == "cuda" and written <= 512 << 20
@@ -814,7 +816,10 @@ class MambaLMTrainer:
                 acc(g["out_proj_w"], y, d_out)
                 _product(go, 1, d_out, lay.w_out, d_y)
                 go.call(scan, lay.scan_b)
-                g["dt_proj_b"].add_(torch.sum(d_delta, 0, dtype=torch.float32))
+                if plan.ones is not None:
+                    acc(g["dt_proj_b"].view(1, di), plan.ones, d_delta)
+                else:
+                    g["dt_proj_b"].add_(torch.sum(d_delta, 0, dtype=torch.float32))
                 acc(g["dt_proj_w"], xdbl[:, :dr], d_delta)
                 _product(go, 1, d_delta, lay.w_dt, d_dt_in)
                 d_bc_out.copy_(d_bc_in)
