@@ -575,6 +575,14 @@ __global__ void __launch_bounds__(256, 1) m3_ssd_fwd_tc_kernel(const __grid_cons
                                           : 0.0f;
         }
     };
+    // and as what the first chunk walked in full starts from
+    auto enter_state = [&]() {
+        float sv[32];
+        carried_state(sv);
+        tmem_st32(lane_addr + cS + half * 32, sv);
+        copy_state(sv);
+        fence_proxy_async();
+    };
     // w o V of chunk j (and its remainders): the B operand of the state update
     auto weigh_v = [&](const float* dA, const float* scl, int nv, uint32_t tV) {
         const float wt = tid < nv ? ex2((dA[nv - 1] - dA[tid]) * kLog2e) * scl[tid] : 0.0f;
@@ -695,6 +703,8 @@ __global__ void __launch_bounds__(256, 1) m3_ssd_fwd_tc_kernel(const __grid_cons
             copy_state(sv);
             fence_proxy_async();  // (published by the barriers ahead of the first MMA group)
         }
+        // ahead of the barrier: past it the CTA of the last chunk may already replace the carried state in place
+        if (CARRY && rank == 0) enter_state();
         cluster_sync();  // nobody reads this CTA's shared memory any more
     } else {
         if (CARRY) {
@@ -705,13 +715,7 @@ __global__ void __launch_bounds__(256, 1) m3_ssd_fwd_tc_kernel(const __grid_cons
         }
         stage_scalars(0);
         if (GEN) load_vel(0);
-    }
-    if (CARRY && rank == 0) {
-        float sv[32];
-        carried_state(sv);
-        tmem_st32(lane_addr + cS + half * 32, sv);
-        copy_state(sv);
-        fence_proxy_async();
+        if (CARRY) enter_state();
     }
 
     for (int c = c_lo; c < c_hi; ++c) {

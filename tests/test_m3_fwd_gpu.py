@@ -215,3 +215,30 @@ def test_chunks_divided_over_a_cluster_match_sequential(cuda_dev, shape, carry):
     assert rel_err(out[0][1], out[1][1]) <= (1e-4 if carry else TOL["bf16"])
     np.testing.assert_array_equal(out[0][2], out[1][2])
     np.testing.assert_array_equal(out[0][3], out[1][3])
+
+
+@pytest.mark.parametrize("T,nh", [(7169, 1), (7177, 3)])
+def test_a_divided_window_starts_from_the_state_that_entered(cuda_dev, T, nh):
+    """57 chunks over eight CTAs: the last has one short chunk and then replaces the state in place, while the
+    first still has eight to walk in full from the one that entered.  Every call must be the same."""
+    import torch
+
+    import mamba_rs_b200 as mb
+    i = rounded(synth.m3_ssd_inputs(1, T, nh, 64, 128, seed=T), "bf16")
+    args = [to_dev(i[k], cuda_dev, torch.bfloat16 if k in ("x", "K", "Q") else None) for k in ARGS]
+    g = torch.Generator().manual_seed(T)
+    st0 = [100 * torch.randn(*s, generator=g).to(cuda_dev) for s in ((1, nh, 64, 128), (1, nh, 128), (1, nh, 64))]
+
+    def call(seq):
+        ssm, ks, vs = (t.clone() for t in st0)
+        y = mb.m3_ssd_fwd(*args, ssm_state=ssm, k_state=ks, v_state=vs, carry_in=True, force_sequential=seq)
+        return y, ssm
+    y, ssm = call(False)
+    ry, rs = call(True)
+    # the state that entered fills the first rows of y (100 against the inputs' 1), so a wrong one shows there
+    assert rel_err(y.float().cpu().numpy(), ry.float().cpu().numpy()) <= TOL["bf16"]
+    assert rel_err(ssm.cpu().numpy(), rs.cpu().numpy()) <= 1e-4
+    for _ in range(20):
+        y2, ssm2 = call(False)
+        assert torch.equal(y2, y) and torch.equal(ssm2, ssm)
+    mb.ffi.default_handle(0).check_status()
