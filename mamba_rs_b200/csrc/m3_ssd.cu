@@ -10,7 +10,7 @@
 //    Y2 = Q S_in^T, S^T <- exp(dA_end) S^T + K^T (w o V).
 //    With a carried state the same kernel starts from it (CARRY).
 //  * m3_ssd_seq_kernel — the sequential definition (eight rows p per warp, state in
-//    registers) for every other shape / dtype and for short carried windows.
+//    registers) for every other shape / dtype, and for carried windows that are short or f16.
 #include <string.h>
 
 #include <type_traits>
@@ -203,9 +203,9 @@ constexpr int CS = 128, HD = 64, NS = 128;
 // 16-bit copy of the new state for the next chunk's Y2; then f32 vectors, barriers.
 constexpr uint32_t kQ0 = 0, kK0 = 65536, kV0 = 131072, kQKStride = 32768, kVStride = 16384;
 constexpr uint32_t kM = 163840, kVw = 196608, kS = 196608;
-// carried state: one Q, K and V buffer; remainders of M, w o V and the state copy behind them
-constexpr uint32_t kCarryK = 32768, kCarryV = 65536, kMlo = 81920, kVwLo = 114688, kSlo = kVwLo;
-static_assert(kVwLo + 16384 <= kM, "carry layout");
+// carried state: one Q, K and V buffer; remainders of M, w o V (two) and the state copy behind them
+constexpr uint32_t kCarryK = 32768, kCarryV = 65536, kMlo = 81920, kVwLo = 114688, kSlo = kVwLo, kVwRest = 131072;
+static_assert(kVwRest + 16384 <= kM, "carry layout");
 // f32 dA[128], scale[128], gamma[128], dA*log2(e)[128], dt[128] per chunk, two sets: a chunk's
 // set is written while slower threads may still read the previous chunk's
 constexpr uint32_t kVec = 212992, kVecSet = 5 * 128;
@@ -233,12 +233,15 @@ constexpr uint32_t cG = 0, cY1 = 256, cY2 = 320, cS = 384, kTmemCols = 512;
 // CARRY: continue from ssm_state / k_state / v_state.  In the shifted form the state that enters
 // is S = h + dt_0 (1 - trap_0) k_prev v_prev^T, so it is loaded into TMEM and the first chunk is
 // a chunk like any other.  A carried state is kept to f32 accuracy as the sequential definition
-// keeps it: every rounded MMA operand (M, w o V, the state copy) is a 16-bit value plus a second
-// one with the rounding that was left, two products each (K, Q and V are 16-bit inputs and
-// exact), which leaves 2^-17 of each term.  The second tiles take the room of the second Q / K /
-// V buffers: Q of the next chunk is requested when the first MMA group has read it, K and V when
-// the second has.  8 x 256 steps x 32 heads of 64 x 128, bf16: 43 us (2050 us sequentially), the
-// state within 3e-6 of the sequential kernel's.
+// keeps it (K, Q and V are 16-bit inputs and exact): w o V, which the state is made of, is three
+// bf16 values, f32's 24 bits, with a product each; M and the state copy, which only y is made of,
+// are two, 2^-17 of each term against the 2^-9 that y is rounded to.  The further tiles take the
+// room of the second Q / K / V buffers: Q of the next chunk is requested when the first MMA group
+// has read it, K and V when the second has.  8 x 256 steps x 32 heads of 64 x 128: 44 us (393 us by
+// the sequential kernel).  The state's error against 64 bits there is 1.1e-6 (sequentially 3.2e-6),
+// over 1 x 1000 steps 6.2e-7 (5.4e-7; 2.5e-6 with w o V of two values).  bf16 only: f16's range
+// does not hold the remainders (x of 1e-3 left an error of 4e-3) nor products beyond 65504, so a
+// carried f16 window is the sequential kernel's.
 //
 // SEG: the chunks of a (sample, head) are divided over the CTAs of a thread-block cluster, for shapes
 // with fewer (sample, head) pairs than SMs.  Every CTA but the last first walks its chunks for the state
@@ -589,19 +592,23 @@ __global__ void __launch_bounds__(256, 1) m3_ssd_fwd_tc_kernel(const __grid_cons
 #pragma unroll
         for (int jj = half * (HD / 16); jj < (half + 1) * (HD / 16); ++jj) {
             const uint4 v = *reinterpret_cast<const uint4*>(smem + tV + sw_chunk(tid, jj));
-            uint32_t w4[4] = {v.x, v.y, v.z, v.w}, lo[4];
+            uint32_t w4[4] = {v.x, v.y, v.z, v.w}, lo[4], rest[4];
 #pragma unroll
             for (int q4 = 0; q4 < 4; ++q4) {
                 const float2 f = unpack2<Th>(w4[q4]);
                 w4[q4] = pack2<Th>(f.x * wt, f.y * wt);
                 if (CARRY) {
-                    const float2 r = unpack2<Th>(w4[q4]);
-                    lo[q4] = pack2<Th>(f.x * wt - r.x, f.y * wt - r.y);
+                    const float2 hi = unpack2<Th>(w4[q4]), r = make_float2(f.x * wt - hi.x, f.y * wt - hi.y);
+                    lo[q4] = pack2<Th>(r.x, r.y);
+                    const float2 mid = unpack2<Th>(lo[q4]);
+                    rest[q4] = pack2<Th>(r.x - mid.x, r.y - mid.y);
                 }
             }
             *reinterpret_cast<uint4*>(smem + kVw + sw_chunk(tid, jj)) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
-            if (CARRY)
+            if (CARRY) {
                 *reinterpret_cast<uint4*>(smem + kVwLo + sw_chunk(tid, jj)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+                *reinterpret_cast<uint4*>(smem + kVwRest + sw_chunk(tid, jj)) = make_uint4(rest[0], rest[1], rest[2], rest[3]);
+            }
         }
     };
     auto decay_state = [&](float e_end) {  // S^T row `tid` (state index n = tid) *= exp(dA_end)
@@ -620,6 +627,9 @@ __global__ void __launch_bounds__(256, 1) m3_ssd_fwd_tc_kernel(const __grid_cons
 #pragma unroll
             for (int k = 0; k < CS / 16; ++k)
                 mma(tmem + cS, desc_sw_mn(sbase + tK, k), desc_sw_mn(sbase + kVwLo, k), idS, true);
+#pragma unroll
+            for (int k = 0; k < CS / 16; ++k)
+                mma(tmem + cS, desc_sw_mn(sbase + tK, k), desc_sw_mn(sbase + kVwRest, k), idS, true);
         }
     };
 
@@ -970,16 +980,14 @@ cudaError_t launch_cluster(const void* fn, dim3 grid, dim3 block, size_t smem, c
 }
 
 int m3_configure(Ctx* c) {
-    const void* fns[10] = {reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, false, false>),
+    const void* fns[8] = {reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, false, false>),
                           reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__half, false, false, false>),
                           reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, true, false, false>),
                           reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__half, true, false, false>),
                           reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, true, false>),
-                          reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__half, false, true, false>),
                           reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, false, true>),
                           reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__half, false, false, true>),
-                          reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, true, true>),
-                          reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__half, false, true, true>)};
+                          reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, true, true>)};
     for (const void* fn : fns)
         MB200_CUDA_CHECK(c, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::kSmem));
     return MAMBA_B200_OK;
@@ -1050,7 +1058,7 @@ extern "C" MAMBA_B200_API int mamba_b200_m3_ssd_fwd(void* handle, void* stream,
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
     bool tensor_core = a.dtype != MAMBA_B200_F32 && a.hd <= tc::HD && a.hd % 8 == 0 && a.N <= tc::NS &&
-                       a.N % 8 == 0 && (!a.carry_in || (!gen && a.T > kCarrySeqSteps)) &&
+                       a.N % 8 == 0 && (!a.carry_in || (!gen && a.dtype == MAMBA_B200_BF16 && a.T > kCarrySeqSteps)) &&
                        !a.force_sequential && al16(a.x) && al16(a.y) &&
                        (gen ? al16(a.Bn) && al16(a.Cn) && al16(a.angle_vel) : al16(a.K) && al16(a.Q));
     // the tile maps; when the driver refuses one (no encoder, a stride beyond its range) the
@@ -1079,8 +1087,7 @@ extern "C" MAMBA_B200_API int mamba_b200_m3_ssd_fwd(void* handle, void* stream,
         if (ranks > 1) {
             const void* fn = bf ? (a.carry_in ? reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, true, true>)
                                               : reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, false, true>))
-                                : (a.carry_in ? reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__half, false, true, true>)
-                                              : reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__half, false, false, true>));
+                                : reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__half, false, false, true>);
             void* args[1] = {&p};
             MB200_CUDA_CHECK(c, launch_cluster(fn, dim3(a.nh * ranks, a.B), dim3(256), tc::kSmem, st, ranks, args));
         } else if (bf) {
@@ -1089,7 +1096,6 @@ extern "C" MAMBA_B200_API int mamba_b200_m3_ssd_fwd(void* handle, void* stream,
             else tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, false, false><<<grid, 256, tc::kSmem, st>>>(p);
         } else {
             if (gen) tc::m3_ssd_fwd_tc_kernel<__half, true, false, false><<<grid, 256, tc::kSmem, st>>>(p);
-            else if (a.carry_in) tc::m3_ssd_fwd_tc_kernel<__half, false, true, false><<<grid, 256, tc::kSmem, st>>>(p);
             else tc::m3_ssd_fwd_tc_kernel<__half, false, false, false><<<grid, 256, tc::kSmem, st>>>(p);
         }
     } else {

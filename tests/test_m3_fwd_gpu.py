@@ -242,3 +242,47 @@ def test_a_divided_window_starts_from_the_state_that_entered(cuda_dev, T, nh):
         y2, ssm2 = call(False)
         assert torch.equal(y2, y) and torch.equal(ssm2, ssm)
     mb.ffi.default_handle(0).check_status()
+
+
+def window_f64(i, st):
+    """The sequential definition in 64 bits: y [B,T,nh*hd] and the state after the window."""
+    B, T, nh, N = i["K"].shape
+    h, kp, vp = (s.astype(np.float64) for s in st)
+    d = {k: i[k].astype(np.float64) for k in ARGS}
+    y = np.empty((B, T, nh, h.shape[2]))
+    for t in range(T):
+        al, v = np.exp(d["adt"][:, t]), d["x"][:, t].reshape(B, nh, -1)
+        be, ga = al * d["dt"][:, t] * (1 - d["trap"][:, t]), d["trap"][:, t] * d["dt"][:, t]
+        h = al[..., None, None] * h + (be[..., None] * vp)[..., None] * kp[:, :, None] + (ga[..., None] * v)[..., None] * d["K"][:, t][:, :, None]
+        y[:, t] = np.einsum("bhpn,bhn->bhp", h, d["Q"][:, t]) + d["Dh"][:, None] * v
+        kp, vp = d["K"][:, t], v
+    return y.reshape(B, T, -1), h
+
+
+# (dtype, T, factor on x and the state, factor on K and Q): the divided form, one CTA a head, and what f16 cannot
+# hold as products (65504) or remainders (6e-8)
+@pytest.mark.parametrize("dt,T,nh,fx,fk", [("bf16", 1000, 4, 1, 1), ("bf16", 200, 160, 1, 1), ("bf16", 300, 2, 1e-3, 1),
+                                           ("f16", 1000, 4, 1, 1), ("f16", 300, 2, 1e-3, 1), ("f16", 300, 2, 1, 1e-2),
+                                           ("f16", 300, 2, 1e-2, 200)])
+def test_a_carried_window_is_as_exact_as_the_sequential_definition(cuda_dev, dt, T, nh, fx, fk):
+    import torch
+
+    import mamba_rs_b200 as mb
+    hd, N = 64, 128
+    i = synth.m3_ssd_inputs(1, T, nh, hd, N, seed=T)
+    i["Dh"] = 0 * i["Dh"]  # (the skip would hide the scan's part of y)
+    i["x"], i["K"], i["Q"] = i["x"] * np.float32(fx), i["K"] * np.float32(fk), i["Q"] * np.float32(fk)
+    i = rounded(i, dt)
+    rng = np.random.default_rng(T)
+    st0 = [(f * rng.standard_normal(s)).astype(np.float32) for f, s in ((fx * fk, (1, nh, hd, N)), (fk, (1, nh, N)), (fx, (1, nh, hd)))]
+    ref = window_f64(i, st0)
+    args = [to_dev(i[k], cuda_dev, torch_dtype(dt) if k in ("x", "K", "Q") else None) for k in ARGS]
+    err = []
+    for seq in (False, True):
+        ssm, ks, vs = (to_dev(s, cuda_dev) for s in st0)
+        y = mb.m3_ssd_fwd(*args, ssm_state=ssm, k_state=ks, v_state=vs, carry_in=True, force_sequential=seq)
+        err.append([np.linalg.norm(a.double().cpu().numpy() - r) / np.linalg.norm(r) for a, r in zip((y, ssm), ref)])
+    mb.ffi.default_handle(0).check_status()
+    # y: both are the rounding of the store; state: f32 sums in another order, a few 2^-24 of 128 terms a chunk
+    assert err[0][0] <= 1.01 * err[1][0], err
+    assert err[0][1] <= max(err[1][1], 2e-6), err
