@@ -500,7 +500,10 @@ MAMBA_B200_API int mamba_b200_adamw_step(void* handle, void* stream, float* para
 
 /*
  * One token per sequence through every layer of a Mamba-1 backbone, in one cooperative launch
- * (the grid stays resident and meets at barriers in `workspace`): replaces the per-layer launch
+ * (the grid stays resident, its CTAs hand one another values through `workspace`; with a vocabulary
+ * or from d_model 600 on (f32: 300) that is one CTA on every SM, so nothing else runs beside it, and it
+ * starts when the other streams' kernels have left the SMs: call the operators one by one where
+ * decoding has to overlap with other work): replaces the per-layer launch
  * sequence of GpuMambaBackbone::step (src/mamba_ssm/gpu/inference.rs:1515-1855, :1062-1215) and,
  * with next_ids != NULL, GpuMambaLM's greedy decode step around it (src/module/gpu_lm.rs:560-679).
  * Weights are two arenas with the same layout, the compute-dtype copy `lp` (in_proj, x_proj,
@@ -517,8 +520,14 @@ MAMBA_B200_API int mamba_b200_adamw_step(void* handle, void* stream, float* para
  *   (lowest index among equals).
  * mamba_b200_decode_workspace_bytes returns what `workspace` must hold, 0 when the kernel does not
  * take this model or batch (N 16, K 4, d_model a multiple of 8 up to 1024, B <= 64): call the
- * operators one by one then.  The workspace's first 256 bytes must be zero before the first
- * launch and are zero again after each; one workspace serves one launch at a time.
+ * operators one by one then.  The WHOLE workspace must be zero before its first launch and is
+ * the library's own from then on: it keeps what the next launch tells its values from the last
+ * one's by, so nothing in it may be cleared or overwritten between launches (clearing all of it
+ * again is a first launch again).  It may pass from one model or batch size to another that it is
+ * large enough for; it serves one launch at a time.  Its third 32-bit word is the caller's: how
+ * many polls a wait inside the kernel may take before it gives up, which mamba_b200_check_status
+ * then reports (0: about two seconds' worth).  After a launch that gave up the states, residual
+ * and outputs are undefined, the workspace is ready for the next one.
  */
 typedef struct mamba_b200_decode_args {
     int dtype;

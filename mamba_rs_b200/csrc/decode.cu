@@ -62,7 +62,8 @@ struct Params {
     uint2* p_x;                         // [ks, B, ncg * 8] partial sums of x_proj
     uint2* r_x;                         // [B, dm] residual stream
     uint4* a_x;                         // [B, ncta] best logit and its index
-    unsigned* ctl;                      // [0] tags used so far, [1] CTAs done; [1] is zero between launches
+    unsigned* ctl;                      // [0] tags used so far, [1] CTAs done (zero between launches), [2] polls a
+                                        // wait may take (zero: kMaxPolls)
     void* out;                          // backbone: rmsnorm(residual) in the compute dtype
     int *next_ids, *tokens;             // LM: ids in / next ids out; tokens[b * tok_ld] = id taken in
     long long tok_ld;
@@ -153,6 +154,7 @@ struct Step {
     const int tid, lane, warp, cta, ncta;
     bool alive = true;
     unsigned base_tag = 0;
+    int polls = kMaxPolls;
     float* pair;     // sums that two warps of a row exchange
     uint64_t* bars;  // landed: W_in, W_out, W_x, small operands; then free: the same
     volatile int* dead;
@@ -200,9 +202,9 @@ struct Step {
             for (int i = 0; i < N; ++i) miss |= (v[i].y ^ tag) | (v[i].w ^ tag);
             if (!__any_sync(0xffffffffu, miss != 0)) break;
             if (lane == 0)
-                while ((v[0].y != tag || v[0].w != tag) && ++it < kMaxPolls) v[0] = get2(src + min(j, last));
+                while (alive && (v[0].y != tag || v[0].w != tag) && ++it < polls) v[0] = get2(src + min(j, last));
             it = __shfl_sync(0xffffffffu, it, 0) + 1;
-            if (it >= kMaxPolls || !alive) {
+            if (it >= polls || !alive) {
                 alive = false;
                 if (lane == 0) atomicCAS(p.status, kStatusOk, kStatusBarrierTimeout);
                 break;
@@ -998,7 +1000,9 @@ struct Step {
     }
 
     __device__ void run() {
-        base_tag = *reinterpret_cast<volatile unsigned*>(p.ctl);
+        const volatile unsigned* ctl = p.ctl;
+        base_tag = ctl[0];
+        if (ctl[2] > 0 && ctl[2] < static_cast<unsigned>(kMaxPolls)) polls = static_cast<int>(ctl[2]);
         float own = 0.0f;
         enter(own);
         const int n = channels(), per = p.ncg * 4;
@@ -1036,11 +1040,9 @@ struct Step {
             final_norm();
         }
         meet();
-        if (!alive) {
-            *dead = 1;
-            return;
-        }
-        // the last CTA to get here (all have read the tag base) hands the next launch tags of its own
+        if (!alive) *dead = 1;
+        // the last CTA to get here (all have read the tag base) hands the next launch tags of its own; a CTA that
+        // has given up counts like any other, or the next launch would take this one's words for its own
         if (tid == 0) {
             __threadfence();
             if (atomicAdd(p.ctl + 1, 1u) == static_cast<unsigned>(ncta) - 1) {

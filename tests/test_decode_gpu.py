@@ -75,3 +75,59 @@ def test_one_launch_greedy_decode_matches_the_operators(cuda_dev, size, dt):
     assert rel_err(got[0][1], got[1][1]) <= tol
     assert rel_err(got[0][3], got[1][3]) <= tol
     mb.ffi.default_handle(0).check_status()
+
+
+def filled(bb, seed):
+    import torch
+    g = torch.Generator(device=bb.conv.device).manual_seed(seed)
+    bb.conv.copy_(torch.randn(bb.conv.shape, device=bb.conv.device, generator=g))
+    bb.ssm.copy_(torch.randn(bb.ssm.shape, device=bb.conv.device, generator=g))
+    return torch.randn(bb.batch, bb.cfg.d_model, device=bb.conv.device, generator=g)
+
+
+@pytest.mark.parametrize("dt,d,L,B", [("bf16", 128, 3, 4), ("f32", 256, 2, 3), ("bf16", 768, 2, 20)])
+def test_a_step_after_one_that_gave_up_is_right(cuda_dev, dt, d, L, B):
+    """A launch whose waits may take one poll gives up, says so, and leaves a workspace that the next launch
+    can use: no word of the one that failed may pass for its own."""
+    import torch
+
+    import mamba_rs_b200 as mb
+    h = mb.ffi.default_handle(0)
+    h.check_status()
+    w = mb.MambaWeights(mb.MambaConfig(d_model=d, n_layers=L), cuda_dev, dtype=torch_dtype(dt)).init_random(3)
+    bb, ref = mb.GpuMambaBackbone(w, B), mb.GpuMambaBackbone(w, B)
+    ctl = bb._plan(B).ws[:16].view(torch.int32)
+    for n in range(1, 4):
+        x = filled(bb, n)
+        ctl[2] = 1
+        bb.step(x)
+        with pytest.raises(RuntimeError, match="bounded wait"):
+            h.check_status()
+        assert ctl.tolist()[:2] == [(2 * n - 1) * (L + 2), 0]
+        ctl[2] = 0
+        x = filled(bb, 10 + n)
+        want = ref.step(filled(ref, 10 + n))
+        got = bb.step(x)
+        assert torch.equal(got, want) and torch.equal(bb.ssm, ref.ssm) and torch.equal(bb.conv, ref.conv)
+        h.check_status()
+        assert ctl.tolist()[:2] == [2 * n * (L + 2), 0]
+
+
+def test_a_workspace_passes_from_one_batch_size_to_another(cuda_dev):
+    """The same memory for 9, 2 and 9 sequences without clearing, then cleared and used again."""
+    import torch
+
+    import mamba_rs_b200 as mb
+    w = mb.MambaWeights(mb.MambaConfig(d_model=128, n_layers=2), cuda_dev).init_random(3)
+    big, small = mb.GpuMambaBackbone(w, 9), mb.GpuMambaBackbone(w, 2)
+    ws = big._plan(9).ws
+    small._plan(2).ws = ws
+    small._plan(2).args.workspace = ws.data_ptr()
+    for n, bb in enumerate((big, small, big, small)):
+        if n == 3:
+            ws.zero_()
+        ref = mb.GpuMambaBackbone(w, bb.batch)
+        want = ref.step(filled(ref, n))
+        got = bb.step(filled(bb, n))
+        assert torch.equal(got, want) and torch.equal(bb.ssm, ref.ssm)
+    mb.ffi.default_handle(0).check_status()
