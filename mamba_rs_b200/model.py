@@ -448,8 +448,9 @@ class GpuMambaBackbone:
     def _prefill(self, temporal, last_only):
         B, T, dm = temporal.shape
         ops._require_cuda(temporal)
-        if temporal.dtype != torch.float32 or not temporal.is_contiguous() or dm != self.cfg.d_model:
-            raise TypeError("temporal is contiguous float32 [B, T, d_model]")
+        if (temporal.dtype != torch.float32 or not temporal.is_contiguous() or dm != self.cfg.d_model
+                or temporal.device != self.w.master.device):
+            raise TypeError("temporal is contiguous float32 [B, T, d_model] on the weights' device")
         if B > self.batch:
             raise ValueError(f"{B} sequences, the engine's state holds {self.batch}")
         return self._prefill_plan(B, T).run(temporal, last_only)
@@ -468,6 +469,8 @@ class GpuMambaBackbone:
         model where ``mamba_b200_decode_step`` takes it, else the operators one by one."""
         c, w = self.cfg, self.w
         B, dm = temporal.shape
+        if dm != c.d_model or temporal.device != w.master.device:
+            raise TypeError(f"temporal is [B, {c.d_model}] on {w.master.device}, not {list(temporal.shape)} on {temporal.device}")
         plan = self._plan(B)
         if (plan.ok and B <= self.batch and temporal.is_cuda and temporal.dtype == torch.float32
                 and temporal.is_contiguous() and temporal.data_ptr() % 16 == 0):
@@ -528,7 +531,7 @@ class GpuMambaLM:
         """ids [B, T] int32 -> logits of the last position [B, vocab]; leaves the greedy
         next token in ``next_ids``."""
         B, T = ids.shape
-        if (B == self.batch and ids.is_cuda and ids.dtype == torch.int32 and T > 0
+        if (B == self.batch and ids.device == self.w.master.device and ids.is_cuda and ids.dtype == torch.int32 and T > 0
                 and not torch.cuda.is_current_stream_capturing()):
             p = self.backbone._prefill_plan(B, T)
             if p.launch_bound:
@@ -865,7 +868,8 @@ class MambaLMTrainer:
 
     def step(self, ids: torch.Tensor) -> torch.Tensor:
         B, T1 = ids.shape
-        if (ids.is_cuda and ids.dtype == torch.int32 and B > 0 and T1 > 1 and self._pending == 0 and self._acts is None
+        if (ids.device == self.w.master.device and ids.is_cuda and ids.dtype == torch.int32 and B > 0 and T1 > 1
+                and self._pending == 0 and self._acts is None
                 and not torch.distributed.is_initialized() and not torch.cuda.is_current_stream_capturing()):
             plan = self._plan(B, T1 - 1)
             if plan.launch_bound:
