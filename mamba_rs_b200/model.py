@@ -69,7 +69,7 @@ class MambaWeights:
     (src/weights.rs:8-65).  GEMM weights are [in, out] row-major, as in the reference."""
 
     def __init__(self, cfg: MambaConfig, device, dtype=torch.bfloat16, vocab: int | None = None):
-        self.cfg, self.device, self.dtype, self.vocab = cfg, device, dtype, vocab
+        self.cfg, self.dtype, self.vocab = cfg, dtype, vocab
         dm, di, N, K, dr, xd = cfg.d_model, cfg.d_inner, cfg.d_state, cfg.d_conv, cfg.dt_rank, cfg.xdbl_dim
         self.shapes = dict(norm_w=(dm,), in_proj_w=(dm, 2 * di), conv_w=(di, K), conv_b=(di,), x_proj_w=(di, xd),
                            dt_proj_w=(dr, di), dt_proj_b=(di,), a_log=(di, N), d_param=(di,), out_proj_w=(di, dm))
@@ -78,6 +78,7 @@ class MambaWeights:
         extra = dm + (vocab * dm if vocab else 0)
         self.n = cfg.n_layers * self.layer_size + extra
         self.master = torch.zeros(self.n, device=device)
+        device = self.device = self.master.device  # with its index, also where `device` is a name or has none
         self.grad = torch.zeros(self.n, device=device)
         self.lp = torch.zeros(self.n, device=device, dtype=dtype) if dtype != torch.float32 else self.master
         self._a_neg_all = torch.empty(cfg.n_layers, di, N, device=device)

@@ -1,5 +1,5 @@
 """Host side of the engines (mamba_rs_b200/model.py) that needs no GPU: what a call refuses before anything is
-launched."""
+launched, and devices by name."""
 import pytest
 import torch
 
@@ -23,3 +23,10 @@ def test_calls_refuse_rows_on_another_device():
     bb = mb.GpuMambaBackbone(weights(), 2)
     with pytest.raises(TypeError, match="device|meta"):
         bb.step(torch.zeros(2, 16, device="meta"))
+
+
+@pytest.mark.parametrize("device", ["cpu", torch.device("cpu")])
+def test_weights_take_a_device_by_name(device):
+    w = weights(device).init_random(1)
+    assert w.device == w.master.device == torch.device("cpu") and bool(w.master.abs().sum() > 0)
+    assert mb.MambaLMTrainer(w)._plans == {}

@@ -236,3 +236,15 @@ def test_steps_by_operators_that_come_again_equal_the_first_ones(cuda_dev):
         ref = once.step(y)
         assert rel_err(out.cpu().numpy(), ref.cpu().numpy()) <= 1e-6 and rel_err(res.cpu().numpy(), y.cpu().numpy()) <= 1e-6
     assert not once._plan(3).replay.kept and torch.equal(again.ssm, once.ssm) and torch.equal(again.conv, once.conv)
+
+
+def test_an_engine_made_on_a_device_by_name(cuda_dev):
+    import torch
+
+    import mamba_rs_b200 as mb
+    w = mb.MambaWeights(mb.MambaConfig(d_model=64, n_layers=1), "cuda", vocab=50).init_random(3)
+    lm, ids = mb.GpuMambaLM(w, 2), torch.randint(0, 50, (2, 9), device=cuda_dev, dtype=torch.int32)
+    for _ in range(4):
+        assert bool(torch.isfinite(lm.prefill(ids).float()).all())
+    assert lm.generate_greedy(3).shape == (2, 3)
+    assert np.isfinite(float(mb.MambaLMTrainer(w).step(ids)))
