@@ -271,7 +271,7 @@ class _PrefillPlan:
 
     def __init__(self, bb: "GpuMambaBackbone", B: int, T: int):
         w, c = bb.w, bb.cfg
-        self.key = self.pointers(bb)
+        self.key = _DecodePlan.made_from(bb)
         self.cfg, self.dtype, self.B, self.T, self.where = c, w.dtype, B, T, None  # (not bb: it keeps this plan)
         self.run_on = _Launcher(w.device)
         di, N, dr, xd = c.d_inner, c.d_state, c.dt_rank, c.xdbl_dim
@@ -294,10 +294,6 @@ class _PrefillPlan:
         self.replay, self.ids = _Replay(w.device), None
         written = B * T * ((c.d_model + 5 * di + xd) * self.es + 4 * c.d_model) + self.ws_bytes
         self.launch_bound = w.device.type == "cuda" and written <= 64 << 20
-
-    @staticmethod
-    def pointers(bb):
-        return _DecodePlan.pointers(bb) + tuple(a.data_ptr() for a in bb.w.a_neg)
 
     def point(self, proj, u, xdbl, delta, y, ws):
         di, N, dr, es = self.cfg.d_inner, self.cfg.d_state, self.cfg.dt_rank, self.es
@@ -366,14 +362,14 @@ class _DecodePlan:
 
     def __init__(self, bb: "GpuMambaBackbone", B: int, lm: "GpuMambaLM | None" = None):
         w, c = bb.w, bb.cfg
-        self.key = self.pointers(bb)
+        self.key = self.made_from(bb)
         self.handle = ffi.default_handle(w.device.index or 0)
         a = self.args = ffi.DecodeArgs()
         a.dtype = ops.dtype_code(w.dtype)
         a.B, a.batch_capacity, a.d_model, a.d_inner = B, bb.batch, c.d_model, c.d_inner
         a.N, a.K, a.dt_rank, a.n_layers = c.d_state, c.d_conv, c.dt_rank, c.n_layers
         a.vocab, a.eps = (w.vocab if lm else 0), c.rms_norm_eps
-        a.lp, a.master, a.a_neg, a.conv_state, a.ssm_state = self.key
+        a.lp, a.master, a.a_neg, a.conv_state, a.ssm_state = self.key[:5]
         a.layer_stride = w.layer_size
         offset, o = {}, 0
         for k in _LAYER_FIELDS:
@@ -399,9 +395,12 @@ class _DecodePlan:
         self._call, self._ref = lib.mamba_b200_decode_step, C.byref(a)
 
     @staticmethod
-    def pointers(bb):
+    def made_from(bb):
+        """All that the structs and recorded launches of a plan hold of their engine: addresses (a layer's
+        decay rates may have been replaced by another tensor) and the norm's epsilon."""
         w = bb.w
-        return (w.lp.data_ptr(), w.master.data_ptr(), w._a_neg_all.data_ptr(), bb.conv.data_ptr(), bb.ssm.data_ptr())
+        return (w.lp.data_ptr(), w.master.data_ptr(), w._a_neg_all.data_ptr(), bb.conv.data_ptr(), bb.ssm.data_ptr(),
+                bb.cfg.rms_norm_eps, *[a.data_ptr() for a in w.a_neg])
 
     def launch(self):
         dev = self.handle.device
@@ -431,7 +430,7 @@ class GpuMambaBackbone:
     def _plan(self, B):
         """The decode launch for B sequences, rebuilt when a buffer it points at was replaced."""
         p = self._plans.get(B)
-        if p is None or p.key != _DecodePlan.pointers(self):
+        if p is None or p.key != _DecodePlan.made_from(self):
             if len(self._plans) >= 8:
                 self._plans.clear()
             p = self._plans[B] = _DecodePlan(self, B)
@@ -458,7 +457,7 @@ class GpuMambaBackbone:
 
     def _prefill_plan(self, B, T):
         p = self._prefills.get((B, T))
-        if p is None or p.key != _PrefillPlan.pointers(self):
+        if p is None or p.key != _DecodePlan.made_from(self):
             if len(self._prefills) >= 64:
                 self._prefills.clear()
             p = self._prefills[B, T] = _PrefillPlan(self, B, T)
@@ -562,7 +561,7 @@ class GpuMambaLM:
     def generate_greedy(self, n: int, use_graph: bool = True) -> torch.Tensor:
         """n greedy tokens after a prefill; returns them as [B, n] int32."""
         out = torch.empty(self.batch, n, dtype=torch.int32, device=self.w.device)
-        if self._dec is None or self._dec.key != _DecodePlan.pointers(self.backbone):
+        if self._dec is None or self._dec.key != _DecodePlan.made_from(self.backbone):
             self._dec = _DecodePlan(self.backbone, self.batch, self)
         if self._dec.ok and n > 0:
             a = self._dec.args
@@ -604,7 +603,7 @@ class _TrainPlan:
 
     def __init__(self, w: MambaWeights, B: int, T: int, save: int):
         c = w.cfg
-        self.key, self.B, self.T, self.w = self.pointers(w), B, T, w
+        self.key, self.B, self.T, self.w = self.made_from(w), B, T, w
         self.run_on = _Launcher(w.device)
         di, N, K, xd, S = c.d_inner, c.d_state, c.d_conv, c.xdbl_dim, save
         self.blocks = (T + S - 1) // S
@@ -646,8 +645,8 @@ class _TrainPlan:
             self.layers.append(lay)
 
     @staticmethod
-    def pointers(w):
-        return (w.lp.data_ptr(), w.master.data_ptr(), w.grad.data_ptr()) + tuple(a.data_ptr() for a in w.a_neg)
+    def made_from(w):
+        return (w.lp.data_ptr(), w.master.data_ptr(), w.grad.data_ptr(), w.cfg.rms_norm_eps, *[a.data_ptr() for a in w.a_neg])
 
     def _at(self, l, proj, u, xdbl, delta, cs):
         """Addresses of layer l's saved x, z, u, B, C, delta and block states."""
@@ -758,7 +757,7 @@ class MambaLMTrainer:
 
     def _plan(self, B, T):
         p = self._plans.get((B, T))
-        if p is None or p.key != _TrainPlan.pointers(self.w):
+        if p is None or p.key != _TrainPlan.made_from(self.w):
             if len(self._plans) >= 16:
                 self._plans.clear()
             p = self._plans[B, T] = _TrainPlan(self.w, B, T, self.SAVE)

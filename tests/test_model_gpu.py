@@ -248,3 +248,53 @@ def test_an_engine_made_on_a_device_by_name(cuda_dev):
         assert bool(torch.isfinite(lm.prefill(ids).float()).all())
     assert lm.generate_greedy(3).shape == (2, 3)
     assert np.isfinite(float(mb.MambaLMTrainer(w).step(ids)))
+
+
+@pytest.mark.parametrize("N", [16, 8])  # the one-launch kernel, and operators that are replayed
+def test_a_step_follows_replaced_decay_rates_and_a_changed_epsilon(cuda_dev, N):
+    import torch
+
+    import mamba_rs_b200 as mb
+    make = lambda: mb.MambaWeights(mb.MambaConfig(d_model=64, n_layers=2, d_state=N), cuda_dev, dtype=torch.float32).init_random(3)  # noqa: E731
+    bb = mb.GpuMambaBackbone(make(), 3)
+    buf, x = torch.empty(3, 64, device=cuda_dev), torch.randn(3, 64, device=cuda_dev)
+
+    def run(b, n=4):
+        b.reset()
+        b.ssm.fill_(0.3)
+        for _ in range(n):
+            buf.copy_(x)
+            out = b.step(buf)
+        return out
+    run(bb)
+    bb.w.a_neg[1] = 3 * bb.w.a_neg[1].clone()
+    bb.cfg.rms_norm_eps = 0.5
+    fresh = mb.GpuMambaBackbone(make(), 3)
+    fresh.w.a_neg[1].mul_(3)
+    fresh.cfg.rms_norm_eps = 0.5
+    fresh._plan(3).ok = False
+    got, want = run(bb), run(fresh, 2)
+    want = run(fresh)
+    assert rel_err(got.cpu().numpy(), want.cpu().numpy()) <= 1e-5
+    assert rel_err(bb.ssm.cpu().numpy(), fresh.ssm.cpu().numpy()) <= 1e-5
+
+
+def test_prefill_and_training_follow_a_changed_epsilon(cuda_dev):
+    import torch
+
+    import mamba_rs_b200 as mb
+    make = lambda: mb.MambaWeights(mb.MambaConfig(d_model=64, n_layers=2), cuda_dev, dtype=torch.float32, vocab=50).init_random(3)  # noqa: E731
+    ids = torch.randint(0, 50, (2, 21), device=cuda_dev, dtype=torch.int32)
+    lm, ref = mb.GpuMambaLM(make(), 2), mb.GpuMambaLM(make(), 2)
+    tr, tref = mb.MambaLMTrainer(make()), mb.MambaLMTrainer(make())
+    for _ in range(4):
+        lm.backbone.reset()
+        lm.prefill(ids)
+        tr.step(ids)
+        tref.step(ids)
+    for c in (lm.w.cfg, ref.w.cfg, tr.cfg, tref.cfg):
+        c.rms_norm_eps = 0.5
+    lm.backbone.reset()
+    assert rel_err(lm.prefill(ids).cpu().numpy(), ref.prefill(ids).cpu().numpy()) <= 1e-6
+    tref._plan(2, 20).launch_bound = False
+    assert abs(float(tr.step(ids)) - float(tref.step(ids))) <= 1e-6
