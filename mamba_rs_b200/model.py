@@ -185,6 +185,16 @@ class MambaWeights:
         return self
 
 
+def _capturing(t):
+    """Whether the current stream of t's device is being captured.  What is made then (a zeroed workspace, a
+    row of ones) is filled by the graph's replays alone, so no later call may be given it: plans made
+    inside a capture serve that call and go."""
+    if not t.is_cuda:
+        return False
+    with ops._on(t.device):
+        return torch.cuda.is_current_stream_capturing()
+
+
 class _Launcher:
     """The library's entry points on one device's current stream, with the arguments a plan has
     prepared: what a layer's launches cost on the host is then the call itself."""
@@ -431,9 +441,11 @@ class GpuMambaBackbone:
         """The decode launch for B sequences, rebuilt when a buffer it points at was replaced."""
         p = self._plans.get(B)
         if p is None or p.key != _DecodePlan.made_from(self):
-            if len(self._plans) >= 8:
-                self._plans.clear()
-            p = self._plans[B] = _DecodePlan(self, B)
+            p = _DecodePlan(self, B)
+            if not _capturing(self.w.master):
+                if len(self._plans) >= 8:
+                    self._plans.clear()
+                self._plans[B] = p
         return p
 
     def reset(self):
@@ -561,13 +573,16 @@ class GpuMambaLM:
     def generate_greedy(self, n: int, use_graph: bool = True) -> torch.Tensor:
         """n greedy tokens after a prefill; returns them as [B, n] int32."""
         out = torch.empty(self.batch, n, dtype=torch.int32, device=self.w.device)
-        if self._dec is None or self._dec.key != _DecodePlan.made_from(self.backbone):
-            self._dec = _DecodePlan(self.backbone, self.batch, self)
-        if self._dec.ok and n > 0:
-            a = self._dec.args
+        dec = self._dec
+        if dec is None or dec.key != _DecodePlan.made_from(self.backbone):
+            dec = _DecodePlan(self.backbone, self.batch, self)
+            if not _capturing(self.w.master):
+                self._dec = dec
+        if dec.ok and n > 0:
+            a = dec.args
             a.next_ids, a.logits, a.steps = self.next_ids.data_ptr(), self.logits.data_ptr(), n
             a.tokens, a.tokens_ld = out.data_ptr(), n
-            self._dec.launch()
+            dec.launch()
             return out
         if use_graph and self._graph is None:
             dev = self.w.device
@@ -758,9 +773,11 @@ class MambaLMTrainer:
     def _plan(self, B, T):
         p = self._plans.get((B, T))
         if p is None or p.key != _TrainPlan.made_from(self.w):
-            if len(self._plans) >= 16:
-                self._plans.clear()
-            p = self._plans[B, T] = _TrainPlan(self.w, B, T, self.SAVE)
+            p = _TrainPlan(self.w, B, T, self.SAVE)
+            if not _capturing(self.w.master):
+                if len(self._plans) >= 16:
+                    self._plans.clear()
+                self._plans[B, T] = p
         return p
 
     def _accumulate(self, g, a, b):

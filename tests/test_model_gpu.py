@@ -298,3 +298,41 @@ def test_prefill_and_training_follow_a_changed_epsilon(cuda_dev):
     assert rel_err(lm.prefill(ids).cpu().numpy(), ref.prefill(ids).cpu().numpy()) <= 1e-6
     tref._plan(2, 20).launch_bound = False
     assert abs(float(tr.step(ids)) - float(tref.step(ids))) <= 1e-6
+
+
+def test_what_a_capture_makes_serves_no_later_call(cuda_dev):
+    """The first call of an engine inside a capture: its workspaces are filled by the graph's replays alone, so
+    an eager call before the first replay makes its own."""
+    import torch
+
+    import mamba_rs_b200 as mb
+    make = lambda: mb.MambaWeights(mb.MambaConfig(d_model=64, n_layers=2), cuda_dev, dtype=torch.float32, vocab=50).init_random(3)  # noqa: E731
+    x, ids = torch.randn(3, 64, device=cuda_dev), torch.randint(0, 50, (3, 9), device=cuda_dev, dtype=torch.int32)
+    warm, wt = mb.GpuMambaLM(make(), 3), mb.MambaLMTrainer(make())
+    want_step = warm.backbone.step(x.clone())  # (and kernels are loaded)
+    warm.backbone.reset()
+    want = warm.generate_greedy(3), warm.backbone.ssm.clone()
+    want_loss = wt.forward(ids)
+    wt.backward_step(accumulate_only=True)
+    lm, tr = mb.GpuMambaLM(make(), 3), mb.MambaLMTrainer(make())
+    bb = mb.GpuMambaBackbone(lm.w, 3)
+    bufs, graph = torch.empty(3, 64, device=cuda_dev), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = bb.step(bufs)
+        toks = lm.generate_greedy(3)
+        loss = tr.forward(ids)
+        tr.backward_step(accumulate_only=True)
+    assert not bb._plans and lm._dec is None and not tr._plans
+    for again in (False, True):
+        bb.reset(), lm.backbone.reset()
+        lm.next_ids.zero_(), tr.w.grad.zero_()
+        if not again:
+            assert torch.equal(bb.step(x.clone()), want_step)
+            assert torch.equal(lm.generate_greedy(3), want[0]) and torch.equal(lm.backbone.ssm, want[1])
+        else:
+            bufs.copy_(x)
+            graph.replay()
+            assert torch.equal(out, want_step) and torch.equal(toks, want[0]) and torch.equal(lm.backbone.ssm, want[1])
+            assert float(loss) == float(want_loss)
+            assert rel_err(tr.w.grad.cpu().numpy(), wt.w.grad.cpu().numpy()) <= 1e-6
+    mb.ffi.default_handle(0).check_status()
