@@ -22,6 +22,7 @@ from __future__ import annotations
 
 import ctypes as C
 import math
+import weakref
 from dataclasses import dataclass
 
 import torch
@@ -230,47 +231,123 @@ def _product(go, op, a, b, out):
 
 
 class _Replay:
-    """Sequences of launches that come again with the same addresses, as CUDA graphs.  A model small
-    enough for its launches to cost more than its work spends a fifth to a half of a pass between
-    kernels (130m, 1021 tokens: 1.96 ms launched one by one, 1.60 replayed; d_model 128, two layers:
-    0.18 and 0.125; a training step of 32 tokens in f32: 7.6 and 6.1 ms).  A sequence is recorded when it comes for the third time, so lengths or buffers
-    that change from call to call never pay for a recording; at most four are kept, each with the
-    activations it writes (the users' limits on them are where the gaps become a few per cent of the
-    work)."""
+    """Sequences of a plan's launches that come again with the same addresses, as CUDA graphs.  A model small
+    enough for its launches to cost more than its work spends a fifth to a half of a pass between kernels
+    (130m, 1021 tokens: 1.96 ms launched one by one, 1.60 replayed; d_model 128, two layers: 0.18 and 0.125;
+    a training step of 32 tokens in f32: 7.6 and 6.1 ms).  A sequence is recorded when it comes for the
+    third time, if its engine's shelf has room for the `nbytes` of activations that stay with it."""
 
-    KEEP = 4
-
-    def __init__(self, device):
-        self.device, self.seen, self.kept = device, {}, {}
+    def __init__(self, shelf, nbytes):
+        self.shelf, self.nbytes, self.seen, self.kept = shelf, nbytes, {}, {}
 
     def run(self, key, launch):
         """launch() now: by its graph where there is one.  What it returns lives until the next call
         with this key.  launch() reads and writes fixed addresses, apart from what it allocates."""
-        hit = self.kept.get(key)
+        shelf, hit = self.shelf, self.kept.get(key)
+        shelf.calls += 1
         if hit is not None:
-            with ops._on(self.device):
+            hit[2].used = shelf.calls
+            with ops._on(shelf.device):
                 hit[0].replay()
             return hit[1]
-        n = self.seen[key] = self.seen.get(key, 0) + 1
-        if n < 3:
-            if len(self.seen) > 64:
-                self.seen.clear()
+        n = self.seen[key] = self.seen.pop(key, 0) + 1
+        if len(self.seen) > 64:
+            del self.seen[next(iter(self.seen))]
+        if n < 3 or not shelf.room(self.nbytes):
             return launch()
-        while len(self.kept) >= self.KEEP:
-            self.kept.pop(next(iter(self.kept)))
+        del self.seen[key]
+        got = shelf.record(launch)
+        if got is None:  # (no memory for it, say: launch() does without, or says so itself)
+            return launch()
+        self.kept[key] = *got, shelf.put(self, key)
+        got[0].replay()
+        return got[1]
+
+    def __del__(self):
+        for _, _, place in self.kept.values():
+            self.shelf.places.discard(place)
+
+
+class _Shelf:
+    """What an engine keeps recorded: no more than KEEP sequences and `limit` bytes of activations, over all
+    its plans.  When there is no room, the one whose last use lies PATIENCE calls back gives way; while all
+    are in use, further ones are launched one by one, so buffers or lengths in rotation cost at most KEEP
+    recordings in PATIENCE calls (a recording takes about as long as five passes)."""
+
+    KEEP, PATIENCE = 16, 1024
+
+    class Place:
+        __slots__ = ("replay", "key", "nbytes", "used")
+
+    def __init__(self, device, limit):
+        self.device, self.limit, self.places, self.calls, self.stream = device, limit, set(), 0, None
+
+    def room(self, nbytes):
+        if nbytes > self.limit:
+            return False
+        while self.places and (len(self.places) >= self.KEEP or nbytes + sum(p.nbytes for p in self.places) > self.limit):
+            last = min(self.places, key=lambda p: p.used)
+            if self.calls - last.used < self.PATIENCE:
+                return False
+            self.places.discard(last)
+            owner = last.replay()
+            if owner is not None:
+                owner.kept.pop(last.key, None)
+        return True
+
+    def put(self, replay, key):
+        place = self.Place()
+        place.replay, place.key, place.nbytes, place.used = weakref.ref(replay), key, replay.nbytes, self.calls
+        self.places.add(place)
+        return place
+
+    def record(self, launch):
+        """(graph, result) of launch(), whose work is still to be done; None where it could not be recorded."""
+        if self.stream is None:
+            self.stream = _RecordingStream(self.device)
         with torch.cuda.device(self.device):
-            graph, here, side = torch.cuda.CUDAGraph(), torch.cuda.current_stream(), torch.cuda.Stream()
+            graph, here, side = torch.cuda.CUDAGraph(), torch.cuda.current_stream(), self.stream.stream
             side.wait_stream(here)
-            with torch.cuda.stream(side):
-                graph.capture_begin(capture_error_mode="thread_local")
-                try:
-                    out = launch()
-                finally:
-                    graph.capture_end()
-            here.wait_stream(side)
-            self.kept[key] = graph, out
-            graph.replay()
-        return out
+            try:
+                with torch.cuda.stream(side):
+                    graph.capture_begin(capture_error_mode="thread_local")
+                    try:
+                        out = launch()
+                    finally:
+                        graph.capture_end()
+            except RuntimeError:
+                return None
+            finally:
+                here.wait_stream(side)
+        return graph, out
+
+
+class _RecordingStream:
+    """A stream that belongs to one engine's recordings.  The workspace that library GEMMs use is one per
+    thread and stream, and a recording keeps its address: on a stream of torch's pool, which hands each out
+    many times, it could be the workspace of another engine's recording or of a program's own GEMMs, running
+    at the same time elsewhere.  An engine's own recordings never run beside each other."""
+
+    spare = {}  # device index -> streams of engines that are gone
+
+    def __init__(self, device):
+        self.index = device.index or 0
+        free = self.spare.setdefault(self.index, [])
+        if free:
+            self.raw = free.pop()
+        else:
+            raw = C.c_void_p()
+            with torch.cuda.device(self.index):
+                torch.cuda.current_stream().query()  # (the device's context is this thread's own from here on)
+                rc = C.CDLL("libcuda.so.1").cuStreamCreate(C.byref(raw), 1)  # CU_STREAM_NON_BLOCKING
+            if rc != 0:
+                raise RuntimeError(f"cuStreamCreate failed ({rc})")
+            self.raw = raw.value
+        self.stream = torch.cuda.ExternalStream(self.raw, device=torch.device("cuda", self.index))
+
+    def __del__(self):
+        if getattr(self, "raw", None):
+            self.spare[self.index].append(self.raw)
 
 
 class _PrefillPlan:
@@ -301,8 +378,9 @@ class _PrefillPlan:
             self.layers.append((pm["norm_w"].data_ptr(), p["in_proj_w"], C.byref(cv), p["x_proj_w"], p["dt_proj_b"],
                                 p["dt_proj_w"], C.byref(sc), p["out_proj_w"], cv, sc))
         self.norm_f = w.tail("master")["norm_f"].data_ptr()
-        self.replay, self.ids = _Replay(w.device), None
         written = B * T * ((c.d_model + 5 * di + xd) * self.es + 4 * c.d_model) + self.ws_bytes
+        self.replay, self.ids = _Replay(bb._shelf, written), None
+        # (beyond 64 MB of activations the gaps are a few per cent of the work)
         self.launch_bound = w.device.type == "cuda" and written <= 64 << 20
 
     def point(self, proj, u, xdbl, delta, y, ws):
@@ -395,7 +473,8 @@ class _DecodePlan:
         whole = all(t.data_ptr() == w._a_neg_all[l].data_ptr() for l, t in enumerate(w.a_neg))
         a.workspace_bytes = lib.mamba_b200_decode_workspace_bytes(self.handle.ptr, C.byref(a)) if whole else 0
         self.ok = a.workspace_bytes > 0
-        self.replay = _Replay(w.device)  # of the operators' launches where the kernel does not take the model
+        # of the operators' launches where the kernel does not take the model
+        self.replay = _Replay(bb._shelf, 4 * B * c.n_layers * (2 * c.d_model + 6 * c.d_inner + c.xdbl_dim))
         if self.ok:
             self.ws = torch.zeros(a.workspace_bytes, dtype=torch.uint8, device=w.device)
             a.workspace = self.ws.data_ptr()
@@ -435,7 +514,7 @@ class GpuMambaBackbone:
         dev, c = weights.device, weights.cfg
         self.conv = torch.zeros(c.n_layers, batch, c.d_inner, c.d_conv, device=dev)
         self.ssm = torch.zeros(c.n_layers, batch, c.d_inner, c.d_state, device=dev)
-        self._plans, self._prefills = {}, {}
+        self._plans, self._prefills, self._shelf = {}, {}, _Shelf(weights.device, 256 << 20)
 
     def _plan(self, B):
         """The decode launch for B sequences, rebuilt when a buffer it points at was replaced."""
@@ -616,7 +695,7 @@ class _TrainPlan:
         __slots__ = ("norm_w", "g_norm", "w_in", "w_x", "w_x_t", "b_dt", "w_dt", "w_out",
                      "conv", "scan", "conv_b", "scan_b", "structs")
 
-    def __init__(self, w: MambaWeights, B: int, T: int, save: int):
+    def __init__(self, w: MambaWeights, B: int, T: int, save: int, shelf: _Shelf):
         c = w.cfg
         self.key, self.B, self.T, self.w = self.made_from(w), B, T, w
         self.run_on = _Launcher(w.device)
@@ -630,12 +709,14 @@ class _TrainPlan:
                           lib.mamba_b200_residual_rmsnorm_bwd_workspace_bytes(B * T, c.d_model), 1)
         self.norm_f = w.tail("master")["norm_f"].data_ptr()
         self.fwd_at = self.bwd_at = None
-        self.replay, self.ids = _Replay(w.device), None
+        self.ids = None
         # few f32 rows: their sum is one more product (of the rows kernel)
         self.ones = torch.ones(B * T, 1, device=w.device) if w.dtype == torch.float32 and B * T <= 32 else None
         a_layer = B * T * (4 * (c.d_model + 1) + self.es * (c.d_model + 5 * di + xd)) + 4 * B * self.blocks * di * N
         written = c.n_layers * a_layer + B * T * self.es * (w.vocab or 0) + self.fwd_ws + self.bwd_ws
+        # (beyond 512 MB of activations the gaps are a few per cent of the work)
         self.launch_bound = w.device.type == "cuda" and written <= 512 << 20
+        self.replay = _Replay(shelf, written)
         self.layers = []
         for l in range(c.n_layers):
             p, pm, g, lay = w.layer(l), w.layer(l, "master"), w.layer(l, "grad"), self.Layer()
@@ -720,7 +801,7 @@ class MambaLMTrainer:
         self.bias = torch.ones(2, device=weights.device)
         self._acts = None
         self._pending = 0
-        self._plans = {}
+        self._plans, self._shelf = {}, _Shelf(weights.device, 1 << 30)
 
     # ---- forward ----
     def forward(self, ids: torch.Tensor) -> torch.Tensor:
@@ -773,7 +854,7 @@ class MambaLMTrainer:
     def _plan(self, B, T):
         p = self._plans.get((B, T))
         if p is None or p.key != _TrainPlan.made_from(self.w):
-            p = _TrainPlan(self.w, B, T, self.SAVE)
+            p = _TrainPlan(self.w, B, T, self.SAVE, self._shelf)
             if not _capturing(self.w.master):
                 if len(self._plans) >= 16:
                     self._plans.clear()

@@ -336,3 +336,28 @@ def test_what_a_capture_makes_serves_no_later_call(cuda_dev):
             assert float(loss) == float(want_loss)
             assert rel_err(tr.w.grad.cpu().numpy(), wt.w.grad.cpu().numpy()) <= 1e-6
     mb.ffi.default_handle(0).check_status()
+
+
+def test_input_buffers_in_rotation_are_right_and_record_a_bounded_number_of_times(cuda_dev, monkeypatch):
+    import torch
+
+    import mamba_rs_b200 as mb
+    from mamba_rs_b200 import model
+    monkeypatch.setattr(model._Shelf, "KEEP", 3)
+    recorded = []
+    record = model._Shelf.record
+    monkeypatch.setattr(model._Shelf, "record", lambda self, launch: recorded.append(1) or record(self, launch))
+    w = mb.MambaWeights(mb.MambaConfig(d_model=64, n_layers=2), cuda_dev, dtype=torch.float32).init_random(3)
+    bb, one = mb.GpuMambaBackbone(w, 2), mb.GpuMambaBackbone(w, 2)
+    one._prefill_plan(2, 20).launch_bound = False
+    x = torch.randn(2, 20, 64, device=cuda_dev)
+    bufs = [torch.empty_like(x) for _ in range(7)]
+    for i in range(10):
+        for b in bufs:
+            for e in (bb, one):
+                e.reset()
+            b.copy_(x * (i + 1))
+            got = bb.prefill_sequence(b)
+            want = one.prefill_sequence(x * (i + 1))
+            assert torch.equal(got, want)
+    assert len(recorded) == 3 == len(bb._prefill_plan(2, 20).replay.kept)
