@@ -875,9 +875,11 @@ class MambaLMTrainer:
 
     # ---- backward + optimiser ----
     def backward_step(self, accumulate_only: bool = False):
-        self._backward(accumulate_only, True)
+        self._gradients(accumulate_only)
+        if not accumulate_only:
+            self._update()
 
-    def _backward(self, accumulate_only, advance):
+    def _gradients(self, accumulate_only):
         c, w, a = self.cfg, self.w, self._acts
         if a is None:
             raise RuntimeError("backward_step needs a forward first")
@@ -937,31 +939,28 @@ class MambaLMTrainer:
         gt["embedding"].index_add_(0, a["inp"].view(-1), d_res)
         self._acts = None
         self._pending += 1
-        if accumulate_only:
-            return
-        red.bucket_ready(L)
-        red.finish()
+        if red is not None:
+            red.bucket_ready(L)
+            red.finish()
+
+    def _update(self):
+        """AdamW on the gradients in the arena, which is zero again afterwards."""
+        w = self.w
         if self._pending > 1:
             w.grad.div_(self._pending)
         self._pending = 0
-        if advance:
-            self._advance()
+        self.t += 1
         b1, b2 = self.betas
+        self.bias[:1].fill_(1.0 / (1.0 - b1 ** self.t))
+        self.bias[1:].fill_(1.0 / (1.0 - b2 ** self.t))
         ops.adamw_step(w.master, w.grad, self.m, self.v, self.bias, lr=self.lr, beta1=b1, beta2=b2, eps=self.eps,
                        weight_decay=self.wd, param_lp=None if w.lp is w.master else w.lp)
         w.refresh_a_neg()
         w.grad.zero_()
 
-    def _advance(self):
-        """The step count, and the bias corrections that follow from it."""
-        self.t += 1
-        b1, b2 = self.betas
-        self.bias[:1].fill_(1.0 / (1.0 - b1 ** self.t))
-        self.bias[1:].fill_(1.0 / (1.0 - b2 ** self.t))
-
-    def _whole_step(self, ids):
+    def _loss_and_gradients(self, ids):
         loss = self.forward(ids)
-        self._backward(False, False)
+        self._gradients(False)
         return loss
 
     def step(self, ids: torch.Tensor) -> torch.Tensor:
@@ -975,9 +974,10 @@ class MambaLMTrainer:
                     if plan.ids is None:
                         plan.ids = torch.empty(B, T1, dtype=torch.int32, device=self.w.device)
                     plan.ids.copy_(ids)
-                    self._advance()
-                    key = (self.lr, tuple(self.betas), self.eps, self.wd, self.m.data_ptr(), self.v.data_ptr(), self.bias.data_ptr())
-                    return plan.replay.run(key, lambda: self._whole_step(plan.ids)).clone()
+                    # (the update stays outside: a schedule changes its numbers from step to step)
+                    loss = plan.replay.run((), lambda: self._loss_and_gradients(plan.ids)).clone()
+                    self._update()
+                    return loss
         loss = self.forward(ids)
         self.backward_step()
         return loss

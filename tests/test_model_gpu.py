@@ -361,3 +361,40 @@ def test_input_buffers_in_rotation_are_right_and_record_a_bounded_number_of_time
             want = one.prefill_sequence(x * (i + 1))
             assert torch.equal(got, want)
     assert len(recorded) == 3 == len(bb._prefill_plan(2, 20).replay.kept)
+
+
+def test_a_learning_rate_schedule_keeps_the_recorded_step(cuda_dev):
+    import torch
+
+    import mamba_rs_b200 as mb
+    make = lambda: mb.MambaWeights(mb.MambaConfig(d_model=64, n_layers=2), cuda_dev, dtype=torch.float32, vocab=50).init_random(3)  # noqa: E731
+    ids = torch.randint(0, 50, (2, 21), device=cuda_dev, dtype=torch.int32)
+    tr, ref = mb.MambaLMTrainer(make()), mb.MambaLMTrainer(make())
+    ref._plan(2, 20).launch_bound = False
+    for i in range(8):
+        for t in (tr, ref):
+            t.lr, t.wd = 1e-3 * (i + 1) / 8, 0.1 / (i + 1)
+        assert abs(float(tr.step(ids)) - float(ref.step(ids))) <= 1e-5
+    assert len(tr._plan(2, 20).replay.kept) == 1 and tr.t == ref.t == 8 and not ref._plan(2, 20).replay.kept
+    for a, b in ((tr.w.master, ref.w.master), (tr.m, ref.m), (tr.v, ref.v)):
+        assert rel_err(a.cpu().numpy(), b.cpu().numpy()) <= 1e-5
+
+
+def test_a_step_that_fails_leaves_the_step_count(cuda_dev):
+    import torch
+
+    import mamba_rs_b200 as mb
+    w = mb.MambaWeights(mb.MambaConfig(d_model=64, n_layers=1), cuda_dev, dtype=torch.float32, vocab=50).init_random(3)
+    tr, ids = mb.MambaLMTrainer(w), torch.randint(0, 50, (1, 9), device=cuda_dev, dtype=torch.int32)
+    forward = tr.forward
+    for i in range(5):  # (the third would be recorded)
+        def fail(ids):
+            forward(ids)
+            raise torch.OutOfMemoryError("no room")
+        tr.forward = fail
+        with pytest.raises(torch.OutOfMemoryError):
+            tr.step(ids)
+        tr._acts = None
+        assert tr.t == 0 and not tr._plan(1, 8).replay.kept
+    tr.forward = forward
+    assert np.isfinite(float(tr.step(ids))) and tr.t == 1
