@@ -574,9 +574,14 @@ class GpuMambaBackbone:
             branch = plan.replay.run(temporal.data_ptr(), lambda: self._step_layers(temporal))
         else:
             branch = self._step_layers(temporal)
-        # (the caller keeps the result, so the norm that writes it is no part of a replay)
-        out, _ = ops.residual_rmsnorm_fwd(temporal, branch, w.tail("master")["norm_f"], eps=c.rms_norm_eps, out_dtype=w.dtype)
-        return out
+        return self._step_norm(temporal, branch)  # (the caller keeps it, so it is no part of a replay)
+
+    def _step_operators(self, temporal):
+        return self._step_norm(temporal, self._step_layers(temporal))
+
+    def _step_norm(self, temporal, branch):
+        return ops.residual_rmsnorm_fwd(temporal, branch, self.w.tail("master")["norm_f"], eps=self.cfg.rms_norm_eps,
+                                        out_dtype=self.w.dtype)[0]
 
     def _step_layers(self, res):
         c, w, B = self.cfg, self.w, res.shape[0]
@@ -642,22 +647,24 @@ class GpuMambaLM:
         torch.matmul(hidden, emb.t(), out=self.logits)
         self.next_ids.copy_(self.logits.argmax(dim=1))
 
-    def _decode_once(self):
+    def _decode_once(self, operators=False):
         emb = self.w.tail()["embedding"]
         temporal = ops.embedding_gather(emb, self.next_ids)
-        hidden = self.backbone.step(temporal)
+        hidden = self.backbone._step_operators(temporal) if operators else self.backbone.step(temporal)
         torch.matmul(hidden, emb.t(), out=self.logits)
         self.next_ids.copy_(self.logits.argmax(dim=1))
 
     def generate_greedy(self, n: int, use_graph: bool = True) -> torch.Tensor:
-        """n greedy tokens after a prefill; returns them as [B, n] int32."""
+        """n greedy tokens after a prefill; returns them as [B, n] int32.  use_graph=False: operator by
+        operator, also where the one-launch kernel would take the step (it needs every SM at once, the
+        operators run beside other streams' work)."""
         out = torch.empty(self.batch, n, dtype=torch.int32, device=self.w.device)
         dec = self._dec
         if dec is None or dec.key != _DecodePlan.made_from(self.backbone):
             dec = _DecodePlan(self.backbone, self.batch, self)
             if not _capturing(self.w.master):
                 self._dec = dec
-        if dec.ok and n > 0:
+        if use_graph and dec.ok and n > 0:
             a = dec.args
             a.next_ids, a.logits, a.steps = self.next_ids.data_ptr(), self.logits.data_ptr(), n
             a.tokens, a.tokens_ld = out.data_ptr(), n
@@ -682,7 +689,7 @@ class GpuMambaLM:
             if use_graph:
                 self._graph.replay()
             else:
-                self._decode_once()
+                self._decode_once(operators=True)
         return out
 
 

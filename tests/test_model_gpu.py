@@ -398,3 +398,33 @@ def test_a_step_that_fails_leaves_the_step_count(cuda_dev):
         assert tr.t == 0 and not tr._plan(1, 8).replay.kept
     tr.forward = forward
     assert np.isfinite(float(tr.step(ids))) and tr.t == 1
+
+
+def test_greedy_decode_by_operators_eager_captured_and_the_one_launch_kernel_agree(cuda_dev):
+    """The three ways generate_greedy has: operators launched one by one (use_graph=False), the captured step
+    where the kernel does not take the model, and the kernel."""
+    import torch
+
+    import mamba_rs_b200 as mb
+    from mamba_rs_b200 import model
+    w = mb.MambaWeights(mb.MambaConfig(d_model=128, n_layers=3), cuda_dev, vocab=997).init_random(11)
+    w.tail("master")["embedding"].mul_(50.0)
+    w.refresh()
+    ids = torch.randint(0, 997, (4, 60), device=cuda_dev, dtype=torch.int32, generator=torch.Generator(device=cuda_dev).manual_seed(2))
+    got = {}
+    for way in ("eager", "captured", "kernel"):
+        lm = mb.GpuMambaLM(w, 4)
+        lm.prefill(ids)
+        lm._dec = model._DecodePlan(lm.backbone, 4, lm)
+        if way == "captured":
+            lm._dec.ok = False
+            lm.backbone._plan(4).ok = False
+        before = lm._dec.ws[:4].view(torch.int32).item()
+        got[way] = lm.generate_greedy(12, use_graph=way != "eager").cpu().numpy(), lm.backbone.ssm.cpu().numpy()
+        assert (lm._graph is not None) == (way == "captured")
+        assert (lm._dec.ws[:4].view(torch.int32).item() > before) == (way == "kernel")  # tags used by launches
+        assert lm.backbone._plan(4).ok == (way != "captured") and (way == "kernel" or not int(lm.backbone._plan(4).ws[:4].view(torch.int32)))
+    np.testing.assert_array_equal(got["eager"][0], got["captured"][0])
+    np.testing.assert_array_equal(got["eager"][1], got["captured"][1])
+    np.testing.assert_array_equal(got["kernel"][0], got["eager"][0])
+    assert rel_err(got["kernel"][1], got["eager"][1]) <= 2e-2
