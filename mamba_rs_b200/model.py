@@ -196,6 +196,22 @@ def _capturing(t):
         return torch.cuda.is_current_stream_capturing()
 
 
+class _Lent:
+    """Buffers that a plan keeps between calls.  Where a call runs on another stream than the one they were
+    made on, the allocator is told, so that a plan which is dropped does not hand memory on that the call
+    still reads."""
+
+    def __init__(self, *tensors):
+        self.tensors, self.dev = tensors, tensors[0].device.index
+        self.home = torch._C._cuda_getCurrentRawStream(self.dev)
+
+    def use(self):
+        if torch._C._cuda_getCurrentRawStream(self.dev) != self.home and not torch.cuda.is_current_stream_capturing():
+            here = torch.cuda.current_stream(self.dev)
+            for t in self.tensors:
+                t.record_stream(here)
+
+
 class _Launcher:
     """The library's entry points on one device's current stream, with the arguments a plan has
     prepared: what a layer's launches cost on the host is then the call itself."""
@@ -478,9 +494,11 @@ class _DecodePlan:
         if self.ok:
             self.ws = torch.zeros(a.workspace_bytes, dtype=torch.uint8, device=w.device)
             a.workspace = self.ws.data_ptr()
+            self.lent = _Lent(self.ws)
             if lm is not None:
                 self.res = torch.empty(B, c.d_model, device=w.device)
                 a.residual = self.res.data_ptr()
+                self.lent = _Lent(self.ws, self.res)
         self._call, self._ref = lib.mamba_b200_decode_step, C.byref(a)
 
     @staticmethod
@@ -492,6 +510,7 @@ class _DecodePlan:
                 bb.cfg.rms_norm_eps, *[a.data_ptr() for a in w.a_neg])
 
     def launch(self):
+        self.lent.use()
         dev = self.handle.device
         stream = torch.cuda.current_stream(dev).cuda_stream
         if torch.cuda.current_device() == dev:
@@ -634,6 +653,8 @@ class GpuMambaLM:
                 with torch.cuda.device(ids.device):
                     if p.ids is None:
                         p.ids = torch.empty(B, T, dtype=torch.int32, device=ids.device)
+                        p.lent = _Lent(p.ids)
+                    p.lent.use()
                     p.ids.copy_(ids)
                     p.replay.run((self.logits.data_ptr(), self.next_ids.data_ptr()), lambda: self._prefill(p.ids))
                 return self.logits
@@ -716,9 +737,10 @@ class _TrainPlan:
                           lib.mamba_b200_residual_rmsnorm_bwd_workspace_bytes(B * T, c.d_model), 1)
         self.norm_f = w.tail("master")["norm_f"].data_ptr()
         self.fwd_at = self.bwd_at = None
-        self.ids = None
+        self.ids = torch.empty(B, T + 1, dtype=torch.int32, device=w.device)
         # few f32 rows: their sum is one more product (of the rows kernel)
         self.ones = torch.ones(B * T, 1, device=w.device) if w.dtype == torch.float32 and B * T <= 32 else None
+        self.lent = _Lent(self.ids, *(() if self.ones is None else (self.ones,)))
         a_layer = B * T * (4 * (c.d_model + 1) + self.es * (c.d_model + 5 * di + xd)) + 4 * B * self.blocks * di * N
         written = c.n_layers * a_layer + B * T * self.es * (w.vocab or 0) + self.fwd_ws + self.bwd_ws
         # (beyond 512 MB of activations the gaps are a few per cent of the work)
@@ -927,6 +949,7 @@ class MambaLMTrainer:
                 _product(go, 1, d_out, lay.w_out, d_y)
                 go.call(scan, lay.scan_b)
                 if plan.ones is not None:
+                    plan.lent.use()
                     acc(g["dt_proj_b"].view(1, di), plan.ones, d_delta)
                 else:
                     g["dt_proj_b"].add_(torch.sum(d_delta, 0, dtype=torch.float32))
@@ -978,8 +1001,7 @@ class MambaLMTrainer:
             plan = self._plan(B, T1 - 1)
             if plan.launch_bound:
                 with torch.cuda.device(self.w.device):
-                    if plan.ids is None:
-                        plan.ids = torch.empty(B, T1, dtype=torch.int32, device=self.w.device)
+                    plan.lent.use()
                     plan.ids.copy_(ids)
                     # (the update stays outside: a schedule changes its numbers from step to step)
                     loss = plan.replay.run((), lambda: self._loss_and_gradients(plan.ids)).clone()

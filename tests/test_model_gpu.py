@@ -428,3 +428,30 @@ def test_greedy_decode_by_operators_eager_captured_and_the_one_launch_kernel_agr
     np.testing.assert_array_equal(got["eager"][1], got["captured"][1])
     np.testing.assert_array_equal(got["kernel"][0], got["eager"][0])
     assert rel_err(got["kernel"][1], got["eager"][1]) <= 2e-2
+
+
+def test_a_workspace_is_not_handed_on_while_another_stream_uses_it(cuda_dev):
+    """A step on a stream that is held up, its plan dropped meanwhile: memory asked for on the plan's own stream
+    must not be the workspace that the step has yet to use."""
+    import torch
+
+    import mamba_rs_b200 as mb
+    w = mb.MambaWeights(mb.MambaConfig(d_model=256, n_layers=2), cuda_dev).init_random(3)
+    bb, side = mb.GpuMambaBackbone(w, 16), torch.cuda.Stream(device=cuda_dev)
+    x = torch.randn(16, 256, device=cuda_dev)
+    want = bb.step(x.clone())
+    for again in (False, True):
+        bb.reset()
+        y, held = x.clone(), bb._plan(16).ws
+        at, size = held.data_ptr(), held.numel()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(side):
+            torch.cuda._sleep(50_000_000)
+            got = bb.step(y)
+        del held
+        bb._plans.clear()
+        taken = [torch.full((size,), 255, dtype=torch.uint8, device=cuda_dev) for _ in range(4)]
+        assert at not in [t.data_ptr() for t in taken]
+        side.synchronize()
+        assert torch.equal(got, want)
+        del taken
