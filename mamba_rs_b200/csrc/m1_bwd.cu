@@ -651,9 +651,8 @@ static int bwd_segments(int B, int T, int D, int N) {
 static int bwd_ns(int N) { return N <= 4 ? 4 : (N <= 8 ? 8 : 16); }
 
 
-static void bwd_ws_layout(int B, int T, int D, int N, size_t* off_a, size_t* off_d, size_t* off_dense,
+static void bwd_ws_layout(int B, int T, int D, int N, size_t segs, size_t* off_a, size_t* off_d, size_t* off_dense,
                           size_t* total, size_t* off_dh = nullptr, size_t* off_sum = nullptr) {
-    const size_t segs = bwd_segments(B, T, D, N);
     // channel tiles of the dB/dC partials: 16 channels per CTA for the two-lane
     // kernel (d_state > 8), 32 for the one-lane kernel
     size_t tiles = N > 8 ? (D + 15) / 16 : (D + 31) / 32, V = 2 * bwd_ns(N);
@@ -686,7 +685,7 @@ using namespace mb200;
 extern "C" MAMBA_B200_API long long mamba_b200_sscan_bwd_workspace_bytes(int B, int T, int D, int N) {
     if (B <= 0 || T <= 0 || D <= 0 || N <= 0 || N > 256) return 0;
     size_t a, d, dn, total;
-    bwd_ws_layout(B, T, D, N, &a, &d, &dn, &total);
+    bwd_ws_layout(B, T, D, N, bwd_segments(B, T, D, N), &a, &d, &dn, &total);
     return static_cast<long long>(total);
 }
 
@@ -709,7 +708,12 @@ static int launch_bwd(Ctx* c, void* stream, const mamba_b200_sscan_bwd_args& a, 
         a.ld_ddelta < a.D || (a.z_mode && (a.ld_z < a.D || a.ld_dz < a.D)))
         return fail(c, MAMBA_B200_ERR_ARG, "sscan_bwd: a row stride is smaller than its row");
     size_t off_a, off_d, off_dense, total, off_dh, off_sum;
-    bwd_ws_layout(a.B, a.T, a.D, a.N, &off_a, &off_d, &off_dense, &total, &off_dh, &off_sum);
+    // A smaller batch may be cut into more segments and then needs more than a larger one: a workspace sized
+    // for the largest has room for every call, in fewer segments where it must be.
+    int segs = bwd_segments(a.B, a.T, a.D, a.N) + 1;
+    do
+        bwd_ws_layout(a.B, a.T, a.D, a.N, --segs, &off_a, &off_d, &off_dense, &total, &off_dh, &off_sum);
+    while (segs > 1 && a.workspace_bytes < static_cast<long long>(total));
     if (a.workspace_bytes < static_cast<long long>(total))
         return fail(c, MAMBA_B200_ERR_ARG, "sscan_bwd: workspace %lld < %zu bytes", a.workspace_bytes, total);
     if (reinterpret_cast<uintptr_t>(a.workspace) % 256)
@@ -785,12 +789,10 @@ static int launch_bwd(Ctx* c, void* stream, const mamba_b200_sscan_bwd_args& a, 
     const int flags = (a.delta_softplus ? 1 : 0) | (a.z_mode ? 2 : 0);
     const int tiles = (a.D + DT - 1) / DT;
     dim3 grid(tiles, a.B);
-    int segs = 1;
     if (two_lane) {
         const Bwd2Table& t2 = bwd2_table();
         const unsigned loads = kBU | kBDl | kBZ | kBDy | kBB | kBC;
         const int flags2 = flags | ((m & loads) != loads ? 8 : 0);
-        segs = bwd_segments(a.B, a.T, a.D, a.N);
         if (segs > 1) {
             const int nblk = (a.T + S - 1) / S;
             p.seg_blocks = (nblk + segs - 1) / segs;

@@ -177,3 +177,27 @@ def test_sums_over_channel_tiles_of_small_and_large_calls_agree(cuda_dev, D):
         for k in ("dB", "dC"):
             assert rel_err(g[k][0], whole[k][b]) <= 1e-5
     torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("dt", ["f32", "bf16"])
+def test_a_workspace_for_a_larger_batch_serves_a_smaller_one(cuda_dev, dt):
+    """22 sequences are cut into time segments and would take more than 23, which are not: with the memory of
+    23 they run in fewer segments."""
+    import torch
+
+    import mamba_rs_b200 as mb
+    B, T, D, N, S = 22, 128, 640, 16, 32
+    size = mb.selective_scan_bwd_workspace_bytes
+    assert size(B, T, D, N) > size(B + 1, T, D, N)
+    q = quantised_inputs(B, T, D, N, 0, dt, seed=1)
+    td = torch_dtype(dt)
+    t = lambda k, d=None: to_dev(q[k], cuda_dev, d)  # noqa: E731
+    args = [t("x", td), t("delta_raw", td), t("Bm", td), t("Cm", td), t("a_neg"), t("Dp")]
+    z, dy = t("z", td), torch.randn(B, T, D, device=cuda_dev, generator=torch.Generator(device=cuda_dev).manual_seed(2)).to(td)
+    cs = torch.empty(B, T // S, D, N, device=cuda_dev)
+    mb.selective_scan_fwd(*args, z, chunk_states=cs, save_stride=S)
+    run = lambda n: mb.selective_scan_bwd(*args, dy, cs, S, z, workspace=torch.empty(n, dtype=torch.uint8, device=cuda_dev))  # noqa: E731
+    own, lent = run(size(B, T, D, N)), run(size(B + 1, T, D, N))
+    for k in own:
+        assert rel_err(lent[k].float().cpu().numpy(), own[k].float().cpu().numpy()) <= (1e-5 if dt == "f32" else TOL[dt]), k
+    mb.ffi.default_handle(0).check_status()
