@@ -1190,11 +1190,14 @@ static void m3_bwd_ws(bool tc, int B, int T, int nh, int hd, int N, size_t* o_g,
 }
 
 // The line of pairs cut into one length per SM (WRAP): from one pair per SM on, where whole waves would
-// leave more than 4 % of the SMs' time idle.
+// leave more than 4 % of the SMs' time idle, and where that is at least 1.3 chunks of an SM's time, which a
+// cooperative launch and the two hand-overs of a CTA cost.  Whole waves and the line, 64 x 128, bf16: 256
+// pairs (0.27 of a wave idle) of 256 steps 67 and 80 us, 512: 125 and 130, 1024: 240 and 235; 192 (0.70) of
+// 200: 56 and 60, 256: 63 and 61; 150 (0.99) of 128: 31 and 37, 200: 57 and 55, 1024: 267 and 169.
 constexpr int kWrapSms = 160;  // hand-overs the workspace has room for
-static bool m3_bwd_wraps(long long heads, int sms) {
-    const long long waves = (heads + sms - 1) / sms;
-    return heads > sms && sms < kWrapSms && heads * 100 < waves * sms * 96;
+static bool m3_bwd_wraps(long long heads, int T, int sms) {
+    const long long waves = (heads + sms - 1) / sms, idle = waves * sms - heads;
+    return heads > sms && sms < kWrapSms && heads * 100 < waves * sms * 96 && 10 * idle * T >= 13LL * tcb::CS * sms;
 }
 static size_t m3_bwd_wrap_bytes() { return 1024 + sizeof(float) * kWrapSms * tcb::kHand; }
 
@@ -1293,7 +1296,7 @@ extern "C" MAMBA_B200_API int mamba_b200_m3_ssd_bwd(void* handle, void* stream,
         const bool f16 = a.dtype == MAMBA_B200_F16;
         // (the outer CTAs of a cluster have one pass more than an undivided one, those between them two.)  bf16,
         // 64 x 128: 4 heads x 4096 steps 114 us (one CTA each: 446), 24 x 2048 104 (224), 64 x 4096 285 (450)
-        const bool wrap = m3_bwd_wraps(static_cast<long long>(a.B) * a.nh, c->sm_count) &&
+        const bool wrap = m3_bwd_wraps(static_cast<long long>(a.B) * a.nh, a.T, c->sm_count) &&
                           a.workspace_bytes >= static_cast<long long>(total + m3_bwd_wrap_bytes());
         // 8 x 4096 steps x 32 heads of 64 x 128, bf16: 861 us (931 in two waves).  False: plain launch.
         auto wrap_launch = [&]() {

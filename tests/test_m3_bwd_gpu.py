@@ -166,3 +166,14 @@ def test_tensor_core_backward_is_linear_in_dy_at_config4_size(cuda_dev):
         want = g1[k].float() + g2[k].float()
         err = float((g12[k].float() - want).abs().max() / want.abs().max())
         assert err <= TOL["bf16"], (k, err)
+
+
+# where the cut line begins to pay: pairs of two chunks that nearly fill one wave, of seven that leave a quarter
+# of two waves; and one step less than the rule asks for
+@pytest.mark.parametrize("shape", [(3, 169, 50, 64, 128), (3, 168, 50, 64, 128), (4, 616, 64, 64, 128), (4, 615, 64, 64, 128)],
+                         ids=lambda s: "B%dT%dnh%dhd%dN%d" % s)
+def test_pairs_on_both_sides_of_the_cut_rule_match_cuda_core_path(cuda_dev, shape):
+    i, dy = case(shape, "bf16", seed=shape[1])
+    got, ref = run_gpu(i, dy, "bf16", cuda_dev), run_gpu(i, dy, "f32", cuda_dev)
+    for k in ("dx",) + F32_OUT:
+        assert rel_err(got[k], ref[k]) <= TOL["bf16"], k
