@@ -117,10 +117,11 @@ __global__ void __launch_bounds__(kNormThreads) residual_rmsnorm_fwd_kernel(cons
     }
 }
 
-// The same for rows of up to 4096 elements, held in registers: TPR threads a row, NV 16-byte pieces
+// The same for rows of up to 8192 elements, held in registers: TPR threads a row, NV 16-byte pieces
 // each, all of a row's loads in flight at once and no second pass through shared memory.  A row of
-// up to 1024 elements belongs to one warp, without a block barrier.  HBM-bound: at 16384 x 768 (bf16)
-// 25 us against 40 us of the kernel above, which walks rows one at a time per CTA.
+// up to 1024 elements belongs to one warp, without a block barrier (where there are enough of them,
+// launch_norm_fwd).  HBM-bound: at 16384 x 768 (bf16) 25 us against 40 us of the kernel above, which
+// walks rows one at a time per CTA; at 2048 x 5120 13.7 against 17.3.
 template <typename Tact, int TPR, int NV>
 __global__ void __launch_bounds__(kNormThreads) residual_rmsnorm_fwd_reg_kernel(const NormParams p) {
     constexpr int RP = kNormThreads / TPR;
@@ -200,17 +201,27 @@ __global__ void __launch_bounds__(kNormThreads) residual_rmsnorm_fwd_reg_kernel(
     }
 }
 
+// Below six rows an SM a row has a whole CTA, one or two pieces a thread: a warp with eight pieces of its own
+// row takes longer than all of its loads together (f32, 32 x 1024: 1.9 us for 2.9, 400 x 768: 2.3 for 2.8; from
+// 1184 x 768 on 3.2 for 3.1).  Rows of up to 128 elements are one piece a lane and stay with the warp (800 x 128:
+// 1.9 us, 2.2 by CTAs).
+constexpr int kNormFewRows = 6 * 148;
+
 template <typename Tact>
 static void launch_norm_fwd(const NormParams& p, bool vec, int ctas, cudaStream_t st) {
     const int q = p.dim / 4;
+    const bool few = p.rows < kNormFewRows && q > 32;
 #define MB200_NORM_REG(TPR, NV)                                                                              \
     residual_rmsnorm_fwd_reg_kernel<Tact, TPR, NV>                                                           \
         <<<(p.rows + kNormThreads / TPR - 1) / (kNormThreads / TPR), kNormThreads, 0, st>>>(p)
-    if (vec && q <= 64) MB200_NORM_REG(32, 2);
+    if (vec && few && q <= 256) MB200_NORM_REG(256, 1);
+    else if (vec && few && q <= 512) MB200_NORM_REG(256, 2);
+    else if (vec && q <= 64) MB200_NORM_REG(32, 2);
     else if (vec && q <= 128) MB200_NORM_REG(32, 4);
     else if (vec && q <= 256) MB200_NORM_REG(32, 8);
     else if (vec && q <= 512) MB200_NORM_REG(128, 4);
     else if (vec && q <= 1024) MB200_NORM_REG(256, 4);
+    else if (vec && q <= 2048) MB200_NORM_REG(256, 8);
     else if (vec) residual_rmsnorm_fwd_kernel<Tact, true><<<ctas, kNormThreads, sizeof(float) * p.dim, st>>>(p);
     else residual_rmsnorm_fwd_kernel<Tact, false><<<ctas, kNormThreads, sizeof(float) * p.dim, st>>>(p);
 #undef MB200_NORM_REG

@@ -142,3 +142,23 @@ def test_sgemm_rows_matches_f64(cuda_dev, size, op):
         h.check(rc, "sgemm_rows")
         torch.cuda.synchronize()
         assert float((c.double() - ref).abs().max()) <= 3e-6 * K ** 0.5 * max(1.0, float(ref.abs().max()) / K ** 0.5)
+
+
+@pytest.mark.parametrize("dt", ["f32", "bf16"])
+@pytest.mark.parametrize("dim", [128, 132, 1024, 1028, 2048, 2052, 4096, 4100, 8192, 8196])
+def test_residual_rmsnorm_forward_at_the_edges_of_its_kernels(cuda_dev, dim, dt):
+    """Widths where the pieces of a thread or the threads of a row change, on both sides of few rows."""
+    import torch
+
+    import mamba_rs_b200 as mb
+    td = torch_dtype(dt)
+    g = torch.Generator(device=cuda_dev).manual_seed(dim)
+    rn = lambda *s: torch.randn(*s, device=cuda_dev, generator=g)  # noqa: E731
+    for rows in (1, 887, 888):
+        res, br, sc = rn(rows, dim), rn(rows, dim).to(td), rn(dim)
+        x = res.double() + br.double()
+        rms = (x.square().mean(1) + 1e-5).sqrt()
+        y, r = mb.residual_rmsnorm_fwd(res, br, sc)
+        want = x / rms[:, None] * sc.double()
+        assert float((res.double() - x).abs().max()) <= 1e-6 and float((r.double() / rms - 1).abs().max()) <= 1e-6
+        assert float((y.double() - want).abs().max() / want.abs().max()) <= (1e-6 if dt == "f32" else 2 ** -8)
