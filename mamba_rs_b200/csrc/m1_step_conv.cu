@@ -307,9 +307,9 @@ __device__ __forceinline__ void conv_load_taps(const ConvParams& p, int d, float
     }
 }
 
-template <typename Tact>
+template <typename Tact, int VEC>
 __global__ void __launch_bounds__(32 * kConvWarps) conv1d_fwd_rows_kernel(const ConvParams p) {
-    constexpr int VEC = 4, KV = kConvKV, R = kConvRT + KV - 1;
+    constexpr int KV = kConvKV, R = kConvRT + KV - 1;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int d = (blockIdx.x * 32 + lane) * VEC, t0 = blockIdx.y * kConvTT + warp * kConvRT, b = blockIdx.z;
     if (d >= p.D || t0 >= p.T) return;
@@ -605,12 +605,20 @@ extern "C" MAMBA_B200_API int mamba_b200_conv1d_fwd(void* handle, void* stream,
     dim3 grid((a.D + 127) / 128, chunks, a.B);
     const unsigned sb = static_cast<unsigned>((static_cast<long long>(a.B) * a.D + 127) / 128);
     const size_t es = a.dtype == MAMBA_B200_F32 ? 4 : 2;
-    if (conv_vec_ok(a.K, a.D, 4, es, {a.x, a.u}, {a.ld_x, a.ld_u}) && reinterpret_cast<uintptr_t>(a.conv_w) % 16 == 0) {
-        dim3 vgrid((a.D / 4 + 31) / 32, chunks, a.B);
+    // four channels a lane; of f32 two where rows allow no more (8 x 2048 x 1538: 38 us, 86 by the scalar kernel)
+    // and where a warp has all steps, so that twice as many share them (16 x 1 x 5120: 3.2 us for 4.9, 16 x 8 x
+    // 5120: 3.2 for 4.4)
+    auto vec = [&](int v) {
+        return conv_vec_ok(a.K, a.D, v, es, {a.x, a.u}, {a.ld_x, a.ld_u}) && reinterpret_cast<uintptr_t>(a.conv_w) % 16 == 0;
+    };
+    const int v = a.dtype == MAMBA_B200_F32 && vec(2) && (a.T <= kConvRT || !vec(4)) ? 2 : vec(4) ? 4 : 0;
+    if (v) {
+        dim3 vgrid((a.D / v + 31) / 32, chunks, a.B);
         const int threads = 32 * std::min(kConvWarps, (a.T + kConvRT - 1) / kConvRT);
-        if (a.dtype == MAMBA_B200_F32) conv1d_fwd_rows_kernel<float><<<vgrid, threads, 0, st>>>(p);
-        else if (a.dtype == MAMBA_B200_F16) conv1d_fwd_rows_kernel<__half><<<vgrid, threads, 0, st>>>(p);
-        else conv1d_fwd_rows_kernel<__nv_bfloat16><<<vgrid, threads, 0, st>>>(p);
+        if (v == 2) conv1d_fwd_rows_kernel<float, 2><<<vgrid, threads, 0, st>>>(p);
+        else if (a.dtype == MAMBA_B200_F32) conv1d_fwd_rows_kernel<float, 4><<<vgrid, threads, 0, st>>>(p);
+        else if (a.dtype == MAMBA_B200_F16) conv1d_fwd_rows_kernel<__half, 4><<<vgrid, threads, 0, st>>>(p);
+        else conv1d_fwd_rows_kernel<__nv_bfloat16, 4><<<vgrid, threads, 0, st>>>(p);
     } else if (a.dtype == MAMBA_B200_F32) {
         conv1d_fwd_kernel<float><<<grid, 128, 0, st>>>(p);
         if (a.conv_state) conv1d_state_kernel<float><<<sb, 128, 0, st>>>(p);
@@ -653,7 +661,8 @@ extern "C" MAMBA_B200_API int mamba_b200_conv1d_bwd(void* handle, void* stream,
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     dim3 grid((a.D + 127) / 128, chunks, a.B);
     const size_t es = a.dtype == MAMBA_B200_F32 ? 4 : 2;
-    if (conv_vec_ok(a.K, a.D, 2, es, {a.x, a.d_u, a.d_x}, {a.ld_x, a.ld_du, a.ld_dx}) &&
+    // (a single step has no rows to share: 1 x 1 x 1536 4.9 us by the scalar kernel, 5.6 by rows)
+    if (a.T > 1 && conv_vec_ok(a.K, a.D, 2, es, {a.x, a.d_u, a.d_x}, {a.ld_x, a.ld_du, a.ld_dx}) &&
         reinterpret_cast<uintptr_t>(a.conv_w) % 16 == 0) {
         dim3 vgrid((a.D / 2 + 31) / 32, chunks, a.B);
         const int threads = 32 * std::min(kConvWarps, (a.T + kConvRT - 1) / kConvRT);

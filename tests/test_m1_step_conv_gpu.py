@@ -154,3 +154,22 @@ def test_decode_step_with_state_slices_that_are_only_4_byte_aligned(cuda_dev, dt
                          q["Dp"], q["conv_w"], q["conv_b"], cst0, ssm0)
     assert rel_err(y.float().cpu().numpy(), ref["y"]) <= TOL[dt]
     assert rel_err(ssm.cpu().numpy(), ref["ssm_state"]) <= 1e-4
+
+
+@pytest.mark.parametrize("K", [2, 4])
+@pytest.mark.parametrize("T", [1, 2, 8, 9, 64, 65, 130])
+def test_f32_channel_counts_that_are_even_but_no_multiple_of_four(cuda_dev, T, K):
+    """Two channels a lane: short sequences of any even count, longer ones where four do not fit."""
+    import torch
+
+    import mamba_rs_b200 as mb
+    for B, D in ((2, 66), (1, 6), (2, 68)):
+        g = torch.Generator(device=cuda_dev).manual_seed(T + D)
+        rn = lambda *s: torch.randn(*s, device=cuda_dev, generator=g)  # noqa: E731
+        x, w, b, st = rn(B, T, D), rn(D, K), rn(D), rn(B, D, K)
+        full = torch.cat([st.transpose(1, 2)[:, 1:], x], 1).double()  # the K-1 steps before the first, then x
+        want = b.double() + sum(full[:, k:k + T] * w[:, k].double() for k in range(K))
+        want = want * torch.sigmoid(want)
+        left = torch.cat([st.transpose(1, 2), x], 1)[:, -K:].transpose(1, 2)
+        u = mb.conv1d_fwd(x, w, b, st)
+        assert float((u.double() - want).abs().max()) <= 1e-5 and torch.equal(st, left)
