@@ -162,3 +162,24 @@ def test_residual_rmsnorm_forward_at_the_edges_of_its_kernels(cuda_dev, dim, dt)
         want = x / rms[:, None] * sc.double()
         assert float((res.double() - x).abs().max()) <= 1e-6 and float((r.double() / rms - 1).abs().max()) <= 1e-6
         assert float((y.double() - want).abs().max() / want.abs().max()) <= (1e-6 if dt == "f32" else 2 ** -8)
+
+
+@pytest.mark.parametrize("op", [0, 1])
+@pytest.mark.parametrize("size", [(32, 768, 50280), (12, 64, 50277), (33, 100, 4096), (32, 80, 1536)], ids=lambda s: "m%dn%dk%d" % s)
+def test_sgemm_rows_stays_as_exact_over_a_long_contraction(cuda_dev, size, op):
+    """One chain of f32 sums drifts by its length (1.4e-6 at 50280); chains of 256 whose sums are added up do
+    not: about 2^-24 of the root of 256 steps each."""
+    import torch
+
+    from mamba_rs_b200 import ffi
+    M, N, K = size
+    h = ffi.default_handle(0)
+    g = torch.Generator(device=cuda_dev).manual_seed(K)
+    a = torch.randn(M, K, device=cuda_dev, generator=g)
+    b = torch.randn(*((K, N) if op == 0 else (N, K)), device=cuda_dev, generator=g)
+    bt, c = (b if op == 0 else b.t()), torch.empty(M, N, device=cuda_dev)
+    rc = ffi.lib().mamba_b200_sgemm_rows(h.ptr, torch.cuda.current_stream().cuda_stream, op, a.data_ptr(), K, b.data_ptr(),
+                                         b.stride(0), None, c.data_ptr(), N, M, N, K)
+    h.check(rc, "sgemm_rows")
+    ref = a.double() @ bt.double()
+    assert float((c.double() - ref).norm() / ref.norm()) <= 4e-7
