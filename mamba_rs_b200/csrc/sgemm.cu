@@ -157,7 +157,8 @@ template <bool VEC>
 __global__ void __launch_bounds__(256) grad_kernel(const Params p) {
     constexpr int BC = 64;
     __shared__ __align__(16) float A[BK][BC], B[BK][BC];
-    const int tid = threadIdx.x, m0 = blockIdx.y * BC, n0 = blockIdx.x * BC, tx = tid & 15, ty = tid >> 4;
+    const int tid = threadIdx.x, nx = (p.N + BC - 1) / BC, tx = tid & 15, ty = tid >> 4;
+    const int m0 = static_cast<int>(blockIdx.x / nx) * BC, n0 = static_cast<int>(blockIdx.x % nx) * BC;
     float acc[4][4];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
@@ -235,8 +236,9 @@ extern "C" MAMBA_B200_API int mamba_b200_sgemm_rows(void* handle, void* stream, 
         p.kper = 0;
         // a row's groups of four are whole where both sides are multiples of four
         const bool vec = al(a, lda) && al(b, ldb) && al(out, ldc) && M % 4 == 0 && N % 4 == 0;
-        const dim3 grid((N + 63) / 64, (M + 63) / 64);
-        if (grid.y > 65535) return fail(c, MAMBA_B200_ERR_SHAPE, "sgemm_rows: %d rows of a gradient", M);
+        const long long tiles = ((N + 63LL) / 64) * ((M + 63LL) / 64);  // one row of them: a vocabulary may have more than 65535
+        if (tiles > 0x7fffffff) return fail(c, MAMBA_B200_ERR_SHAPE, "sgemm_rows: a gradient of %d x %d", M, N);
+        const dim3 grid(static_cast<unsigned>(tiles));
         if (vec) sg::grad_kernel<true><<<grid, 256, 0, st>>>(p);
         else sg::grad_kernel<false><<<grid, 256, 0, st>>>(p);
         MB200_CUDA_CHECK(c, cudaGetLastError());

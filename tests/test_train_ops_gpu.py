@@ -183,3 +183,18 @@ def test_sgemm_rows_stays_as_exact_over_a_long_contraction(cuda_dev, size, op):
     h.check(rc, "sgemm_rows")
     ref = a.double() @ bt.double()
     assert float((c.double() - ref).norm() / ref.norm()) <= 4e-7
+
+
+def test_sgemm_rows_gradient_takes_more_than_65535_tiles_of_rows(cuda_dev):
+    import torch
+
+    from mamba_rs_b200 import ffi
+    M, N, K = 64 * 65536 + 1, 3, 2
+    h = ffi.default_handle(0)
+    g = torch.Generator(device=cuda_dev).manual_seed(1)
+    a, b, c = (torch.randn(*s, device=cuda_dev, generator=g) for s in ((K, M), (K, N), (M, N)))
+    ref = c.double() + a.double().t() @ b.double()
+    rc = ffi.lib().mamba_b200_sgemm_rows(h.ptr, torch.cuda.current_stream().cuda_stream, 2, a.data_ptr(), M, b.data_ptr(), N, None,
+                                         c.data_ptr(), N, M, N, K)
+    h.check(rc, "sgemm_rows")
+    assert float((c.double() - ref).abs().max()) <= 1e-5
