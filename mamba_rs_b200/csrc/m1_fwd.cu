@@ -2,30 +2,48 @@
 // Host side of the fused forward: argument validation, TMA descriptors, variant
 // selection, the time-segment plan and launch.  The kernels live in
 // m1_fwd_kernel.cuh.
+#include <algorithm>
+
 #include "m1_fwd_kernel.cuh"
 
 namespace mb200 {
 
 constexpr int kMaxSegments = 64;
 
-// Time segments of a launch that was lent a workspace (see launch_fwd), chosen from the consumer warps
-// it has per warp scheduler.  A warp alone on its scheduler takes 225 cycles a step, with 2.6 beside
-// each other 340 for all of them, and the state-only first pass costs half of a full one, so from 1.15
-// warps per scheduler one piece is as fast (8 x 2048 x 1536: 288 us in one piece, 303 in four; at 6
-// sequences 248 and 239).  Below that the sequence is cut into at least 16 pieces, and into more until
-// the schedulers are full (1 x 8192 x 64), none shorter than about 32 steps; sequences under 192 steps
-// stay whole (1 x 128 x 1536: 21 us whole, 24 in four).
-static int fwd_segments(int B, int T, int D, int N) {
+// Time segments of a launch that was lent a workspace (see launch_fwd): the count with the least estimated
+// time.  In one piece a step takes 0.1155 us with one CTA per SM and 0.137 with two; both passes of a cut take
+// kCut[2 x] with x CTAs per SM on average (d_state 16, bf16; f32 takes 1.08 times as long throughout), a piece
+// costs its steps and 16 more for its pipeline to fill, and the call 8 us with two more launches.  Beyond 1.15 CTAs
+// per SM one piece is as fast, and under 192 steps (1 x 128 x 2560 whole 17.6, in four 18.9).  Fitted to 300 measured shapes of 64 to 4096 steps: half of the estimates are within 5 %, and
+// the counts chosen take 0.8 % longer than the best that was measured on average, 9 % at most.  Whole and as cut
+// here, bf16 and f32 in us: 1 x 1021 x 1536 118 and 31, 129 and 32; 2 x 192 x 1536 25 and 20, 27 and 19; 4 x 512 x
+// 1536 61 and 51, 66 and 53; 6 x 2048 x 1344 236 and 208, 259 and 213.
+constexpr int kFwdMaxPerSm = 9, kFwdMaxCtas = 170;
+static long long fwd_ctas(int B, int D, int N) {  // of four consumer warps, one a scheduler
     int lpc = 1;
     while (8 * lpc < N) lpc *= 2;
     const int cw = lpc >= 16 ? 8 : 4, dt = cw * (32 / lpc);
-    const double per_sched = static_cast<double>(B) * ((D + dt - 1) / dt) * cw / (4 * 148);
-    if (per_sched >= 1.15 || T < 192) return 1;
-    int s = static_cast<int>(2.6 / per_sched) + 1;
-    if (s < 16) s = 16;
-    if (s > kMaxSegments) s = kMaxSegments;
-    const int most = (T + 31) / 32;
-    return s < most ? s : most;
+    return static_cast<long long>(B) * ((D + dt - 1) / dt) * (cw / 4);
+}
+static int fwd_segments(int B, int T, int D, int N) {
+    static const double kCut[2 * kFwdMaxPerSm + 2] = {0.175, 0.180, 0.191, 0.221, 0.239, 0.275, 0.312, 0.395, 0.429, 0.460,
+                                                      0.508, 0.536, 0.568, 0.619, 0.669, 0.712, 0.753, 0.806, 0.860, 0.860};
+    const long long ctas = fwd_ctas(B, D, N);
+    if (ctas > kFwdMaxCtas || T < 192) return 1;
+    const int blocks = (T + 31) / 32;
+    int best = 1;
+    double cost = 3.5 + T * (ctas <= 148 ? 0.1155 : 0.137);
+    for (int s = 2; s <= kMaxSegments && s <= blocks && ctas * s <= kFwdMaxPerSm * 148; ++s) {
+        const int per = (blocks + s - 1) / s;
+        const double x = 2.0 * ctas * s / 148, f = x - static_cast<int>(x);
+        const double* at = kCut + static_cast<int>(x);
+        const double c = 8 + (32 * per + 16) * (at[0] + f * (at[1] - at[0]));
+        if (c < cost) {
+            cost = c;
+            best = s;
+        }
+    }
+    return best;
 }
 
 struct FwdTable {

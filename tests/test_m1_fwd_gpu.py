@@ -332,3 +332,26 @@ def test_unaligned_rows_take_plain_loads(cuda_dev, case, dt):
     torch.cuda.synchronize()
     mb.ffi.default_handle(0).check_status()
     assert rel_err(y.float().cpu().numpy(), ref["y"]) <= TOL[dt]
+
+
+# (B, T, D) either side of where the number of time segments changes: whole, four, eight, as many as fill the chip
+@pytest.mark.parametrize("dt", ["bf16", "f32"])
+@pytest.mark.parametrize("shape", [(2, 191, 320), (2, 192, 320), (3, 255, 1536), (11, 256, 640), (11, 255, 640), (6, 511, 1344), (6, 512, 1344),
+                                   (7, 999, 1344), (7, 1000, 1344), (7, 1536, 1344), (8, 1536, 1536), (1, 1021, 1536), (1, 2100, 64)],
+                         ids=lambda s: "B%dT%dD%d" % s)
+def test_time_segments_equal_one_piece(cuda_dev, shape, dt):
+    import torch
+
+    import mamba_rs_b200 as mb
+    (B, T, D), N, td = shape, 16, torch_dtype(dt)
+    g = torch.Generator(device=cuda_dev).manual_seed(T)
+    rn = lambda *s: torch.randn(*s, device=cuda_dev, generator=g)  # noqa: E731
+    args = [rn(B, T, D).to(td), (0.5 * rn(B, T, D) - 3).to(td), rn(B, T, N).to(td), rn(B, T, N).to(td), -torch.exp(rn(D, N)), rn(D)]
+    z, h = rn(B, T, D).to(td), rn(B, D, N)
+    ws = torch.empty(mb.selective_scan_fwd_workspace_bytes(B, T, D, N), dtype=torch.uint8, device=cuda_dev)
+    h1, h2 = h.clone(), h.clone()
+    whole, cut = mb.selective_scan_fwd(*args, z, ssm_state=h1), mb.selective_scan_fwd(*args, z, ssm_state=h2, workspace=ws)
+    mb.ffi.default_handle(0).check_status()
+    tol = 1e-5 if dt == "f32" else 2e-2
+    assert float((cut.float() - whole.float()).abs().max() / whole.float().abs().max()) <= tol
+    assert float((h2 - h1).abs().max() / h1.abs().max()) <= 1e-5
