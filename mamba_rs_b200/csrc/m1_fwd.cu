@@ -256,8 +256,15 @@ using namespace mb200;
 
 extern "C" MAMBA_B200_API long long mamba_b200_sscan_fwd_workspace_bytes(int B, int T, int D, int N) {
     if (B <= 0 || T <= 0 || D <= 0 || N <= 0 || N > 256) return 0;
-    size_t o1, o2, o3;
-    return static_cast<long long>(fwd_ws_bytes(B, D, N, fwd_segments(B, T, D, N), &o1, &o2, &o3));
+    // room for every batch up to B and length up to T, whose counts of segments may be larger
+    size_t o1, o2, o3, most = 0;
+    for (int b = 1; b <= B; ++b) {
+        const long long ctas = fwd_ctas(b, D, N);
+        if (ctas > kFwdMaxCtas) b = B;
+        const long long segs = ctas > kFwdMaxCtas ? 1 : std::min<long long>({kFwdMaxPerSm * 148 / ctas, (T + 31) / 32, kMaxSegments});
+        most = std::max(most, fwd_ws_bytes(b, D, N, static_cast<int>(segs), &o1, &o2, &o3));
+    }
+    return static_cast<long long>(most);
 }
 
 extern "C" MAMBA_B200_API int mamba_b200_sscan_fwd(void* handle, void* stream, const mamba_b200_sscan_fwd_args* args) {
