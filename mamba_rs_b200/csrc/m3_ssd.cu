@@ -54,7 +54,7 @@ struct M3Params {
 // row with 128 states in registers and two block barriers a step, which it replaces, took 8 us.
 // grid (nh, B, ceil(hd / rows of a CTA)).
 // ---------------------------------------------------------------------------
-template <typename Tact, int NI, int R>
+template <typename Tact, int NI, int R, bool PART>  // PART: the last 32 states are not all there
 __global__ void __launch_bounds__(256) m3_ssd_seq_kernel(const M3Params p) {
     constexpr int PF = 4;  // steps requested ahead
     const int h = blockIdx.x, b = blockIdx.y, lane = threadIdx.x & 31;
@@ -136,6 +136,7 @@ __global__ void __launch_bounds__(256) m3_ssd_seq_kernel(const M3Params p) {
                     acc[r] = 0.0f;
 #pragma unroll
                     for (int i = 0; i < NI; ++i) {
+                        if (PART && !nok[i]) continue;  // (an infinite x would make a NaN of the zeros there)
                         st[r][i] = fmaf(alpha, st[r][i], fmaf(bv, kp[i], gx * k[i]));
                         acc[r] = fmaf(st[r][i], q[i], acc[r]);
                     }
@@ -995,20 +996,32 @@ int m3_configure(Ctx* c) {
 
 // Eight rows a warp share one K / Q load and one butterfly; two rows a warp when that leaves
 // fewer than eight warps per SM (the step's chain, not the arithmetic, is then the time).
-template <typename Tact, int NI>
-static void launch_seq_ni(const M3Params& p, int sms, cudaStream_t st) {
-    const bool few = static_cast<long long>(p.B) * p.nh * ((p.hd + 7) / 8) < 8LL * sms;
-    const int rows = few ? 2 : 8, warps = min(8, (p.hd + rows - 1) / rows);
-    const dim3 grid(p.nh, p.B, (p.hd + rows * warps - 1) / (rows * warps));
-    if (few) m3_ssd_seq_kernel<Tact, NI, 2><<<grid, warps * 32, 0, st>>>(p);
-    else m3_ssd_seq_kernel<Tact, NI, 8><<<grid, warps * 32, 0, st>>>(p);
+template <typename Tact, int NI, int R, bool PART>
+static void launch_seq_rows(const M3Params& p, cudaStream_t st) {
+    const int warps = min(8, (p.hd + R - 1) / R);
+    const dim3 grid(p.nh, p.B, (p.hd + R * warps - 1) / (R * warps));
+    m3_ssd_seq_kernel<Tact, NI, R, PART><<<grid, warps * 32, 0, st>>>(p);
     if (grid.z > 1 && p.k_state) m3_seq_kstate_kernel<Tact><<<dim3(p.nh, p.B), 128, 0, st>>>(p);
 }
 template <typename Tact>
 static void launch_seq(const M3Params& p, int sms, cudaStream_t st) {
-    if (p.N <= 32) launch_seq_ni<Tact, 1>(p, sms, st);
-    else if (p.N <= 64) launch_seq_ni<Tact, 2>(p, sms, st);
-    else launch_seq_ni<Tact, 4>(p, sms, st);
+    const bool few = static_cast<long long>(p.B) * p.nh * ((p.hd + 7) / 8) < 8LL * sms, part = p.N % 32 != 0;
+#define MB200_SEQ(NI, R)                                               \
+    do {                                                               \
+        if (part) launch_seq_rows<Tact, NI, R, true>(p, st);           \
+        else launch_seq_rows<Tact, NI, R, false>(p, st);               \
+    } while (0)
+    if (few) {
+        if (p.N <= 32) MB200_SEQ(1, 2);
+        else if (p.N <= 64) MB200_SEQ(2, 2);
+        // (96 states in three pieces: 36 us for 24 at 1 x 64 steps x 4 heads)
+        else if (p.N < 128) launch_seq_rows<Tact, 4, 2, true>(p, st);
+        else launch_seq_rows<Tact, 4, 2, false>(p, st);
+    } else if (p.N <= 32) MB200_SEQ(1, 8);
+    else if (p.N <= 64) MB200_SEQ(2, 8);
+    else if (p.N <= 96) MB200_SEQ(3, 8);  // (8 x 64 steps x 32 heads, 96 states: 59 us for 93 in four pieces)
+    else MB200_SEQ(4, 8);
+#undef MB200_SEQ
 }
 
 }  // namespace mb200

@@ -286,3 +286,15 @@ def test_a_carried_window_is_as_exact_as_the_sequential_definition(cuda_dev, dt,
     # y: both are the rounding of the store; state: f32 sums in another order, a few 2^-24 of 128 terms a chunk
     assert err[0][0] <= 1.01 * err[1][0], err
     assert err[0][1] <= max(err[1][1], 2e-6), err
+
+
+@pytest.mark.parametrize("N", [8, 40, 96, 100])
+def test_an_infinite_input_stays_infinite_beside_the_states_that_are_not_there(cuda_dev, N):
+    """The lanes past d_state hold zeros; an infinite x must not make a NaN of them and carry it into y."""
+    i = synth.m3_ssd_inputs(1, 12, 1, 16, N, seed=N)
+    for k in ("K", "Q"):
+        i[k] = np.abs(i[k]) + np.float32(0.1)
+    i["Dh"], i["x"][0, 5, 3] = np.abs(i["Dh"]), np.inf
+    y, ssm, _, _ = run_gpu(i, "f32", cuda_dev, force_sequential=True)
+    assert np.isinf(y[0, 5:, 3]).all() and np.isfinite(np.delete(y, 3, axis=2)).all()
+    assert np.isinf(ssm[0, 0, 3]).all()
