@@ -584,19 +584,19 @@ static const BwdTable& bwd_table() {
     return table;
 }
 
-// Two-lane kernels (8 < d_state <= 16, save stride 32): [dtype][0][flags].
+// Two-lane kernels (8 < d_state <= 16, save stride 32): [dtype][flags].
 struct Bwd2Table {
-    BwdKernelFn fn[3][1][16];
-    size_t smem[3][1];
+    BwdKernelFn fn[3][16];
+    size_t smem[3];
 };
 
 static const Bwd2Table& bwd2_table() {
     static const Bwd2Table table = [] {
         Bwd2Table t;
         memset(&t, 0, sizeof(t));
-        bwd2_kernels_f32(t.fn[MAMBA_B200_F32], t.smem[MAMBA_B200_F32]);
-        bwd2_kernels_f16(t.fn[MAMBA_B200_F16], t.smem[MAMBA_B200_F16]);
-        bwd2_kernels_bf16(t.fn[MAMBA_B200_BF16], t.smem[MAMBA_B200_BF16]);
+        bwd2_kernels_f32(t.fn[MAMBA_B200_F32], &t.smem[MAMBA_B200_F32]);
+        bwd2_kernels_f16(t.fn[MAMBA_B200_F16], &t.smem[MAMBA_B200_F16]);
+        bwd2_kernels_bf16(t.fn[MAMBA_B200_BF16], &t.smem[MAMBA_B200_BF16]);
         return t;
     }();
     return table;
@@ -606,16 +606,15 @@ int m1_bwd_configure(Ctx* c) {
     MB200_CUDA_CHECK(c, bwd_wide_configure());
     const Bwd2Table& t2 = bwd2_table();
     for (int dt = 0; dt < 3; ++dt)
-        for (int si = 0; si < 1; ++si)
-            for (int f = 0; f < 16; ++f) {
-                MB200_CUDA_CHECK(c, cudaFuncSetAttribute(reinterpret_cast<const void*>(t2.fn[dt][si][f]),
-                                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                         static_cast<int>(t2.smem[dt][si])));
-                // many small CTAs per SM: ask for the largest shared-memory carve-out
-                MB200_CUDA_CHECK(c, cudaFuncSetAttribute(reinterpret_cast<const void*>(t2.fn[dt][si][f]),
-                                                         cudaFuncAttributePreferredSharedMemoryCarveout,
-                                                         cudaSharedmemCarveoutMaxShared));
-            }
+        for (int f = 0; f < 16; ++f) {
+            MB200_CUDA_CHECK(c, cudaFuncSetAttribute(reinterpret_cast<const void*>(t2.fn[dt][f]),
+                                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                     static_cast<int>(t2.smem[dt])));
+            // many small CTAs per SM: ask for the largest shared-memory carve-out
+            MB200_CUDA_CHECK(c, cudaFuncSetAttribute(reinterpret_cast<const void*>(t2.fn[dt][f]),
+                                                     cudaFuncAttributePreferredSharedMemoryCarveout,
+                                                     cudaSharedmemCarveoutMaxShared));
+        }
     const BwdTable& t = bwd_table();
     for (int dt = 0; dt < 3; ++dt)
         for (int v = 0; v < 3; ++v)
@@ -802,7 +801,7 @@ static int launch_bwd(Ctx* c, void* stream, const mamba_b200_sscan_bwd_args& a, 
             p.seg_dh = reinterpret_cast<float*>(ws + off_dh);
             p.seg_sum = reinterpret_cast<float*>(ws + off_sum);
             grid.z = segs - 1;
-            t2.fn[a.dtype][0][4 | flags2]<<<grid, 32, t2.smem[a.dtype][0], st>>>(p);
+            t2.fn[a.dtype][4 | flags2]<<<grid, 32, t2.smem[a.dtype], st>>>(p);
             MB200_CUDA_CHECK(c, cudaGetLastError());
             const long long n = static_cast<long long>(a.B) * a.D * a.N;
             sscan_bwd_carry_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, st>>>(p.seg_dh, p.seg_sum, a.a_neg, a.B, segs,
@@ -812,7 +811,7 @@ static int launch_bwd(Ctx* c, void* stream, const mamba_b200_sscan_bwd_args& a, 
         } else {
             p.seg_blocks = 0;
         }
-        t2.fn[a.dtype][0][flags2]<<<grid, 32, t2.smem[a.dtype][0], st>>>(p);
+        t2.fn[a.dtype][flags2]<<<grid, 32, t2.smem[a.dtype], st>>>(p);
     } else {
         t.fn[a.dtype][vi][flags]<<<grid, 32, t.smem[a.dtype][vi], st>>>(p);
     }

@@ -2,5 +2,5 @@
 #include "m1_bwd2_kernel.cuh"
 
 namespace mb200 {
-void bwd2_kernels_f32(BwdKernelFn (*fn)[16], size_t* smem) { fill_bwd2<float>(fn, smem); }
+void bwd2_kernels_f32(BwdKernelFn* fn, size_t* smem) { fill_bwd2<float>(fn, smem); }
 }  // namespace mb200

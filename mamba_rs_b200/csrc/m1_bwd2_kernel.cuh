@@ -465,14 +465,14 @@ static void fill_bwd2_flags(BwdKernelFn* fn, std::integer_sequence<int, F...>) {
     ((fn[F] = sscan_bwd2_kernel<Tact, 32, F>), ...);
 }
 template <typename Tact>
-static void fill_bwd2(BwdKernelFn (*fn)[16], size_t* smem) {
-    fill_bwd2_flags<Tact>(fn[0], std::make_integer_sequence<int, 16>{});
-    smem[0] = Bwd2Traits<Tact, 32>::SMEM;
+static void fill_bwd2(BwdKernelFn* fn, size_t* smem) {
+    fill_bwd2_flags<Tact>(fn, std::make_integer_sequence<int, 16>{});
+    *smem = Bwd2Traits<Tact, 32>::SMEM;
 }
 
-// [0][flags] (save stride 32); one translation unit per storage dtype
-void bwd2_kernels_f32(BwdKernelFn (*fn)[16], size_t* smem);
-void bwd2_kernels_f16(BwdKernelFn (*fn)[16], size_t* smem);
-void bwd2_kernels_bf16(BwdKernelFn (*fn)[16], size_t* smem);
+// [flags]; one translation unit per storage dtype
+void bwd2_kernels_f32(BwdKernelFn* fn, size_t* smem);
+void bwd2_kernels_f16(BwdKernelFn* fn, size_t* smem);
+void bwd2_kernels_bf16(BwdKernelFn* fn, size_t* smem);
 
 }  // namespace mb200
