@@ -122,3 +122,51 @@ def test_mamba3_tensor_core_kernels_replay_bit_identically_from_a_graph(cuda_dev
         for k, v in eager.items():
             np.testing.assert_array_equal(replayed[k], v, err_msg=k)
     mb.ffi.default_handle(0).check_status()
+
+def test_kernels_whose_blocks_wait_on_one_another_replay_bit_identically_from_a_graph(cuda_dev):
+    """The cooperative and clustered launches in a caller's graph: the whole-model decode step, the Mamba-3 forward
+    and backward over a cluster (4 heads), and the backward's pairs cut between CTAs (192 heads)."""
+    import torch
+
+    import mamba_rs_b200 as mb
+    bf = torch.bfloat16
+    g = torch.Generator(device=cuda_dev).manual_seed(6)
+    rn = lambda *s: torch.randn(*s, device=cuda_dev, generator=g)  # noqa: E731
+    bb = mb.GpuMambaBackbone(mb.MambaWeights(mb.MambaConfig(d_model=128, n_layers=2), cuda_dev).init_random(3), 5)
+    x, out, calls = rn(5, 128), {}, []
+    for B, T, nh in ((1, 1100, 4), (6, 300, 32)):
+        step = torch.nn.functional.softplus(rn(B, T, nh) - 3)
+        args = [rn(B, T, nh * 64).to(bf), (0.3 * rn(B, T, nh, 128)).to(bf), (0.3 * rn(B, T, nh, 128)).to(bf), step, torch.sigmoid(rn(B, T, nh)),
+                -2 * step, torch.ones(nh, device=cuda_dev)]
+        size = mb.ffi.lib().mamba_b200_m3_ssd_bwd_workspace_bytes_for(mb.dtype_code(bf), B, T, nh, 64, 128)
+        calls.append((args, torch.empty_like(args[0]), rn(B, T, nh * 64).to(bf), torch.zeros(nh, device=cuda_dev),
+                      torch.empty(size, dtype=torch.uint8, device=cuda_dev)))
+
+    def work():
+        bb.reset()
+        for i in range(2):
+            out["step%d" % i] = bb.step(x.clone())
+        out["ssm"], out["conv"] = bb.ssm, bb.conv
+        for n, (args, y, dy, dD, ws) in enumerate(calls):
+            dD.zero_()
+            out["y%d" % n] = mb.m3_ssd_fwd(*args, y=y)
+            out.update({"%s%d" % (k, n): v for k, v in mb.m3_ssd_bwd(*args, dy, dD=dD, workspace=ws).items()})
+
+    def snapshot():
+        torch.cuda.synchronize()
+        return {k: v.float().cpu().numpy().copy() for k, v in out.items()}
+    work()
+    eager = snapshot()
+    side = torch.cuda.Stream(device=cuda_dev)
+    side.wait_stream(torch.cuda.current_stream(cuda_dev))
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        work()
+    for _ in range(3):
+        for v in out.values():
+            v.zero_()
+        graph.replay()
+        replayed = snapshot()
+        for k, v in eager.items():
+            np.testing.assert_array_equal(replayed[k], v, err_msg=k)
+    mb.ffi.default_handle(0).check_status()

@@ -159,6 +159,7 @@ def test_greedy_decode_from_a_captured_graph_equals_eager_decode(cuda_dev):
     import torch
 
     import mamba_rs_b200 as mb
+    from mamba_rs_b200 import model
     cfg = mb.MambaConfig(d_model=128, n_layers=3)
     V, B, T, n = 997, 4, 60, 12
     w = mb.MambaWeights(cfg, cuda_dev, dtype=torch.bfloat16, vocab=V).init_random(11)
@@ -168,7 +169,10 @@ def test_greedy_decode_from_a_captured_graph_equals_eager_decode(cuda_dev):
     for use_graph in (False, True):
         lm = mb.GpuMambaLM(w, B)
         lm.prefill(ids)
+        lm._dec = model._DecodePlan(lm.backbone, B, lm)
+        lm._dec.ok = lm.backbone._plan(B).ok = False  # (the one-launch kernel would take both)
         outs.append(lm.generate_greedy(n, use_graph=use_graph).cpu().numpy())
+        assert (lm._graph is not None) == use_graph
     np.testing.assert_array_equal(outs[0], outs[1])
     assert outs[0].min() >= 0 and outs[0].max() < V
 
@@ -455,3 +459,22 @@ def test_a_workspace_is_not_handed_on_while_another_stream_uses_it(cuda_dev):
         side.synchronize()
         assert torch.equal(got, want)
         del taken
+
+def test_one_launch_steps_from_the_start_match_the_cpu_backbone(cuda_dev):
+    """Every step of a sequence by the whole-model decode launch, against the CPU oracle's token loop."""
+    import torch
+
+    import mamba_rs_b200 as mb
+    ocfg, flat, lv, _, w = reference_weights(cuda_dev)
+    B, T = 3, 40
+    inp = np.random.default_rng(9).standard_normal((B, T, 128)).astype(np.float32)
+    refs = [oracle.m1_prefill(ocfg, flat, inp[b]) for b in range(B)]
+    temporal = (inp.astype(np.float64) @ lv["input_proj_w"].astype(np.float64) + lv["input_proj_b"]).astype(np.float32)
+    bb = mb.GpuMambaBackbone(w, B)
+    assert bb._plan(B).ok
+    outs = [bb.step(torch.from_numpy(np.ascontiguousarray(temporal[:, t])).to(cuda_dev)) for t in range(T)]
+    got = torch.stack(outs, 1)
+    assert rel_err(host(got), np.stack([r["out"] for r in refs])) <= 1e-4
+    assert rel_err(host(bb.ssm), np.stack([r["ssm_state"] for r in refs], axis=1)) <= 1e-4
+    np.testing.assert_allclose(host(bb.conv), np.stack([r["conv_state"] for r in refs], axis=1), rtol=0, atol=2e-5)
+    mb.ffi.default_handle(0).check_status()
