@@ -582,14 +582,16 @@ class GpuMambaBackbone:
         B, dm = temporal.shape
         if dm != c.d_model or temporal.device != w.master.device:
             raise TypeError(f"temporal is [B, {c.d_model}] on {w.master.device}, not {list(temporal.shape)} on {temporal.device}")
+        if B > self.batch:
+            raise ValueError(f"{B} sequences, the engine's state holds {self.batch}")
         plan = self._plan(B)
-        if (plan.ok and B <= self.batch and temporal.is_cuda and temporal.dtype == torch.float32
+        if (plan.ok and temporal.is_cuda and temporal.dtype == torch.float32
                 and temporal.is_contiguous() and temporal.data_ptr() % 16 == 0):
             out = torch.empty(B, dm, device=temporal.device, dtype=w.dtype)
             plan.args.residual, plan.args.out = temporal.data_ptr(), out.data_ptr()
             plan.launch()
             return out
-        if (B <= self.batch and temporal.is_cuda and temporal.dtype == torch.float32 and temporal.is_contiguous()
+        if (temporal.is_cuda and temporal.dtype == torch.float32 and temporal.is_contiguous()
                 and not torch.cuda.is_current_stream_capturing()):
             branch = plan.replay.run(temporal.data_ptr(), lambda: self._step_layers(temporal))
         else:

@@ -21,6 +21,12 @@ def test_a_step_refuses_rows_of_another_width(width):
         bb.step(torch.zeros(2, width))
 
 
+def test_a_step_refuses_more_sequences_than_the_state_holds():
+    bb = mb.GpuMambaBackbone(weights(), 2)
+    with pytest.raises(ValueError, match="holds 2"):
+        bb.step(torch.zeros(3, 16))
+
+
 def test_calls_refuse_rows_on_another_device():
     bb = mb.GpuMambaBackbone(weights(), 2)
     with pytest.raises(TypeError, match="device|meta"):
