@@ -11,9 +11,10 @@
 //
 // ops 0 and 1: a CTA of 128 threads has 32 rows x 64 columns, a 4 x 4 block per thread, and a part of K; the
 // parts of a tile form a cluster and add their blocks through distributed shared memory, in rank order, so
-// the result does not depend on scheduling.  Tiles of 32 K steps come by cp.async, three stages.  Every 256
-// steps the running sums are added to a second set: in one chain the product over a vocabulary (32 x 50280 x
-// 768) was 1.4e-6 from the exact one, with two 3.0e-7, the library's 9.3e-7.
+// the result does not depend on scheduling.  Tiles of 32 K steps come by cp.async, three stages.  Where a part
+// has more than 256 steps the running sums are added to a second set every 256: in one chain the product over a
+// vocabulary (32 x 50280 x 768) was 1.4e-6 from the exact one, with two 3.1e-7, the library's 9.3e-7 (150 us in
+// one chain, 171 in two; transposed 174 and 156).
 // op 2: a CTA of 256 threads has 64 x 64 of C, requested before the products so that its read, which is
 // what the call costs, overlaps them.
 #include <string.h>
@@ -45,7 +46,7 @@ __device__ __forceinline__ void copy4(float* dst, const float* src, int have) { 
     }
 }
 
-template <int OP, bool VEC>
+template <int OP, bool VEC, bool LONG>  // LONG: a part of K has more than 256 steps
 __global__ void __launch_bounds__(128) rows_kernel(const Params p) {
     constexpr int LB = OP == 0 ? BN : LA, WB = OP == 0 ? BK * BN : BN * LA, WA = BM * LA;
     extern __shared__ __align__(16) float sm[];  // [STAGES][A | B]
@@ -90,36 +91,39 @@ __global__ void __launch_bounds__(128) rows_kernel(const Params p) {
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = sum[i][j] = 0.0f;
-    for (int s = 0; s < steps; ++s) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
-        __syncthreads();
-        fetch(s + STAGES - 1);
-        const float* A = sm + (s % STAGES) * (WA + WB);
-        const float* B = A + WA;
+        for (int j = 0; j < 4; ++j) acc[i][j] = sum[i][j] = 0.0f;  // (sum: LONG)
+    for (int s = 0; s < steps;) {
+        const int top = LONG ? min(steps, s + 8) : steps;
+        for (; s < top; ++s) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+            __syncthreads();
+            fetch(s + STAGES - 1);
+            const float* A = sm + (s % STAGES) * (WA + WB);
+            const float* B = A + WA;
 #pragma unroll
-        for (int k = 0; k < BK; k += 4) {
-            float4 a[4], b[4];
+            for (int k = 0; k < BK; k += 4) {
+                float4 a[4], b[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float4*>(A + (ty + 8 * i) * LA + k);
+                for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float4*>(A + (ty + 8 * i) * LA + k);
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
-                b[j] = *reinterpret_cast<const float4*>(OP == 0 ? B + (k + j) * LB + 4 * tx : B + (tx + 16 * j) * LB + k);
+                for (int j = 0; j < 4; ++j)
+                    b[j] = *reinterpret_cast<const float4*>(OP == 0 ? B + (k + j) * LB + 4 * tx : B + (tx + 16 * j) * LB + k);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float av[4] = {a[i].x, a[i].y, a[i].z, a[i].w};
+                for (int i = 0; i < 4; ++i) {
+                    const float av[4] = {a[i].x, a[i].y, a[i].z, a[i].w};
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const float bv[4] = {b[j].x, b[j].y, b[j].z, b[j].w};
+                    for (int j = 0; j < 4; ++j) {
+                        const float bv[4] = {b[j].x, b[j].y, b[j].z, b[j].w};
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        if (OP == 0) acc[i][q] = fmaf(av[j], bv[q], acc[i][q]);
-                        else acc[i][j] = fmaf(av[q], bv[q], acc[i][j]);
+                        for (int q = 0; q < 4; ++q) {
+                            if (OP == 0) acc[i][q] = fmaf(av[j], bv[q], acc[i][q]);
+                            else acc[i][j] = fmaf(av[q], bv[q], acc[i][j]);
+                        }
                     }
                 }
             }
         }
-        if ((s & 7) == 7) {
+        if (LONG) {
 #pragma unroll
             for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -134,7 +138,7 @@ __global__ void __launch_bounds__(128) rows_kernel(const Params p) {
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) sm[(ty + 8 * i) * BN + (OP == 0 ? 4 * tx + j : tx + 16 * j)] = sum[i][j] + acc[i][j];
+        for (int j = 0; j < 4; ++j) sm[(ty + 8 * i) * BN + (OP == 0 ? 4 * tx + j : tx + 16 * j)] = LONG ? sum[i][j] : acc[i][j];
     if (parts > 1) cluster_sync();
     else __syncthreads();
     // this rank's rows of the sum
@@ -153,12 +157,11 @@ __global__ void __launch_bounds__(128) rows_kernel(const Params p) {
     if (parts > 1) cluster_sync();  // nobody reads this CTA's shared memory any more
 }
 
-template <bool VEC>
+template <bool VEC, bool TALL>  // TALL: grid.x counts the tiles of rows
 __global__ void __launch_bounds__(256) grad_kernel(const Params p) {
     constexpr int BC = 64;
     __shared__ __align__(16) float A[BK][BC], B[BK][BC];
-    const int tid = threadIdx.x, nx = (p.N + BC - 1) / BC, tx = tid & 15, ty = tid >> 4;
-    const int m0 = static_cast<int>(blockIdx.x / nx) * BC, n0 = static_cast<int>(blockIdx.x % nx) * BC;
+    const int tid = threadIdx.x, m0 = (TALL ? blockIdx.x : blockIdx.y) * BC, n0 = (TALL ? blockIdx.y : blockIdx.x) * BC, tx = tid & 15, ty = tid >> 4;
     float acc[4][4];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
@@ -236,11 +239,15 @@ extern "C" MAMBA_B200_API int mamba_b200_sgemm_rows(void* handle, void* stream, 
         p.kper = 0;
         // a row's groups of four are whole where both sides are multiples of four
         const bool vec = al(a, lda) && al(b, ldb) && al(out, ldc) && M % 4 == 0 && N % 4 == 0;
-        const long long tiles = ((N + 63LL) / 64) * ((M + 63LL) / 64);  // one row of them: a vocabulary may have more than 65535
-        if (tiles > 0x7fffffff) return fail(c, MAMBA_B200_ERR_SHAPE, "sgemm_rows: a gradient of %d x %d", M, N);
-        const dim3 grid(static_cast<unsigned>(tiles));
-        if (vec) sg::grad_kernel<true><<<grid, 256, 0, st>>>(p);
-        else sg::grad_kernel<false><<<grid, 256, 0, st>>>(p);
+        // tiles of columns side by side; of rows where there are too many for the other dimension (a vocabulary)
+        dim3 grid((N + 63) / 64, (M + 63) / 64);
+        const bool tall = grid.y > 65535;
+        if (tall) grid = dim3(grid.y, grid.x);
+        if (grid.y > 65535) return fail(c, MAMBA_B200_ERR_SHAPE, "sgemm_rows: a gradient of %d x %d", M, N);
+        if (vec && !tall) sg::grad_kernel<true, false><<<grid, 256, 0, st>>>(p);
+        else if (vec) sg::grad_kernel<true, true><<<grid, 256, 0, st>>>(p);
+        else if (!tall) sg::grad_kernel<false, false><<<grid, 256, 0, st>>>(p);
+        else sg::grad_kernel<false, true><<<grid, 256, 0, st>>>(p);
         MB200_CUDA_CHECK(c, cudaGetLastError());
         return MAMBA_B200_OK;
     }
@@ -252,11 +259,13 @@ extern "C" MAMBA_B200_API int mamba_b200_sgemm_rows(void* handle, void* stream, 
     while (parts < 8 && static_cast<long long>(tiles) * rows * parts < 2 * 148 && K >= parts * 4 * sg::BK) parts *= 2;
     p.kper = ((K + parts - 1) / parts + sg::BK - 1) / sg::BK * sg::BK;
     const bool vec = al(a, lda) && al(b, ldb) && K % 4 == 0 && (op == 1 || N % 4 == 0);
-    const void* fns[4] = {reinterpret_cast<const void*>(sg::rows_kernel<0, false>), reinterpret_cast<const void*>(sg::rows_kernel<0, true>),
-                          reinterpret_cast<const void*>(sg::rows_kernel<1, false>), reinterpret_cast<const void*>(sg::rows_kernel<1, true>)};
+    const bool lng = p.kper > 8 * sg::BK;
+#define MB200_ROWS(OP, VEC) {reinterpret_cast<const void*>(sg::rows_kernel<OP, VEC, false>), reinterpret_cast<const void*>(sg::rows_kernel<OP, VEC, true>)}
+    const void* fns[4][2] = {MB200_ROWS(0, false), MB200_ROWS(0, true), MB200_ROWS(1, false), MB200_ROWS(1, true)};
+#undef MB200_ROWS
     const size_t smem = sizeof(float) * sg::STAGES * (sg::BM * sg::LA + (op == 0 ? sg::BK * sg::BN : sg::BN * sg::LA));
     static_assert(sizeof(float) * sg::STAGES * (sg::BM * sg::LA + sg::BN * sg::LA) <= 48 * 1024, "within what needs no opt-in");
     void* args[1] = {&p};
-    MB200_CUDA_CHECK(c, launch_cluster(fns[op * 2 + (vec ? 1 : 0)], dim3(tiles * parts, rows), dim3(128), smem, st, parts, args));
+    MB200_CUDA_CHECK(c, launch_cluster(fns[op * 2 + (vec ? 1 : 0)][lng ? 1 : 0], dim3(tiles * parts, rows), dim3(128), smem, st, parts, args));
     return MAMBA_B200_OK;
 }

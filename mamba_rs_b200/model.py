@@ -236,7 +236,7 @@ def _product(go, op, a, b, out):
     """out = a b (op 0) or a b^T (op 1), inside go.begin().  In f32 with few output tiles and a long
     contraction the rows kernel has the parts of K that the library's tiles leave to one SM (us, with the
     library's: 32 rows, 768 x 3072 8.9 and 14.6, 1536 x 768 8.5 and 18.2, 512 x 512 5.1 and 8.5; a vocabulary of
-    50280 to 768 168 and 165, transposed 159 and 242).  The last size it takes, 96 tiles of 32 x 64, is 64 x 768 x
+    50280 to 768 171 and 165, transposed 156 and 240).  The last size it takes, 96 tiles of 32 x 64, is 64 x 768 x
     3072: 13.9 and 15.8; 96 rows, 144 tiles, are 20.0 and 15.9."""
     M, K = a.shape
     N = out.shape[1]
@@ -895,9 +895,9 @@ class MambaLMTrainer:
 
     def _accumulate(self, g, a, b):
         """g (f32) += a.T @ b, the product accumulated into g by the GEMM itself."""
-        # up to 32 rows are one pass over the tiles of the rows kernel (us, with the library's: 32 rows, 768 x 3072 6.7
-        # and 8.9, 1536 x 80 3.0 and 4.0, 50280 x 768 89 and 101, but 8 rows there 86 and 81); 33 are two (10.7 and
-        # 10.1, 4.2 and 4.3, 141 and 105)
+        # up to 32 rows are one pass over the tiles of the rows kernel (us, with the library's: 32 rows, 768 x 3072 6.2
+        # and 8.9, 1536 x 80 2.9 and 4.0, 50280 x 768 82 and 101); 33 are two (10.0 and
+        # 9.9, 4.2 and 4.3, 131 and 105)
         if a.dtype == torch.float32 and a.shape[0] <= 32:
             go = self._acts["plan"].run_on
             with go.begin():
