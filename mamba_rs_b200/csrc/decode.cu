@@ -154,10 +154,9 @@ struct Step {
     const int tid, lane, warp, cta, ncta;
     bool alive = true;
     unsigned base_tag = 0;
-    int polls = kMaxPolls;
     float* pair;     // sums that two warps of a row exchange
     uint64_t* bars;  // landed: W_in, W_out, W_x, small operands; then free: the same
-    volatile int* dead;
+    volatile int* dead;  // [1]: polls a wait may take (in shared memory, read after a miss: in a register it cost 3 %)
 
     __device__ Step(const Params& p_, unsigned char* sm_, float* pair_, uint64_t* bars_, int* dead_)
         : p(p_), sm(sm_), tid(threadIdx.x), lane(threadIdx.x & 31), warp(threadIdx.x >> 5), cta(blockIdx.x),
@@ -201,8 +200,9 @@ struct Step {
 #pragma unroll
             for (int i = 0; i < N; ++i) miss |= (v[i].y ^ tag) | (v[i].w ^ tag);
             if (!__any_sync(0xffffffffu, miss != 0)) break;
+            const int polls = dead[1];
             if (lane == 0)
-                while (alive && (v[0].y != tag || v[0].w != tag) && ++it < polls) v[0] = get2(src + min(j, last));
+                while ((v[0].y != tag || v[0].w != tag) && ++it < polls) v[0] = get2(src + min(j, last));
             it = __shfl_sync(0xffffffffu, it, 0) + 1;
             if (it >= polls || !alive) {
                 alive = false;
@@ -1002,7 +1002,6 @@ struct Step {
     __device__ void run() {
         const volatile unsigned* ctl = p.ctl;
         base_tag = ctl[0];
-        if (ctl[2] > 0 && ctl[2] < static_cast<unsigned>(kMaxPolls)) polls = static_cast<int>(ctl[2]);
         float own = 0.0f;
         enter(own);
         const int n = channels(), per = p.ncg * 4;
@@ -1057,15 +1056,17 @@ template <typename Tact>
 __global__ void __launch_bounds__(kThreads + 32, 1) decode_step_kernel(const __grid_constant__ Params p) {
     extern __shared__ __align__(128) unsigned char sm[];
     __shared__ float pair[kWarps];
-    __shared__ int dead;
+    __shared__ int dead[2];
     __shared__ __align__(8) uint64_t bars[8];
     if (threadIdx.x == 0) {
         for (int i = 0; i < 8; ++i) mbar_init(&bars[i], 1);
-        dead = 0;
+        dead[0] = 0;
+        const unsigned limit = *reinterpret_cast<const volatile unsigned*>(p.ctl + 2);
+        dead[1] = limit > 0 && limit < static_cast<unsigned>(kMaxPolls) ? static_cast<int>(limit) : kMaxPolls;
         fence_barrier_init();
     }
     __syncthreads();
-    Step<Tact> s(p, sm, pair, bars, &dead);
+    Step<Tact> s(p, sm, pair, bars, dead);
     if (threadIdx.x >= kThreads) s.feed();
     else s.run();
 }
