@@ -14,11 +14,15 @@ constexpr int kMaxSegments = 64;
 // time.  In one piece a step takes 0.1155 us with one CTA per SM and 0.137 with two; both passes of a cut take
 // kCut[2 x] with x CTAs per SM on average (d_state 16, bf16; f32 takes 1.08 times as long throughout), a piece
 // costs its steps and 16 more for its pipeline to fill, and the call 8 us with two more launches.  Beyond 1.15 CTAs
-// per SM one piece is as fast, and under 192 steps (1 x 128 x 2560 whole 17.6, in four 18.9).  Fitted to 300 measured shapes of 64 to 4096 steps: half of the estimates are within 5 %, and
-// the counts chosen take 0.8 % longer than the best that was measured on average, 9 % at most.  Whole and as cut
-// here, bf16 and f32 in us: 1 x 1021 x 1536 118 and 31, 129 and 32; 2 x 192 x 1536 25 and 20, 27 and 19; 4 x 512 x
-// 1536 61 and 51, 66 and 53; 6 x 2048 x 1344 236 and 208, 259 and 213.
+// per SM one piece is as fast, and under 192 steps (1 x 128 x 2560 whole 17.6, in four 18.9).  Fitted to 300
+// measured shapes of 64 to 4096 steps: half of the estimates are within 5 %, and the counts chosen take 0.8 % longer
+// than the best that was measured on average, 9 % at most.  Whole and as cut here, bf16 and f32 in us: 1 x 1021 x
+// 1536 118 and 31, 129 and 32; 2 x 192 x 1536 25 and 20, 27 and 19; 4 x 512 x 1536 61 and 51, 66 and 53.
+// From 1536 steps on the pieces are long whatever their number, and their number goes by what was measured: eight
+// from 0.7 CTAs per SM on (0.85 x 2048 steps 207 us, 16: 209; 1.1: 253, 261), else 16 (0.65: 168, eight 171; 0.32 x
+// 4096: 174, eight 183), or as many as fill the chip (0.03 x 2048: 24 in 64, 35 in 16).
 constexpr int kFwdMaxPerSm = 9, kFwdMaxCtas = 170;
+constexpr int kFwdMaxPieces = 12 * 148;  // of all CTAs together, by either rule
 static long long fwd_ctas(int B, int D, int N) {  // of four consumer warps, one a scheduler
     int lpc = 1;
     while (8 * lpc < N) lpc *= 2;
@@ -31,6 +35,10 @@ static int fwd_segments(int B, int T, int D, int N) {
     const long long ctas = fwd_ctas(B, D, N);
     if (ctas > kFwdMaxCtas || T < 192) return 1;
     const int blocks = (T + 31) / 32;
+    if (T >= 1536) {
+        const double w = ctas / 148.0;
+        return w >= 0.7 ? 8 : std::min({std::max(16, static_cast<int>(2.6 / w) + 1), blocks, kMaxSegments});
+    }
     int best = 1;
     double cost = 3.5 + T * (ctas <= 148 ? 0.1155 : 0.137);
     for (int s = 2; s <= kMaxSegments && s <= blocks && ctas * s <= kFwdMaxPerSm * 148; ++s) {
@@ -261,7 +269,7 @@ extern "C" MAMBA_B200_API long long mamba_b200_sscan_fwd_workspace_bytes(int B, 
     for (int b = 1; b <= B; ++b) {
         const long long ctas = fwd_ctas(b, D, N);
         if (ctas > kFwdMaxCtas) b = B;
-        const long long segs = ctas > kFwdMaxCtas ? 1 : std::min<long long>({kFwdMaxPerSm * 148 / ctas, (T + 31) / 32, kMaxSegments});
+        const long long segs = ctas > kFwdMaxCtas ? 1 : std::min<long long>({kFwdMaxPieces / ctas, (T + 31) / 32, kMaxSegments});
         most = std::max(most, fwd_ws_bytes(b, D, N, static_cast<int>(segs), &o1, &o2, &o3));
     }
     return static_cast<long long>(most);
