@@ -1,17 +1,17 @@
 // Mamba-1 fused selective-scan forward for sm_100a.
 // Host side of the fused forward: argument validation, TMA descriptors, variant
 // selection, the time-segment plan and launch.  The kernels live in
-// m1_fwd_kernel.cuh.
+// m1_fwd_kernel.cuh (all sizes) and m1_fwd16_kernel.cuh (warp roles, d_state 9 .. 16).
 #include <algorithm>
 
-#include "m1_fwd_kernel.cuh"
+#include "m1_fwd16_kernel.cuh"
 
 namespace mb200 {
 
 constexpr int kMaxSegments = 64;
 
-// Time segments of a launch that was lent a workspace (see launch_fwd): the count with the least estimated
-// time.  In one piece a step takes 0.1155 us with one CTA per SM and 0.137 with two; both passes of a cut take
+// Time segments of sscan_fwd_kernel when it was lent a workspace (see launch_fwd): the count with the least estimated
+// time, which it returns in *us.  In one piece a step takes 0.1155 us with one CTA per SM and 0.137 with two; both passes of a cut take
 // kCut[2 x] with x CTAs per SM on average (d_state 16, bf16; f32 takes 1.08 times as long throughout), a piece
 // costs its steps and 16 more for its pipeline to fill, and the call 8 us with two more launches.  Beyond 1.15 CTAs
 // per SM one piece is as fast, and under 192 steps (1 x 128 x 2560 whole 17.6, in four 18.9).  Fitted to 300
@@ -29,30 +29,53 @@ static long long fwd_ctas(int B, int D, int N) {  // of four consumer warps, one
     const int cw = lpc >= 16 ? 8 : 4, dt = cw * (32 / lpc);
     return static_cast<long long>(B) * ((D + dt - 1) / dt) * (cw / 4);
 }
-static int fwd_segments(int B, int T, int D, int N) {
+static int fwd_segments(int B, int T, int D, int N, double* us) {
     static const double kCut[2 * kFwdMaxPerSm + 2] = {0.175, 0.180, 0.191, 0.221, 0.239, 0.275, 0.312, 0.395, 0.429, 0.460,
                                                       0.508, 0.536, 0.568, 0.619, 0.669, 0.712, 0.753, 0.806, 0.860, 0.860};
     const long long ctas = fwd_ctas(B, D, N);
+    // whole: three CTAs share an SM, 0.165 us a step together
+    const long long rounds = ctas / (3 * 148), rest = ctas % (3 * 148);
+    *us = rounds * (3.2 + 0.165 * T) + (rest ? 3.2 + T * (rest <= 148 ? 0.1155 : rest <= 296 ? 0.137 : 0.165) : 0.0);
     if (ctas > kFwdMaxCtas || T < 192) return 1;
     const int blocks = (T + 31) / 32;
+    auto cut = [&](int s) {
+        const int per = (blocks + s - 1) / s;
+        const double x = std::min(2.0 * ctas * s / 148, 2.0 * kFwdMaxPerSm), f = x - static_cast<int>(x);
+        const double* at = kCut + static_cast<int>(x);
+        return 8 + (32 * per + 16) * (at[0] + f * (at[1] - at[0]));
+    };
     if (T >= 1536) {
         const double w = ctas / 148.0;
-        return w >= 0.7 ? 8 : std::min({std::max(16, static_cast<int>(2.6 / w) + 1), blocks, kMaxSegments});
+        const int s = w >= 0.7 ? 8 : std::min({std::max(16, static_cast<int>(2.6 / w) + 1), blocks, kMaxSegments});
+        *us = cut(s);
+        return s;
     }
     int best = 1;
-    double cost = 3.5 + T * (ctas <= 148 ? 0.1155 : 0.137);
-    for (int s = 2; s <= kMaxSegments && s <= blocks && ctas * s <= kFwdMaxPerSm * 148; ++s) {
-        const int per = (blocks + s - 1) / s;
-        const double x = 2.0 * ctas * s / 148, f = x - static_cast<int>(x);
-        const double* at = kCut + static_cast<int>(x);
-        const double c = 8 + (32 * per + 16) * (at[0] + f * (at[1] - at[0]));
-        if (c < cost) {
-            cost = c;
+    for (int s = 2; s <= kMaxSegments && s <= blocks && ctas * s <= kFwdMaxPerSm * 148; ++s)
+        if (cut(s) < *us) {
+            *us = cut(s);
             best = s;
         }
-    }
     return best;
 }
+
+// The kernel by warp roles: how a call is laid out and what that takes, in us.  One CTA has an SM to itself (three at
+// two consumer warps).  Whole: w0 + w1 a step and round of CTAs; cut, where all pieces run side by side: c0 + c1 a step
+// of a piece, both passes and the carry.  Fitted to 200 shapes of 8 to 5600 steps (as CUDA graphs): half of the
+// estimates are within 5 % (whole) and 8 % (cut).  16-bit storage; f32 takes 1.05 times as long.
+struct Fwd16Kind {
+    int ns, workers, helpers, stages;
+    double w0, w1, c0, c1;
+};
+static const Fwd16Kind kFwd16Kinds[] = {{4, 2, 2, 3, 3.7, 0.0623, 8.6, 0.1022},
+                                        {4, 4, 4, 4, 3.5, 0.0712, 8.7, 0.1175},
+                                        {4, 6, 4, 4, 4.3, 0.0888, 10.0, 0.1501},
+                                        {4, 8, 4, 4, 4.0, 0.1068, 9.5, 0.1813},
+                                        {8, 6, 4, 4, 5.4, 0.1527, 13.1, 0.2608}};
+struct Fwd16Plan {
+    const Fwd16Kind* kind = nullptr;  // null: sscan_fwd_kernel
+    int segs = 1;
+};
 
 struct FwdTable {
     FwdVariant v[3][kMaxFwdVariants];
@@ -72,7 +95,27 @@ static const FwdTable& fwd_table() {
     return table;
 }
 
+// Built once, like the other table.
+struct Fwd16Tables {
+    Fwd16Table t[3];
+};
+static const Fwd16Tables& fwd16_tables() {
+    static const Fwd16Tables tables = [] {
+        Fwd16Tables t;
+        fwd16_f32(&t.t[MAMBA_B200_F32]);
+        fwd16_f16(&t.t[MAMBA_B200_F16]);
+        fwd16_bf16(&t.t[MAMBA_B200_BF16]);
+        return t;
+    }();
+    return tables;
+}
+
 int m1_fwd_configure(Ctx* c) {
+    for (int dt = 0; dt < 3; ++dt)
+        for (int i = 0; i < 2; ++i)
+            for (int f = 0; f < 6; ++f)
+                MB200_CUDA_CHECK(c, cudaFuncSetAttribute(reinterpret_cast<const void*>(fwd16_tables().t[dt].fn[i][f]),
+                                                         cudaFuncAttributeMaxDynamicSharedMemorySize, kF16MaxSmem));
     const FwdTable& t = fwd_table();
     for (int dt = 0; dt < 3; ++dt)
         for (int i = 0; i < t.n[dt]; ++i)
@@ -132,9 +175,121 @@ static size_t fwd_ws_bytes(int B, int D, int N, int segs, size_t* o_sum, size_t*
     return off;
 }
 
+// The layout with the least estimate, if that is at most 0.95 (cut: 0.9) of what sscan_fwd_kernel is estimated to take.
+// Against it, on the 200 shapes: 12 % less time on average, 4 % more at most (1 x 471 x 5024 in f32), 1 % more than the
+// best layout of either kernel.  8 x 2048 x 1536 with general rates 284 -> 196 us, 2 x 8192 x 5120 with progressions 762
+// -> 645, 16 x 2048 x 1536 367 -> 342 and 303 -> 287, 1 x 1021 x 1536 39 -> 34.  Under 24 steps the shorter prologue of
+// the other kernel wins (12 x 9 x 144 4.5 us, here 5.8), and past three rounds of CTAs its three CTAs an SM do (19 x 33 x
+// 5360 32 us, here 59).
+static Fwd16Plan fwd16_plan(const Fwd16Table& t, bool f32, int B, int T, int D, int N, double us, long long workspace_bytes) {
+    Fwd16Plan best;
+    if (T < 24) return best;
+    us *= 0.95;
+    for (const Fwd16Kind& k : kFwd16Kinds) {
+        const int steps = t.steps[k.ns == 8], chunks = (T + steps - 1) / steps, dt = 4 * k.ns * k.workers;
+        const long long ctas = static_cast<long long>(B) * ((D + dt - 1) / dt);
+        const double scale = f32 ? 1.05 : 1.0;
+        double c = scale * ((ctas + 147) / 148) * (k.w0 + k.w1 * T);
+        if (k.workers == 2 && ctas > 148) c = scale * ((ctas + 443) / 444) * (4.5 + 0.0931 * T);
+        if (c < us && ctas <= 3 * 148) {
+            us = c;
+            best = {&k, 1};
+        }
+        if (T < 192) continue;
+        for (int s = 2; ctas * s <= 148 && s <= 32; ++s) {
+            const int per = (chunks + s - 1) / s, segs = (chunks + per - 1) / per;
+            size_t o1, o2, o3;
+            if (segs != s || per * steps < 32 || fwd_ws_bytes(B, D, N, s, &o1, &o2, &o3) > static_cast<size_t>(workspace_bytes)) continue;
+            c = scale * (k.c0 + k.c1 * per * steps) * (0.95 / 0.9);
+            if (c < us) {
+                us = c;
+                best = {&k, s};
+            }
+        }
+    }
+    return best;
+}
+
 static bool overlaps(const void* a, size_t na, const void* b, size_t nb) {
     const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
     return a && b && x < y + nb && y < x + na;
+}
+
+// The caller's workspace, divided for `segs` time segments.
+struct SegmentBuffers {
+    float *states, *sums, *ssm, *conv;
+};
+static SegmentBuffers segment_buffers(const mamba_b200_sscan_fwd_args& a, int segs) {
+    size_t o_sum, o_h0, o_c0;
+    fwd_ws_bytes(a.B, a.D, a.N, segs, &o_sum, &o_h0, &o_c0);
+    unsigned char* ws = static_cast<unsigned char*>(a.workspace);
+    return {reinterpret_cast<float*>(ws), reinterpret_cast<float*>(ws + o_sum), reinterpret_cast<float*>(ws + o_h0),
+            reinterpret_cast<float*>(ws + o_c0)};
+}
+static void launch_seg_carry(cudaStream_t stream, const mamba_b200_sscan_fwd_args& a, const SegmentBuffers& w, int segs) {
+    const long long n = static_cast<long long>(a.B) * a.D * a.N;
+    sscan_seg_carry_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, stream>>>(w.states, w.sums, a.a_neg, a.B, segs, a.D,
+                                                                                      a.N);
+}
+
+// The call by warp roles; `p` holds what both kernels need, its tensor maps are made again for this one's tiles.
+static int launch_fwd16(Ctx* c, cudaStream_t stream, const mamba_b200_sscan_fwd_args& a, const FwdParams& p, const Fwd16Table& t,
+                        const Fwd16Plan& plan) {
+    const Fwd16Kind& k = *plan.kind;
+    const int i = k.ns == 8, steps = t.steps[i], dt = 4 * k.ns * k.workers;
+    Fwd16Params q;
+    memset(&q, 0, sizeof(q));
+    q.f = p;
+    q.dt = dt;
+    q.stages = k.stages;
+    while (t.smem[i](dt, q.stages) > kF16MaxSmem) --q.stages;
+    // a helper goes to the scheduler (warp % 4) that has the least to do
+    int load[4] = {}, warps = k.workers;
+    for (int w = 0; w < k.workers; ++w) {
+        q.consumers |= 1u << w;
+        load[w % 4] += 2;
+    }
+    for (int h = 0; h < k.helpers; ++h) {
+        int best = -1;
+        for (int w = k.workers; w < k.workers + 8; ++w)
+            if (!(q.helpers >> w & 1) && (best < 0 || load[w % 4] < load[best % 4])) best = w;
+        q.helpers |= 1u << best;
+        load[best % 4] += 1;
+        warps = std::max(warps, best + 1);
+    }
+    const int threads = 32 * (warps + 1);  // and the producer
+    auto tile = [&](CUtensorMap* map, const void* base, long long ld) {
+        return make_tmap_3d(c, map, a.dtype, base, ld, a.D, a.T, a.B, dt, steps);
+    };
+    if (!tile(&q.f.tm_x, a.x, a.ld_x) || !tile(&q.f.tm_dl, a.delta, a.ld_delta) || (a.z_mode && !tile(&q.f.tm_z, a.z, a.ld_z)))
+        return fail(c, MAMBA_B200_ERR_CUDA, "sscan_fwd: no tensor map for %d channels", dt);
+    q.f.tma_mask = 0;
+    if (make_tmap_3d(c, &q.f.tm_b, a.dtype, a.Bm, a.ld_bc, a.N, a.T, a.B, a.N, steps)) q.f.tma_mask |= kTmaB;
+    if (make_tmap_3d(c, &q.f.tm_c, a.dtype, a.Cm, a.ld_bc, a.N, a.T, a.B, a.N, steps)) q.f.tma_mask |= kTmaC;
+    q.vec_y = reinterpret_cast<uintptr_t>(a.y) % (2 * dtype_size(a.dtype)) == 0 && a.ld_y % 2 == 0;
+    auto aligned = [](const void* ptr) { return reinterpret_cast<uintptr_t>(ptr) % 16 == 0; };
+    q.vec_state = a.N == 16 && aligned(a.ssm_state) && aligned(a.chunk_states) && p.cs_ld_b % 4 == 0 && p.cs_ld_k % 4 == 0;
+
+    const int flags = (a.delta_softplus ? 1 : 0) | (a.z_mode ? 2 : 0);
+    const size_t smem = t.smem[i](dt, q.stages);
+    dim3 grid((a.D + dt - 1) / dt, a.B, plan.segs);
+    if (plan.segs > 1) {
+        const int chunks = (a.T + steps - 1) / steps;
+        q.f.seg_chunks = (chunks + plan.segs - 1) / plan.segs;
+        const SegmentBuffers w = segment_buffers(a, plan.segs);
+        q.f.seg_states = w.states;
+        q.f.seg_sumdl = w.sums;
+        Fwd16Params q1 = q;
+        q1.f.ssm_copy = w.ssm;
+        t.fn[i][4 + (flags & 1)]<<<grid, threads, smem, stream>>>(q1);
+        MB200_CUDA_CHECK(c, cudaGetLastError());
+        launch_seg_carry(stream, a, w, plan.segs);
+        MB200_CUDA_CHECK(c, cudaGetLastError());
+        q.f.ssm_in = w.ssm;
+    }
+    t.fn[i][flags]<<<grid, threads, smem, stream>>>(q);
+    MB200_CUDA_CHECK(c, cudaGetLastError());
+    return MAMBA_B200_OK;
 }
 
 static int launch_fwd(Ctx* c, cudaStream_t stream, const mamba_b200_sscan_fwd_args& a, long long cs_ld_b = 0,
@@ -203,6 +358,21 @@ static int launch_fwd(Ctx* c, cudaStream_t stream, const mamba_b200_sscan_fwd_ar
     if (make_tmap_3d(c, &p.tm_c, a.dtype, a.Cm, a.ld_bc, a.N, a.T, a.B, a.N, v->tc)) m |= kTmaC;
     p.tma_mask = m;
 
+    const bool lent = a.workspace && a.workspace_bytes > 0;
+    double us = 0.0;
+    int segs = fwd_segments(a.B, a.T, a.D, a.N, &us);
+    if (!lent) segs = 1;
+    // d_state 9 .. 16 without the conv, channels that TMA can bring: by warp roles where that is estimated to be faster
+    if (v->ns * v->lpc == 16 && !a.conv_w && (m & kTmaX) && (m & kTmaDl) && (!a.z_mode || (m & kTmaZ))) {
+        const Fwd16Table& t16 = fwd16_tables().t[a.dtype];
+        const Fwd16Plan plan = fwd16_plan(t16, a.dtype == MAMBA_B200_F32, a.B, a.T, a.D, a.N, us, lent ? a.workspace_bytes : 0);
+        if (plan.kind) {
+            if (plan.segs > 1 && reinterpret_cast<uintptr_t>(a.workspace) % 256)
+                return fail(c, MAMBA_B200_ERR_ARG, "sscan_fwd: workspace must be 256-byte aligned");
+            return launch_fwd16(c, stream, a, p, t16, plan);
+        }
+    }
+
     const int flags = (a.delta_softplus ? 1 : 0) | (a.z_mode ? 2 : 0) | (a.conv_w ? 4 : 0);
     FwdKernelFn fn = v->fn[flags];
     FwdKernelFn fn_state = v->fn[8 | (flags & 5)];
@@ -218,9 +388,7 @@ static int launch_fwd(Ctx* c, cudaStream_t stream, const mamba_b200_sscan_fwd_ar
     // entering states, and the second launch runs every segment in full.
     const int tiles = (a.D + v->dt - 1) / v->dt;
     const int nchunks = (a.T + v->tc - 1) / v->tc;
-    int segs = 1;
-    if (a.workspace && a.workspace_bytes > 0) {
-        segs = fwd_segments(a.B, a.T, a.D, a.N);
+    if (segs > 1) {
         size_t o1, o2, o3;
         while (segs > 1 && fwd_ws_bytes(a.B, a.D, a.N, segs, &o1, &o2, &o3) > static_cast<size_t>(a.workspace_bytes))
             segs /= 2;
@@ -233,20 +401,16 @@ static int launch_fwd(Ctx* c, cudaStream_t stream, const mamba_b200_sscan_fwd_ar
         segs = (nchunks + p.seg_chunks - 1) / p.seg_chunks;
     }
     if (segs > 1) {
-        size_t o_sum, o_h0, o_c0;
-        fwd_ws_bytes(a.B, a.D, a.N, segs, &o_sum, &o_h0, &o_c0);
-        unsigned char* ws = static_cast<unsigned char*>(a.workspace);
-        p.seg_states = reinterpret_cast<float*>(ws);
-        p.seg_sumdl = reinterpret_cast<float*>(ws + o_sum);
         grid.z = segs;
-        FwdParams p1 = p;  // state-only pass: also keeps the entering states for the second pass
-        p1.ssm_copy = reinterpret_cast<float*>(ws + o_h0);
-        p1.conv_copy = p.K ? reinterpret_cast<float*>(ws + o_c0) : nullptr;
+        FwdParams p1 = p;
+        const SegmentBuffers w = segment_buffers(a, segs);
+        p.seg_states = p1.seg_states = w.states;
+        p.seg_sumdl = p1.seg_sumdl = w.sums;
+        p1.ssm_copy = w.ssm;  // the state-only pass also keeps the entering states for the second pass
+        p1.conv_copy = p.K ? w.conv : nullptr;
         fn_state<<<grid, v->threads, v->smem, stream>>>(p1);
         MB200_CUDA_CHECK(c, cudaGetLastError());
-        const long long n = static_cast<long long>(a.B) * a.D * a.N;
-        sscan_seg_carry_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, stream>>>(
-            p.seg_states, p.seg_sumdl, a.a_neg, a.B, segs, a.D, a.N);
+        launch_seg_carry(stream, a, w, segs);
         MB200_CUDA_CHECK(c, cudaGetLastError());
         // segment 0 of the second pass reads the copies: the last segment overwrites the
         // caller's state arrays while other segments may still be starting

@@ -355,3 +355,59 @@ def test_time_segments_equal_one_piece(cuda_dev, shape, dt):
     tol = 1e-5 if dt == "f32" else 2e-2
     assert float((cut.float() - whole.float()).abs().max() / whole.float().abs().max()) <= tol
     assert float((h2 - h1).abs().max() / h1.abs().max()) <= 1e-5
+
+
+# The kernel by warp roles (d_state 9 .. 16, TMA-able channels, 24 steps or more), one shape for each of its layouts:
+# two, four, six and eight consumer warps of four states a lane, six of eight; whole and cut into segments.  Ragged
+# lengths, d_state below 16, a tile that reaches past d_inner (rows longer than the channels), B and C that no tensor
+# map describes, rows of y off every word, saves every 32 and 64 steps, all gate modes.  y is held to half a unit of its storage
+# and the decay rates' f32 rounding (TOL), the states to 1e-4, as everywhere in this file.
+@pytest.mark.parametrize("dt", ["f32", "bf16", "f16"])
+@pytest.mark.parametrize("case", [
+    # B, T, D, N, a_mode, workspace, z_mode, save_stride, odd (views: longer rows, B / C and y off by one element)
+    (1, 24, 64, 16, "s4d", False, 1, 32, False), (2, 25, 40, 9, "random", False, 1, 64, True),
+    (3, 75, 2048, 16, "random", False, 1, 32, False), (8, 79, 1536, 16, "s4d", False, 1, 64, False),
+    (10, 95, 1832, 16, "random", False, 2, 32, True), (16, 700, 1536, 12, "random", False, 0, 64, False),
+    (1, 1021, 328, 16, "random", True, 1, 32, True), (2, 333, 136, 13, "s4d", True, 1, 64, False),
+    (1, 300, 1536, 16, "s4d", True, 0, 32, False),
+], ids=lambda c: "B%dT%dD%dN%d%sws%dz%ds%dodd%d" % c)
+def test_warp_roles_match_oracle(cuda_dev, case, dt):
+    import torch
+
+    import mamba_rs_b200 as mb
+    B, T, D, N, a_mode, lent, z_mode, S, odd = case
+    q = quantised_inputs(B, T, D, N, 0, dt, seed=T + D, a_mode=a_mode)
+    ssm0, _ = random_states(B, D, N, 0, seed=T)
+    ref = oracle.m1_fused_fwd(q["x"], q["delta_raw"], q["Bm"], q["Cm"], q["z"] if z_mode == 1 else None, q["a_neg"], q["Dp"],
+                              None, None, None, ssm0, want_h=B * D * T < 300000)
+    want = ref["y"] * q["z"] if z_mode == 2 else ref["y"]
+    td = torch_dtype(dt)
+
+    def view(a, extra, off):
+        t = to_dev(a, cuda_dev, td)
+        if not odd:
+            return t
+        buf = torch.full((B, T, t.shape[-1] + extra), float("nan"), device=cuda_dev, dtype=td)
+        buf[..., off:off + t.shape[-1]] = t
+        return buf[..., off:off + t.shape[-1]]
+
+    D8 = 8 * ((D + 7) // 8) - D + 8
+    ssm = to_dev(ssm0, cuda_dev)
+    cs = torch.full((B, (T + S - 1) // S, D, N), float("nan"), device=cuda_dev)
+    ws = torch.empty(mb.selective_scan_fwd_workspace_bytes(B, T, D, N), dtype=torch.uint8, device=cuda_dev) if lent else None
+    ybuf = torch.zeros(B, T, D + 3, device=cuda_dev, dtype=td)
+    y = mb.selective_scan_fwd(view(q["x"], D8, 0), view(q["delta_raw"], D8, 0), view(q["Bm"], 3, 1), view(q["Cm"], 3, 1),
+                              to_dev(q["a_neg"], cuda_dev), to_dev(q["Dp"], cuda_dev), view(q["z"], D8, 0) if z_mode else None,
+                              z_mode=z_mode, ssm_state=ssm, chunk_states=cs, save_stride=S, workspace=ws,
+                              y=ybuf[..., 1:1 + D] if odd else None)
+    torch.cuda.synchronize()
+    mb.ffi.default_handle(0).check_status()
+    assert rel_err(y.float().cpu().numpy(), want) <= TOL[dt]
+    assert float(ybuf[..., 0].abs().max()) == 0.0 and float(ybuf[..., 1 + D:].abs().max()) == 0.0
+    assert rel_err(ssm.cpu().numpy(), ref["ssm_state"]) <= 1e-4
+    got = cs.cpu().numpy()
+    assert np.isfinite(got).all()
+    np.testing.assert_array_equal(got[:, 0], ssm0)
+    if "h_all" in ref and ref["h_all"] is not None:
+        for k in range(got.shape[1]):
+            assert rel_err(got[:, k], ref["h_all"][:, k * S]) <= 1e-4, k
