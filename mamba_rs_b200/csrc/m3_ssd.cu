@@ -224,6 +224,19 @@ constexpr uint32_t kLoc = kM;             // SEG: f32 local state [128 n][64 p],
 // TMEM columns: G; Y1; Y2; S^T.
 constexpr uint32_t cG = 0, cY1 = 256, cY2 = 320, cS = 384, kTmemCols = 512;
 
+// LEAN: two CTAs per SM, so that one's tensor-core and copy waits (3000 of a chunk's 7300 cycles) are the other's time.
+// One buffer for Q, K and V, asked for again when the last MMA of a chunk is done; M over the Q tile, Y1 over G, which
+// have been read by then.  8 x 4096 steps x 32 heads of 64 x 128: 250 -> 195 us (0.63 of the measured HBM rate), the same
+// bits.  What is left is the chain of a chunk, 11600 cycles long with the copies in it.  Not kept: the next chunk's tiles
+// brought into L2 ahead (201 us), V on a barrier of its own and another warp for the copies (196).
+namespace lean {
+constexpr uint32_t kK0 = 32768, kV0 = 65536, kVw = 81920, kVec = 98304, kStage = kVec + 2 * kVecSet * 4;
+static_assert(kStage % 128 == 0, "scalar staging");
+constexpr uint32_t kBar = kStage + 3 * kStageArr + 16, kTmemSlot = kBar + 48, kSmem = kTmemSlot + 16;
+static_assert(2 * (kSmem + 1024) <= 228 * 1024, "two CTAs per SM");
+constexpr uint32_t cY2 = 128, cS = 192, kTmemCols = 256;
+}  // namespace lean
+
 // GEN: build the K and Q tiles of a chunk in the kernel instead of reading them:
 //   K[t,h,:] = rope(Bn[t,g,:] + b_bias[h,:], angle[t,h,:]),  Q likewise from Cn / c_bias,
 //   angle[t,h,a] = (angle_in[h,a] + sum_{s<=t} angle_vel[s,a] * dt[s,h]) mod 2 pi
@@ -249,8 +262,16 @@ constexpr uint32_t cG = 0, cY1 = 256, cY2 = 320, cS = 384, kTmemCols = 512;
 // alone (K, V, one product a chunk) from zero; the CTAs then read one another's local states and decays
 // through distributed shared memory, which gives each the exact state entering its chunks, and walk them
 // in full.
-template <typename Th, bool GEN, bool CARRY, bool SEG>
-__global__ void __launch_bounds__(256, 1) m3_ssd_fwd_tc_kernel(const __grid_constant__ M3Params p) {
+template <typename Th, bool GEN, bool CARRY, bool SEG, bool LEAN>
+__global__ void __launch_bounds__(256, LEAN ? 2 : 1) m3_ssd_fwd_tc_kernel(const __grid_constant__ M3Params p) {
+    static_assert(!LEAN || !(GEN || CARRY || SEG), "the other forms need the room");
+    constexpr uint32_t kK0 = LEAN ? lean::kK0 : tc::kK0, kV0 = LEAN ? lean::kV0 : tc::kV0, kM = LEAN ? kQ0 : tc::kM;
+    constexpr uint32_t kVw = LEAN ? lean::kVw : tc::kVw, kS = kVw, kVec = LEAN ? lean::kVec : tc::kVec;
+    constexpr uint32_t kStage = LEAN ? lean::kStage : tc::kStage, kBar = LEAN ? lean::kBar : tc::kBar;
+    constexpr uint32_t kTmemSlot = LEAN ? lean::kTmemSlot : tc::kTmemSlot, kTmemCols = LEAN ? lean::kTmemCols : tc::kTmemCols;
+    constexpr uint32_t cY1 = LEAN ? cG : tc::cY1, cY2 = LEAN ? lean::cY2 : tc::cY2, cS = LEAN ? lean::cS : tc::cS;
+    constexpr uint32_t kQKStride = LEAN ? 0 : tc::kQKStride, kVStride = LEAN ? 0 : tc::kVStride;  // to the second buffer
+    constexpr uint32_t kQKBytes = tc::kQKStride, kVBytes = tc::kVStride;
     extern __shared__ __align__(1024) unsigned char smem[];
     // two threads per step: thread (row, half) owns row `row` of the chunk (TMEM lane
     // `row`) and half of that row's columns in every elementwise stage
@@ -511,7 +532,7 @@ __global__ void __launch_bounds__(256, 1) m3_ssd_fwd_tc_kernel(const __grid_cons
     // arrive as zeros.
     auto issue_carry_q = [&](int c) {
         if (threadIdx.x == 0) {
-            mbar_expect_tx(&full[0], kQKStride);
+            mbar_expect_tx(&full[0], kQKBytes);
 #pragma unroll
             for (int sub = 0; sub < 2; ++sub)
                 tma_load_4d(smem + kQ0 + sub * kSwSub, &p.tm_q, &full[0], 64 * sub, h, c * CS, b);
@@ -519,7 +540,7 @@ __global__ void __launch_bounds__(256, 1) m3_ssd_fwd_tc_kernel(const __grid_cons
     };
     auto issue_carry_kv = [&](int c) {
         if (threadIdx.x == 0) {
-            mbar_expect_tx(&full[1], kQKStride + kVStride);
+            mbar_expect_tx(&full[1], kQKBytes + kVBytes);
 #pragma unroll
             for (int sub = 0; sub < 2; ++sub)
                 tma_load_4d(smem + kCarryK + sub * kSwSub, &p.tm_k, &full[1], 64 * sub, h, c * CS, b);
@@ -529,7 +550,7 @@ __global__ void __launch_bounds__(256, 1) m3_ssd_fwd_tc_kernel(const __grid_cons
     auto issue_kv = [&](int c, int j) {  // state pass
         if (threadIdx.x == 0) {
             const int buf = j & 1, t0 = c * CS;
-            mbar_expect_tx(&full[buf], kQKStride + kVStride);
+            mbar_expect_tx(&full[buf], kQKBytes + kVBytes);
 #pragma unroll
             for (int sub = 0; sub < 2; ++sub)
                 tma_load_4d(smem + kK0 + buf * kQKStride + sub * kSwSub, &p.tm_k, &full[buf], 64 * sub, h, t0, b);
@@ -538,9 +559,9 @@ __global__ void __launch_bounds__(256, 1) m3_ssd_fwd_tc_kernel(const __grid_cons
     };
     auto issue_tiles = [&](int c, int j) {
         if (threadIdx.x == 0) {
-            const int buf = j & 1, t0 = c * CS;
+            const int buf = LEAN ? 0 : j & 1, t0 = c * CS;
             const int hq = GEN ? h / (nh / p.ng) : h;
-            mbar_expect_tx(&full[buf], 2 * kQKStride + kVStride);
+            mbar_expect_tx(&full[buf], 2 * kQKBytes + kVBytes);
 #pragma unroll
             for (int sub = 0; sub < 2; ++sub) {
                 tma_load_4d(smem + kQ0 + buf * kQKStride + sub * kSwSub, &p.tm_q, &full[buf], 64 * sub, hq, t0, b);
@@ -741,11 +762,13 @@ __global__ void __launch_bounds__(256, 1) m3_ssd_fwd_tc_kernel(const __grid_cons
         const uint32_t tV = CARRY ? kCarryV : kV0 + (j & 1) * kVStride;
         // ---- 1. copies of the next chunk's tiles into the other buffers (their last readers,
         //         the MMAs of chunk c - 1, have completed); per-row scalars; this chunk's tiles ----
-        if (!CARRY && c + 1 < c_hi) issue_tiles(c + 1, j + 1);
+        if (!CARRY && !LEAN && c + 1 < c_hi) issue_tiles(c + 1, j + 1);
         scalars(j);
         if (CARRY) {
             ok = mbar_wait(&full[0], i0 & 1, p.status) && ok;
             ok = mbar_wait(&full[1], j & 1, p.status) && ok;
+        } else if (LEAN) {
+            ok = mbar_wait(&full[0], j & 1, p.status) && ok;
         } else {
             ok = mbar_wait(&full[j & 1], (j >> 1) & 1, p.status) && ok;
         }
@@ -868,6 +891,7 @@ __global__ void __launch_bounds__(256, 1) m3_ssd_fwd_tc_kernel(const __grid_cons
         ok = mbar_wait(&bars[1], j & 1, p.status) && ok;
         fence_after();
         if (CARRY && c + 1 < c_hi) issue_carry_kv(c + 1);
+        if (LEAN && c + 1 < c_hi) issue_tiles(c + 1, j + 1);
         // ---- 5. epilogue: y row; 16-bit copy of the new state for the next chunk ----
         {
             const float e_t = ex2(dA[tid] * kLog2e);
@@ -963,6 +987,12 @@ int m3_cluster_ranks(int heads, int nchunks, double full, double pair, double ma
     return best;
 }
 
+// Two CTAs per SM (LEAN) or one: 5.9 us a chunk for both together against 3.7 for one, which has its next tiles on the
+// way while it works.  16 chunks of 64 x 128 in us, one / two per SM: 152 pairs 127 and 99, 256 131 and 104, 296 148
+// and 132, 352 191 and 188, 384 192 and 193, 440 220 and 223, 464 284 and 232, 512 256 and 198, 592 309 and 264, 896 443
+// and 362.  So one wave of one CTA per SM stays, and three nearly full ones.
+static bool m3_two_per_sm(int pairs) { return pairs > 148 && (pairs <= 360 || pairs > 3 * 148); }
+
 cudaError_t launch_cluster(const void* fn, dim3 grid, dim3 block, size_t smem, cudaStream_t st, int ranks, void** args) {
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
@@ -981,16 +1011,22 @@ cudaError_t launch_cluster(const void* fn, dim3 grid, dim3 block, size_t smem, c
 }
 
 int m3_configure(Ctx* c) {
-    const void* fns[8] = {reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, false, false>),
-                          reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__half, false, false, false>),
-                          reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, true, false, false>),
-                          reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__half, true, false, false>),
-                          reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, true, false>),
-                          reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, false, true>),
-                          reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__half, false, false, true>),
-                          reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, true, true>)};
+    const void* fns[8] = {reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, false, false, false>),
+                          reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__half, false, false, false, false>),
+                          reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, true, false, false, false>),
+                          reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__half, true, false, false, false>),
+                          reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, true, false, false>),
+                          reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, false, true, false>),
+                          reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__half, false, false, true, false>),
+                          reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, true, true, false>)};
     for (const void* fn : fns)
         MB200_CUDA_CHECK(c, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::kSmem));
+    const void* lean_fns[2] = {reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, false, false, true>),
+                               reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__half, false, false, false, true>)};
+    for (const void* fn : lean_fns) {
+        MB200_CUDA_CHECK(c, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::lean::kSmem));
+        MB200_CUDA_CHECK(c, cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+    }
     return MAMBA_B200_OK;
 }
 
@@ -1098,18 +1134,21 @@ extern "C" MAMBA_B200_API int mamba_b200_m3_ssd_fwd(void* handle, void* stream,
         const int ranks = gen ? 1 : a.carry_in ? m3_cluster_ranks(a.B * a.nh, nchunks, 5.5, 6.6, 6.6, 3.2)
                                                : m3_cluster_ranks(a.B * a.nh, nchunks, 3.7, 5.15, 5.15, 2.6);
         if (ranks > 1) {
-            const void* fn = bf ? (a.carry_in ? reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, true, true>)
-                                              : reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, false, true>))
-                                : reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__half, false, false, true>);
+            const void* fn = bf ? (a.carry_in ? reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, true, true, false>)
+                                              : reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, false, true, false>))
+                                : reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__half, false, false, true, false>);
             void* args[1] = {&p};
             MB200_CUDA_CHECK(c, launch_cluster(fn, dim3(a.nh * ranks, a.B), dim3(256), tc::kSmem, st, ranks, args));
+        } else if (!gen && !a.carry_in && m3_two_per_sm(a.B * a.nh)) {
+            if (bf) tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, false, false, true><<<grid, 256, tc::lean::kSmem, st>>>(p);
+            else tc::m3_ssd_fwd_tc_kernel<__half, false, false, false, true><<<grid, 256, tc::lean::kSmem, st>>>(p);
         } else if (bf) {
-            if (gen) tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, true, false, false><<<grid, 256, tc::kSmem, st>>>(p);
-            else if (a.carry_in) tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, true, false><<<grid, 256, tc::kSmem, st>>>(p);
-            else tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, false, false><<<grid, 256, tc::kSmem, st>>>(p);
+            if (gen) tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, true, false, false, false><<<grid, 256, tc::kSmem, st>>>(p);
+            else if (a.carry_in) tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, true, false, false><<<grid, 256, tc::kSmem, st>>>(p);
+            else tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, false, false, false><<<grid, 256, tc::kSmem, st>>>(p);
         } else {
-            if (gen) tc::m3_ssd_fwd_tc_kernel<__half, true, false, false><<<grid, 256, tc::kSmem, st>>>(p);
-            else tc::m3_ssd_fwd_tc_kernel<__half, false, false, false><<<grid, 256, tc::kSmem, st>>>(p);
+            if (gen) tc::m3_ssd_fwd_tc_kernel<__half, true, false, false, false><<<grid, 256, tc::kSmem, st>>>(p);
+            else tc::m3_ssd_fwd_tc_kernel<__half, false, false, false, false><<<grid, 256, tc::kSmem, st>>>(p);
         }
     } else {
         if (a.dtype == MAMBA_B200_F32) launch_seq<float>(p, c->sm_count, st);

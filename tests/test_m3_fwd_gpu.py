@@ -298,3 +298,35 @@ def test_an_infinite_input_stays_infinite_beside_the_states_that_are_not_there(c
     y, ssm, _, _ = run_gpu(i, "f32", cuda_dev, force_sequential=True)
     assert np.isinf(y[0, 5:, 3]).all() and np.isfinite(np.delete(y, 3, axis=2)).all()
     assert np.isinf(ssm[0, 0, 3]).all()
+
+
+# More (sample, head) pairs than SMs run two CTAs per SM, fewer one: the same arithmetic in the same order, so a batch
+# of 150 or more pairs must give, bit for bit, what its first and its last samples give in calls of fewer than 148.
+@pytest.mark.parametrize("dt", ["bf16", "f16"])
+@pytest.mark.parametrize("case", [(10, 1, 16, 64, 128), (10, 127, 15, 32, 64), (10, 128, 16, 8, 16), (10, 129, 15, 64, 128),
+                                  (10, 300, 16, 64, 72), (10, 513, 16, 56, 128)], ids=lambda c: "B%dT%dnh%dhd%dN%d" % c)
+def test_two_ctas_per_sm_give_the_same_bits(cuda_dev, case, dt):
+    import torch
+
+    import mamba_rs_b200 as mb
+    B, T, nh, hd, N = case
+    td = {"bf16": torch.bfloat16, "f16": torch.float16}[dt]
+    g = torch.Generator(device=cuda_dev).manual_seed(T)
+    rn = lambda *s: torch.randn(*s, device=cuda_dev, generator=g)  # noqa: E731
+    x, K, Q = rn(B, T, nh * hd).to(td), (0.3 * rn(B, T, nh, N)).to(td), (0.3 * rn(B, T, nh, N)).to(td)
+    dt_, trap = torch.nn.functional.softplus(rn(B, T, nh) - 2), torch.sigmoid(rn(B, T, nh))
+    adt, Dh = -dt_ * torch.rand(nh, device=cuda_dev, generator=g) * 4, rn(nh)
+
+    def call(lo, hi):
+        st = dict(ssm_state=torch.full((hi - lo, nh, hd, N), float("nan"), device=cuda_dev),
+                  k_state=torch.full((hi - lo, nh, N), float("nan"), device=cuda_dev),
+                  v_state=torch.full((hi - lo, nh, hd), float("nan"), device=cuda_dev))
+        c = lambda t: t[lo:hi].contiguous()  # noqa: E731
+        y = mb.m3_ssd_fwd(c(x), c(K), c(Q), c(dt_), c(trap), c(adt), Dh, **st)
+        return [y, st["ssm_state"], st["k_state"], st["v_state"]]
+
+    whole = call(0, B)
+    for lo, hi in ((0, B - 1), (1, B)):
+        for a, b in zip(whole, call(lo, hi)):
+            assert torch.isfinite(a.float()).all() and torch.equal(a[lo:hi], b)
+    mb.ffi.default_handle(0).check_status()
