@@ -40,9 +40,9 @@ static int fwd_segments(int B, int T, int D, int N, double* us) {
     const int blocks = (T + 31) / 32;
     auto cut = [&](int s) {
         const int per = (blocks + s - 1) / s;
-        const double x = std::min(2.0 * ctas * s / 148, 2.0 * kFwdMaxPerSm), f = x - static_cast<int>(x);
-        const double* at = kCut + static_cast<int>(x);
-        return 8 + (32 * per + 16) * (at[0] + f * (at[1] - at[0]));
+        const double x = 2.0 * ctas * s / 148, f = x - static_cast<int>(x);
+        const double* at = kCut + std::min(static_cast<int>(x), 2 * kFwdMaxPerSm);
+        return 8 + (32 * per + 16) * (x < 2 * kFwdMaxPerSm ? at[0] + f * (at[1] - at[0]) : at[0] * x / (2 * kFwdMaxPerSm));
     };
     if (T >= 1536) {
         const double w = ctas / 148.0;
@@ -61,17 +61,17 @@ static int fwd_segments(int B, int T, int D, int N, double* us) {
 
 // The kernel by warp roles: how a call is laid out and what that takes, in us.  One CTA has an SM to itself (three at
 // two consumer warps).  Whole: w0 + w1 a step and round of CTAs; cut, where all pieces run side by side: c0 + c1 a step
-// of a piece, both passes and the carry.  Fitted to 200 shapes of 8 to 5600 steps (as CUDA graphs): half of the
+// of a piece, both passes.  Fitted to 200 shapes of 8 to 5600 steps (as CUDA graphs): half of the
 // estimates are within 5 % (whole) and 8 % (cut).  16-bit storage; f32 takes 1.05 times as long.
 struct Fwd16Kind {
     int ns, workers, helpers, stages;
     double w0, w1, c0, c1;
 };
-static const Fwd16Kind kFwd16Kinds[] = {{4, 2, 2, 3, 3.7, 0.0623, 8.6, 0.1022},
-                                        {4, 4, 4, 4, 3.5, 0.0712, 8.7, 0.1175},
-                                        {4, 6, 4, 4, 4.3, 0.0888, 10.0, 0.1501},
-                                        {4, 8, 4, 4, 4.0, 0.1068, 9.5, 0.1813},
-                                        {8, 6, 4, 4, 5.4, 0.1527, 13.1, 0.2608}};
+static const Fwd16Kind kFwd16Kinds[] = {{4, 2, 2, 3, 3.7, 0.0623, 5.6, 0.1022},
+                                        {4, 4, 4, 4, 3.5, 0.0712, 5.7, 0.1175},
+                                        {4, 6, 4, 4, 4.3, 0.0888, 7.0, 0.1501},
+                                        {4, 8, 4, 4, 4.0, 0.1068, 6.5, 0.1813},
+                                        {8, 6, 4, 4, 5.4, 0.1527, 10.1, 0.2608}};
 struct Fwd16Plan {
     const Fwd16Kind* kind = nullptr;  // null: sscan_fwd_kernel
     int segs = 1;
@@ -175,12 +175,12 @@ static size_t fwd_ws_bytes(int B, int D, int N, int segs, size_t* o_sum, size_t*
     return off;
 }
 
-// The layout with the least estimate, if that is at most 0.95 (cut: 0.9) of what sscan_fwd_kernel is estimated to take.
-// Against it, on the 200 shapes: 12 % less time on average, 4 % more at most (1 x 471 x 5024 in f32), 1 % more than the
-// best layout of either kernel.  8 x 2048 x 1536 with general rates 284 -> 196 us, 2 x 8192 x 5120 with progressions 762
-// -> 645, 16 x 2048 x 1536 367 -> 342 and 303 -> 287, 1 x 1021 x 1536 39 -> 34.  Under 24 steps the shorter prologue of
-// the other kernel wins (12 x 9 x 144 4.5 us, here 5.8), and past three rounds of CTAs its three CTAs an SM do (19 x 33 x
-// 5360 32 us, here 59).
+// The layout with the least estimate, if that is at most 0.95 (eight states a lane: 0.935, cut: 0.9) of what
+// sscan_fwd_kernel is estimated to take.  Against that kernel alone, 160 shapes of 64 to 8192 steps, both kinds of rates:
+// 14 % less time on average, no shape more than 2 % more.  8 x 2048 x 1536 with general rates 284 -> 196 us, 2 x 8192 x
+// 5120 with progressions 757 -> 663, 16 x 2048 x 1536 363 -> 339 (10 x 750 x 2600 with progressions would be 117 -> 124),
+// 1 x 1021 x 1536 32.0 -> 28.5, 4 x 512 x 256 19.7 -> 15.5.  Under 24 steps the shorter prologue of the other kernel wins
+// (12 x 9 x 144 4.5 us, here 5.8), and past three rounds of CTAs its three CTAs an SM do (19 x 33 x 5360 32 us, here 59).
 static Fwd16Plan fwd16_plan(const Fwd16Table& t, bool f32, int B, int T, int D, int N, double us, long long workspace_bytes) {
     Fwd16Plan best;
     if (T < 24) return best;
@@ -191,7 +191,7 @@ static Fwd16Plan fwd16_plan(const Fwd16Table& t, bool f32, int B, int T, int D, 
         const double scale = f32 ? 1.05 : 1.0;
         double c = scale * ((ctas + 147) / 148) * (k.w0 + k.w1 * T);
         if (k.workers == 2 && ctas > 148) c = scale * ((ctas + 443) / 444) * (4.5 + 0.0931 * T);
-        if (c < us && ctas <= 3 * 148) {
+        if (c < (k.ns == 8 ? 0.935 / 0.95 * us : us) && ctas <= 3 * 148) {
             us = c;
             best = {&k, 1};
         }
@@ -283,9 +283,7 @@ static int launch_fwd16(Ctx* c, cudaStream_t stream, const mamba_b200_sscan_fwd_
         q1.f.ssm_copy = w.ssm;
         t.fn[i][4 + (flags & 1)]<<<grid, threads, smem, stream>>>(q1);
         MB200_CUDA_CHECK(c, cudaGetLastError());
-        launch_seg_carry(stream, a, w, plan.segs);
-        MB200_CUDA_CHECK(c, cudaGetLastError());
-        q.f.ssm_in = w.ssm;
+        q.f.ssm_in = w.ssm;  // the last segment writes the caller's state while others may still be starting
     }
     t.fn[i][flags]<<<grid, threads, smem, stream>>>(q);
     MB200_CUDA_CHECK(c, cudaGetLastError());

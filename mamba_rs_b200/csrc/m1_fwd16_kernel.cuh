@@ -346,9 +346,7 @@ sscan_fwd16_kernel(const __grid_constant__ Fwd16Params q) {
     float2 h[2][NS / 2], a2[NS], a_inc;
     bool progression = true;
     {
-        const float* h0 = nullptr;
-        if (seg == 0) h0 = p.ssm_in ? p.ssm_in + static_cast<long long>(b) * D * N : nullptr;
-        else if (!kStateOnly) h0 = p.seg_states + (static_cast<long long>(b) * nseg + (seg - 1)) * D * N;
+        const float* h0 = seg == 0 && p.ssm_in ? p.ssm_in + static_cast<long long>(b) * D * N : nullptr;
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             float av[NS], hv[NS];
@@ -373,6 +371,48 @@ sscan_fwd16_kernel(const __grid_constant__ Fwd16Params q) {
                 else a2[j].x = av[j];
                 if (j & 1) h[i][j / 2] = make_float2(hv[j - 1], hv[j]);
             }
+        }
+    }
+    // The state that enters a later segment: h = exp(a * sum of its deltas) h + what it leaves from zero, over the
+    // segments before this one (the first of which started from the real state).  Every CTA does this for itself, from
+    // L2, a few segments' loads at a time: with a launch of its own between the passes it took 3 us more.
+    if (!kStateOnly && seg > 0) {
+        const long long row = static_cast<long long>(D) * N;
+        const float* left = p.seg_states + static_cast<long long>(b) * nseg * row + static_cast<long long>(d) * N + n0;
+        const float* sums = p.seg_sumdl + static_cast<long long>(b) * nseg * D + d;
+        constexpr int U = NS == 8 ? 2 : 4;
+        for (int s0 = 0; s0 < seg; s0 += U) {
+            float w[U][2][NS], dl[U][2];
+#pragma unroll
+            for (int k = 0; k < U; ++k) {
+                const int s = min(s0 + k, seg - 1);
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const bool ok = d + i < D;
+                    dl[k][i] = ok ? sums[static_cast<long long>(s) * D + i] : 0.0f;
+                    if (N == 16 && ok) {
+#pragma unroll
+                        for (int v = 0; v < NS; v += 4) {
+                            const float4 f = *reinterpret_cast<const float4*>(left + s * row + i * 16 + v);
+                            w[k][i][v] = f.x, w[k][i][v + 1] = f.y, w[k][i][v + 2] = f.z, w[k][i][v + 3] = f.w;
+                        }
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < NS; ++j) w[k][i][j] = ok && n0 + j < N ? left[s * row + i * N + j] : 0.0f;
+                    }
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < U; ++k)
+                if (s0 + k < seg) {
+#pragma unroll
+                    for (int i = 0; i < 2; ++i)
+#pragma unroll
+                        for (int j = 0; j < NS; ++j) {
+                            float& x = j & 1 ? h[i][j / 2].y : h[i][j / 2].x;
+                            x = s0 + k ? fmaf(ex2((i ? a2[j].y : a2[j].x) * dl[k][i]), x, w[k][i][j]) : w[k][i][j];
+                        }
+                }
         }
     }
     const bool geo = __all_sync(0xffffffffu, progression);
