@@ -69,6 +69,7 @@ struct Fwd16Kind {
 };
 static const Fwd16Kind kFwd16Kinds[] = {{4, 2, 2, 3, 3.7, 0.0623, 5.6, 0.1022},
                                         {4, 4, 4, 4, 3.5, 0.0712, 5.7, 0.1175},
+                                        {4, 5, 4, 4, 4.2, 0.0852, 6.8, 0.1400},
                                         {4, 6, 4, 4, 4.3, 0.0888, 7.0, 0.1501},
                                         {4, 8, 4, 4, 4.0, 0.1068, 6.5, 0.1813},
                                         {8, 6, 4, 4, 5.4, 0.1527, 10.1, 0.2608}};
@@ -178,7 +179,7 @@ static size_t fwd_ws_bytes(int B, int D, int N, int segs, size_t* o_sum, size_t*
 // The layout with the least estimate, if that is at most 0.95 (eight states a lane: 0.935, cut: 0.9) of what
 // sscan_fwd_kernel is estimated to take.  Against that kernel alone, 160 shapes of 64 to 8192 steps, both kinds of rates:
 // 14 % less time on average, no shape more than 2 % more.  8 x 2048 x 1536 with general rates 284 -> 196 us, 2 x 8192 x
-// 5120 with progressions 757 -> 663, 16 x 2048 x 1536 363 -> 339 (10 x 750 x 2600 with progressions would be 117 -> 124),
+// 5120 with progressions 757 -> 640, 16 x 2048 x 1536 363 -> 339 (10 x 750 x 2600 with progressions would be 117 -> 124),
 // 1 x 1021 x 1536 32.0 -> 28.5, 4 x 512 x 256 19.7 -> 15.5.  Under 24 steps the shorter prologue of the other kernel wins
 // (12 x 9 x 144 4.5 us, here 5.8), and past three rounds of CTAs its three CTAs an SM do (19 x 33 x 5360 32 us, here 59).
 static Fwd16Plan fwd16_plan(const Fwd16Table& t, bool f32, int B, int T, int D, int N, double us, long long workspace_bytes) {
