@@ -229,6 +229,11 @@ constexpr uint32_t cG = 0, cY1 = 256, cY2 = 320, cS = 384, kTmemCols = 512;
 // have been read by then.  8 x 4096 steps x 32 heads of 64 x 128: 250 -> 195 us (0.63 of the measured HBM rate), the same
 // bits.  What is left is the chain of a chunk, 11600 cycles long with the copies in it.  Not kept: the next chunk's tiles
 // brought into L2 ahead (201 us), V on a barrier of its own and another warp for the copies (196).
+// Carried windows (CARRY) do this too, although they have five more operand tiles: the remainders take turns in the tiles
+// of the first products (S_lo after S, M_lo after M, the second and third part of w o V after the first), five MMA groups
+// a chunk for two, whose waits are the other CTA's time.  Y2 takes its rows' decay in tensor memory and M V on top, which
+// leaves G readable.  The state's sums keep their order, and its bits.  8 x 256 steps x 32 heads: 62 -> 47 us with inputs
+// that are new to the caches.
 namespace lean {
 constexpr uint32_t kK0 = 32768, kV0 = 65536, kVw = 81920, kVec = 98304, kStage = kVec + 2 * kVecSet * 4;
 static_assert(kStage % 128 == 0, "scalar staging");
@@ -264,7 +269,8 @@ constexpr uint32_t cY2 = 128, cS = 192, kTmemCols = 256;
 // in full.
 template <typename Th, bool GEN, bool CARRY, bool SEG, bool LEAN>
 __global__ void __launch_bounds__(256, LEAN ? 2 : 1) m3_ssd_fwd_tc_kernel(const __grid_constant__ M3Params p) {
-    static_assert(!LEAN || !(GEN || CARRY || SEG), "the other forms need the room");
+    static_assert(!LEAN || !(GEN || SEG), "the other forms need the room");
+    constexpr bool TURNS = CARRY && LEAN;  // the remainders' products take turns in the tiles of the first ones
     constexpr uint32_t kK0 = LEAN ? lean::kK0 : tc::kK0, kV0 = LEAN ? lean::kV0 : tc::kV0, kM = LEAN ? kQ0 : tc::kM;
     constexpr uint32_t kVw = LEAN ? lean::kVw : tc::kVw, kS = kVw, kVec = LEAN ? lean::kVec : tc::kVec;
     constexpr uint32_t kStage = LEAN ? lean::kStage : tc::kStage, kBar = LEAN ? lean::kBar : tc::kBar;
@@ -571,6 +577,7 @@ __global__ void __launch_bounds__(256, LEAN ? 2 : 1) m3_ssd_fwd_tc_kernel(const 
         }
     };
     // 16-bit copy of this thread's state row (and the remainders): the B operand of Y2
+    uint32_t s_lo[TURNS ? 16 : 1], m_lo[TURNS ? 2 : 1][16];  // TURNS: remainders that wait for their turn
     auto copy_state = [&](const float* sv) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -584,9 +591,13 @@ __global__ void __launch_bounds__(256, LEAN ? 2 : 1) m3_ssd_fwd_tc_kernel(const 
                 }
             }
             *reinterpret_cast<uint4*>(smem + kS + sw_chunk(tid, half * 4 + j)) = make_uint4(w[0], w[1], w[2], w[3]);
-            if (CARRY)
+            if constexpr (TURNS) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) s_lo[4 * j + i] = lo[i];
+            } else if (CARRY) {
                 *reinterpret_cast<uint4*>(smem + kSlo + sw_chunk(tid, half * 4 + j)) =
                     make_uint4(lo[0], lo[1], lo[2], lo[3]);
+            }
         }
     };
     // the carried state as this thread's row: h + dt_0 (1 - trap_0) k_prev v_prev^T
@@ -608,8 +619,8 @@ __global__ void __launch_bounds__(256, LEAN ? 2 : 1) m3_ssd_fwd_tc_kernel(const 
         copy_state(sv);
         fence_proxy_async();
     };
-    // w o V of chunk j (and its remainders): the B operand of the state update
-    auto weigh_v = [&](const float* dA, const float* scl, int nv, uint32_t tV) {
+    // w o V of chunk j (and its remainders; TURNS: which of the three): the B operand of the state update
+    auto weigh_v = [&](const float* dA, const float* scl, int nv, uint32_t tV, int turn) {
         const float wt = tid < nv ? ex2((dA[nv - 1] - dA[tid]) * kLog2e) * scl[tid] : 0.0f;
 #pragma unroll
         for (int jj = half * (HD / 16); jj < (half + 1) * (HD / 16); ++jj) {
@@ -626,8 +637,12 @@ __global__ void __launch_bounds__(256, LEAN ? 2 : 1) m3_ssd_fwd_tc_kernel(const 
                     rest[q4] = pack2<Th>(r.x - mid.x, r.y - mid.y);
                 }
             }
+            if (TURNS && turn > 0) {
+#pragma unroll
+                for (int q4 = 0; q4 < 4; ++q4) w4[q4] = turn == 1 ? lo[q4] : rest[q4];
+            }
             *reinterpret_cast<uint4*>(smem + kVw + sw_chunk(tid, jj)) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
-            if (CARRY) {
+            if (CARRY && !TURNS) {
                 *reinterpret_cast<uint4*>(smem + kVwLo + sw_chunk(tid, jj)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
                 *reinterpret_cast<uint4*>(smem + kVwRest + sw_chunk(tid, jj)) = make_uint4(rest[0], rest[1], rest[2], rest[3]);
             }
@@ -645,7 +660,7 @@ __global__ void __launch_bounds__(256, LEAN ? 2 : 1) m3_ssd_fwd_tc_kernel(const 
 #pragma unroll
         for (int k = 0; k < CS / 16; ++k)  // M = n, N = p, K = t
             mma(tmem + cS, desc_sw_mn(sbase + tK, k), desc_sw_mn(sbase + kVw, k), idS, accumulate || k > 0);
-        if (CARRY) {
+        if (CARRY && !TURNS) {
 #pragma unroll
             for (int k = 0; k < CS / 16; ++k)
                 mma(tmem + cS, desc_sw_mn(sbase + tK, k), desc_sw_mn(sbase + kVwLo, k), idS, true);
@@ -676,7 +691,7 @@ __global__ void __launch_bounds__(256, LEAN ? 2 : 1) m3_ssd_fwd_tc_kernel(const 
                 ok = mbar_wait(CARRY ? &full[1] : &full[j & 1], CARRY ? j & 1 : (j >> 1) & 1, p.status) && ok;
                 __syncthreads();  // the per-row vectors of every row
                 stage_scalars(c + 1);
-                weigh_v(dA, dA + 128, nv, tV);
+                weigh_v(dA, dA + 128, nv, tV, 0);
                 const bool have = c > c_lo || (CARRY && rank == 0);
                 if (have) decay_state(ex2(dA[nv - 1] * kLog2e));
                 tot += dA[nv - 1];
@@ -739,7 +754,7 @@ __global__ void __launch_bounds__(256, LEAN ? 2 : 1) m3_ssd_fwd_tc_kernel(const 
         if (CARRY && rank == 0) enter_state();
         cluster_sync();  // nobody reads this CTA's shared memory any more
     } else {
-        if (CARRY) {
+        if (CARRY && !LEAN) {
             issue_carry_q(0);
             issue_carry_kv(0);
         } else {
@@ -758,17 +773,17 @@ __global__ void __launch_bounds__(256, LEAN ? 2 : 1) m3_ssd_fwd_tc_kernel(const 
         const float* scl = dA + 128;
         const float* gam = dA + 256;
         const uint32_t tQ = kQ0 + (CARRY ? 0u : (j & 1) * kQKStride);
-        const uint32_t tK = CARRY ? kCarryK : kK0 + (j & 1) * kQKStride;
-        const uint32_t tV = CARRY ? kCarryV : kV0 + (j & 1) * kVStride;
+        const uint32_t tK = CARRY && !LEAN ? kCarryK : kK0 + (j & 1) * kQKStride;
+        const uint32_t tV = CARRY && !LEAN ? kCarryV : kV0 + (j & 1) * kVStride;
         // ---- 1. copies of the next chunk's tiles into the other buffers (their last readers,
         //         the MMAs of chunk c - 1, have completed); per-row scalars; this chunk's tiles ----
         if (!CARRY && !LEAN && c + 1 < c_hi) issue_tiles(c + 1, j + 1);
         scalars(j);
-        if (CARRY) {
+        if (LEAN) {
+            ok = mbar_wait(&full[0], j & 1, p.status) && ok;
+        } else if (CARRY) {
             ok = mbar_wait(&full[0], i0 & 1, p.status) && ok;
             ok = mbar_wait(&full[1], j & 1, p.status) && ok;
-        } else if (LEAN) {
-            ok = mbar_wait(&full[0], j & 1, p.status) && ok;
         } else {
             ok = mbar_wait(&full[j & 1], (j >> 1) & 1, p.status) && ok;
         }
@@ -794,20 +809,39 @@ __global__ void __launch_bounds__(256, LEAN ? 2 : 1) m3_ssd_fwd_tc_kernel(const 
                 for (int k = 0; k < NS / 16; ++k)  // N = p, K = n
                     mma(tmem + cY2, desc_sw_k(sbase + tQ, k), desc_sw_mn(sbase + kS, k), idY, k > 0);
             }
-            if (CARRY) {
+            if (CARRY && !LEAN) {
 #pragma unroll
                 for (int k = 0; k < NS / 16; ++k)
                     mma(tmem + cY2, desc_sw_k(sbase + tQ, k), desc_sw_mn(sbase + kSlo, k), idY, true);
             }
             commit(&bars[0]);
         }
-        ok = mbar_wait(&bars[0], i0 & 1, p.status) && ok;
+        ok = mbar_wait(&bars[0], TURNS ? 0 : i0 & 1, p.status) && ok;
         fence_after();
-        if (CARRY && c + 1 < c_hi) issue_carry_q(c + 1);
+        if constexpr (TURNS) {  // Y2 += Q S_lo, S_lo where the state copy was
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                *reinterpret_cast<uint4*>(smem + kS + sw_chunk(tid, half * 4 + q)) =
+                    make_uint4(s_lo[4 * q], s_lo[4 * q + 1], s_lo[4 * q + 2], s_lo[4 * q + 3]);
+            fence_proxy_async();
+            fence_before();
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                fence_after();
+                const uint32_t idY = instr_desc(fmt, 0, 1, 64);
+#pragma unroll
+                for (int k = 0; k < NS / 16; ++k)
+                    mma(tmem + cY2, desc_sw_k(sbase + tQ, k), desc_sw_mn(sbase + kS, k), idY, true);
+                commit(&bars[0]);
+            }
+            ok = mbar_wait(&bars[0], 1, p.status) && ok;
+            fence_after();
+        }
+        if (CARRY && !LEAN && c + 1 < c_hi) issue_carry_q(c + 1);
         // ---- 3. decay / causal mask -> M (over the Q tile); w o V (over the old state
         //         copy); rescale the running state ----
         {
-            weigh_v(dA, scl, nv, tV);
+            weigh_v(dA, scl, nv, tV, 0);
             const float* dAl = dA + 384;  // dA * log2(e)
             const float dAlt = dAl[tid], gt = gam[tid];
             // One 32-column block of row `tid`.  Blocks left of the diagonal block need no
@@ -846,18 +880,29 @@ __global__ void __launch_bounds__(256, LEAN ? 2 : 1) m3_ssd_fwd_tc_kernel(const 
                 for (int j = 0; j < 4; ++j)
                     *reinterpret_cast<uint4*>(smem + kM + sw_chunk(tid, q4 * 4 + j)) =
                         make_uint4(packed[4 * j], packed[4 * j + 1], packed[4 * j + 2], packed[4 * j + 3]);
-                if (CARRY)
+                if constexpr (TURNS) {
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) {
+                        if (q4 & 1) m_lo[1][j] = rest[j];
+                        else m_lo[0][j] = rest[j];
+                    }
+                } else if (CARRY) {
 #pragma unroll
                     for (int j = 0; j < 4; ++j)
                         *reinterpret_cast<uint4*>(smem + kMlo + sw_chunk(tid, q4 * 4 + j)) =
                             make_uint4(rest[4 * j], rest[4 * j + 1], rest[4 * j + 2], rest[4 * j + 3]);
+                }
             };
+            if constexpr (TURNS) {
+#pragma unroll
+                for (int j = 0; j < 16; ++j) m_lo[0][j] = m_lo[1][j] = 0;
+            }
             for (int q4 = 2 * half; q4 < 2 * half + 2; ++q4) {
                 if (q4 > warp) {  // wholly above the diagonal for every row of this warp
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
                         *reinterpret_cast<uint4*>(smem + kM + sw_chunk(tid, q4 * 4 + j)) = make_uint4(0, 0, 0, 0);
-                        if (CARRY)
+                        if (CARRY && !TURNS)
                             *reinterpret_cast<uint4*>(smem + kMlo + sw_chunk(tid, q4 * 4 + j)) = make_uint4(0, 0, 0, 0);
                     }
                 } else if (q4 == warp) {
@@ -867,6 +912,14 @@ __global__ void __launch_bounds__(256, LEAN ? 2 : 1) m3_ssd_fwd_tc_kernel(const 
                 }
             }
             if (CARRY || c > 0) decay_state(ex2(dA[nv - 1] * kLog2e));
+            if constexpr (TURNS) {  // Y2 takes its rows' decay here and M V on top
+                const float e_t = ex2(dA[tid] * kLog2e);
+                float y2[32];
+                tmem_ld32(lane_addr + cY2 + half * 32, y2);
+#pragma unroll
+                for (int i = 0; i < 32; ++i) y2[i] *= e_t;
+                tmem_st32(lane_addr + cY2 + half * 32, y2);
+            }
         }
         fence_proxy_async();
         fence_before();
@@ -879,8 +932,8 @@ __global__ void __launch_bounds__(256, LEAN ? 2 : 1) m3_ssd_fwd_tc_kernel(const 
             const uint32_t idY = instr_desc(fmt, 0, 1, 64);
 #pragma unroll
             for (int k = 0; k < CS / 16; ++k)  // N = p, K = s
-                mma(tmem + cY1, desc_sw_k(sbase + kM, k), desc_sw_mn(sbase + tV, k), idY, k > 0);
-            if (CARRY) {
+                mma(tmem + (TURNS ? cY2 : cY1), desc_sw_k(sbase + kM, k), desc_sw_mn(sbase + tV, k), idY, TURNS || k > 0);
+            if (CARRY && !TURNS) {
 #pragma unroll
                 for (int k = 0; k < CS / 16; ++k)
                     mma(tmem + cY1, desc_sw_k(sbase + kMlo, k), desc_sw_mn(sbase + tV, k), idY, true);
@@ -888,16 +941,48 @@ __global__ void __launch_bounds__(256, LEAN ? 2 : 1) m3_ssd_fwd_tc_kernel(const 
             update_state(tK, CARRY || c > 0);
             commit(&bars[1]);
         }
-        ok = mbar_wait(&bars[1], j & 1, p.status) && ok;
+        ok = mbar_wait(&bars[1], (TURNS ? 3 * j : j) & 1, p.status) && ok;
         fence_after();
-        if (CARRY && c + 1 < c_hi) issue_carry_kv(c + 1);
+        if constexpr (TURNS) {
+            // the remainders' turns: M_lo V and K^T (w o V)_lo, then K^T (w o V)_rest
+#pragma unroll
+            for (int turn = 1; turn < 3; ++turn) {
+                weigh_v(dA, scl, nv, tV, turn);
+                if (turn == 1) {
+#pragma unroll
+                    for (int q = 0; q < 8; ++q)
+                        *reinterpret_cast<uint4*>(smem + kM + sw_chunk(tid, half * 8 + q)) =
+                            make_uint4(m_lo[q / 4][4 * (q % 4)], m_lo[q / 4][4 * (q % 4) + 1], m_lo[q / 4][4 * (q % 4) + 2],
+                                       m_lo[q / 4][4 * (q % 4) + 3]);
+                }
+                fence_proxy_async();
+                fence_before();
+                __syncthreads();
+                if (threadIdx.x == 0) {
+                    fence_after();
+                    const uint32_t idY = instr_desc(fmt, 0, 1, 64);
+                    if (turn == 1) {
+#pragma unroll
+                        for (int k = 0; k < CS / 16; ++k)
+                            mma(tmem + cY2, desc_sw_k(sbase + kM, k), desc_sw_mn(sbase + tV, k), idY, true);
+                    }
+                    update_state(tK, true);
+                    commit(&bars[1]);
+                }
+                ok = mbar_wait(&bars[1], (3 * j + turn) & 1, p.status) && ok;
+                fence_after();
+            }
+        }
+        if (CARRY && !LEAN && c + 1 < c_hi) issue_carry_kv(c + 1);
         if (LEAN && c + 1 < c_hi) issue_tiles(c + 1, j + 1);
         // ---- 5. epilogue: y row; 16-bit copy of the new state for the next chunk ----
         {
             const float e_t = ex2(dA[tid] * kLog2e);
             const int q2 = half;
             float y1[32], y2[32];
-            if (CARRY || c > 0) {
+            if (TURNS) {
+                tmem_ld32(lane_addr + cY2 + q2 * 32, y1);
+            } else if (CARRY || c > 0) {
                 tmem_ld32x2(lane_addr + cY1 + q2 * 32, y1, lane_addr + cY2 + q2 * 32, y2);
 #pragma unroll
                 for (int i = 0; i < 32; ++i) y1[i] = fmaf(e_t, y2[i], y1[i]);
@@ -993,6 +1078,13 @@ int m3_cluster_ranks(int heads, int nchunks, double full, double pair, double ma
 // and 362.  So one wave of one CTA per SM stays, and three nearly full ones.
 static bool m3_two_per_sm(int pairs) { return pairs > 148 && (pairs <= 360 || pairs > 3 * 148); }
 
+// The same for carried windows, in us: 152 pairs x 256 steps 49 and 42, 256 62 and 47, 512 121 and 90; x 1024 steps 123
+// and 108, 126 and 110, 247 and 214; in the third wave of one CTA per SM, 384 pairs, 91 and 86 x 256 but 186 and 202 x
+// 1024, so there only up to two chunks.  256 pairs x 21 steps 33 and 26.
+static bool m3_two_carried_per_sm(int pairs, int nchunks) {
+    return pairs > 148 && (pairs <= 2 * 148 || pairs > 3 * 148 || nchunks <= 2);
+}
+
 cudaError_t launch_cluster(const void* fn, dim3 grid, dim3 block, size_t smem, cudaStream_t st, int ranks, void** args) {
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
@@ -1021,7 +1113,8 @@ int m3_configure(Ctx* c) {
                           reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, true, true, false>)};
     for (const void* fn : fns)
         MB200_CUDA_CHECK(c, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::kSmem));
-    const void* lean_fns[2] = {reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, false, false, true>),
+    const void* lean_fns[3] = {reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, true, false, true>),
+                               reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, false, false, true>),
                                reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__half, false, false, false, true>)};
     for (const void* fn : lean_fns) {
         MB200_CUDA_CHECK(c, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::lean::kSmem));
@@ -1139,6 +1232,8 @@ extern "C" MAMBA_B200_API int mamba_b200_m3_ssd_fwd(void* handle, void* stream,
                                 : reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__half, false, false, true, false>);
             void* args[1] = {&p};
             MB200_CUDA_CHECK(c, launch_cluster(fn, dim3(a.nh * ranks, a.B), dim3(256), tc::kSmem, st, ranks, args));
+        } else if (a.carry_in && m3_two_carried_per_sm(a.B * a.nh, nchunks)) {
+            tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, true, false, true><<<grid, 256, tc::lean::kSmem, st>>>(p);
         } else if (!gen && !a.carry_in && m3_two_per_sm(a.B * a.nh)) {
             if (bf) tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, false, false, true><<<grid, 256, tc::lean::kSmem, st>>>(p);
             else tc::m3_ssd_fwd_tc_kernel<__half, false, false, false, true><<<grid, 256, tc::lean::kSmem, st>>>(p);

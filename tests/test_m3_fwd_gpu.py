@@ -301,8 +301,10 @@ def test_an_infinite_input_stays_infinite_beside_the_states_that_are_not_there(c
 
 
 # More (sample, head) pairs than SMs run two CTAs per SM, fewer one: the same arithmetic in the same order, so a batch
-# of 150 or more pairs must give, bit for bit, what its first and its last samples give in calls of fewer than 148.
-@pytest.mark.parametrize("dt", ["bf16", "f16"])
+# of 150 or more pairs must give, bit for bit, what its first and its last samples give in calls of fewer than 148.  Of a
+# carried window y's sums are in another order there: f32 sums of up to 500 terms differ by less than 1e-5 of the
+# largest value, and then by one rounding to the storage type at most.
+@pytest.mark.parametrize("dt", ["bf16", "f16", "carried"])
 @pytest.mark.parametrize("case", [(10, 1, 16, 64, 128), (10, 127, 15, 32, 64), (10, 128, 16, 8, 16), (10, 129, 15, 64, 128),
                                   (10, 300, 16, 64, 72), (10, 513, 16, 56, 128)], ids=lambda c: "B%dT%dnh%dhd%dN%d" % c)
 def test_two_ctas_per_sm_give_the_same_bits(cuda_dev, case, dt):
@@ -310,23 +312,29 @@ def test_two_ctas_per_sm_give_the_same_bits(cuda_dev, case, dt):
 
     import mamba_rs_b200 as mb
     B, T, nh, hd, N = case
-    td = {"bf16": torch.bfloat16, "f16": torch.float16}[dt]
+    carried = dt == "carried"
+    td = torch.float16 if dt == "f16" else torch.bfloat16
     g = torch.Generator(device=cuda_dev).manual_seed(T)
     rn = lambda *s: torch.randn(*s, device=cuda_dev, generator=g)  # noqa: E731
     x, K, Q = rn(B, T, nh * hd).to(td), (0.3 * rn(B, T, nh, N)).to(td), (0.3 * rn(B, T, nh, N)).to(td)
     dt_, trap = torch.nn.functional.softplus(rn(B, T, nh) - 2), torch.sigmoid(rn(B, T, nh))
     adt, Dh = -dt_ * torch.rand(nh, device=cuda_dev, generator=g) * 4, rn(nh)
+    h0, k0, v0 = rn(B, nh, hd, N), 0.3 * rn(B, nh, N), rn(B, nh, hd)
 
     def call(lo, hi):
-        st = dict(ssm_state=torch.full((hi - lo, nh, hd, N), float("nan"), device=cuda_dev),
-                  k_state=torch.full((hi - lo, nh, N), float("nan"), device=cuda_dev),
-                  v_state=torch.full((hi - lo, nh, hd), float("nan"), device=cuda_dev))
         c = lambda t: t[lo:hi].contiguous()  # noqa: E731
-        y = mb.m3_ssd_fwd(c(x), c(K), c(Q), c(dt_), c(trap), c(adt), Dh, **st)
+        new = lambda t: t[lo:hi].clone() if carried else torch.full_like(t[lo:hi], float("nan"))  # noqa: E731
+        st = dict(ssm_state=new(h0), k_state=new(k0), v_state=new(v0))
+        y = mb.m3_ssd_fwd(c(x), c(K), c(Q), c(dt_), c(trap), c(adt), Dh, carry_in=carried, **st)
         return [y, st["ssm_state"], st["k_state"], st["v_state"]]
 
     whole = call(0, B)
     for lo, hi in ((0, B - 1), (1, B)):
-        for a, b in zip(whole, call(lo, hi)):
-            assert torch.isfinite(a.float()).all() and torch.equal(a[lo:hi], b)
+        for i, (a, b) in enumerate(zip(whole, call(lo, hi))):
+            assert torch.isfinite(a.float()).all()
+            if carried and i == 0:
+                a, b = a[lo:hi].float(), b.float()
+                assert bool(((a - b).abs() <= b.abs() / 128 + 1e-5 * b.abs().max()).all())
+            else:
+                assert torch.equal(a[lo:hi], b)
     mb.ffi.default_handle(0).check_status()
