@@ -578,7 +578,7 @@ def ncu_traffic_bytes():
     p = os.path.join(ROOT, "profiles", "sscan_fwd_traffic.txt")
     try:
         kv = dict(line.strip().split("=", 1) for line in open(p) if "=" in line)
-        src = open(os.path.join(ROOT, "mamba_rs_b200", "csrc", "m1_fwd_kernel.cuh"), "rb").read()
+        src = open(os.path.join(ROOT, "mamba_rs_b200", "csrc", "m1_fwd16_kernel.cuh"), "rb").read()
         if kv.get("kernel_source_sha1") != hashlib.sha1(src).hexdigest():
             return None
         return int(kv["dram_bytes_per_launch_full_workload"])
@@ -806,7 +806,7 @@ def main():
                              "host's root complexes, which the GPUs of one box share"}),
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": ncu_traffic_bytes(), "peak_source": peak_src,
-                         "kernel": "sscan_fwd_kernel", "kernel_ms": kern_ms,
+                         "kernel": "sscan_fwd16_kernel", "kernel_ms": kern_ms,
                          "algorithmic_bytes": by},
         }
         if extra is not None:
