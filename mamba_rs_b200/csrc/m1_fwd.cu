@@ -29,14 +29,14 @@ static long long fwd_ctas(int B, int D, int N) {  // of four consumer warps, one
     const int cw = lpc >= 16 ? 8 : 4, dt = cw * (32 / lpc);
     return static_cast<long long>(B) * ((D + dt - 1) / dt) * (cw / 4);
 }
-static int fwd_segments(int B, int T, int D, int N, double* us) {
+static int fwd_segments(int B, int T, int D, int N, bool lent, double* us) {
     static const double kCut[2 * kFwdMaxPerSm + 2] = {0.175, 0.180, 0.191, 0.221, 0.239, 0.275, 0.312, 0.395, 0.429, 0.460,
                                                       0.508, 0.536, 0.568, 0.619, 0.669, 0.712, 0.753, 0.806, 0.860, 0.860};
     const long long ctas = fwd_ctas(B, D, N);
     // whole: three CTAs share an SM, 0.165 us a step together
     const long long rounds = ctas / (3 * 148), rest = ctas % (3 * 148);
     *us = rounds * (3.2 + 0.165 * T) + (rest ? 3.2 + T * (rest <= 148 ? 0.1155 : rest <= 296 ? 0.137 : 0.165) : 0.0);
-    if (ctas > kFwdMaxCtas || T < 192) return 1;
+    if (!lent || ctas > kFwdMaxCtas || T < 192) return 1;
     const int blocks = (T + 31) / 32;
     auto cut = [&](int s) {
         const int per = (blocks + s - 1) / s;
@@ -359,17 +359,20 @@ static int launch_fwd(Ctx* c, cudaStream_t stream, const mamba_b200_sscan_fwd_ar
 
     const bool lent = a.workspace && a.workspace_bytes > 0;
     double us = 0.0;
-    int segs = fwd_segments(a.B, a.T, a.D, a.N, &us);
-    if (!lent) segs = 1;
+    int segs = fwd_segments(a.B, a.T, a.D, a.N, lent, &us);
+    {
+        size_t o1, o2, o3;
+        while (segs > 1 && fwd_ws_bytes(a.B, a.D, a.N, segs, &o1, &o2, &o3) > static_cast<size_t>(a.workspace_bytes))
+            segs /= 2;
+    }
+    const bool ws_aligned = reinterpret_cast<uintptr_t>(a.workspace) % 256 == 0;
+    if (segs > 1 && !ws_aligned) return fail(c, MAMBA_B200_ERR_ARG, "sscan_fwd: workspace must be 256-byte aligned");
     // d_state 9 .. 16 without the conv, channels that TMA can bring: by warp roles where that is estimated to be faster
     if (v->ns * v->lpc == 16 && !a.conv_w && (m & kTmaX) && (m & kTmaDl) && (!a.z_mode || (m & kTmaZ))) {
         const Fwd16Table& t16 = fwd16_tables().t[a.dtype];
-        const Fwd16Plan plan = fwd16_plan(t16, a.dtype == MAMBA_B200_F32, a.B, a.T, a.D, a.N, us, lent ? a.workspace_bytes : 0);
-        if (plan.kind) {
-            if (plan.segs > 1 && reinterpret_cast<uintptr_t>(a.workspace) % 256)
-                return fail(c, MAMBA_B200_ERR_ARG, "sscan_fwd: workspace must be 256-byte aligned");
-            return launch_fwd16(c, stream, a, p, t16, plan);
-        }
+        const Fwd16Plan plan = fwd16_plan(t16, a.dtype == MAMBA_B200_F32, a.B, a.T, a.D, a.N, us,
+                                          lent && ws_aligned ? a.workspace_bytes : 0);
+        if (plan.kind) return launch_fwd16(c, stream, a, p, t16, plan);
     }
 
     const int flags = (a.delta_softplus ? 1 : 0) | (a.z_mode ? 2 : 0) | (a.conv_w ? 4 : 0);
@@ -387,13 +390,6 @@ static int launch_fwd(Ctx* c, cudaStream_t stream, const mamba_b200_sscan_fwd_ar
     // entering states, and the second launch runs every segment in full.
     const int tiles = (a.D + v->dt - 1) / v->dt;
     const int nchunks = (a.T + v->tc - 1) / v->tc;
-    if (segs > 1) {
-        size_t o1, o2, o3;
-        while (segs > 1 && fwd_ws_bytes(a.B, a.D, a.N, segs, &o1, &o2, &o3) > static_cast<size_t>(a.workspace_bytes))
-            segs /= 2;
-        if (segs > 1 && reinterpret_cast<uintptr_t>(a.workspace) % 256)
-            return fail(c, MAMBA_B200_ERR_ARG, "sscan_fwd: workspace must be 256-byte aligned");
-    }
     dim3 grid(tiles, a.B, 1);
     if (segs > 1) {
         p.seg_chunks = (nchunks + segs - 1) / segs;
