@@ -307,16 +307,16 @@ __device__ __forceinline__ void conv_load_taps(const ConvParams& p, int d, float
     }
 }
 
-template <typename Tact, int VEC>
-__global__ void __launch_bounds__(32 * kConvWarps) conv1d_fwd_rows_kernel(const ConvParams p) {
-    constexpr int KV = kConvKV, R = kConvRT + KV - 1;
+template <typename Tact, int VEC, int RT>
+__global__ void __launch_bounds__(32 * kConvTT / RT) conv1d_fwd_rows_kernel(const ConvParams p) {
+    constexpr int KV = kConvKV, R = RT + KV - 1;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int d = (blockIdx.x * 32 + lane) * VEC, t0 = blockIdx.y * kConvTT + warp * kConvRT, b = blockIdx.z;
+    const int d = (blockIdx.x * 32 + lane) * VEC, t0 = blockIdx.y * kConvTT + warp * RT, b = blockIdx.z;
     if (d >= p.D || t0 >= p.T) return;
     const int K = p.K;
     const Tact* xb = static_cast<const Tact*>(p.x) + static_cast<long long>(b) * p.T * p.ld_x + d;
     Tact* ub = static_cast<Tact*>(p.u) + (static_cast<long long>(b) * p.T + t0) * p.ld_u + d;
-    RawVec<Tact, VEC> x[R];  // rows t0 - 3 .. t0 + 7
+    RawVec<Tact, VEC> x[R];  // rows t0 - 3 .. t0 + RT - 1
 #pragma unroll
     for (int r = 0; r < R; ++r) {
         const int t = t0 - (KV - 1) + r;
@@ -343,7 +343,7 @@ __global__ void __launch_bounds__(32 * kConvWarps) conv1d_fwd_rows_kernel(const 
             if (p.T - KV + k >= 0) last[k].load(xb + static_cast<long long>(p.T - KV + k) * p.ld_x);
     }
 #pragma unroll
-    for (int i = 0; i < kConvRT; ++i) {
+    for (int i = 0; i < RT; ++i) {
         float o[VEC];
 #pragma unroll
         for (int v = 0; v < VEC; ++v) {
@@ -614,11 +614,22 @@ extern "C" MAMBA_B200_API int mamba_b200_conv1d_fwd(void* handle, void* stream,
     const int v = a.dtype == MAMBA_B200_F32 && vec(2) && (a.T <= kConvRT || !vec(4)) ? 2 : vec(4) ? 4 : 0;
     if (v) {
         dim3 vgrid((a.D / v + 31) / 32, chunks, a.B);
-        const int threads = 32 * std::min(kConvWarps, (a.T + kConvRT - 1) / kConvRT);
-        if (v == 2) conv1d_fwd_rows_kernel<float, 2><<<vgrid, threads, 0, st>>>(p);
-        else if (a.dtype == MAMBA_B200_F32) conv1d_fwd_rows_kernel<float, 4><<<vgrid, threads, 0, st>>>(p);
-        else if (a.dtype == MAMBA_B200_F16) conv1d_fwd_rows_kernel<__half, 4><<<vgrid, threads, 0, st>>>(p);
-        else conv1d_fwd_rows_kernel<__nv_bfloat16, 4><<<vgrid, threads, 0, st>>>(p);
+        // Sixteen steps a warp where that leaves 16 warps for every SM: its taps (64 bytes a lane) and its three rows of
+        // halo are then read for twice as many outputs.  In us, 8 and 16 steps: 8 x 2048 x 1536 bf16 24.4 and 21.8, f32
+        // 35.4 and 32.6, 2 x 8192 x 5120 71.7 and 61.8, 2 x 2048 x 2048 10.6 and 10.1; 1 x 1021 x 1536 4.2 and 4.4 (and with
+        // 32 steps, in the registers of a third of the warps, 26.5 at the first).
+        const bool tall = v == 4 && static_cast<long long>(a.B) * ((a.T + 15) / 16) * vgrid.x >= 16 * 148;
+        const int rt = tall ? 16 : kConvRT, threads = 32 * std::min(kConvTT / rt, (a.T + rt - 1) / rt);
+#define MB200_CONV(T)                                                              \
+    do {                                                                           \
+        if (tall) conv1d_fwd_rows_kernel<T, 4, 16><<<vgrid, threads, 0, st>>>(p);  \
+        else conv1d_fwd_rows_kernel<T, 4, kConvRT><<<vgrid, threads, 0, st>>>(p);  \
+    } while (0)
+        if (v == 2) conv1d_fwd_rows_kernel<float, 2, kConvRT><<<vgrid, threads, 0, st>>>(p);
+        else if (a.dtype == MAMBA_B200_F32) MB200_CONV(float);
+        else if (a.dtype == MAMBA_B200_F16) MB200_CONV(__half);
+        else MB200_CONV(__nv_bfloat16);
+#undef MB200_CONV
     } else if (a.dtype == MAMBA_B200_F32) {
         conv1d_fwd_kernel<float><<<grid, 128, 0, st>>>(p);
         if (a.conv_state) conv1d_state_kernel<float><<<sb, 128, 0, st>>>(p);

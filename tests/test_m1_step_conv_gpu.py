@@ -173,3 +173,23 @@ def test_f32_channel_counts_that_are_even_but_no_multiple_of_four(cuda_dev, T, K
         left = torch.cat([st.transpose(1, 2), x], 1)[:, -K:].transpose(1, 2)
         u = mb.conv1d_fwd(x, w, b, st)
         assert float((u.double() - want).abs().max()) <= 1e-5 and torch.equal(st, left)
+
+
+# Long batches give a warp sixteen steps, a sample of them alone eight: the same arithmetic for every output, so the same
+# bits.  Lengths around both counts, a width that is no multiple of a warp's 128 channels, d_conv 4 and 2.
+@pytest.mark.parametrize("dt", ["f32", "bf16", "f16"])
+@pytest.mark.parametrize("case", [(8, 1009, 644, 4), (8, 1024, 640, 2), (150, 17, 1024, 4)], ids=lambda c: "B%dT%dD%dK%d" % c)
+def test_conv_sixteen_steps_a_warp_give_the_bits_of_eight(cuda_dev, case, dt):
+    import torch
+
+    import mamba_rs_b200 as mb
+    B, T, D, K = case
+    td = {"f32": torch.float32, "bf16": torch.bfloat16, "f16": torch.float16}[dt]
+    g = torch.Generator(device=cuda_dev).manual_seed(T)
+    rn = lambda *s: torch.randn(*s, device=cuda_dev, generator=g)  # noqa: E731
+    x, w, b, st = rn(B, T, D).to(td), rn(D, K), rn(D), rn(B, D, K)
+    st0 = st.clone()
+    u = mb.conv1d_fwd(x, w, b, conv_state=st)
+    for i in (0, B // 2, B - 1):
+        si = st0[i:i + 1].clone()
+        assert torch.equal(mb.conv1d_fwd(x[i:i + 1], w, b, conv_state=si), u[i:i + 1]) and torch.equal(si, st[i:i + 1])
