@@ -115,6 +115,14 @@ MAMBA_B200_API long long mamba_b200_sscan_fwd_workspace_bytes(int B, int T, int 
 MAMBA_B200_API int mamba_b200_sscan_fwd(void* handle, void* stream, const mamba_b200_sscan_fwd_args* args);
 
 /*
+ * How mamba_b200_sscan_fwd lays such a call out, without a device: no fused conv, rows of x, delta and z that TMA can
+ * describe (16-byte aligned), an aligned workspace of workspace_bytes (0: none).  out[0]: states a lane of the kernel by
+ * warp roles (4 or 8), or 0 for the general kernel; out[1]: its consumer warps; out[2]: time segments (1: one piece).
+ */
+MAMBA_B200_API int mamba_b200_sscan_fwd_layout(int dtype, int B, int T, int D, int N, int z_mode, long long workspace_bytes,
+                                               int* out);
+
+/*
  * Reference-compatible unfused entry point: same argument list and meaning as
  * ssm_parallel_scan_fwd_nosave_{f32,bf16,f16}
  * (kernels/mamba_ssm_parallel.cu:544-553, :969-980; launch

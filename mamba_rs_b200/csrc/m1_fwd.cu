@@ -29,14 +29,32 @@ static long long fwd_ctas(int B, int D, int N) {  // of four consumer warps, one
     const int cw = lpc >= 16 ? 8 : 4, dt = cw * (32 / lpc);
     return static_cast<long long>(B) * ((D + dt - 1) / dt) * (cw / 4);
 }
-static int fwd_segments(int B, int T, int D, int N, bool lent, double* us) {
+static size_t fwd_ws_bytes(int B, int D, int N, int segs, size_t* o_sum, size_t* o_h0, size_t* o_c0) {
+    auto al = [](size_t v) { return (v + 255) & ~size_t(255); };
+    size_t off = al(sizeof(float) * static_cast<size_t>(B) * segs * D * N);
+    *o_sum = off;
+    off += al(sizeof(float) * static_cast<size_t>(B) * segs * D);
+    *o_h0 = off;
+    off += al(sizeof(float) * static_cast<size_t>(B) * D * N);
+    *o_c0 = off;
+    off += al(sizeof(float) * static_cast<size_t>(B) * D * kKMax);
+    return off;
+}
+static bool fwd_ws_holds(long long bytes, int B, int D, int N, int segs) {
+    size_t o1, o2, o3;
+    return bytes > 0 && fwd_ws_bytes(B, D, N, segs, &o1, &o2, &o3) <= static_cast<size_t>(bytes);
+}
+// `lent`: bytes of the workspace.  Where they do not hold the count that was wanted, *us is what the count that they
+// do hold takes (1 x 1021 x 1536 with 4 KB is walked whole, 121 us, and not in the 31 of sixteen segments).
+static int fwd_segments(int B, int T, int D, int N, long long lent, double* us) {
     static const double kCut[2 * kFwdMaxPerSm + 2] = {0.175, 0.180, 0.191, 0.221, 0.239, 0.275, 0.312, 0.395, 0.429, 0.460,
                                                       0.508, 0.536, 0.568, 0.619, 0.669, 0.712, 0.753, 0.806, 0.860, 0.860};
     const long long ctas = fwd_ctas(B, D, N);
     // whole: three CTAs share an SM, 0.165 us a step together
     const long long rounds = ctas / (3 * 148), rest = ctas % (3 * 148);
-    *us = rounds * (3.2 + 0.165 * T) + (rest ? 3.2 + T * (rest <= 148 ? 0.1155 : rest <= 296 ? 0.137 : 0.165) : 0.0);
-    if (!lent || ctas > kFwdMaxCtas || T < 192) return 1;
+    const double whole = rounds * (3.2 + 0.165 * T) + (rest ? 3.2 + T * (rest <= 148 ? 0.1155 : rest <= 296 ? 0.137 : 0.165) : 0.0);
+    *us = whole;
+    if (lent <= 0 || ctas > kFwdMaxCtas || T < 192) return 1;
     const int blocks = (T + 31) / 32;
     auto cut = [&](int s) {
         const int per = (blocks + s - 1) / s;
@@ -44,18 +62,19 @@ static int fwd_segments(int B, int T, int D, int N, bool lent, double* us) {
         const double* at = kCut + std::min(static_cast<int>(x), 2 * kFwdMaxPerSm);
         return 8 + (32 * per + 16) * (x < 2 * kFwdMaxPerSm ? at[0] + f * (at[1] - at[0]) : at[0] * x / (2 * kFwdMaxPerSm));
     };
+    int best = 1;
     if (T >= 1536) {
         const double w = ctas / 148.0;
-        const int s = w >= 0.7 ? 8 : std::min({std::max(16, static_cast<int>(2.6 / w) + 1), blocks, kMaxSegments});
-        *us = cut(s);
-        return s;
+        best = w >= 0.7 ? 8 : std::min({std::max(16, static_cast<int>(2.6 / w) + 1), blocks, kMaxSegments});
+    } else {
+        for (int s = 2; s <= kMaxSegments && s <= blocks && ctas * s <= kFwdMaxPerSm * 148; ++s)
+            if (cut(s) < *us) {
+                *us = cut(s);
+                best = s;
+            }
     }
-    int best = 1;
-    for (int s = 2; s <= kMaxSegments && s <= blocks && ctas * s <= kFwdMaxPerSm * 148; ++s)
-        if (cut(s) < *us) {
-            *us = cut(s);
-            best = s;
-        }
+    while (best > 1 && !fwd_ws_holds(lent, B, D, N, best)) best /= 2;
+    *us = best > 1 ? cut(best) : whole;
     return best;
 }
 
@@ -94,6 +113,14 @@ static const FwdTable& fwd_table() {
         return t;
     }();
     return table;
+}
+
+// The smallest one that holds N states.
+static const FwdVariant* fwd_variant(int dtype, int N) {
+    const FwdTable& tab = fwd_table();
+    for (int i = 0; i < tab.n[dtype]; ++i)
+        if (tab.v[dtype][i].ns * tab.v[dtype][i].lpc >= N) return &tab.v[dtype][i];
+    return nullptr;
 }
 
 // Built once, like the other table.
@@ -164,18 +191,6 @@ __global__ void sscan_seg_carry_kernel(float* seg_states, const float* seg_sumdl
     }
 }
 
-static size_t fwd_ws_bytes(int B, int D, int N, int segs, size_t* o_sum, size_t* o_h0, size_t* o_c0) {
-    auto al = [](size_t v) { return (v + 255) & ~size_t(255); };
-    size_t off = al(sizeof(float) * static_cast<size_t>(B) * segs * D * N);
-    *o_sum = off;
-    off += al(sizeof(float) * static_cast<size_t>(B) * segs * D);
-    *o_h0 = off;
-    off += al(sizeof(float) * static_cast<size_t>(B) * D * N);
-    *o_c0 = off;
-    off += al(sizeof(float) * static_cast<size_t>(B) * D * kKMax);
-    return off;
-}
-
 // The layout with the least estimate, if that is at most 0.95 (eight states a lane: 0.935, cut: 0.9) of what
 // sscan_fwd_kernel is estimated to take.  Against that kernel alone, 160 shapes of 64 to 8192 steps, both kinds of rates:
 // 14 % less time on average, no shape more than 2 % more.  8 x 2048 x 1536 with general rates 284 -> 196 us, 2 x 8192 x
@@ -199,8 +214,7 @@ static Fwd16Plan fwd16_plan(const Fwd16Table& t, bool f32, int B, int T, int D, 
         if (T < 192) continue;
         for (int s = 2; ctas * s <= 148 && s <= 32; ++s) {
             const int per = (chunks + s - 1) / s, segs = (chunks + per - 1) / per;
-            size_t o1, o2, o3;
-            if (segs != s || per * steps < 32 || fwd_ws_bytes(B, D, N, s, &o1, &o2, &o3) > static_cast<size_t>(workspace_bytes)) continue;
+            if (segs != s || per * steps < 32 || !fwd_ws_holds(workspace_bytes, B, D, N, s)) continue;
             c = scale * (k.c0 + k.c1 * per * steps) * (0.95 / 0.9);
             if (c < us) {
                 us = c;
@@ -321,11 +335,7 @@ static int launch_fwd(Ctx* c, cudaStream_t stream, const mamba_b200_sscan_fwd_ar
                                           (static_cast<size_t>(a.B) * a.T - 1) * a.ld_u * es + a.D * es))))
         return fail(c, MAMBA_B200_ERR_ARG, "sscan_fwd: with the conv fused, y and u_out must not overlap x");
 
-    const FwdTable& tab = fwd_table();
-    const FwdVariant* vs = tab.v[a.dtype];
-    const FwdVariant* v = nullptr;
-    for (int i = 0; i < tab.n[a.dtype]; ++i)
-        if (vs[i].ns * vs[i].lpc >= a.N) { v = &vs[i]; break; }
+    const FwdVariant* v = fwd_variant(a.dtype, a.N);
     if (!v) return fail(c, MAMBA_B200_ERR_SHAPE, "sscan_fwd: no variant for d_state %d", a.N);
     if (a.chunk_states && (a.save_stride <= 0 || a.save_stride % 32 != 0 || a.save_stride > 64))
         return fail(c, MAMBA_B200_ERR_ARG, "sscan_fwd: save_stride %d must be 32 or 64", a.save_stride);
@@ -357,21 +367,16 @@ static int launch_fwd(Ctx* c, cudaStream_t stream, const mamba_b200_sscan_fwd_ar
     if (make_tmap_3d(c, &p.tm_c, a.dtype, a.Cm, a.ld_bc, a.N, a.T, a.B, a.N, v->tc)) m |= kTmaC;
     p.tma_mask = m;
 
-    const bool lent = a.workspace && a.workspace_bytes > 0;
+    const long long lent = a.workspace ? a.workspace_bytes : 0;
     double us = 0.0;
     int segs = fwd_segments(a.B, a.T, a.D, a.N, lent, &us);
-    {
-        size_t o1, o2, o3;
-        while (segs > 1 && fwd_ws_bytes(a.B, a.D, a.N, segs, &o1, &o2, &o3) > static_cast<size_t>(a.workspace_bytes))
-            segs /= 2;
-    }
     const bool ws_aligned = reinterpret_cast<uintptr_t>(a.workspace) % 256 == 0;
     if (segs > 1 && !ws_aligned) return fail(c, MAMBA_B200_ERR_ARG, "sscan_fwd: workspace must be 256-byte aligned");
     // d_state 9 .. 16 without the conv, channels that TMA can bring: by warp roles where that is estimated to be faster
     if (v->ns * v->lpc == 16 && !a.conv_w && (m & kTmaX) && (m & kTmaDl) && (!a.z_mode || (m & kTmaZ))) {
         const Fwd16Table& t16 = fwd16_tables().t[a.dtype];
         const Fwd16Plan plan = fwd16_plan(t16, a.dtype == MAMBA_B200_F32, a.B, a.T, a.D, a.N, us,
-                                          lent && ws_aligned ? a.workspace_bytes : 0);
+                                          ws_aligned ? lent : 0);
         if (plan.kind) return launch_fwd16(c, stream, a, p, t16, plan);
     }
 
@@ -432,6 +437,26 @@ extern "C" MAMBA_B200_API long long mamba_b200_sscan_fwd_workspace_bytes(int B, 
         most = std::max(most, fwd_ws_bytes(b, D, N, static_cast<int>(segs), &o1, &o2, &o3));
     }
     return static_cast<long long>(most);
+}
+
+extern "C" MAMBA_B200_API int mamba_b200_sscan_fwd_layout(int dtype, int B, int T, int D, int N, int z_mode, long long workspace_bytes,
+                                                            int* out) {
+    (void)z_mode;
+    if (!out || !dtype_ok(dtype) || B <= 0 || T <= 0 || D <= 0 || N <= 0 || N > 256) return MAMBA_B200_ERR_ARG;
+    const FwdVariant* v = fwd_variant(dtype, N);
+    double us = 0.0;
+    int segs = fwd_segments(B, T, D, N, workspace_bytes, &us);
+    Fwd16Plan plan;
+    if (v->ns * v->lpc == 16)
+        plan = fwd16_plan(fwd16_tables().t[dtype], dtype == MAMBA_B200_F32, B, T, D, N, us, workspace_bytes);
+    if (!plan.kind) {
+        const int chunks = (T + v->tc - 1) / v->tc, per = (chunks + segs - 1) / segs;
+        segs = (chunks + per - 1) / per;
+    }
+    out[0] = plan.kind ? plan.kind->ns : 0;
+    out[1] = plan.kind ? plan.kind->workers : 0;
+    out[2] = plan.kind ? plan.segs : segs;
+    return MAMBA_B200_OK;
 }
 
 extern "C" MAMBA_B200_API int mamba_b200_sscan_fwd(void* handle, void* stream, const mamba_b200_sscan_fwd_args* args) {

@@ -153,6 +153,7 @@ def lib() -> C.CDLL:
         bind("mamba_b200_selftest_wait_timeout", [vp, vp, C.c_int])
         bind("mamba_b200_sscan_fwd", [vp, vp, C.POINTER(SscanFwdArgs)])
         bind("mamba_b200_sscan_fwd_workspace_bytes", [C.c_int] * 4, C.c_longlong)
+        bind("mamba_b200_sscan_fwd_layout", [C.c_int] * 6 + [C.c_longlong, C.POINTER(C.c_int)])
         bind("mamba_b200_sscan_bwd", [vp, vp, C.POINTER(SscanBwdArgs)])
         bind("mamba_b200_ssm_scan_fwd_nosave", [vp, vp, C.c_int] + [vp] * 8 + [C.c_int] * 4)
         bind("mamba_b200_ssm_scan_fwd_save", [vp, vp, C.c_int] + [vp] * 9 + [C.c_int] * 4)
