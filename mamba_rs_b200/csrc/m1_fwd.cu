@@ -12,7 +12,7 @@ constexpr int kMaxSegments = 64;
 
 // Time segments of sscan_fwd_kernel when it was lent a workspace (see launch_fwd): the count with the least estimated
 // time, which it returns in *us.  In one piece a step takes 0.1155 us with one CTA per SM and 0.137 with two; both passes of a cut take
-// kCut[2 x] with x CTAs per SM on average (d_state 16, bf16; f32 takes 1.08 times as long throughout), a piece
+// kCut[2 x] with x CTAs per SM on average (d_state 16; f32 takes 1.03 times as long), a piece
 // costs its steps and 16 more for its pipeline to fill, and the call 8 us with two more launches.  Beyond 1.15 CTAs
 // per SM one piece is as fast, and under 192 steps (1 x 128 x 2560 whole 17.6, in four 18.9).  Fitted to 300
 // measured shapes of 64 to 4096 steps: half of the estimates are within 5 %, and the counts chosen take 0.8 % longer
@@ -44,8 +44,8 @@ static bool fwd_ws_holds(long long bytes, int B, int D, int N, int segs) {
     size_t o1, o2, o3;
     return bytes > 0 && fwd_ws_bytes(B, D, N, segs, &o1, &o2, &o3) <= static_cast<size_t>(bytes);
 }
-// `lent`: bytes of the workspace.  Where they do not hold the count that was wanted, *us is what the count that they
-// do hold takes (1 x 1021 x 1536 with 4 KB is walked whole, 121 us, and not in the 31 of sixteen segments).
+// `lent`: bytes of the workspace.  Where they do not hold the count that was wanted, it is one that they do hold, and
+// *us what that takes (1 x 1021 x 1536 with 4 KB is walked whole, and not in the 31 us of sixteen segments); whole: 0.
 static int fwd_segments(int B, int T, int D, int N, long long lent, double* us) {
     static const double kCut[2 * kFwdMaxPerSm + 2] = {0.175, 0.180, 0.191, 0.221, 0.239, 0.275, 0.312, 0.395, 0.429, 0.460,
                                                       0.508, 0.536, 0.568, 0.619, 0.669, 0.712, 0.753, 0.806, 0.860, 0.860};
@@ -53,7 +53,7 @@ static int fwd_segments(int B, int T, int D, int N, long long lent, double* us) 
     // whole: three CTAs share an SM, 0.165 us a step together
     const long long rounds = ctas / (3 * 148), rest = ctas % (3 * 148);
     const double whole = rounds * (3.2 + 0.165 * T) + (rest ? 3.2 + T * (rest <= 148 ? 0.1155 : rest <= 296 ? 0.137 : 0.165) : 0.0);
-    *us = whole;
+    *us = 0.0;
     if (lent <= 0 || ctas > kFwdMaxCtas || T < 192) return 1;
     const int blocks = (T + 31) / 32;
     auto cut = [&](int s) {
@@ -63,35 +63,56 @@ static int fwd_segments(int B, int T, int D, int N, long long lent, double* us) 
         return 8 + (32 * per + 16) * (x < 2 * kFwdMaxPerSm ? at[0] + f * (at[1] - at[0]) : at[0] * x / (2 * kFwdMaxPerSm));
     };
     int best = 1;
+    double least = whole;
     if (T >= 1536) {
         const double w = ctas / 148.0;
         best = w >= 0.7 ? 8 : std::min({std::max(16, static_cast<int>(2.6 / w) + 1), blocks, kMaxSegments});
     } else {
         for (int s = 2; s <= kMaxSegments && s <= blocks && ctas * s <= kFwdMaxPerSm * 148; ++s)
-            if (cut(s) < *us) {
-                *us = cut(s);
+            if (cut(s) < least) {
+                least = cut(s);
                 best = s;
             }
     }
     while (best > 1 && !fwd_ws_holds(lent, B, D, N, best)) best /= 2;
-    *us = best > 1 ? cut(best) : whole;
+    if (best > 1) *us = cut(best);
     return best;
 }
+// What sscan_fwd_kernel (d_state 9 .. 16) takes in one piece, in us: kWhole[f32][plain][0] and a step by CTAs per SM,
+// three, without a gate four of f32; the CTAs past full waves run beside the end of the last one.  plain: rows of B and C
+// that no tensor map describes, brought by one warp's loads.  Means of rates in progression and general ones, which lie
+// 12 % below and above them in 16-bit storage, 6 % in f32.
+static double fwd_whole_us(bool f32, bool gated, bool plain, int T, long long ctas) {
+    static const double kWhole[2][2][5] = {{{4.4, 0.102, 0.123, 0.161}, {9.0, 0.121, 0.190, 0.235}},
+                                           {{4.2, 0.118, 0.1395, 0.175, 0.210}, {6.0, 0.180, 0.262, 0.275, 0.360}}};
+    static const double kTail[4] = {0.83, 0.93, 0.96, 1.0};
+    const double* at = kWhole[f32][plain];
+    double base = at[0];
+    if (!f32 && T <= 64) base = T <= 32 ? (plain ? 5.5 : 4.2) : (plain ? 11.0 : 4.9);  // one chunk, two
+    const int per = f32 && !gated ? 4 : 3;
+    const long long full = ctas / (per * 148), rest = ctas % (per * 148);
+    const int k = static_cast<int>((rest + 147) / 148);
+    return full * (base + at[per] * T) + (rest ? at[k] * T * (full ? kTail[k - 1] : 1.0) + (full ? 0.0 : base) : 0.0);
+}
 
-// The kernel by warp roles: how a call is laid out and what that takes, in us.  One CTA has an SM to itself (three at
-// two consumer warps).  Whole: w0 + w1 a step and round of CTAs; cut, where all pieces run side by side: c0 + c1 a step
-// of a piece, both passes.  Fitted to 200 shapes of 8 to 5600 steps (as CUDA graphs): half of the
-// estimates are within 5 % (whole) and 8 % (cut).  16-bit storage; f32 takes 1.05 times as long.
+// The kernel by warp roles: how a call is laid out and what that takes, in us, by storage (16-bit, f32).  One CTA has an
+// SM to itself (three at two consumer warps).  Whole: w0 + w1 a step and round of CTAs; cut, where all pieces run side by
+// side: c0 + c1 a step of a piece, both passes, + cs a segment, whose states every CTA chains.  Steps are those of whole
+// chunks, which the kernel walks whatever the length (34 steps of 16-bit storage take what 64 do).  Means of rates in
+// progression and general ones, which lie 6 % below and above them (cut 8 %).  Fitted to 2400 shapes of 16 to 8192 steps
+// (as CUDA graphs): nine in ten of the estimates are within 3 % of either kind (cut 5 %).
 struct Fwd16Kind {
     int ns, workers, helpers, stages;
-    double w0, w1, c0, c1;
+    double w0, w1[2], c0, c1[2], cs;
 };
-static const Fwd16Kind kFwd16Kinds[] = {{4, 2, 2, 3, 3.7, 0.0623, 5.6, 0.1022},
-                                        {4, 4, 4, 4, 3.5, 0.0712, 5.7, 0.1175},
-                                        {4, 5, 4, 4, 4.2, 0.0852, 6.8, 0.1400},
-                                        {4, 6, 4, 4, 4.3, 0.0888, 7.0, 0.1501},
-                                        {4, 8, 4, 4, 4.0, 0.1068, 6.5, 0.1813},
-                                        {8, 6, 4, 4, 5.4, 0.1527, 10.1, 0.2608}};
+static const Fwd16Kind kFwd16Kinds[] = {{4, 2, 2, 3, 4.2, {0.0600, 0.0680}, 6.6, {0.1000, 0.1130}, 0.27},
+                                        {4, 4, 4, 4, 3.8, {0.0680, 0.0800}, 6.1, {0.1140, 0.1337}, 0.27},
+                                        {4, 5, 4, 4, 4.6, {0.0822, 0.0984}, 7.0, {0.1443, 0.1662}, 0.26},
+                                        {4, 6, 4, 4, 4.7, {0.0850, 0.0999}, 7.1, {0.1474, 0.1690}, 0.26},
+                                        {4, 8, 4, 4, 4.4, {0.1020, 0.1184}, 6.8, {0.1754, 0.1986}, 0.30},
+                                        {8, 6, 4, 4, 5.8, {0.1491, 0.1640}, 9.9, {0.2700, 0.2900}, 0.50}};
+// Two consumer warps, two or three CTAs an SM: the base and a step.
+static const double kFwd16Shared[2][3] = {{4.8, 0.0845, 0.0972}, {4.2, 0.0930, 0.1080}};
 struct Fwd16Plan {
     const Fwd16Kind* kind = nullptr;  // null: sscan_fwd_kernel
     int segs = 1;
@@ -191,12 +212,15 @@ __global__ void sscan_seg_carry_kernel(float* seg_states, const float* seg_sumdl
     }
 }
 
-// The layout with the least estimate, if that is at most 0.95 (eight states a lane: 0.935, cut: 0.9) of what
-// sscan_fwd_kernel is estimated to take.  Against that kernel alone, 160 shapes of 64 to 8192 steps, both kinds of rates:
-// 14 % less time on average, no shape more than 2 % more.  8 x 2048 x 1536 with general rates 284 -> 196 us, 2 x 8192 x
-// 5120 with progressions 757 -> 640, 16 x 2048 x 1536 363 -> 339 (10 x 750 x 2600 with progressions would be 117 -> 124),
-// 1 x 1021 x 1536 32.0 -> 28.5, 4 x 512 x 256 19.7 -> 15.5.  Under 24 steps the shorter prologue of the other kernel wins
-// (12 x 9 x 144 4.5 us, here 5.8), and past three rounds of CTAs its three CTAs an SM do (19 x 33 x 5360 32 us, here 59).
+// The layout with the least estimate, if that is at most 0.95 of `us`, what sscan_fwd_kernel is estimated to take.
+// Against that kernel alone, 2400 shapes of 16 to 8192 steps with and without a workspace, both kinds of rates: 25 % less
+// time on average, six calls in a thousand more than 2 % more, 11 % at most.  Rates in progression decide where the line
+// lies: they help the other kernel more, so that at the border they are even and general ones gain a tenth.  8 x 2048 x
+// 1536 with general rates 284 -> 196 us, 2 x 8192 x 5120 with progressions 757 -> 640, 16 x 2048 x 1536 363 -> 339, 1 x
+// 1021 x 1536 32.0 -> 28.5, 4 x 512 x 256 19.7 -> 15.5.  Under 24 steps the shorter prologue of the other kernel wins (12 x
+// 9 x 144 4.5 us, here 5.8), with 34 to 36 steps of 16-bit storage its shorter chunks of rows do (14 x 37 x 2416 15.3, here
+// 19.8), in f32 without a gate its four CTAs an SM (10 x 544 x 3096 110, here 127), and past three rounds of CTAs its three
+// (19 x 33 x 5360 32, here 59).
 static Fwd16Plan fwd16_plan(const Fwd16Table& t, bool f32, int B, int T, int D, int N, double us, long long workspace_bytes) {
     Fwd16Plan best;
     if (T < 24) return best;
@@ -204,10 +228,11 @@ static Fwd16Plan fwd16_plan(const Fwd16Table& t, bool f32, int B, int T, int D, 
     for (const Fwd16Kind& k : kFwd16Kinds) {
         const int steps = t.steps[k.ns == 8], chunks = (T + steps - 1) / steps, dt = 4 * k.ns * k.workers;
         const long long ctas = static_cast<long long>(B) * ((D + dt - 1) / dt);
-        const double scale = f32 ? 1.05 : 1.0;
-        double c = scale * ((ctas + 147) / 148) * (k.w0 + k.w1 * T);
-        if (k.workers == 2 && ctas > 148) c = scale * ((ctas + 443) / 444) * (4.5 + 0.0931 * T);
-        if (c < (k.ns == 8 ? 0.935 / 0.95 * us : us) && ctas <= 3 * 148) {
+        double c = ((ctas + 147) / 148) * (k.w0 + k.w1[f32] * chunks * steps);
+        if (k.workers == 2 && ctas > 148) c = kFwd16Shared[f32][0] + kFwd16Shared[f32][ctas > 2 * 148 ? 2 : 1] * chunks * steps;
+        // a tile that reaches past the channels stores element by element, which progressions leave no time for
+        if (k.ns == 8 && !f32 && D % dt != 0) c *= 1.06;
+        if (c < us && ctas <= 3 * 148) {
             us = c;
             best = {&k, 1};
         }
@@ -215,7 +240,7 @@ static Fwd16Plan fwd16_plan(const Fwd16Table& t, bool f32, int B, int T, int D, 
         for (int s = 2; ctas * s <= 148 && s <= 32; ++s) {
             const int per = (chunks + s - 1) / s, segs = (chunks + per - 1) / per;
             if (segs != s || per * steps < 32 || !fwd_ws_holds(workspace_bytes, B, D, N, s)) continue;
-            c = scale * (k.c0 + k.c1 * per * steps) * (0.95 / 0.9);
+            c = k.c0 + k.c1[f32] * per * steps + k.cs * s;
             if (c < us) {
                 us = c;
                 best = {&k, s};
@@ -223,6 +248,15 @@ static Fwd16Plan fwd16_plan(const Fwd16Table& t, bool f32, int B, int T, int D, 
         }
     }
     return best;
+}
+
+// How a call is laid out that both kernels can take (no conv, d_state 9 .. 16, x, delta and z by TMA); segs: of the
+// general kernel, with `us` from fwd_segments, which is for 16-bit storage and B and C by TMA.
+static Fwd16Plan fwd16_choose(int dtype, int B, int T, int D, int N, bool gated, bool plain, int segs, double us, long long lent) {
+    const bool f32 = dtype == MAMBA_B200_F32;
+    us += 0.17 * std::max(0, segs - 18);  // the kernel between the passes
+    us = segs > 1 ? us * (plain ? 1.3 : 1.0) * (f32 ? 1.03 : 1.0) : fwd_whole_us(f32, gated, plain, T, fwd_ctas(B, D, N));
+    return fwd16_plan(fwd16_tables().t[dtype], f32, B, T, D, N, us, lent);
 }
 
 static bool overlaps(const void* a, size_t na, const void* b, size_t nb) {
@@ -374,10 +408,9 @@ static int launch_fwd(Ctx* c, cudaStream_t stream, const mamba_b200_sscan_fwd_ar
     if (segs > 1 && !ws_aligned) return fail(c, MAMBA_B200_ERR_ARG, "sscan_fwd: workspace must be 256-byte aligned");
     // d_state 9 .. 16 without the conv, channels that TMA can bring: by warp roles where that is estimated to be faster
     if (v->ns * v->lpc == 16 && !a.conv_w && (m & kTmaX) && (m & kTmaDl) && (!a.z_mode || (m & kTmaZ))) {
-        const Fwd16Table& t16 = fwd16_tables().t[a.dtype];
-        const Fwd16Plan plan = fwd16_plan(t16, a.dtype == MAMBA_B200_F32, a.B, a.T, a.D, a.N, us,
-                                          ws_aligned ? lent : 0);
-        if (plan.kind) return launch_fwd16(c, stream, a, p, t16, plan);
+        const bool plain = (m & (kTmaB | kTmaC)) != (kTmaB | kTmaC);
+        const Fwd16Plan plan = fwd16_choose(a.dtype, a.B, a.T, a.D, a.N, a.z_mode != 0, plain, segs, us, ws_aligned ? lent : 0);
+        if (plan.kind) return launch_fwd16(c, stream, a, p, fwd16_tables().t[a.dtype], plan);
     }
 
     const int flags = (a.delta_softplus ? 1 : 0) | (a.z_mode ? 2 : 0) | (a.conv_w ? 4 : 0);
@@ -441,14 +474,13 @@ extern "C" MAMBA_B200_API long long mamba_b200_sscan_fwd_workspace_bytes(int B, 
 
 extern "C" MAMBA_B200_API int mamba_b200_sscan_fwd_layout(int dtype, int B, int T, int D, int N, int z_mode, long long workspace_bytes,
                                                             int* out) {
-    (void)z_mode;
     if (!out || !dtype_ok(dtype) || B <= 0 || T <= 0 || D <= 0 || N <= 0 || N > 256) return MAMBA_B200_ERR_ARG;
     const FwdVariant* v = fwd_variant(dtype, N);
     double us = 0.0;
     int segs = fwd_segments(B, T, D, N, workspace_bytes, &us);
     Fwd16Plan plan;
     if (v->ns * v->lpc == 16)
-        plan = fwd16_plan(fwd16_tables().t[dtype], dtype == MAMBA_B200_F32, B, T, D, N, us, workspace_bytes);
+        plan = fwd16_choose(dtype, B, T, D, N, z_mode != 0, N * dtype_size(dtype) % 16 != 0, segs, us, workspace_bytes);
     if (!plan.kind) {
         const int chunks = (T + v->tc - 1) / v->tc, per = (chunks + segs - 1) / segs;
         segs = (chunks + per - 1) / per;

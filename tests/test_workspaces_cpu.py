@@ -31,3 +31,22 @@ def layout(dtype, B, T, D, N=16, z_mode=1, lent=None):
 def test_a_workspace_that_is_too_small_to_cut_with_is_like_none(dtype, shape):
     assert layout(dtype, *shape)[2] > 1
     assert layout(dtype, *shape, lent=4096) == layout(dtype, *shape, lent=0)
+
+
+# Calls without a workspace on both sides of the line between the two kernels, by what was measured (us by the general
+# kernel, by warp roles): steps past whole chunks, f32 without a gate, f32 with one, lengths that go on like the longer ones.
+@pytest.mark.parametrize("case", [
+    (ffi.BF16, 14, 37, 2416, 16, 1, False),   # 15.3, 19.8: 64 steps are walked
+    (ffi.BF16, 9, 34, 1448, 16, 1, False),    # 8.3, 10.1
+    (ffi.BF16, 8, 64, 1536, 16, 1, True),
+    (ffi.F32, 25, 240, 1248, 16, 0, False),   # 51.3, 58.9: four CTAs of the general kernel an SM
+    (ffi.F32, 10, 544, 3096, 16, 0, False),   # 110, 127
+    (ffi.F32, 14, 1549, 1392, 16, 1, True),   # 254, 227
+    (ffi.F32, 16, 2048, 1536, 16, 1, True),
+    (ffi.BF16, 16, 2048, 1536, 16, 1, True),  # 363, 339
+    (ffi.BF16, 16, 1504, 1536, 16, 1, True),
+    (ffi.BF16, 16, 1065, 1544, 12, 1, True),  # 269, 185: B and C by plain loads
+], ids=lambda c: "-".join(map(str, c)))
+def test_the_scan_forward_takes_the_faster_kernel(case):
+    *call, z_mode, roles = case
+    assert (layout(*call, z_mode=z_mode, lent=0)[0] > 0) == roles
