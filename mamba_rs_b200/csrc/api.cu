@@ -13,15 +13,20 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
-bool make_tmap_3d(Ctx* c, CUtensorMap* map, int dtype, const void* base, long long ld, int cols,
-                  int T, int B, int box_cols, int box_rows) {
+bool tmap_3d_fits(Ctx* c, int dtype, const void* base, long long ld, int cols, int T, int box_cols, int box_rows) {
     if (!c->encode_tiled || !base) return false;
     const size_t es = dtype_size(dtype);
     if ((reinterpret_cast<uintptr_t>(base) & 15) != 0) return false;
     if ((static_cast<size_t>(ld) * es) % 16 != 0) return false;
     if ((static_cast<size_t>(box_cols) * es) % 16 != 0) return false;
     if (box_cols > 256 || box_rows > 256 || box_cols < 1 || box_rows < 1) return false;
-    if (ld < cols) return false;
+    return ld >= cols && static_cast<cuuint64_t>(ld) * es * static_cast<cuuint64_t>(T) < (1ull << 40);
+}
+
+bool make_tmap_3d(Ctx* c, CUtensorMap* map, int dtype, const void* base, long long ld, int cols,
+                  int T, int B, int box_cols, int box_rows) {
+    if (!tmap_3d_fits(c, dtype, base, ld, cols, T, box_cols, box_rows)) return false;
+    const size_t es = dtype_size(dtype);
     CUtensorMapDataType dt = dtype == MAMBA_B200_F32   ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
                              : dtype == MAMBA_B200_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
                                                        : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
@@ -29,7 +34,6 @@ bool make_tmap_3d(Ctx* c, CUtensorMap* map, int dtype, const void* base, long lo
                           static_cast<cuuint64_t>(B)};
     cuuint64_t strides[2] = {static_cast<cuuint64_t>(ld) * es,
                              static_cast<cuuint64_t>(ld) * es * static_cast<cuuint64_t>(T)};
-    if (strides[1] >= (1ull << 40)) return false;
     cuuint32_t box[3] = {static_cast<cuuint32_t>(box_cols), static_cast<cuuint32_t>(box_rows), 1};
     cuuint32_t estr[3] = {1, 1, 1};
     CUresult r = reinterpret_cast<EncodeTiledFn>(c->encode_tiled)(

@@ -40,6 +40,8 @@ inline bool dtype_ok(int dtype) {
 // in which case the caller uses the plain-load path for that tensor.
 bool make_tmap_3d(Ctx* c, CUtensorMap* map, int dtype, const void* base, long long ld, int cols,
                   int T, int B, int box_cols, int box_rows);
+// Those rules alone, for a choice that comes before the tile is known.
+bool tmap_3d_fits(Ctx* c, int dtype, const void* base, long long ld, int cols, int T, int box_cols, int box_rows);
 
 // Describes `layers` row-major [rows, cols] matrices, `stride` elements apart, as a 3-D TMA tensor
 // with a box of box_rows x box_cols of one matrix (no swizzle; outside reads as zero).

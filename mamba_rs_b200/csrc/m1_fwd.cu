@@ -281,15 +281,25 @@ static void launch_seg_carry(cudaStream_t stream, const mamba_b200_sscan_fwd_arg
                                                                                       a.N);
 }
 
-// The call by warp roles; `p` holds what both kernels need, its tensor maps are made again for this one's tiles.
-static int launch_fwd16(Ctx* c, cudaStream_t stream, const mamba_b200_sscan_fwd_args& a, const FwdParams& p, const Fwd16Table& t,
-                        const Fwd16Plan& plan) {
+// The call by warp roles.  q.f holds what both kernels need, and the tensor maps of this one's tiles after fwd16_maps.
+static bool fwd16_maps(Ctx* c, const mamba_b200_sscan_fwd_args& a, const Fwd16Table& t, const Fwd16Plan& plan, Fwd16Params* q) {
     const Fwd16Kind& k = *plan.kind;
-    const int i = k.ns == 8, steps = t.steps[i], dt = 4 * k.ns * k.workers;
-    Fwd16Params q;
-    memset(&q, 0, sizeof(q));
-    q.f = p;
-    q.dt = dt;
+    const int steps = t.steps[k.ns == 8], dt = 4 * k.ns * k.workers;
+    auto tile = [&](CUtensorMap* map, const void* base, long long ld, int cols, int box) {
+        return make_tmap_3d(c, map, a.dtype, base, ld, cols, a.T, a.B, box, steps);
+    };
+    q->dt = dt;
+    if (!tile(&q->f.tm_x, a.x, a.ld_x, a.D, dt) || !tile(&q->f.tm_dl, a.delta, a.ld_delta, a.D, dt) ||
+        (a.z_mode && !tile(&q->f.tm_z, a.z, a.ld_z, a.D, dt)))
+        return false;
+    if (tile(&q->f.tm_b, a.Bm, a.ld_bc, a.N, a.N)) q->f.tma_mask |= kTmaB;
+    if (tile(&q->f.tm_c, a.Cm, a.ld_bc, a.N, a.N)) q->f.tma_mask |= kTmaC;
+    return true;
+}
+static int launch_fwd16(Ctx* c, cudaStream_t stream, const mamba_b200_sscan_fwd_args& a, const Fwd16Table& t, const Fwd16Plan& plan,
+                        Fwd16Params& q) {
+    const Fwd16Kind& k = *plan.kind;
+    const int i = k.ns == 8, steps = t.steps[i], dt = q.dt;
     q.stages = k.stages;
     while (t.smem[i](dt, q.stages) > kF16MaxSmem) --q.stages;
     // a helper goes to the scheduler (warp % 4) that has the least to do
@@ -307,17 +317,9 @@ static int launch_fwd16(Ctx* c, cudaStream_t stream, const mamba_b200_sscan_fwd_
         warps = std::max(warps, best + 1);
     }
     const int threads = 32 * (warps + 1);  // and the producer
-    auto tile = [&](CUtensorMap* map, const void* base, long long ld) {
-        return make_tmap_3d(c, map, a.dtype, base, ld, a.D, a.T, a.B, dt, steps);
-    };
-    if (!tile(&q.f.tm_x, a.x, a.ld_x) || !tile(&q.f.tm_dl, a.delta, a.ld_delta) || (a.z_mode && !tile(&q.f.tm_z, a.z, a.ld_z)))
-        return fail(c, MAMBA_B200_ERR_CUDA, "sscan_fwd: no tensor map for %d channels", dt);
-    q.f.tma_mask = 0;
-    if (make_tmap_3d(c, &q.f.tm_b, a.dtype, a.Bm, a.ld_bc, a.N, a.T, a.B, a.N, steps)) q.f.tma_mask |= kTmaB;
-    if (make_tmap_3d(c, &q.f.tm_c, a.dtype, a.Cm, a.ld_bc, a.N, a.T, a.B, a.N, steps)) q.f.tma_mask |= kTmaC;
     q.vec_y = reinterpret_cast<uintptr_t>(a.y) % (2 * dtype_size(a.dtype)) == 0 && a.ld_y % 2 == 0;
     auto aligned = [](const void* ptr) { return reinterpret_cast<uintptr_t>(ptr) % 16 == 0; };
-    q.vec_state = a.N == 16 && aligned(a.ssm_state) && aligned(a.chunk_states) && p.cs_ld_b % 4 == 0 && p.cs_ld_k % 4 == 0;
+    q.vec_state = a.N == 16 && aligned(a.ssm_state) && aligned(a.chunk_states) && q.f.cs_ld_b % 4 == 0 && q.f.cs_ld_k % 4 == 0;
 
     const int flags = (a.delta_softplus ? 1 : 0) | (a.z_mode ? 2 : 0);
     const size_t smem = t.smem[i](dt, q.stages);
@@ -392,6 +394,28 @@ static int launch_fwd(Ctx* c, cudaStream_t stream, const mamba_b200_sscan_fwd_ar
         p.cs_ld_b = cs_ld_b ? cs_ld_b : p.cs_ld_k * ((a.T + a.save_stride - 1) / a.save_stride);
     }
     p.status = c->d_status;
+    const long long lent = a.workspace ? a.workspace_bytes : 0;
+    double us = 0.0;
+    int segs = fwd_segments(a.B, a.T, a.D, a.N, lent, &us);
+    const bool ws_aligned = reinterpret_cast<uintptr_t>(a.workspace) % 256 == 0;
+    if (segs > 1 && !ws_aligned) return fail(c, MAMBA_B200_ERR_ARG, "sscan_fwd: workspace must be 256-byte aligned");
+    // d_state 9 .. 16 without the conv, channels that TMA can bring: by warp roles where that is estimated to be faster
+    auto fits = [&](const void* base, long long ld, int cols, int box) {
+        return tmap_3d_fits(c, a.dtype, base, ld, cols, a.T, box, v->tc);
+    };
+    if (v->ns * v->lpc == 16 && !a.conv_w && fits(a.x, a.ld_x, a.D, v->dt) && fits(a.delta, a.ld_delta, a.D, v->dt) &&
+        (!a.z_mode || fits(a.z, a.ld_z, a.D, v->dt))) {
+        const Fwd16Table& t16 = fwd16_tables().t[a.dtype];
+        const bool plain = !fits(a.Bm, a.ld_bc, a.N, a.N) || !fits(a.Cm, a.ld_bc, a.N, a.N);
+        const Fwd16Plan plan = fwd16_choose(a.dtype, a.B, a.T, a.D, a.N, a.z_mode != 0, plain, segs, us, ws_aligned ? lent : 0);
+        Fwd16Params q;
+        if (plan.kind) {
+            memset(&q, 0, sizeof(q));
+            q.f = p;
+            if (fwd16_maps(c, a, t16, plan, &q)) return launch_fwd16(c, stream, a, t16, plan, q);
+        }
+    }
+
     unsigned m = 0;
     const int xrows = a.conv_w ? v->tc + kHaloRows : v->tc;
     if (make_tmap_3d(c, &p.tm_x, a.dtype, a.x, a.ld_x, a.D, a.T, a.B, v->dt, xrows)) m |= kTmaX;
@@ -400,18 +424,6 @@ static int launch_fwd(Ctx* c, cudaStream_t stream, const mamba_b200_sscan_fwd_ar
     if (make_tmap_3d(c, &p.tm_b, a.dtype, a.Bm, a.ld_bc, a.N, a.T, a.B, a.N, v->tc)) m |= kTmaB;
     if (make_tmap_3d(c, &p.tm_c, a.dtype, a.Cm, a.ld_bc, a.N, a.T, a.B, a.N, v->tc)) m |= kTmaC;
     p.tma_mask = m;
-
-    const long long lent = a.workspace ? a.workspace_bytes : 0;
-    double us = 0.0;
-    int segs = fwd_segments(a.B, a.T, a.D, a.N, lent, &us);
-    const bool ws_aligned = reinterpret_cast<uintptr_t>(a.workspace) % 256 == 0;
-    if (segs > 1 && !ws_aligned) return fail(c, MAMBA_B200_ERR_ARG, "sscan_fwd: workspace must be 256-byte aligned");
-    // d_state 9 .. 16 without the conv, channels that TMA can bring: by warp roles where that is estimated to be faster
-    if (v->ns * v->lpc == 16 && !a.conv_w && (m & kTmaX) && (m & kTmaDl) && (!a.z_mode || (m & kTmaZ))) {
-        const bool plain = (m & (kTmaB | kTmaC)) != (kTmaB | kTmaC);
-        const Fwd16Plan plan = fwd16_choose(a.dtype, a.B, a.T, a.D, a.N, a.z_mode != 0, plain, segs, us, ws_aligned ? lent : 0);
-        if (plan.kind) return launch_fwd16(c, stream, a, p, fwd16_tables().t[a.dtype], plan);
-    }
 
     const int flags = (a.delta_softplus ? 1 : 0) | (a.z_mode ? 2 : 0) | (a.conv_w ? 4 : 0);
     FwdKernelFn fn = v->fn[flags];
