@@ -1224,17 +1224,21 @@ extern "C" MAMBA_B200_API int mamba_b200_m3_ssd_fwd(void* handle, void* stream,
         // bf16, 64 x 128: 4 heads x 4096 steps 44 us (one CTA each: 123), 24 x 2048 34 (63), 64 x 4096 91 (124);
         // continued from a state 4 x 4096 62 us
         const int nchunks = (a.T + tc::CS - 1) / tc::CS;
-        const int ranks = gen ? 1 : a.carry_in ? m3_cluster_ranks(a.B * a.nh, nchunks, 5.5, 6.6, 6.6, 3.2)
-                                               : m3_cluster_ranks(a.B * a.nh, nchunks, 3.7, 5.15, 5.15, 2.6);
+        // Pairs that two CTAs per SM take are not divided, whose costs are one CTA's: 180 pairs continued over 4096 steps 535
+        // us in clusters of four, 352 undivided; 150 x 16384 from zero 1023 and 825.
+        const int pairs = a.B * a.nh;
+        const bool two = !gen && (a.carry_in ? m3_two_carried_per_sm(pairs, nchunks) : m3_two_per_sm(pairs));
+        const int ranks = gen || two ? 1 : a.carry_in ? m3_cluster_ranks(pairs, nchunks, 5.5, 6.6, 6.6, 3.2)
+                                                      : m3_cluster_ranks(pairs, nchunks, 3.7, 5.15, 5.15, 2.6);
         if (ranks > 1) {
             const void* fn = bf ? (a.carry_in ? reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, true, true, false>)
                                               : reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, false, true, false>))
                                 : reinterpret_cast<const void*>(tc::m3_ssd_fwd_tc_kernel<__half, false, false, true, false>);
             void* args[1] = {&p};
             MB200_CUDA_CHECK(c, launch_cluster(fn, dim3(a.nh * ranks, a.B), dim3(256), tc::kSmem, st, ranks, args));
-        } else if (a.carry_in && m3_two_carried_per_sm(a.B * a.nh, nchunks)) {
+        } else if (two && a.carry_in) {
             tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, true, false, true><<<grid, 256, tc::lean::kSmem, st>>>(p);
-        } else if (!gen && !a.carry_in && m3_two_per_sm(a.B * a.nh)) {
+        } else if (two) {
             if (bf) tc::m3_ssd_fwd_tc_kernel<__nv_bfloat16, false, false, false, true><<<grid, 256, tc::lean::kSmem, st>>>(p);
             else tc::m3_ssd_fwd_tc_kernel<__half, false, false, false, true><<<grid, 256, tc::lean::kSmem, st>>>(p);
         } else if (bf) {

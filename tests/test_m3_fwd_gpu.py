@@ -338,3 +338,27 @@ def test_two_ctas_per_sm_give_the_same_bits(cuda_dev, case, dt):
             else:
                 assert torch.equal(a[lo:hi], b)
     mb.ffi.default_handle(0).check_status()
+
+
+# Pairs that two CTAs per SM take are not divided over clusters, however long: the state has the bits that nine tenths
+# of the batch, which are undivided pairs of one CTA, give in a call of their own.
+@pytest.mark.parametrize("case", [(10, 4096, 15, True), (10, 16384, 15, False)], ids=lambda c: "B%dT%dnh%dcarry%d" % c)
+def test_more_pairs_than_sms_are_not_divided(cuda_dev, case):
+    import torch
+
+    import mamba_rs_b200 as mb
+    (B, T, nh, carried), hd, N = case, 64, 128
+    g = torch.Generator(device=cuda_dev).manual_seed(T)
+    rn = lambda *s: torch.randn(*s, device=cuda_dev, generator=g)  # noqa: E731
+    x, K, Q = [rn(B, T, nh, n).mul_(0.3).to(torch.bfloat16).view(B, T, -1) for n in (hd, N, N)]
+    dt_, trap = torch.nn.functional.softplus(rn(B, T, nh) - 2), torch.sigmoid(rn(B, T, nh))
+    adt, Dh = -dt_ * 0.01, rn(nh)  # slow enough for every chunk's roundings to reach the end
+    h0, k0, v0 = rn(B, nh, hd, N), 0.3 * rn(B, nh, N), rn(B, nh, hd)
+
+    def call(n):
+        st = dict(ssm_state=h0[:n].clone(), k_state=k0[:n].clone(), v_state=v0[:n].clone())
+        mb.m3_ssd_fwd(x[:n], K[:n].view(n, T, nh, N), Q[:n].view(n, T, nh, N), dt_[:n], trap[:n], adt[:n], Dh, carry_in=carried, **st)
+        return st["ssm_state"]
+
+    assert torch.equal(call(B)[:9], call(9))
+    mb.ffi.default_handle(0).check_status()
