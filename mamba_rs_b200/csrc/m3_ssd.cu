@@ -256,8 +256,8 @@ constexpr uint32_t cY2 = 128, cS = 192, kTmemCols = 256;
 // bf16 values, f32's 24 bits, with a product each; M and the state copy, which only y is made of,
 // are two, 2^-17 of each term against the 2^-9 that y is rounded to.  The further tiles take the
 // room of the second Q / K / V buffers: Q of the next chunk is requested when the first MMA group
-// has read it, K and V when the second has.  8 x 256 steps x 32 heads of 64 x 128: 44 us (393 us by
-// the sequential kernel).  The state's error against 64 bits there is 1.1e-6 (sequentially 3.2e-6),
+// has read it, K and V when the second has.  8 x 256 steps x 32 heads of 64 x 128: 62 us, 47 as LEAN (393
+// by the sequential kernel).  The state's error against 64 bits there is 1.1e-6 (sequentially 3.2e-6),
 // over 1 x 1000 steps 6.2e-7 (5.4e-7; 2.5e-6 with w o V of two values).  bf16 only: f16's range
 // does not hold the remainders (x of 1e-3 left an error of 4e-3) nor products beyond 65504, so a
 // carried f16 window is the sequential kernel's.
@@ -1080,7 +1080,7 @@ static bool m3_two_per_sm(int pairs) { return pairs > 148 && (pairs <= 360 || pa
 
 // The same for carried windows, in us: 152 pairs x 256 steps 49 and 42, 256 62 and 47, 512 121 and 90; x 1024 steps 123
 // and 108, 126 and 110, 247 and 214; in the third wave of one CTA per SM, 384 pairs, 91 and 86 x 256 but 186 and 202 x
-// 1024, so there only up to two chunks.  256 pairs x 21 steps 33 and 26.
+// 1024, so there only up to two chunks.  256 pairs x 21 steps 33 and 23.
 static bool m3_two_carried_per_sm(int pairs, int nchunks) {
     return pairs > 148 && (pairs <= 2 * 148 || pairs > 3 * 148 || nchunks <= 2);
 }
@@ -1157,10 +1157,16 @@ static void launch_seq(const M3Params& p, int sms, cudaStream_t st) {
 
 using namespace mb200;
 
-// A carried window of at most this many steps takes the sequential kernel: a 128-row chunk costs
-// the tensor-core kernel the same time whether it holds 1 step or 128 (15 us at 4 heads, 32 us at
-// 256), and the sequential kernel reaches that after 30 and 18 steps.
-constexpr int kCarrySeqSteps = 20;
+// A carried window of at most this many steps takes the sequential kernel: a 128-row chunk costs the tensor-core kernel the
+// same time whether it holds 1 step or 128 (15 us at 4 heads, 22 at 150 to 296 pairs, 41 to 45 at 297 to 592), and the
+// sequential kernel reaches that after 30 steps at 4 heads.  Its widest form, heads over 48 x 96, takes 1.5 us a step at 150 to
+// 296 pairs and 2.3 to 3.3 beyond: against two CTAs per SM 16 steps of 256 pairs 28 and 23 us, 20 of 512 66 and 45,
+// 17 of 416 43 and 43, 14 of 1024 82 and 88.  Smaller heads get there later (32 x 64 at 21 steps, 48 x 128 at 18 to 21).  The
+// state is closer to 64 bits on the tensor cores at every length: 1.2e-7 and 3.7e-7 after 16 steps.
+static int m3_sequential_steps(int pairs, int hd, int N) {
+    if (pairs <= 148 || hd <= 48 || N <= 96) return 20;
+    return pairs > 2 * 148 && pairs <= 3 * 148 ? 17 : 14;
+}
 
 extern "C" MAMBA_B200_API int mamba_b200_m3_ssd_fwd(void* handle, void* stream,
                                                     const mamba_b200_m3_ssd_args* ap) {
@@ -1200,7 +1206,7 @@ extern "C" MAMBA_B200_API int mamba_b200_m3_ssd_fwd(void* handle, void* stream,
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
     bool tensor_core = a.dtype != MAMBA_B200_F32 && a.hd <= tc::HD && a.hd % 8 == 0 && a.N <= tc::NS &&
-                       a.N % 8 == 0 && (!a.carry_in || (!gen && a.dtype == MAMBA_B200_BF16 && a.T > kCarrySeqSteps)) &&
+                       a.N % 8 == 0 && (!a.carry_in || (!gen && a.dtype == MAMBA_B200_BF16 && a.T > m3_sequential_steps(a.B * a.nh, a.hd, a.N))) &&
                        !a.force_sequential && al16(a.x) && al16(a.y) &&
                        (gen ? al16(a.Bn) && al16(a.Cn) && al16(a.angle_vel) : al16(a.K) && al16(a.Q));
     // the tile maps; when the driver refuses one (no encoder, a stride beyond its range) the
