@@ -42,6 +42,19 @@ def to_dev(a, dev, dtype=None):
     return t.to(dtype) if dtype is not None else t
 
 
+def scan_fwd_layout(dtype, B, T, D, N=16, z_mode=1, lent=None):
+    """(states a lane by warp roles or 0 for the general kernel, its consumer warps, time segments) of such a call;
+    dtype: ffi.F32 / F16 / BF16, lent: bytes of workspace, None what it asks for."""
+    import ctypes
+
+    from mamba_rs_b200 import ffi
+    if lent is None:
+        lent = ffi.lib().mamba_b200_sscan_fwd_workspace_bytes(B, T, D, N)
+    out = (ctypes.c_int * 3)()
+    assert ffi.lib().mamba_b200_sscan_fwd_layout(dtype, B, T, D, N, z_mode, lent, out) == 0
+    return tuple(out)
+
+
 # Committed golden fixtures (tests/golden/m1_fused_<name>.npz, made by
 # tests/golden/gen_golden.py): name, B, T, D, N, K, dtype, a_mode, seed
 GOLDEN_CASES = [

@@ -9,7 +9,8 @@ import pytest
 
 import oracle
 from helpers import (GOLDEN_CASES, TOL, golden_inputs, load_golden, quantised_inputs, random_states,
-                     rel_err, to_dev, torch_dtype)
+                     rel_err, scan_fwd_layout, to_dev, torch_dtype)
+from mamba_rs_b200 import synth
 
 pytestmark = pytest.mark.gpu
 
@@ -334,16 +335,19 @@ def test_unaligned_rows_take_plain_loads(cuda_dev, case, dt):
     assert rel_err(y.float().cpu().numpy(), ref["y"]) <= TOL[dt]
 
 
-# (B, T, D) either side of where the number of time segments changes: whole, four, eight, as many as fill the chip
+# (B, T, D) that a workspace cuts, by either kernel and into few pieces and many, from the shortest length on (192);
+# without one the same call is walked in one piece, by the kernel that it would take then
 @pytest.mark.parametrize("dt", ["bf16", "f32"])
-@pytest.mark.parametrize("shape", [(2, 191, 320), (2, 192, 320), (3, 255, 1536), (11, 256, 640), (11, 255, 640), (6, 511, 1344), (6, 512, 1344),
-                                   (7, 999, 1344), (7, 1000, 1344), (7, 1536, 1344), (8, 1536, 1536), (1, 1021, 1536), (1, 2100, 64)],
-                         ids=lambda s: "B%dT%dD%d" % s)
+@pytest.mark.parametrize("shape", [(2, 192, 320), (3, 255, 1536), (11, 256, 128), (11, 255, 96), (6, 511, 256), (6, 512, 640), (7, 999, 320),
+                                   (4, 1000, 640), (7, 1536, 320), (2, 1536, 1536), (1, 1021, 1536), (1, 2100, 64), (16, 1500, 40),
+                                   (2, 700, 1832), (1, 1535, 5120), (1, 1536, 5120)], ids=lambda s: "B%dT%dD%d" % s)
 def test_time_segments_equal_one_piece(cuda_dev, shape, dt):
     import torch
 
     import mamba_rs_b200 as mb
     (B, T, D), N, td = shape, 16, torch_dtype(dt)
+    code = mb.dtype_code(td)
+    assert scan_fwd_layout(code, *shape)[2] > 1 and scan_fwd_layout(code, *shape, lent=0)[2] == 1
     g = torch.Generator(device=cuda_dev).manual_seed(T)
     rn = lambda *s: torch.randn(*s, device=cuda_dev, generator=g)  # noqa: E731
     args = [rn(B, T, D).to(td), (0.5 * rn(B, T, D) - 3).to(td), rn(B, T, N).to(td), rn(B, T, N).to(td), -torch.exp(rn(D, N)), rn(D)]
@@ -357,29 +361,50 @@ def test_time_segments_equal_one_piece(cuda_dev, shape, dt):
     assert float((h2 - h1).abs().max() / h1.abs().max()) <= 1e-5
 
 
-# The kernel by warp roles (d_state 9 .. 16, TMA-able channels, 24 steps or more), one shape for each of its layouts:
-# two, four, six and eight consumer warps of four states a lane, six of eight; whole and cut into segments.  Ragged
-# lengths, d_state below 16, a tile that reaches past d_inner (rows longer than the channels), B and C that no tensor
-# map describes, rows of y off every word, saves every 32 and 64 steps, all gate modes.  y is held to half a unit of its storage
-# and the decay rates' f32 rounding (TOL), the states to 1e-4, as everywhere in this file.
-@pytest.mark.parametrize("dt", ["f32", "bf16", "f16"])
-@pytest.mark.parametrize("case", [
-    # B, T, D, N, a_mode, workspace, z_mode, save_stride, odd (views: longer rows, B / C and y off by one element)
-    (1, 24, 64, 16, "s4d", False, 1, 32, False), (2, 25, 40, 9, "random", False, 1, 64, True),
-    (3, 75, 2048, 16, "random", False, 1, 32, False), (8, 79, 1536, 16, "s4d", False, 1, 64, False),
-    (10, 95, 1832, 16, "random", False, 2, 32, True), (16, 700, 1536, 12, "random", False, 0, 64, False),
-    (1, 1021, 328, 16, "random", True, 1, 32, True), (2, 333, 136, 13, "s4d", True, 1, 64, False),
-    (1, 300, 1536, 16, "s4d", True, 0, 32, False),
-], ids=lambda c: "B%dT%dD%dN%d%sws%dz%ds%dodd%d" % c)
+# The kernel by warp roles (d_state 9 .. 16, TMA-able channels, 24 steps or more): every layout that the rule chooses,
+# four states a lane with two, four, five, six and eight consumer warps and eight with six, whole and cut into segments,
+# and two warps with more than one CTA per SM (f32).  That a case has the layout it is here for is asserted, so that a
+# line that moves does not leave it behind.  Ragged lengths, d_state below 16, a tile that reaches past d_inner (rows longer
+# than the channels), B and C that no tensor map describes, rows of y off every word, saves every 32 and 64 steps, all
+# gate modes, with softplus and without, each in one piece and cut.  y is held to half a unit of its storage and the decay
+# rates' f32 rounding (TOL), the states to 1e-4, as everywhere in this file.
+ALL = ("f32", "bf16", "f16")
+
+
+@pytest.mark.parametrize("case,dt", [(c, dt) for c in [
+    # B, T, D, N, a_mode, workspace, z_mode, softplus, save_stride, odd (views: longer rows, B / C and y off by one
+    # element), layout: states a lane, consumer warps, cut; storage
+    (1, 33, 40, 9, "random", False, 1, True, 64, True, (4, 2, False), ALL),
+    (12, 33, 968, 13, "s4d", False, 2, True, 32, True, (4, 2, False), ("f32",)),
+    (1, 24, 64, 16, "s4d", False, 1, True, 32, False, (4, 4, False), ALL),
+    (3, 75, 2048, 16, "random", False, 1, True, 32, False, (4, 4, False), ALL),
+    (10, 33, 1000, 13, "random", False, 2, True, 32, True, (4, 5, False), ALL),
+    (8, 79, 1536, 16, "s4d", False, 1, False, 64, False, (4, 6, False), ALL),
+    (8, 24, 1832, 13, "s4d", False, 0, True, 32, True, (4, 8, False), ALL),
+    (16, 75, 1344, 13, "random", False, 1, True, 64, True, (8, 6, False), ALL),
+    (16, 1023, 1536, 16, "s4d", False, 0, True, 64, False, (8, 6, False), ALL),
+    (1, 1021, 40, 9, "s4d", True, 1, True, 32, True, (4, 2, True), ALL),
+    (5, 451, 40, 16, "random", True, 1, True, 64, False, (4, 4, True), ALL),
+    (1, 300, 1536, 16, "s4d", True, 0, True, 32, False, (4, 4, True), ALL),
+    (10, 205, 136, 13, "random", True, 1, True, 32, True, (4, 5, True), ALL),
+    (5, 205, 328, 16, "s4d", True, 0, True, 32, False, (4, 6, True), ALL),
+    (10, 205, 200, 16, "random", True, 2, False, 64, False, (4, 8, True), ALL),
+    (2, 1500, 1832, 9, "random", True, 1, True, 64, True, (8, 6, True), ALL),
+    (10, 1500, 328, 13, "s4d", True, 1, False, 32, False, (8, 6, True), ALL),
+] for dt in c[-1]], ids=lambda c: c if isinstance(c, str) else "B%dT%dD%dN%d%sws%dz%dsp%ds%dodd%d" % c[:10])
 def test_warp_roles_match_oracle(cuda_dev, case, dt):
     import torch
 
     import mamba_rs_b200 as mb
-    B, T, D, N, a_mode, lent, z_mode, S, odd = case
+    B, T, D, N, a_mode, lent, z_mode, softplus, S, odd, layout, _ = case
+    states, warps, segments = scan_fwd_layout(mb.dtype_code(torch_dtype(dt)), B, T, D, N, z_mode, None if lent else 0)
+    assert (states, warps, segments > 1) == layout
     q = quantised_inputs(B, T, D, N, 0, dt, seed=T + D, a_mode=a_mode)
+    if not softplus:
+        q["delta_raw"] = synth.round_to(np.log1p(np.exp(q["delta_raw"])), dt)
     ssm0, _ = random_states(B, D, N, 0, seed=T)
     ref = oracle.m1_fused_fwd(q["x"], q["delta_raw"], q["Bm"], q["Cm"], q["z"] if z_mode == 1 else None, q["a_neg"], q["Dp"],
-                              None, None, None, ssm0, want_h=B * D * T < 300000)
+                              None, None, None, ssm0, delta_softplus=softplus, want_h=B * D * T < 300000)
     want = ref["y"] * q["z"] if z_mode == 2 else ref["y"]
     td = torch_dtype(dt)
 
@@ -398,7 +423,7 @@ def test_warp_roles_match_oracle(cuda_dev, case, dt):
     ybuf = torch.zeros(B, T, D + 3, device=cuda_dev, dtype=td)
     y = mb.selective_scan_fwd(view(q["x"], D8, 0), view(q["delta_raw"], D8, 0), view(q["Bm"], 3, 1), view(q["Cm"], 3, 1),
                               to_dev(q["a_neg"], cuda_dev), to_dev(q["Dp"], cuda_dev), view(q["z"], D8, 0) if z_mode else None,
-                              z_mode=z_mode, ssm_state=ssm, chunk_states=cs, save_stride=S, workspace=ws,
+                              z_mode=z_mode, delta_softplus=softplus, ssm_state=ssm, chunk_states=cs, save_stride=S, workspace=ws,
                               y=ybuf[..., 1:1 + D] if odd else None)
     torch.cuda.synchronize()
     mb.ffi.default_handle(0).check_status()
