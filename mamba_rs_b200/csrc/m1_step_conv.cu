@@ -617,8 +617,11 @@ extern "C" MAMBA_B200_API int mamba_b200_conv1d_fwd(void* handle, void* stream,
         // Sixteen steps a warp where that leaves 16 warps for every SM: its taps (64 bytes a lane) and its three rows of
         // halo are then read for twice as many outputs.  In us, 8 and 16 steps: 8 x 2048 x 1536 bf16 24.4 and 21.8, f32
         // 35.4 and 32.6, 2 x 8192 x 5120 71.7 and 61.8, 2 x 2048 x 2048 10.6 and 10.1; 1 x 1021 x 1536 4.2 and 4.4 (and with
-        // 32 steps, in the registers of a third of the warps, 26.5 at the first).
-        const bool tall = v == 4 && static_cast<long long>(a.B) * ((a.T + 15) / 16) * vgrid.x >= 16 * 148;
+        // 32 steps, in the registers of a third of the warps, 26.5 at the first).  A short batch's last warp must have more
+        // than eight of its steps: 256 x 24 x 640 f32 8.4 and 9.6, 256 x 28 x 640 10.6 and 9.7, 256 x 36 x 640 10.7 and
+        // 12.3, 256 x 44 x 640 13.5 and 12.5; in 16-bit storage two full ones outweigh it (256 x 36 x 1536 21.3 and 18.5).
+        const bool filled = a.T > 40 || (a.T > 24 && (a.T <= 32 || a.dtype != MAMBA_B200_F32));
+        const bool tall = v == 4 && filled && static_cast<long long>(a.B) * ((a.T + 15) / 16) * vgrid.x >= 16 * 148;
         const int rt = tall ? 16 : kConvRT, threads = 32 * std::min(kConvTT / rt, (a.T + rt - 1) / rt);
 #define MB200_CONV(T)                                                              \
     do {                                                                           \

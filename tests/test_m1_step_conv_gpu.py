@@ -176,9 +176,10 @@ def test_f32_channel_counts_that_are_even_but_no_multiple_of_four(cuda_dev, T, K
 
 
 # Long batches give a warp sixteen steps, a sample of them alone eight: the same arithmetic for every output, so the same
-# bits.  Lengths around both counts, a width that is no multiple of a warp's 128 channels, d_conv 4 and 2.
+# bits.  Lengths around both counts and from the shortest that has sixteen (25), a width that is no multiple of a warp's 128
+# channels, d_conv 4 and 2.
 @pytest.mark.parametrize("dt", ["f32", "bf16", "f16"])
-@pytest.mark.parametrize("case", [(8, 1009, 644, 4), (8, 1024, 640, 2), (150, 17, 1024, 4)], ids=lambda c: "B%dT%dD%dK%d" % c)
+@pytest.mark.parametrize("case", [(8, 1009, 644, 4), (8, 1024, 640, 2), (150, 25, 1024, 4), (150, 41, 1020, 3)], ids=lambda c: "B%dT%dD%dK%d" % c)
 def test_conv_sixteen_steps_a_warp_give_the_bits_of_eight(cuda_dev, case, dt):
     import torch
 
