@@ -21,7 +21,7 @@
 // cycles of the SM's return path whether or not its lanes ask for the same words, so B and C cost a cycle per channel
 // and step where a lane has one channel (204 us), half where it has two.  Four states a lane: eight (16 x 2048 x 1536
 // 342 us) need fewer instructions and loads, but leave one warp a scheduler below 256 channels an SM (8 x 2048 x 1536
-// 260 us).  Elementwise work in the consumers, as sscan_fwd_kernel has it, would put its latency into the chain of
+// 260 us); they take all of the 128 registers that 512 threads leave and spill 8 bytes.  Elementwise work in the consumers, as sscan_fwd_kernel has it, would put its latency into the chain of
 // every step and its registers into every lane.  Tried and not kept: packing over the two channels (B and C twice in
 // shared memory, 30 % slower); a fourth of the exponentials by a polynomial on the FMA pipe (196 -> 206 us);
 // chunks unrolled in full (instruction fetch: 141 -> 190 us at four consumer warps).

@@ -227,8 +227,9 @@ constexpr uint32_t cG = 0, cY1 = 256, cY2 = 320, cS = 384, kTmemCols = 512;
 // LEAN: two CTAs per SM, so that one's tensor-core and copy waits (3000 of a chunk's 7300 cycles) are the other's time.
 // One buffer for Q, K and V, asked for again when the last MMA of a chunk is done; M over the Q tile, Y1 over G, which
 // have been read by then.  8 x 4096 steps x 32 heads of 64 x 128: 250 -> 195 us (0.63 of the measured HBM rate), the same
-// bits.  What is left is the chain of a chunk, 11600 cycles long with the copies in it.  Not kept: the next chunk's tiles
-// brought into L2 ahead (201 us), V on a barrier of its own and another warp for the copies (196).
+// bits.  What is left is the chain of a chunk, 11600 cycles long with the copies in it.  Two CTAs leave 128 registers a
+// thread: 76 bytes of each spill (carried windows 116).  Not kept: the next chunk's tiles brought into L2 ahead (201 us),
+// V on a barrier of its own and another warp for the copies (196).
 // Carried windows (CARRY) do this too, although they have five more operand tiles: the remainders take turns in the tiles
 // of the first products (S_lo after S, M_lo after M, the second and third part of w o V after the first), five MMA groups
 // a chunk for two, whose waits are the other CTA's time.  Y2 takes its rows' decay in tensor memory and M V on top, which
