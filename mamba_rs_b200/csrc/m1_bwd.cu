@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(32) sscan_bwd_kernel(const __grid_constant__ B
         const float step = a2[1] - a2[0];
 #pragma unroll
         for (int j = 2; j < NS; ++j)
-            if (fabsf(a2[j] - fmaf(static_cast<float>(j), step, a2[0])) > 4.8e-7f * fabsf(a2[j]))
+            if (!(fabsf(a2[j] - fmaf(static_cast<float>(j), step, a2[0])) <= 4.8e-7f * fabsf(a2[j])))
                 geo_local = false;
     }
     const bool geo = __all_sync(0xffffffffu, geo_local ? 1 : 0) != 0;
@@ -511,7 +511,7 @@ __global__ void __launch_bounds__(32) sscan_densify_kernel(const BwdParams p, fl
     const float step = a2[1] - a2[0];
 #pragma unroll
     for (int j = 2; j < 8; ++j)
-        if (fabsf(a2[j] - fmaf(static_cast<float>(j), step, a2[0])) > 4.8e-7f * fabsf(a2[j])) geo = false;
+        if (!(fabsf(a2[j] - fmaf(static_cast<float>(j), step, a2[0])) <= 4.8e-7f * fabsf(a2[j]))) geo = false;
     geo = __all_sync(__activemask(), geo ? 1 : 0) != 0;
     const bool vec_b = N == 16 && (p.ld_bc % 8) == 0 && (reinterpret_cast<uintptr_t>(p.bm) % 16) == 0;
 #pragma unroll 4

@@ -174,7 +174,7 @@ __global__ void __maxnreg__(kBwd2MaxRegs) sscan_bwd2_kernel(const __grid_constan
         const float step = av[1] - av[0];
 #pragma unroll
         for (int j = 2; j < 8; ++j)
-            if (fabsf(av[j] - fmaf(static_cast<float>(j), step, av[0])) > 4.8e-7f * fabsf(av[j])) geo_local = false;
+            if (!(fabsf(av[j] - fmaf(static_cast<float>(j), step, av[0])) <= 4.8e-7f * fabsf(av[j]))) geo_local = false;
 #pragma unroll
         for (int j = 0; j < 4; ++j) a2[j] = make_float2(av[2 * j], av[2 * j + 1]);
     }

@@ -372,12 +372,12 @@ sscan_fwd16_kernel(const __grid_constant__ Fwd16Params q) {
                 hv[j] = (ok && h0) ? h0[at] : 0.0f;
                 if (kStateOnly && seg == 0 && ok && p.ssm_copy) p.ssm_copy[static_cast<long long>(b) * D * N + at] = hv[j];
             }
-            const float inc = av[1] - av[0];  // a[n] = a[n0] + (n - n0) * inc to 4 ulp
+            const float inc = av[1] - av[0];  // a[n] = a[n0] + (n - n0) * inc to 4 ulp (a NaN is none)
             if (i) a_inc.y = inc;
             else a_inc.x = inc;
 #pragma unroll
             for (int j = 2; j < NS; ++j)
-                if (fabsf(av[j] - fmaf(static_cast<float>(j), inc, av[0])) > 4.8e-7f * fabsf(av[j])) progression = false;
+                if (!(fabsf(av[j] - fmaf(static_cast<float>(j), inc, av[0])) <= 4.8e-7f * fabsf(av[j]))) progression = false;
 #pragma unroll
             for (int j = 0; j < NS; ++j) {
                 if (i) a2[j].y = av[j];

@@ -466,3 +466,34 @@ def test_f32_decays_do_not_drift(cuda_dev, case):
     y = mb.selective_scan_fwd(x, delta, Bm, Cm, a, Dp, z, ssm_state=h, workspace=ws)
     assert float((y - y64).norm() / y64.norm()) <= tol_y
     assert float((h - h64).norm() / h64.norm()) <= tol_h
+
+
+# A decay rate that is no number makes its channel so, also where the rates around it form a progression and only the
+# first two of a lane's states are used: each place that a lane of four or eight states can have it, by warp roles, by the
+# general kernel (with the conv) and in the backward.
+@pytest.mark.parametrize("dt", ["f32", "bf16"])
+@pytest.mark.parametrize("n,N", [(0, 16), (1, 16), (2, 16), (7, 16), (15, 16), (10, 12), (11, 12)])
+def test_a_decay_rate_that_is_no_number_shows(cuda_dev, n, N, dt):
+    import torch
+
+    import mamba_rs_b200 as mb
+    (B, T, D, bad), td = (2, 70, 64, 21), torch_dtype(dt)
+    assert scan_fwd_layout(mb.dtype_code(td), B, T, D, N, lent=0)[0] > 0
+    g = torch.Generator(device=cuda_dev).manual_seed(n)
+    rn = lambda *s: torch.randn(*s, device=cuda_dev, generator=g)  # noqa: E731
+    a = -torch.arange(1.0, N + 1, device=cuda_dev).repeat(D, 1)
+    a[bad, n] = float("nan")
+    x, dl, z, dy = [rn(B, T, D).to(td) for _ in range(4)]
+    args = [x, dl, rn(B, T, N).to(td), rn(B, T, N).to(td), a, rn(D)]
+    cs = torch.empty(B, (T + 31) // 32, D, N, device=cuda_dev)
+    others = torch.arange(D, device=cuda_dev) != bad
+    for conv in (dict(), dict(conv_w=rn(D, 4), conv_b=rn(D), conv_state=torch.zeros(B, D, 4, device=cuda_dev))):
+        h = rn(B, D, N)
+        y = mb.selective_scan_fwd(*args, z, ssm_state=h, chunk_states=cs, save_stride=32, **conv)
+        assert bool(y[..., bad].isnan().all()) and bool(h[:, bad, n].isnan().all())
+        assert bool(y[..., others].isfinite().all()) and bool(h[:, others].isfinite().all())
+        if not conv:
+            ws = torch.empty(mb.selective_scan_bwd_workspace_bytes(B, T, D, N), dtype=torch.uint8, device=cuda_dev)
+            d_u = mb.selective_scan_bwd(*args, dy, cs, 32, z, workspace=ws)["d_u"]
+            assert bool(d_u[:, 1:-1, bad].isnan().all()) and bool(d_u[..., others].isfinite().all())
+    mb.ffi.default_handle(0).check_status()
