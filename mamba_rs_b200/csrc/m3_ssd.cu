@@ -1160,14 +1160,10 @@ using namespace mb200;
 
 // A carried window of at most this many steps takes the sequential kernel: a 128-row chunk costs the tensor-core kernel the
 // same time whether it holds 1 step or 128 (15 us at 4 heads, 22 at 150 to 296 pairs, 41 to 45 at 297 to 592), and the
-// sequential kernel reaches that after 30 steps at 4 heads.  Its widest form, heads over 48 x 96, takes 1.5 us a step at 150 to
-// 296 pairs and 2.3 to 3.3 beyond: against two CTAs per SM 16 steps of 256 pairs 28 and 23 us, 20 of 512 66 and 45,
-// 17 of 416 43 and 43, 14 of 1024 82 and 88.  Smaller heads get there later (32 x 64 at 21 steps, 48 x 128 at 18 to 21).  The
-// state is closer to 64 bits on the tensor cores at every length: 1.2e-7 and 3.7e-7 after 16 steps.
-static int m3_sequential_steps(int pairs, int hd, int N) {
-    if (pairs <= 148 || hd <= 48 || N <= 96) return 20;
-    return pairs > 2 * 148 && pairs <= 3 * 148 ? 17 : 14;
-}
+// sequential kernel reaches that after 30 steps at 4 heads and 18 to 21 at 150 to 296 pairs of 48 x 128.  At 64 x 128 it
+// does after 12 to 17 (16 steps of 256 pairs 28 and 23 us, 20 of 512 66 and 45), but it keeps an infinite input to its own
+// step and row, where 0 * infinity in the chunk's masked products reaches all of them: the line stays for every size.
+constexpr int kCarrySeqSteps = 20;
 
 extern "C" MAMBA_B200_API int mamba_b200_m3_ssd_fwd(void* handle, void* stream,
                                                     const mamba_b200_m3_ssd_args* ap) {
@@ -1207,7 +1203,7 @@ extern "C" MAMBA_B200_API int mamba_b200_m3_ssd_fwd(void* handle, void* stream,
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
     bool tensor_core = a.dtype != MAMBA_B200_F32 && a.hd <= tc::HD && a.hd % 8 == 0 && a.N <= tc::NS &&
-                       a.N % 8 == 0 && (!a.carry_in || (!gen && a.dtype == MAMBA_B200_BF16 && a.T > m3_sequential_steps(a.B * a.nh, a.hd, a.N))) &&
+                       a.N % 8 == 0 && (!a.carry_in || (!gen && a.dtype == MAMBA_B200_BF16 && a.T > kCarrySeqSteps)) &&
                        !a.force_sequential && al16(a.x) && al16(a.y) &&
                        (gen ? al16(a.Bn) && al16(a.Cn) && al16(a.angle_vel) : al16(a.K) && al16(a.Q));
     // the tile maps; when the driver refuses one (no encoder, a stride beyond its range) the

@@ -364,38 +364,22 @@ def test_more_pairs_than_sms_are_not_divided(cuda_dev, case):
     mb.ffi.default_handle(0).check_status()
 
 
-# The longest window that the sequential kernel takes and the next one, which the tensor cores take, by what was measured:
-# few pairs, two CTAs per SM with heads of 64 x 128 in one wave, two and more, with smaller heads.  The route shows in
-# the state's last bits.  The sequential kernel rounds it at every step, the other one decays it once and adds 24 bits of
-# every product: it is the closer one to 64 bits (by half or more where this was measured).
-@pytest.mark.parametrize("case", [(1, 4, 64, 128, 20), (8, 32, 64, 128, 14), (13, 32, 64, 128, 17), (16, 32, 64, 128, 14),
-                                  (8, 32, 48, 128, 20), (8, 32, 64, 96, 20), (8, 32, 32, 64, 20)],
-                         ids=lambda c: "B%dnh%dhd%dN%dT%d" % c)
-def test_the_longest_window_of_the_sequential_kernel(cuda_dev, case):
+# A short carried window keeps an infinite input to its own step, row and what follows, also where two CTAs per SM would
+# be faster: the chunk's masked products would bring 0 * infinity to every step of the row.
+@pytest.mark.parametrize("T", [16, 20])
+def test_a_short_carried_window_keeps_an_infinite_input_to_its_row(cuda_dev, T):
     import torch
 
     import mamba_rs_b200 as mb
-    B, nh, hd, N, steps = case
-    g = torch.Generator(device=cuda_dev).manual_seed(steps + hd)
+    B, nh, hd, N, at = 8, 32, 64, 128, T - 4
+    g = torch.Generator(device=cuda_dev).manual_seed(T)
     rn = lambda *s: torch.randn(*s, device=cuda_dev, generator=g)  # noqa: E731
-    h0, k0, v0, Dh = rn(B, nh, hd, N), 0.3 * rn(B, nh, N), rn(B, nh, hd), rn(nh)
-    for T, sequential in ((steps, True), (steps + 1, False)):
-        x, K, Q = [rn(B, T, nh, n).mul_(0.3).to(torch.bfloat16) for n in (hd, N, N)]
-        dt_, trap = torch.nn.functional.softplus(rn(B, T, nh) - 2), torch.sigmoid(rn(B, T, nh))
-        adt = -dt_ * torch.rand(nh, device=cuda_dev, generator=g)
-        got = []
-        for force in (False, True):
-            st = dict(ssm_state=h0.clone(), k_state=k0.clone(), v_state=v0.clone())
-            mb.m3_ssd_fwd(x.view(B, T, -1), K, Q, dt_, trap, adt, Dh, carry_in=True, force_sequential=force, **st)
-            got.append(st["ssm_state"])
-        assert torch.equal(*got) == sequential
-        if not sequential:
-            h, k, v = h0.double(), k0.double(), v0.double()
-            for t in range(T):
-                al, d, tr = torch.exp(adt[:, t].double()), dt_[:, t].double(), trap[:, t].double()
-                kn, vn = K[:, t].double(), x[:, t].double()
-                h = (al[..., None, None] * (h + (d * (1 - tr))[..., None, None] * v[..., None] * k[:, :, None])
-                     + (d * tr)[..., None, None] * vn[..., None] * kn[:, :, None])
-                k, v = kn, vn
-            assert float((got[0] - h).norm()) <= float((got[1] - h).norm())
+    x, K, Q = [rn(B, T, nh, n).mul_(0.3).to(torch.bfloat16) for n in (hd, N, N)]
+    x[3, at, 7, 21] = float("inf")
+    dt_, trap = torch.nn.functional.softplus(rn(B, T, nh) - 2), torch.sigmoid(rn(B, T, nh))
+    st = dict(ssm_state=rn(B, nh, hd, N), k_state=0.3 * rn(B, nh, N), v_state=rn(B, nh, hd))
+    y = mb.m3_ssd_fwd(x.view(B, T, -1), K, Q, dt_, trap, -dt_, rn(nh), carry_in=True, **st).view(B, T, nh, hd)
+    finite = torch.ones_like(y, dtype=torch.bool)
+    finite[3, at:, 7, 21] = False
+    assert torch.equal(torch.isfinite(y), finite) and bool(torch.isinf(st["ssm_state"][3, 7, 21]).all())
     mb.ffi.default_handle(0).check_status()
